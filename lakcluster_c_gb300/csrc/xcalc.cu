@@ -15,12 +15,12 @@
 // the conversion is one IEEE subtract, one multiply and a truncation, computed
 // here with the same rounding.
 //
-// Device side: the masked min / max is a grid reduction (exact, order-free);
-// the planes are built one warp per (column, 32-row word): every lane
-// quantises one row and each plane word is one __ballot_sync, bit-reversed
-// into the reference's MSB-first byte order.  The planes stay resident on the
-// device for the products that follow, and are copied into M_X->wX for
-// callers that read them on the host.
+// Device side: the masked min / max is a grid reduction (exact, order-free)
+// whose last block forms min, max and mlt; the planes are built by warps that
+// each take 256 rows, quantise in 64-bit fixed point and transpose 32 x 32
+// bits in registers.  The planes stay resident on the device for the products
+// that follow, and are copied into M_X->wX for callers that read them on the
+// host.
 #include <math.h>
 #include <stdint.h>
 
@@ -41,20 +41,33 @@ namespace {
 // solves may use different B_MLT.
 thread_local long long g_d_mlt = 4294967296LL;
 
+// min, max and mlt of one matrix, and the constants of the fixed-point
+// quantisation (quantise_fixed below): frac = -1 when the FP64 operations are
+// used for every value.
+struct XcalcScalars {
+  double lo, hi, mlt;
+  unsigned long long K;       // mlt in fixed point
+  unsigned long long neglo;   // -lo in fixed point
+  unsigned long long span;    // largest value - lo in fixed point
+  int shift0, frac;
+};
+static_assert(sizeof(XcalcScalars) <= 64, "eight doubles of scratch");
+
 struct XcalcParams {
   const double *lf;
   const long long *row_off;  // per a-row of Yn (nrows_a): element offset, -1 = not retained
   int nrows_a;
   const long long *col_off;  // per retained column nc_j
   int ncols_j;
-  double min, mlt;
   unsigned long long dmax;   // D_MLT - 1
   int ncols_per;
   long long brows;           // bytes per plane row
   uint8_t *planes;
+  const uint8_t *row0;       // first plane's bytes (null: zeros)
+  long long row_max;         // largest row offset
   unsigned long long lf_n, planes_n;  // elements of lf, bytes of planes (bounds checks)
   int *bad;                  // set when an index would leave its buffer (access skipped)
-  const double *dev_scalars; // a deferred call: device min, max, mlt (then min / mlt above are unused)
+  const XcalcScalars *sc;
 };
 
 // The masked min / max compare order keys instead of doubles: GB300's FP64
@@ -76,16 +89,73 @@ __device__ __forceinline__ double key_value(unsigned long long k) {
   return __longlong_as_double((long long)((k >> 63) ? (k & 0x7fffffffffffffffull) : ~k));
 }
 
+// |x| < 2^e in units of 2^(e-62), truncated towards zero, negated for x < 0;
+// shift0 = e + 1024.  *ok is false outside that range (and for inf and NaN).
+__device__ __forceinline__ unsigned long long to_fixed(double x, int shift0, bool *ok) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const int r = shift0 - (int)((hi >> 20) & 0x7ffu);
+  *ok = r >= 2;
+  // the significand with its leading bit at bit 63, shifted down (by 64 and
+  // more: zero, as PTX defines the shift)
+  const unsigned long long m = ((unsigned long long)((hi << 11) | (lo >> 21) | 0x80000000u) << 32) | (lo << 11);
+  unsigned long long v;
+  asm("shr.u64 %0, %1, %2;" : "=l"(v) : "l"(m), "r"(r));
+  const unsigned long long sgn = (unsigned long long)((long long)((unsigned long long)hi << 32) >> 63);
+  return (v ^ sgn) - sgn;
+}
+
+// min, max and mlt from the extremes' keys with the reference's operations
+// (xcalc.c:34, :130), and the fixed-point constants: with w = max - min in
+// [2^(e-1), 2^e), values are taken in units of 2^(e-62), and
+// K = mlt 2^(e + 2 + frac) <= 2^63 turns them into quantised values with
+// `frac` fraction bits: T = x_fixed K / 2^64 = mlt (x - min) 2^frac.
+__device__ void make_scalars(unsigned long long kmn, unsigned long long kmx, bool nan_first, long long d_mlt,
+                             XcalcScalars *out) {
+  double mn = 0.0, mx = 0.0;
+  if (kmn <= kmx) { mn = key_value(kmn); mx = key_value(kmx); }
+  if (nan_first) mn = mx = __longlong_as_double(0x7ff8000000000000ll);
+  const double top = mx;
+  if (mn >= mx) mx = __dadd_rn(mn, 1.0);
+  const double range = __dsub_rn(mx, mn);
+  XcalcScalars r;
+  r.lo = __dsub_rn(mn, __dmul_rn(0.0625, range));
+  r.hi = __dadd_rn(mx, __dmul_rn(0.0625, range));
+  const double w = __dsub_rn(r.hi, r.lo);
+  r.mlt = __ddiv_rn((double)d_mlt, w);
+  const int E = (int)(((unsigned long long)__double_as_longlong(w) >> 52) & 0x7ff);
+  const int bits = 64 - __clzll(d_mlt - 1);  // d_mlt <= 2^bits
+  const int e = E - 1022;
+  r.frac = 60 - bits;
+  r.shift0 = e + 1024;
+  r.K = r.neglo = r.span = 0ull;
+  bool ok_lo, ok_top;
+  r.neglo = 0ull - to_fixed(r.lo, r.shift0, &ok_lo);
+  r.span = to_fixed(top, r.shift0, &ok_top) + r.neglo;
+  if (d_mlt < 64 || bits > 38 || E < 200 || E > 1800 || !(w > 0.0) || !(r.mlt > 0.0) || !ok_lo || !ok_top) {
+    r.frac = -1;
+  } else {
+    const unsigned long long mb = (unsigned long long)__double_as_longlong(r.mlt);
+    const int s = (int)(mb >> 52) - 1075 + e + 2 + r.frac;  // 6 <= s <= 10: 2^58 < K <= 2^63
+    r.K = ((mb & 0x000fffffffffffffull) | 0x0010000000000000ull) << s;
+  }
+  *out = r;
+}
+
 // Grid: blockIdx.x * blockDim.x + threadIdx.x strides the retained rows, each
 // thread holding kMinMaxRows row offsets in registers for all its columns;
 // blockIdx.y strides the retained columns, kMinMaxCols per pass, so that
 // kMinMaxRows * kMinMaxCols loads are in flight per thread.  One partial
-// (min, max, any) per block.
+// (min key, max key) per block; the last block to finish reduces them and
+// forms the scalars, so the planes kernel follows with no launch between.
+// SKIP_NAN: a NaN is left out of the extremes unless it is the first retained
+// value, which then gives NaN (the comparisons of xcalc.c:25 in order).
 constexpr int kMinMaxRows = 4, kMinMaxCols = 2, kMinMaxThreads = 256;
+constexpr int kMinMaxBlocks = 152 * 8;  // one full wave
 
-__global__ void xcalc_minmax_kernel(const double *lf, const long long *rows_j, int nr,
-                                    const long long *cols_j, int nc, double *pmin, double *pmax,
-                                    int *pany) {
+template <bool SKIP_NAN>
+__global__ void __launch_bounds__(kMinMaxThreads, 5)
+    xcalc_minmax_kernel(const double *lf, const long long *rows_j, int nr, const long long *cols_j, int nc,
+                        ulonglong2 *part, unsigned *ticket, long long d_mlt, XcalcScalars *out) {
   unsigned long long kmn = ~0ull, kmx = 0ull;  // empty: kmn > kmx
   const int stride = gridDim.x * blockDim.x;
   for (int rb = blockIdx.x * blockDim.x + threadIdx.x; rb < nr; rb += kMinMaxRows * stride) {
@@ -111,232 +181,243 @@ __global__ void xcalc_minmax_kernel(const double *lf, const long long *rows_j, i
 #pragma unroll
       for (int k = 0; k < kMinMaxCols; ++k)
 #pragma unroll
-        for (int u = 0; u < kMinMaxRows; ++u)
-          if (cok[k] && rok[u]) {
+        for (int u = 0; u < kMinMaxRows; ++u) {
+          const unsigned long long b = (unsigned long long)__double_as_longlong(x[k][u]);
+          if (cok[k] && rok[u] && !(SKIP_NAN && (b << 1) > 0xffe0000000000000ull)) {
             const unsigned long long q = order_key(x[k][u]);
             kmn = q < kmn ? q : kmn;
             kmx = q > kmx ? q : kmx;
           }
+        }
     }
   }
-  __shared__ unsigned long long smn[32], smx[32];
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long omn = __shfl_xor_sync(0xffffffffu, kmn, o);
-    const unsigned long long omx = __shfl_xor_sync(0xffffffffu, kmx, o);
-    kmn = omn < kmn ? omn : kmn;
-    kmx = omx > kmx ? omx : kmx;
-  }
+  __shared__ unsigned long long smn[kMinMaxThreads / 32], smx[kMinMaxThreads / 32];
+  __shared__ bool last;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) { smn[warp] = kmn; smx[warp] = kmx; }
+  auto block_reduce = [&]() {  // result in thread 0
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long omn = __shfl_xor_sync(0xffffffffu, kmn, o);
+      const unsigned long long omx = __shfl_xor_sync(0xffffffffu, kmx, o);
+      kmn = omn < kmn ? omn : kmn;
+      kmx = omx > kmx ? omx : kmx;
+    }
+    if (lane == 0) { smn[warp] = kmn; smx[warp] = kmx; }
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int w = 1; w < kMinMaxThreads / 32; ++w) {
+        kmn = smn[w] < kmn ? smn[w] : kmn;
+        kmx = smx[w] > kmx ? smx[w] : kmx;
+      }
+  };
+  block_reduce();
+  const int blocks = gridDim.x * gridDim.y;
+  if (threadIdx.x == 0) {
+    part[blockIdx.x + gridDim.x * blockIdx.y] = make_ulonglong2(kmn, kmx);
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == (unsigned)blocks - 1u;
+  }
   __syncthreads();
+  if (!last) return;
+  __threadfence();
+  kmn = ~0ull;
+  kmx = 0ull;
+  for (int i = threadIdx.x; i < blocks; i += kMinMaxThreads) {
+    const ulonglong2 q = __ldcg(part + i);
+    kmn = q.x < kmn ? q.x : kmn;
+    kmx = q.y > kmx ? q.y : kmx;
+  }
+  block_reduce();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-      kmn = smn[w] < kmn ? smn[w] : kmn;
-      kmx = smx[w] > kmx ? smx[w] : kmx;
-    }
-    const int b = blockIdx.x + gridDim.x * blockIdx.y;
-    const int any = kmn <= kmx;
-    pmin[b] = any ? key_value(kmn) : 0.0;
-    pmax[b] = any ? key_value(kmx) : 0.0;
-    pany[b] = any;
+    bool nan_first = false;
+    if (SKIP_NAN && nr > 0 && nc > 0) nan_first = isnan(lf[rows_j[0] + cols_j[0]]);
+    make_scalars(kmn, kmx, nan_first, d_mlt, out);
+    *ticket = 0u;  // ready for the next launch
   }
 }
 
-// A deferred call's min / max partials reduced on the device (one warp), and
-// min, max and mlt formed from them with the host's operations (xcalc.c:34,
-// :130): out = {min, max, mlt}.
-__global__ void xcalc_scalars_from_partials_kernel(const double *pmin, const double *pmax, const int *pany,
-                                                   int blocks, double d_mlt, double *out) {
-  unsigned long long kmn = ~0ull, kmx = 0ull;
-  for (int i = threadIdx.x; i < blocks; i += 32)
-    if (pany[i]) {
-      const unsigned long long a = order_key(pmin[i]), b = order_key(pmax[i]);
-      kmn = a < kmn ? a : kmn;
-      kmx = b > kmx ? b : kmx;
-    }
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long a = __shfl_xor_sync(0xffffffffu, kmn, o), b = __shfl_xor_sync(0xffffffffu, kmx, o);
-    kmn = a < kmn ? a : kmn;
-    kmx = b > kmx ? b : kmx;
-  }
-  if (threadIdx.x == 0) {
-    double mn = 0.0, mx = 0.0;
-    if (kmn <= kmx) { mn = key_value(kmn); mx = key_value(kmx); }
-    if (mn >= mx) mx = __dadd_rn(mn, 1.0);
-    const double w = __dsub_rn(mx, mn);
-    const double lo = __dsub_rn(mn, __dmul_rn(0.0625, w)), hi = __dadd_rn(mx, __dmul_rn(0.0625, w));
-    out[0] = lo;
-    out[1] = hi;
-    out[2] = __ddiv_rn(d_mlt, __dsub_rn(hi, lo));
-  }
+// floor(mlt * (x - min)) cropped to [1, dmax], as the FP64 operations of
+// xcalc.c:150 give it.
+__device__ __forceinline__ unsigned long long quantise_fp64(double x, const XcalcScalars &s, unsigned long long dmax) {
+  unsigned long long v = __double2ull_rz(__dmul_rn(s.mlt, __dsub_rn(x, s.lo)));
+  if (v < 1ull) v = 1ull;
+  return v > dmax ? dmax : v;
 }
 
-// Warp per (column, 128-row group): lane l quantises rows 128g + 32k + l,
-// k = 0..3 (four independent coalesced loads).  Per k, the 32 x 32 bit
-// matrix (row l = bits nb0 .. nb0+31 of lane l's value) is transposed in
-// registers, so lane j holds the word of bit nb0+j; lane j then writes its
-// plane's four words (128 rows) as one 16-byte store.  Plane rows are
-// bsize(nrows) bytes, a multiple of 240 and so of 16, and a group that starts
-// inside the rows ends inside the 1920-bit padding, so every store is aligned
-// and within its plane row.
-__global__ void xcalc_planes_kernel(XcalcParams p) {
-  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// The same in 64-bit integers: GB300's FP64 pipe takes 80 cycles per warp
+// instruction, and the subtract, the multiply and the conversion are three.
+// T = mlt (x - min) 2^frac is within 5 of the exact product (two truncations
+// to the unit, the product's low words left out, K <= 2^63), and the two FP64
+// roundings move that by at most 2^-52 of 2^60, 2^8.  Only where a multiple
+// of 2^frac lies within kMargin of T could the integer part differ: for those
+// values (about one in 2^17 at 32 bits) and for values above the largest one,
+// below min or not finite, *ok is false and the FP64 operations decide.  A
+// value up to the largest one stays below 17 d_mlt / 18 and so needs no
+// cropping from above (frac is -1 for d_mlt < 64).
+constexpr unsigned kMargin = 1u << 10;
+__device__ __forceinline__ unsigned long long quantise_fixed(double x, const XcalcScalars &s, bool *ok) {
+  bool in;
+  const unsigned long long d = to_fixed(x, s.shift0, &in) + s.neglo;
+  const uint32_t dh = (uint32_t)(d >> 32), kh = (uint32_t)(s.K >> 32);
+  const unsigned long long t =
+      (unsigned long long)dh * kh + __umulhi(dh, (uint32_t)s.K) + __umulhi((uint32_t)d, kh);
+  // frac is 22 to 54; its low 22 bits or more lie in the low word
+  const uint32_t low = (uint32_t)t + kMargin;
+  bool clear = (low & ((1u << min(s.frac, 31)) - 1u)) >= 2u * kMargin;
+  *ok = in && d <= s.span && clear;
+  const unsigned long long v = t >> s.frac;
+  return v < 1ull ? 1ull : v;
+}
+
+// Warp per 256-row group (32 bytes of every plane row), for the columns
+// c, c + step, ...: the row offsets stay in registers, lane l quantises rows
+// 256g + 32k + l, k = 0..7 (eight independent coalesced loads).  Per k, the
+// 32 x 32 bit matrix (row l = bits nb0 .. nb0+31 of lane l's value) is
+// transposed in registers, so lane j holds the word of bit nb0+j; lane j then
+// writes its plane's 32 bytes.  Every byte of the column's plane rows is
+// written, the first plane and (by the last group's warp) the padding past the
+// rows included, so the planes need no zero-fill before.  WIDE: plane rows and the array are 16-byte
+// aligned (16-byte stores); otherwise 4-byte ones.  T: holds b_mlt bits.
+// Bound: the integer pipe (57 % active; about 100 operations per value, 30 of
+// them the transpose), then load latency.  4096 x 4001 values to 32 bits
+// through lakgb_xcalc_noalloc: 1463 us a call before (a warp per 32 rows, FP64
+// operations, 4-byte stores, one thread folding the columns' extremes), 130 us
+// now; this kernel 76 us, the extremes 37 us.
+constexpr int kPlaneRows = 256, kPlaneThreads = 256, kPlaneBlocks = 3;
+template <bool WIDE, typename T>
+__global__ void __launch_bounds__(kPlaneThreads, kPlaneBlocks) xcalc_planes_kernel(XcalcParams p, int cstep) {
+  constexpr int R = kPlaneRows / 32;
+  const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
-  const int ngroups = (p.nrows_a + 127) >> 7;
-  if (warp >= (long long)ngroups * p.ncols_j) return;
-  const int g = (int)(warp % ngroups), c = (int)(warp / ngroups);
-  const long long co = p.col_off[c];
-  unsigned long long cz[4];
+  const int ngroups = max(1, (p.nrows_a + kPlaneRows - 1) / kPlaneRows);
+  const int g = warp % ngroups;
+  if (warp / ngroups >= cstep) return;
+  const long long pad0 = g == ngroups - 1 ? 32ll * ngroups : p.brows;  // padding this warp clears
+  const XcalcScalars s = *p.sc;
+  const Transpose32 tr(lane);
+  long long ro[R];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int r = (g << 7) + (k << 5) + lane;
-    cz[k] = 0ull;
-    const long long ro = r < p.nrows_a ? p.row_off[r] : -1;
-    if (ro >= 0 && (unsigned long long)(ro + co) >= p.lf_n) {
-      atomicCAS(p.bad, 0, 1);
-    } else if (ro >= 0) {
-      const double x = p.lf[ro + co];
-      const double pmin = p.dev_scalars ? p.dev_scalars[0] : p.min;
-      const double pmlt = p.dev_scalars ? p.dev_scalars[2] : p.mlt;
-      unsigned long long v = __double2ull_rz(__dmul_rn(pmlt, __dsub_rn(x, pmin)));
-      if (v < 1ull) v = 1ull;
-      if (v > p.dmax) v = p.dmax;
-      cz[k] = v;
-    }
+  for (int k = 0; k < R; ++k) {
+    const int r = g * kPlaneRows + 32 * k + lane;
+    ro[k] = r < p.nrows_a ? p.row_off[r] : -1;
   }
   const int nbits = p.ncols_per - 1;
-  for (int nb0 = 0; nb0 < nbits; nb0 += 32) {
-    const int nr_ = min(32, nbits - nb0);
-    unsigned mine[4];
+  const long long byte0 = 32ll * g;
+  for (int c = warp / ngroups; c < p.ncols_j; c += cstep) {
+    const long long co = p.col_off[c];
+    const bool inside = (unsigned long long)(p.row_max + co) < p.lf_n;
+    if (!inside) atomicCAS(p.bad, 0, 1);
+    double x[R];
+    unsigned live = 0u;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) mine[k] = transpose32(__brev((uint32_t)(cz[k] >> nb0)), lane);
-    if (lane < nr_ && (mine[0] | mine[1] | mine[2] | mine[3])) {
+    for (int k = 0; k < R; ++k) {
+      const bool l = inside && ro[k] >= 0;
+      live |= (unsigned)l << k;
+      x[k] = l ? __ldg(p.lf + ro[k] + co) : 0.0;
+    }
+    T cz[R];
+    unsigned fp64 = live;
+    if (s.frac >= 0) {
+      fp64 = 0u;
+#pragma unroll
+      for (int k = 0; k < R; ++k) {
+        bool ok;
+        cz[k] = (T)quantise_fixed(x[k], s, &ok);
+        if (!ok) fp64 |= 1u << k;
+      }
+      fp64 &= live;
+    }
+    // one branch for the warp and the eight rows, its values read again: FP64
+    // instructions that the compiler predicates, or hoists above the branch,
+    // cost their 80 cycles for every value
+    if (__any_sync(0xffffffffu, fp64 != 0u)) {
+#pragma unroll
+      for (int k = 0; k < R; ++k)
+        if ((fp64 >> k) & 1u) cz[k] = (T)quantise_fp64(__ldcv(p.lf + ro[k] + co), s, p.dmax);
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k)
+      if (!((live >> k) & 1u)) cz[k] = 0;
+    const long long first = (long long)p.ncols_per * c;
+    for (int nb0 = 0; nb0 < nbits; nb0 += 32) {
       // lane j's word has row i at bit 31-i; memory wants row 8m+q at byte m, bit 7-q.
-      uint4 v;
-      v.x = __byte_perm(mine[0], 0u, 0x0123);
-      v.y = __byte_perm(mine[1], 0u, 0x0123);
-      v.z = __byte_perm(mine[2], 0u, 0x0123);
-      v.w = __byte_perm(mine[3], 0u, 0x0123);
-      const long long plane = (long long)p.ncols_per * c + p.ncols_per - 1 - (nb0 + lane);
-      const unsigned long long off = (unsigned long long)(plane * p.brows + 16ll * g);
-      if (off + 16 > p.planes_n || (off & 15ull)) atomicCAS(p.bad, 0, 2);
-      else *reinterpret_cast<uint4 *>(p.planes + off) = v;
+      uint32_t o[R];
+#pragma unroll
+      for (int k = 0; k < R; ++k) o[k] = __byte_perm(tr(__brev((uint32_t)(cz[k] >> nb0))), 0u, 0x0123);
+      if (lane < nbits - nb0) {
+        const unsigned long long off = (unsigned long long)((first + nbits - (nb0 + lane)) * p.brows + byte0);
+        if (WIDE) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            if (byte0 + 16 * h < p.brows) {
+              if (off + 16 * h + 16 > p.planes_n) atomicCAS(p.bad, 0, 2);
+              else *reinterpret_cast<uint4 *>(p.planes + off + 16 * h) =
+                  make_uint4(o[4 * h], o[4 * h + 1], o[4 * h + 2], o[4 * h + 3]);
+            }
+          for (long long b = pad0; b < p.brows; b += 16)
+            if (off - byte0 + b + 16 <= p.planes_n)
+              *reinterpret_cast<uint4 *>(p.planes + off - byte0 + b) = make_uint4(0u, 0u, 0u, 0u);
+        } else {
+#pragma unroll
+          for (int k = 0; k < R; ++k)
+            if (byte0 + 4 * k < p.brows) {
+              if (off + 4 * k + 4 > p.planes_n) atomicCAS(p.bad, 0, 2);
+              else *reinterpret_cast<uint32_t *>(p.planes + off + 4 * k) = o[k];
+            }
+          for (long long b = pad0; b < p.brows; b += 4)
+            if (off - byte0 + b + 4 <= p.planes_n) *reinterpret_cast<uint32_t *>(p.planes + off - byte0 + b) = 0u;
+        }
+      }
+      if (sizeof(T) == 4) break;
+    }
+    // the column's mask plane: row0 before the first column, zero elsewhere
+    const long long mask_end = pad0 < p.brows ? p.brows : min(p.brows, byte0 + 32);
+    for (long long b = byte0 + lane; b < mask_end; b += 32) {
+      const unsigned long long off = (unsigned long long)(first * p.brows + b);
+      if (off >= p.planes_n) atomicCAS(p.bad, 0, 2);
+      else p.planes[off] = (c == 0 && p.row0) ? p.row0[b] : (uint8_t)0;
     }
   }
+}
+
+// One resident wave of warps (kPlaneBlocks blocks per SM) over the row groups
+// and as many column steps.
+void launch_planes(const XcalcParams &p, cudaStream_t s) {
+  if (p.brows <= 0) return;
+  const long long ngroups = std::max(1, (p.nrows_a + kPlaneRows - 1) / kPlaneRows);
+  const long long resident = 152ll * kPlaneBlocks * (kPlaneThreads / 32);
+  const int cstep = (int)std::max(1ll, std::min<long long>(p.ncols_j, resident / ngroups));
+  const unsigned blocks = (unsigned)((ngroups * cstep * 32 + kPlaneThreads - 1) / kPlaneThreads);
+  const bool wide = (p.brows & 15) == 0 && (reinterpret_cast<uintptr_t>(p.planes) & 15) == 0;
+  const bool narrow = p.ncols_per - 1 <= 32 && p.dmax <= 0xffffffffull;
+  if (wide && narrow)
+    xcalc_planes_kernel<true, uint32_t><<<blocks, kPlaneThreads, 0, s>>>(p, cstep);
+  else if (wide)
+    xcalc_planes_kernel<true, unsigned long long><<<blocks, kPlaneThreads, 0, s>>>(p, cstep);
+  else
+    xcalc_planes_kernel<false, unsigned long long><<<blocks, kPlaneThreads, 0, s>>>(p, cstep);
+  LAKGB_CUDA(cudaGetLastError());
+  count_launch();
+}
+
+// Rows across blockIdx.x (kMinMaxRows per thread), columns across blockIdx.y.
+dim3 minmax_grid(int nr, int nc) {
+  const int gx = std::max(1, std::min((nr + kMinMaxRows * kMinMaxThreads - 1) / (kMinMaxRows * kMinMaxThreads),
+                                      kMinMaxBlocks));
+  return dim3(gx, std::max(1, std::min(nc, kMinMaxBlocks / gx)));
 }
 
 // --- allocation-free variant ---------------------------------------------
 //
-// lakgb_xcalc_noalloc runs the same quantisation on caller-owned device
-// buffers for callers that cannot allocate device memory.  Its only scratch
-// is this file-scope array: per retained column, the column's min, max and a
-// "has values" flag (3 x kNoAllocMaxCols doubles), then min / max / mlt of
-// the whole matrix (4 doubles) -- 786,464 bytes in all.  Every entry a call
-// reads is written earlier in the same call, so nothing needs clearing; the
-// array is shared by every call on a device, so calls whose kernels overlap
-// on the GPU race.
+// lakgb_xcalc_noalloc runs the same kernels on caller-owned device buffers
+// for callers that cannot allocate device memory.  Its only scratch is this
+// file-scope array (786,464 bytes): the blocks' partial extremes, the scalars
+// and the ticket of the last block.  Every entry a call reads is written
+// earlier in the same call; the array is shared by every call on a device, so
+// calls whose kernels overlap on the GPU race.
 constexpr int kNoAllocMaxCols = LAKGB_XCALC_NOALLOC_MAX_COLS;
 static __device__ __align__(256) double g_xcalc_noalloc_scratch[3 * kNoAllocMaxCols + 4];
-
-// Column-wise min / max of the retained entries: one block per column.
-__global__ void xcalc_colminmax_kernel(const double *lf, const long long *rows_j, int nr, const long long *cols_j,
-                                       int nc, double *scratch) {
-  const int c = blockIdx.x;
-  if (c >= nc) return;
-  double mn = 0.0, mx = 0.0;
-  int any = 0;
-  for (int r = threadIdx.x; r < nr; r += blockDim.x) {
-    const double x = lf[rows_j[r] + cols_j[c]];
-    if (!any) { mn = x; mx = x; any = 1; }
-    else { mn = x < mn ? x : mn; mx = x > mx ? x : mx; }
-  }
-  __shared__ double smn[32], smx[32];
-  __shared__ int sany[32];
-  for (int o = 16; o > 0; o >>= 1) {
-    const double omn = __shfl_xor_sync(0xffffffffu, mn, o);
-    const double omx = __shfl_xor_sync(0xffffffffu, mx, o);
-    const int oany = __shfl_xor_sync(0xffffffffu, any, o);
-    if (oany) {
-      if (!any) { mn = omn; mx = omx; any = 1; }
-      else { mn = omn < mn ? omn : mn; mx = omx > mx ? omx : mx; }
-    }
-  }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) { smn[warp] = mn; smx[warp] = mx; sany[warp] = any; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int a = 0;
-    double bmn = 0.0, bmx = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-      if (!sany[w]) continue;
-      if (!a) { bmn = smn[w]; bmx = smx[w]; a = 1; }
-      else { bmn = smn[w] < bmn ? smn[w] : bmn; bmx = smx[w] > bmx ? smx[w] : bmx; }
-    }
-    scratch[c] = bmn;
-    scratch[kNoAllocMaxCols + c] = bmx;
-    scratch[2 * kNoAllocMaxCols + c] = a ? 1.0 : 0.0;
-  }
-}
-
-// One thread folds the column partials in column order (min / max are exact,
-// so the order does not change the result) and derives min, max and mlt with
-// the host formula's operations (xcalc.c:129-130, 240).
-__global__ void xcalc_scalars_kernel(int nc, double d_mlt, double *scratch) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double mn = 0.0, mx = 0.0;
-  int set = 0;
-  for (int c = 0; c < nc; ++c) {
-    if (scratch[2 * kNoAllocMaxCols + c] == 0.0) continue;
-    const double a = scratch[c], b = scratch[kNoAllocMaxCols + c];
-    if (!set) { mn = a; mx = b; set = 1; }
-    else { mn = a < mn ? a : mn; mx = b > mx ? b : mx; }
-  }
-  if (mn >= mx) mx = __dadd_rn(mn, 1.0);
-  const double range = __dsub_rn(mx, mn);
-  const double lo = __dsub_rn(mn, __dmul_rn(0.0625, range));
-  const double hi = __dadd_rn(mx, __dmul_rn(0.0625, range));
-  double mlt = __ddiv_rn(d_mlt, __dsub_rn(hi, lo));
-  double* out = scratch + 3 * kNoAllocMaxCols;
-  out[0] = lo;
-  out[1] = hi;
-  out[2] = mlt;            // used by the plane kernel
-  if (!isfinite(mlt) || mlt <= 0) mlt = 1.0;
-  out[3] = mlt;            // the value wrap_xcalc stores as M_X->mlt_d
-}
-
-// A warp per (32-row word, column); grid-stride over the warps, so any
-// launch size covers every word (the warp index is uniform within a warp, as
-// the ballots need).
-__global__ void xcalc_planes_dev_kernel(XcalcParams p, const double *scalars) {
-  p.min = scalars[0];
-  p.mlt = scalars[2];
-  const int lane = threadIdx.x & 31;
-  const int nwords = (p.nrows_a + 31) >> 5;
-  const long long total = (long long)nwords * p.ncols_j;
-  const long long step = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; warp < total; warp += step) {
-    const int w = (int)(warp % nwords), c = (int)(warp / nwords);
-    const int r = (w << 5) + lane;
-    unsigned long long cz = 0ull;
-    if (r < p.nrows_a) {
-      const long long ro = p.row_off[r];
-      if (ro >= 0) {
-        const double x = p.lf[ro + p.col_off[c]];
-        cz = __double2ull_rz(__dmul_rn(p.mlt, __dsub_rn(x, p.min)));
-        if (cz < 1ull) cz = 1ull;
-        if (cz > p.dmax) cz = p.dmax;
-      }
-    }
-    for (int nb = 0; nb < p.ncols_per - 1; ++nb) {
-      const unsigned bal = __ballot_sync(0xffffffffu, (unsigned)((cz >> nb) & 1ull));
-      if (lane == 0 && bal) {
-        const unsigned word = __byte_perm(__brev(bal), 0u, 0x0123);
-        const long long plane = (long long)p.ncols_per * c + p.ncols_per - 1 - nb;
-        *reinterpret_cast<unsigned *>(p.planes + plane * p.brows + 4ll * w) = word;
-      }
-    }
-  }
-}
+constexpr int kScratchScalars = 2 * kMinMaxBlocks;       // doubles from the start
+constexpr int kScratchTicket = kScratchScalars + 8;
 
 std::mutex g_noalloc_mu;
 void *g_noalloc_scratch[64] = {nullptr};
@@ -389,8 +470,19 @@ int *bad_flag() {
   return d;
 }
 
-// Calls inside a deferral scope: their min, max and mlt stay on the device
-// (three doubles per call, in chunks of kSlots calls) until the scope ends;
+// The ticket of the extremes kernel's last block, per host thread (its
+// launches follow one another on the thread's stream); zero between launches.
+unsigned *minmax_ticket() {
+  thread_local unsigned *d = nullptr;
+  if (!d) {
+    LAKGB_CUDA(cudaMalloc(&d, sizeof(unsigned)));
+    LAKGB_CUDA(cudaMemsetAsync(d, 0, sizeof(unsigned), stream()));
+  }
+  return d;
+}
+
+// Calls inside a deferral scope: their scalars stay on the device (one
+// XcalcScalars per call, in chunks of kSlots calls) until the scope ends;
 // then M_X's fields are set from them.
 constexpr int kSlots = 256;
 struct XcalcDeferred { M_handle *M_X; int slot; };
@@ -398,10 +490,10 @@ thread_local std::vector<DBuf> t_xs_chunks;
 thread_local int t_xs_used = 0;
 thread_local std::vector<XcalcDeferred> t_xs;
 
-double *xcalc_slot(int &slot) {
-  if (t_xs_used == (int)t_xs_chunks.size() * kSlots) t_xs_chunks.emplace_back((size_t)kSlots * 3 * sizeof(double));
+XcalcScalars *xcalc_slot(int &slot) {
+  if (t_xs_used == (int)t_xs_chunks.size() * kSlots) t_xs_chunks.emplace_back((size_t)kSlots * sizeof(XcalcScalars));
   slot = t_xs_used++;
-  return t_xs_chunks[slot / kSlots].as<double>() + (size_t)(slot % kSlots) * 3;
+  return t_xs_chunks[slot / kSlots].as<XcalcScalars>() + slot % kSlots;
 }
 
 void xcalc_deferred_enqueue() {}
@@ -409,19 +501,19 @@ void xcalc_deferred_enqueue() {}
 // After the scope's wait: the scalars into M_X (xcalc.c:240), the planes
 // kernels' bounds flag checked once.
 void xcalc_deferred_finish() {
-  std::vector<double> h((size_t)t_xs_used * 3);
+  std::vector<XcalcScalars> h((size_t)t_xs_used);
   for (size_t c = 0; c < t_xs_chunks.size(); ++c) {
     const int n = std::min(kSlots, t_xs_used - (int)c * kSlots);
     if (n > 0)
-      LAKGB_CUDA(cudaMemcpyAsync(h.data() + c * kSlots * 3, t_xs_chunks[c].p, (size_t)n * 3 * sizeof(double),
+      LAKGB_CUDA(cudaMemcpyAsync(h.data() + c * kSlots, t_xs_chunks[c].p, (size_t)n * sizeof(XcalcScalars),
                                  cudaMemcpyDeviceToHost, stream()));
   }
   int hbad = 0;
   LAKGB_CUDA(cudaMemcpyAsync(&hbad, bad_flag(), sizeof(int), cudaMemcpyDeviceToHost, stream()));
   LAKGB_CUDA(cudaStreamSynchronize(stream()));
   for (const XcalcDeferred &d : t_xs) {
-    const double *v = h.data() + (size_t)d.slot * 3;
-    d.M_X->min_d = v[0]; d.M_X->max_d = v[1]; d.M_X->mlt_d = v[2];
+    const XcalcScalars &v = h[(size_t)d.slot];
+    d.M_X->min_d = v.lo; d.M_X->max_d = v.hi; d.M_X->mlt_d = v.mlt;
     if (!isfinite(d.M_X->mlt_d) || d.M_X->mlt_d <= 0) d.M_X->mlt_d = 1;
   }
   if (hbad) {
@@ -489,8 +581,7 @@ extern "C" void wrap_xcalc(int *tidx, void **vpra, pthread_t *thread_in, unsigne
   const size_t lf_elems = (size_t)(max_off + max_coff + 1);
 
   std::optional<Stager> st;
-  DBuf d_lf, d_rows, d_cols, d_roff_all;
-  double min_data = 0.0, max_data = 0.0;
+  DBuf d_lf, d_rows, d_cols, d_roff_all, d_row0, d_part, d_sc;
   const int nr = (int)rows_j.size(), nc = (int)cols_j.size();
   // A mirrored matrix (lmirror.cu) is read in place.
   Mirror *mlf = (lf_YnWt && YnWt == lf_YnWt->lf) ? find_mirror(lf_YnWt) : nullptr;
@@ -499,9 +590,16 @@ extern "C" void wrap_xcalc(int *tidx, void **vpra, pthread_t *thread_in, unsigne
   // min, max and mlt stay on the device: the planes kernel reads them there
   // and M_X's fields are set when the scope ends, so the call does not wait.
   const bool deferred = defer_active() && !host_planes_wanted();
-  double *dev_scalars = nullptr;
+  const bool values = nr > 0 && nc > 0 && YnWt;
+  XcalcScalars *dev_sc = nullptr;
   int slot = -1;
-  if (nr > 0 && nc > 0 && YnWt) {
+  // Plane 0: the rows set in mr_j (xcalc.c:141).
+  std::vector<unsigned char> row0((size_t)lakbcc::bsize(Yn_nrows), 0);
+  for (int a = 0; a < Yn_nrows; ++a)
+    if (bit_on(mr_j, a)) row0[a / 8] |= (unsigned char)(1 << (7 - a % 8));
+  // no values: min 0, max 1 before the margins (xcalc.c:34)
+  double min = 0.0 - 0.0625, max = 1.0 + 0.0625, mlt = (double)g_d_mlt / (max - min);
+  if (values) {
     if (mlf && lf_elems <= mlf->n) {
       plf = mlf->d;
     } else {
@@ -515,50 +613,23 @@ extern "C" void wrap_xcalc(int *tidx, void **vpra, pthread_t *thread_in, unsigne
     d_rows = upload_vec(rows_j);
     d_cols = upload_vec(cols_j);
     d_roff_all = upload_vec(row_off_a);
+    d_row0 = upload_vec(row0);
     st->flush();
-    // About 16 blocks per SM: rows across blockIdx.x (kMinMaxRows per
-    // thread), columns across blockIdx.y.
-    const int gx = std::min((nr + kMinMaxRows * kMinMaxThreads - 1) / (kMinMaxRows * kMinMaxThreads), 2432);
-    const int gy = std::max(1, std::min(nc, 2432 / gx));
-    const int blocks = gx * gy;
-    DBuf d_min(blocks * sizeof(double)), d_max(blocks * sizeof(double)), d_any(blocks * sizeof(int));
-    xcalc_minmax_kernel<<<dim3(gx, gy), kMinMaxThreads, 0, stream()>>>(plf, d_rows.as<long long>(), nr,
-                                                       d_cols.as<long long>(), nc, d_min.as<double>(),
-                                                       d_max.as<double>(), d_any.as<int>());
+    const dim3 grid = minmax_grid(nr, nc);
+    d_part = DBuf((size_t)grid.x * grid.y * sizeof(ulonglong2));
+    if (deferred) {
+      dev_sc = xcalc_slot(slot);
+    } else {
+      d_sc = DBuf(sizeof(XcalcScalars));
+      dev_sc = d_sc.as<XcalcScalars>();
+    }
+    xcalc_minmax_kernel<false><<<grid, kMinMaxThreads, 0, stream()>>>(plf, d_rows.as<long long>(), nr,
+                                                                      d_cols.as<long long>(), nc,
+                                                                      d_part.as<ulonglong2>(), minmax_ticket(),
+                                                                      g_d_mlt, dev_sc);
     LAKGB_CUDA(cudaGetLastError());
     count_launch();
-    if (deferred) {
-      dev_scalars = xcalc_slot(slot);
-      xcalc_scalars_from_partials_kernel<<<1, 32, 0, stream()>>>(d_min.as<double>(), d_max.as<double>(),
-                                                                 d_any.as<int>(), blocks, (double)g_d_mlt, dev_scalars);
-      LAKGB_CUDA(cudaGetLastError());
-      count_launch();
-    } else {
-      std::vector<double> hmin(blocks), hmax(blocks);
-      std::vector<int> hany(blocks);
-      int hbad = 0;  // an earlier call's planes kernel met an index outside its buffers
-      LAKGB_CUDA(cudaMemcpyAsync(&hbad, bad_flag(), sizeof(int), cudaMemcpyDeviceToHost, stream()));
-      LAKGB_CUDA(cudaMemcpyAsync(hmin.data(), d_min.p, blocks * sizeof(double), cudaMemcpyDeviceToHost, stream()));
-      LAKGB_CUDA(cudaMemcpyAsync(hmax.data(), d_max.p, blocks * sizeof(double), cudaMemcpyDeviceToHost, stream()));
-      LAKGB_CUDA(cudaMemcpyAsync(hany.data(), d_any.p, blocks * sizeof(int), cudaMemcpyDeviceToHost, stream()));
-      LAKGB_CUDA(cudaStreamSynchronize(stream()));
-      if (hbad) {
-        printf(" %% Warning! wrap_xcalc: an earlier call skipped an out-of-range index (code %d)\n", hbad);
-        set_error(5, "wrap_xcalc: an earlier call skipped an out-of-range index (code %d)", hbad);
-        LAKGB_CUDA(cudaMemsetAsync(bad_flag(), 0, sizeof(int), stream()));
-      }
-      bool set = false;
-      for (int i = 0; i < blocks; ++i) {
-        if (!hany[i]) continue;
-        if (!set) { min_data = hmin[i]; max_data = hmax[i]; set = true; }
-        else { min_data = hmin[i] < min_data ? hmin[i] : min_data; max_data = hmax[i] > max_data ? hmax[i] : max_data; }
-      }
-    }
   }
-  if (min_data >= max_data) max_data = min_data + 1;
-  const double min = min_data - 0.0625 * (max_data - min_data);
-  const double max = max_data + 0.0625 * (max_data - min_data);
-  const double mlt = (double)g_d_mlt / (max - min);
 
   int ncols_bZ = 0, nrows_bZ = 0;
   long long brows = 0;
@@ -572,34 +643,42 @@ extern "C" void wrap_xcalc(int *tidx, void **vpra, pthread_t *thread_in, unsigne
       if (!M_X->Ara) { set_error(2, "wrap_xcalc: out of host memory"); return; }
     }
     DBuf planes(nbytes);
-    planes.zero();
-    // Plane 0: the rows set in mr_j (xcalc.c:141).
-    std::vector<unsigned char> row0((size_t)brows, 0);
-    for (int a = 0; a < Yn_nrows; ++a)
-      if (bit_on(mr_j, a)) row0[a / 8] |= (unsigned char)(1 << (7 - a % 8));
-    if (nbytes) planes.upload(row0.data(), (size_t)brows);
-    if (nr > 0 && nc > 0 && YnWt) {
+    if (values) {
       XcalcParams p{};
       p.lf = plf;
       p.row_off = d_roff_all.as<long long>(); p.nrows_a = Yn_nrows;
       p.col_off = d_cols.as<long long>(); p.ncols_j = nc;
-      p.min = min; p.mlt = mlt; p.dmax = (unsigned long long)(g_d_mlt - 1);
-      p.dev_scalars = dev_scalars;
+      p.dmax = (unsigned long long)(g_d_mlt - 1);
+      p.sc = dev_sc;
+      p.row0 = d_row0.as<uint8_t>();
       p.ncols_per = ncols_per; p.brows = brows; p.planes = planes.as<uint8_t>();
+      p.row_max = max_off;
       p.lf_n = (plf == d_lf.p) ? (unsigned long long)lf_elems : (unsigned long long)mlf->n;
       p.planes_n = (unsigned long long)nbytes;
       p.bad = bad_flag();
-      const long long warps = (long long)((Yn_nrows + 127) / 128) * nc;
-      const int blocks = (int)((warps * 32 + 255) / 256);
-      xcalc_planes_kernel<<<blocks, 256, 0, stream()>>>(p);
-      LAKGB_CUDA(cudaGetLastError());
-      count_launch();
+      launch_planes(p, stream());
+    } else {
+      planes.zero();
+      if (nbytes) planes.upload(row0.data(), (size_t)brows);
     }
     if (host_planes_wanted()) {
       if (nbytes) LAKGB_CUDA(cudaMemcpyAsync(M_X->Ara, planes.p, nbytes, cudaMemcpyDeviceToHost, stream()));
       LAKGB_CUDA(cudaStreamSynchronize(stream()));
     }
     resident_put(M_X->Ara, nbytes, std::move(planes));
+  }
+  if (values && !deferred) {
+    XcalcScalars h;
+    int hbad = 0;  // this call or an earlier one met an index outside its buffers
+    LAKGB_CUDA(cudaMemcpyAsync(&hbad, bad_flag(), sizeof(int), cudaMemcpyDeviceToHost, stream()));
+    LAKGB_CUDA(cudaMemcpyAsync(&h, dev_sc, sizeof h, cudaMemcpyDeviceToHost, stream()));
+    LAKGB_CUDA(cudaStreamSynchronize(stream()));
+    if (hbad) {
+      printf(" %% Warning! wrap_xcalc: a call skipped an out-of-range index (code %d)\n", hbad);
+      set_error(5, "wrap_xcalc: a call skipped an out-of-range index (code %d)", hbad);
+      LAKGB_CUDA(cudaMemsetAsync(bad_flag(), 0, sizeof(int), stream()));
+    }
+    min = h.lo; max = h.hi; mlt = h.mlt;
   }
   // M_X fields (xcalc.c:231-241).
   M_X->nrows = ncols_bZ; M_X->ncols = nrows_bZ;
@@ -613,7 +692,7 @@ extern "C" void wrap_xcalc(int *tidx, void **vpra, pthread_t *thread_in, unsigne
   M_X->cpop_b = rpop_b; M_X->cpop_j = rpop_j;
   M_X->wX = M_X->Ara;
   M_X->ncols_per_z = ncols_per;
-  if (dev_scalars) {
+  if (values && deferred) {
     t_xs.push_back(XcalcDeferred{M_X, slot});
     defer_register(xcalc_deferred_enqueue, xcalc_deferred_finish);
   } else {
@@ -655,33 +734,38 @@ extern "C" int lakgb_xcalc_noalloc(const struct lakgb_xcalc_noalloc_args *a) {
   cudaStream_t s = static_cast<cudaStream_t>(a->stream);
   const int ncols_per = a->b_mlt + 1;
   const size_t nbytes = (size_t)ncols_per * (size_t)a->n_cols_j * (size_t)a->brows;
-  if (nbytes) LAKGB_CUDA(cudaMemsetAsync(a->planes, 0, nbytes, s));
-  if (nbytes && a->row0) LAKGB_CUDA(cudaMemcpyAsync(a->planes, a->row0, (size_t)a->brows, cudaMemcpyDeviceToDevice, s));
-  const int nc = (a->n_rows_j > 0) ? a->n_cols_j : 0;
-  if (nc > 0) {
-    xcalc_colminmax_kernel<<<nc, 128, 0, s>>>(a->lf, a->rows_j, a->n_rows_j, a->cols_j, nc, scratch);
-    LAKGB_CUDA(cudaGetLastError());
+  const bool values = a->n_rows_j > 0 && a->n_cols_j > 0;
+  if (!values && nbytes) {
+    LAKGB_CUDA(cudaMemsetAsync(a->planes, 0, nbytes, s));
+    if (a->row0) LAKGB_CUDA(cudaMemcpyAsync(a->planes, a->row0, (size_t)a->brows, cudaMemcpyDeviceToDevice, s));
   }
-  xcalc_scalars_kernel<<<1, 32, 0, s>>>(nc, (double)a->d_mlt, scratch);
+  XcalcScalars *sc = reinterpret_cast<XcalcScalars *>(scratch + kScratchScalars);
+  unsigned *ticket = reinterpret_cast<unsigned *>(scratch + kScratchTicket);
+  // zeroed here, whatever calls that raced on the scratch may have left in it
+  LAKGB_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned), s));
+  const dim3 grid = minmax_grid(values ? a->n_rows_j : 0, values ? a->n_cols_j : 0);
+  xcalc_minmax_kernel<true><<<grid, kMinMaxThreads, 0, s>>>(a->lf, a->rows_j, values ? a->n_rows_j : 0, a->cols_j,
+                                                            values ? a->n_cols_j : 0,
+                                                            reinterpret_cast<ulonglong2 *>(scratch), ticket,
+                                                            (long long)a->d_mlt, sc);
   LAKGB_CUDA(cudaGetLastError());
-  count_launch(nc > 0 ? 2 : 1);
-  if (nc > 0) {
+  count_launch();
+  if (values) {
     XcalcParams p{};
     p.lf = a->lf; p.row_off = a->row_off_a; p.nrows_a = a->nrows_a;
-    p.col_off = a->cols_j; p.ncols_j = nc;
+    p.col_off = a->cols_j; p.ncols_j = a->n_cols_j;
     p.dmax = (unsigned long long)(a->d_mlt - 1); p.ncols_per = ncols_per; p.brows = a->brows;
-    p.planes = a->planes;
-    const long long warps = (long long)((a->nrows_a + 31) / 32) * nc;
-    const long long blocks = std::min<long long>((warps * 32 + 255) / 256, 1ll << 20);  // the kernel grid-strides
-    xcalc_planes_dev_kernel<<<(unsigned)blocks, 256, 0, s>>>(p, scratch + 3 * kNoAllocMaxCols);
-    LAKGB_CUDA(cudaGetLastError());
-    count_launch();
+    p.planes = a->planes; p.row0 = a->row0;
+    p.sc = sc;
+    p.lf_n = ~0ull;  // the caller's offsets are taken as they are
+    p.planes_n = (unsigned long long)nbytes;
+    launch_planes(p, s);
   }
-  double sc[4];
-  LAKGB_CUDA(cudaMemcpyAsync(sc, scratch + 3 * kNoAllocMaxCols, sizeof(sc), cudaMemcpyDeviceToHost, s));
+  XcalcScalars h;
+  LAKGB_CUDA(cudaMemcpyAsync(&h, sc, sizeof(h), cudaMemcpyDeviceToHost, s));
   LAKGB_CUDA(cudaStreamSynchronize(s));
-  a->min_max_mlt[0] = sc[0];
-  a->min_max_mlt[1] = sc[1];
-  a->min_max_mlt[2] = sc[3];
+  a->min_max_mlt[0] = h.lo;
+  a->min_max_mlt[1] = h.hi;
+  a->min_max_mlt[2] = (!isfinite(h.mlt) || h.mlt <= 0) ? 1.0 : h.mlt;  // the value wrap_xcalc stores
   return 0;
 }
