@@ -96,6 +96,7 @@ long long footprint(const lakgb_bcc_problem &p) {
   bytes += 8 * 3 * (long long)p.ncols * cdrop * p.nbins;        // SNP x SNP blocks
   if (p.QR_strategy && strstr(p.QR_strategy, "condense"))
     bytes += 8 * (rows_total + rows_total) * cdrop;             // dense removed columns, their uploads
+  bytes += 64ll << 20;                                          // terms of the bit-plane product
   return bytes + (64ll << 20);                                // staging arena, scratch
 }
 

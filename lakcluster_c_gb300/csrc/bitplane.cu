@@ -83,24 +83,72 @@ __global__ void bitplane_prep_kernel(BitplaneParams p, int nT, int *pm, int *ycn
 }
 
 // T_base[t] = pm[t][0] * min * mlt;  T_tmp[t][mw] = sum_k 2^k pm[t][1 + mw*B + k]
-// (sums of exact integers, accumulated in the reference's order).
-__global__ void bitplane_tsum_kernel(BitplaneParams p, int nT, const int *pm, double *T_base,
-                                     double *T_tmp) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+// in the reference's order.  The partial sums are integers: below 2^53 (EXACT)
+// they are added as such, where the FP64 additions would be a chain of 2 B
+// operations of 80 cycles each.  Thread per (mw, block of A, t); those of
+// block 0 write T_base, T_tmp and (t = 0) ysum, and with q2 each writes
+// (a T_base + a T_tmp) / mlt of its block's a.
+template <bool EXACT>
+__global__ void bitplane_tsum_kernel(BitplaneParams p, const int *pm, double *T_base, double *T_tmp, long long *ysum,
+                                     double *q2) {
+  const int mw = blockIdx.x * blockDim.x + threadIdx.x, blk = blockIdx.y, t = blockIdx.z;
   const int nq = 1 + p.nW * p.B;
-  if (idx >= nT * (p.nW + 1)) return;
-  const int t = idx / (p.nW + 1), mw = idx % (p.nW + 1) - 1;
+  if (mw >= p.nW) return;
   const int *row = pm + (long long)t * nq;
-  if (mw < 0) {
-    T_base[t] = __dmul_rn(__dmul_rn((double)row[0], p.min_d), p.mlt_d);
-    return;
+  const double tb = __dmul_rn(__dmul_rn((double)row[0], p.min_d), p.mlt_d);
+  double s = 0.0;
+  if (EXACT) {
+    long long si = 0;
+    for (int k = 0; k < p.B; ++k) si += (long long)row[1 + mw * p.B + k] << k;
+    s = (double)si;
+  } else {
+    double n2 = 1.0;
+    for (int k = 0; k < p.B; ++k) {
+      s = __dadd_rn(s, __dmul_rn(n2, (double)row[1 + mw * p.B + k]));
+      n2 *= 2.0;
+    }
   }
-  double s = 0.0, n2 = 1.0;
-  for (int k = 0; k < p.B; ++k) {
-    s = __dadd_rn(s, __dmul_rn(n2, (double)row[1 + mw * p.B + k]));
-    n2 *= 2.0;
+  if (blk == 0) {
+    if (mw == 0) T_base[t] = tb;
+    T_tmp[(long long)t * p.nW + mw] = s;
+    if (ysum && t == 0) {
+      long long y = 0;
+      for (int k = 0; k < p.B; ++k) y += (long long)p.ycnt[1 + mw * p.B + k] << k;
+      ysum[mw] = y;
+    }
   }
-  T_tmp[(long long)t * p.nW + mw] = s;
+  if (q2) {
+    const double a = p.aBlk[blk];
+    q2[((long long)t * p.nblk + blk) * p.nW + mw] =
+        __ddiv_rn(__dadd_rn(__dmul_rn(tb, a), __dmul_rn(s, a)), p.mlt_d);
+  }
+}
+
+// Per pair (a warp each): At_base = pmpm0(At, Tt, plane 0) * min * mlt for
+// every t, and the two values of vZ - aZ.
+__global__ void bitplane_pairs_kernel(BitplaneParams p, double *At_base, double2 *zz) {
+  const long long pr = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (pr >= p.npairs) return;
+  const uint32_t *aw = reinterpret_cast<const uint32_t *>(p.At + (long long)p.at_rowb[pr] * p.at_row_bytes);
+  const uint32_t *m = reinterpret_cast<const uint32_t *>(p.mask);
+  const uint32_t *p0 = reinterpret_cast<const uint32_t *>(p.planes);
+  const int nw = p.P * kBlockWords;
+  for (int t = 0; t < p.nT; ++t) {
+    const uint32_t *tw = reinterpret_cast<const uint32_t *>(p.Tt + (long long)p.tt_rowb[t] * p.tt_row_bytes);
+    int c = 0;
+    for (int i = lane; i < nw; i += 32) c += __popc(~(__ldg(aw + i) ^ __ldg(tw + i)) & __ldg(m + i) & __ldg(p0 + i));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    if (lane == 0) {
+      const long long pm = 2ll * c - p.ycnt[0];
+      At_base[(long long)t * p.npairs + pr] = __dmul_rn(__dmul_rn((double)pm, p.min_d), p.mlt_d);
+    }
+  }
+  if (lane == 0) {
+    const double a = p.aZ[pr];
+    zz[pr] = make_double2(__dsub_rn(1.0, a), __dsub_rn(-1.0, a));
+  }
 }
 
 __global__ void __launch_bounds__(kBP_T, 1)
@@ -559,31 +607,40 @@ namespace {
 // calls with the same B run as one grouped launch when the scope ends.
 struct BitplaneDeferred {
   BitplaneParams p{};
-  int nT = 0;
   std::vector<DBuf> keep;
   double *host_out = nullptr;
   unsigned long long length = 0;
 };
 thread_local std::vector<BitplaneDeferred> t_bp;
-thread_local std::vector<DBuf> t_bp_groups;
+// The tensor-core launches of calls of one B: descriptors through `up`
+// (valid once flushed) and the scratch, then, after the flush, the launches.
+struct BitplaneTcRun {
+  std::vector<BitplaneBatch> batches;
+  DBuf ps, segs, scratch;
+  template <class Up>
+  BitplaneTcRun(const std::vector<BitplaneParams> &calls, int B, const Up &up) {
+    std::vector<BitplaneSeg> sg;
+    const size_t n = bitplane_tc_plan(B, calls, &sg, &batches);
+    ps = up(calls);
+    segs = up(sg);
+    scratch = DBuf(n * sizeof(double));
+  }
+  void launch(int B) const {
+    launch_bitplane_tc(B, ps.as<BitplaneParams>(), segs.as<BitplaneSeg>(), batches, scratch.as<double>(), stream());
+  }
+};
+
+thread_local std::vector<BitplaneTcRun> t_bp_runs;
 
 void bitplane_deferred_enqueue() {
   for (int B : {8, 16, 32}) {
     std::vector<BitplaneParams> ps;
-    std::vector<int> tile0;
-    int tiles = 0;
     for (const auto &d : t_bp)
-      if (d.p.B == B) {
-        ps.push_back(d.p);
-        tile0.push_back(tiles);
-        tiles += bitplane_tc_tiles(d.p, d.nT);
-      }
+      if (d.p.B == B) ps.push_back(d.p);
     if (ps.empty()) continue;
-    t_bp_groups.push_back(defer_upload(ps));
-    t_bp_groups.push_back(defer_upload(tile0));
+    t_bp_runs.emplace_back(ps, B, [](const auto &v) { return defer_upload(v); });
     defer_flush();
-    launch_bitplane_tc_group(B, t_bp_groups[t_bp_groups.size() - 2].as<BitplaneParams>(),
-                             t_bp_groups.back().as<int>(), (int)ps.size(), tiles, stream());
+    t_bp_runs.back().launch(B);
   }
   for (const auto &d : t_bp)
     if (d.length)
@@ -592,7 +649,7 @@ void bitplane_deferred_enqueue() {
 
 void bitplane_deferred_clear() {
   t_bp.clear();
-  t_bp_groups.clear();
+  t_bp_runs.clear();
 }
 
 }  // namespace
@@ -629,13 +686,16 @@ extern "C" int wrap_At_T_YnWt_S_Zn_ww__run(int *tidx, void **vpra, pthread_t *th
   const int P = (int)(M_At->mc_length / kBlockBytes);
   const int A_pcols = (int)lakbcc::psize(M_At->nrows);
   const double *a_An = A_ajdk + (size_t)lakbcc::AJDK_1_0 * A_pcols;
+  const bool tensor = g_bitplane_impl.load(std::memory_order_relaxed) == LAKGB_IMPL_TENSOR &&
+                      (B == 8 || B == 16 || B == 32);
 
-  std::vector<uint32_t> at_rowb(npairs), zt_rowb(npairs), tt_rowb(nT), mw_a(nW);
+  std::vector<uint32_t> at_rowb(npairs), zt_rowb(npairs), a_blk(npairs), tt_rowb(nT), mw_a(nW);
   std::vector<double> aA(npairs), aZ(npairs);
   std::vector<unsigned long long> out_off(npairs), t_off(nT);
   for (int i = 0; i < npairs; ++i) {
     at_rowb[i] = M_At->m_b_[i]; zt_rowb[i] = M_Zt->m_b_[i];
-    aA[i] = a_An[M_At->m_a_[i] / lakbcc::POPLENGTH];
+    a_blk[i] = M_At->m_a_[i] / lakbcc::POPLENGTH;
+    aA[i] = a_An[a_blk[i]];
     aZ[i] = a_An[M_Zt->m_a_[i] / lakbcc::POPLENGTH];
     out_off[i] = pick_u(spacing_a, i, M_At->m_b_[i], M_At->m_a_[i]);
   }
@@ -653,9 +713,7 @@ extern "C" int wrap_At_T_YnWt_S_Zn_ww__run(int *tidx, void **vpra, pthread_t *th
   // residency on: the matrices' device copies must stay where they are until
   // the scope ends, which an upload of the same host buffer without residency
   // would not guarantee.
-  const bool defer = defer_active() && residency_enabled() &&
-                     g_bitplane_impl.load(std::memory_order_relaxed) == LAKGB_IMPL_TENSOR &&
-                     (B == 8 || B == 16 || B == 32);
+  const bool defer = defer_active() && residency_enabled() && tensor;
   BitplaneParams p{};
   std::optional<Stager> st;
   if (!defer) st.emplace();
@@ -675,6 +733,23 @@ extern "C" int wrap_At_T_YnWt_S_Zn_ww__run(int *tidx, void **vpra, pthread_t *th
   DBuf d_at = up(at_rowb), d_zt = up(zt_rowb), d_tt = up(tt_rowb), d_mw = up(mw_a);
   DBuf d_vS = up(vS), d_aA = up(aA), d_aZ = up(aZ);
   DBuf d_oo = up(out_off), d_to = up(t_off);
+  DBuf d_ablk, d_aBlk;
+  if (tensor) {
+    d_ablk = up(a_blk);
+    d_aBlk = up(std::vector<double>(a_An, a_An + A_pcols));
+    p.a_blk = d_ablk.as<uint32_t>();
+    p.aBlk = d_aBlk.as<double>();
+    p.nblk = A_pcols;
+    // chunks up to the last retained patient: past it the mask is all zero
+    long last = (long)M_At->mc_length - 1;
+    while (last >= 0 && !M_At->mc_j[last]) --last;
+    p.chunks = (int)(last / 16 + (last >= 0 ? 1 : 0));
+    // The division by mlt as multiplications by its reciprocal (bitplane_tc.cu)
+    // needs quotients and remainders far from overflow and underflow.
+    const double lim = 1.2676506002282294e30;  // 2^100
+    const double m = M_YnWt->mlt_d, lo = M_YnWt->min_d;
+    if (m >= 1.0 / lim && m <= lim && lo >= -lim && lo <= lim) p.inv_mlt = 1.0 / m;
+  }
   if (defer) defer_flush();
   p.at_rowb = d_at.as<uint32_t>(); p.zt_rowb = d_zt.as<uint32_t>(); p.tt_rowb = d_tt.as<uint32_t>();
   p.mw_a = d_mw.as<uint32_t>(); p.nW = nW; p.B = B; p.ncols_per = ncols_per;
@@ -683,44 +758,68 @@ extern "C" int wrap_At_T_YnWt_S_Zn_ww__run(int *tidx, void **vpra, pthread_t *th
   p.out_off = d_oo.as<unsigned long long>(); p.t_off = d_to.as<unsigned long long>();
 
   const int nq = 1 + nW * B;
+  p.nT = nT;
   DBuf d_pm((size_t)nT * nq * sizeof(int)), d_ycnt((size_t)nq * sizeof(int));
   DBuf d_Tb((size_t)nT * sizeof(double)), d_Tt((size_t)nT * nW * sizeof(double));
-  {
-    const long long warps = (long long)nq * nT;
-    if (st) st->flush();
-    bitplane_prep_kernel<<<(int)((warps * 32 + 255) / 256), 256, 0, stream()>>>(p, nT, d_pm.as<int>(), d_ycnt.as<int>());
-    LAKGB_CUDA(cudaGetLastError());
-    const int n = nT * (nW + 1);
-    bitplane_tsum_kernel<<<(n + 255) / 256, 256, 0, stream()>>>(p, nT, d_pm.as<int>(), d_Tb.as<double>(), d_Tt.as<double>());
-    LAKGB_CUDA(cudaGetLastError());
-    count_launch(2);
+  DBuf d_ys, d_q2, d_Ab, d_zz;
+  if (tensor) {
+    d_ys = DBuf((size_t)nW * sizeof(long long));
+    d_q2 = DBuf((size_t)nT * A_pcols * nW * sizeof(double));
+    d_Ab = DBuf((size_t)nT * npairs * sizeof(double));
+    d_zz = DBuf((size_t)npairs * sizeof(double2));
   }
-  p.ycnt = d_ycnt.as<int>(); p.T_base = d_Tb.as<double>(); p.T_tmp = d_Tt.as<double>();
   DBuf d_out(length * sizeof(double));
   d_out.zero();
+  p.ycnt = d_ycnt.as<int>(); p.T_base = d_Tb.as<double>(); p.T_tmp = d_Tt.as<double>();
+  p.At_base = d_Ab.as<double>(); p.zz = d_zz.as<double2>();
+  p.ysum = d_ys.as<long long>(); p.q2 = d_q2.as<double>();
   p.out = d_out.as<double>();
+  std::optional<BitplaneTcRun> run;
+  if (tensor && !defer)
+    run.emplace(std::vector<BitplaneParams>{p}, B, [](const auto &v) { return upload_vec(v); });
+  if (st) st->flush();
+  {
+    const long long warps = (long long)nq * nT;
+    bitplane_prep_kernel<<<(int)((warps * 32 + 255) / 256), 256, 0, stream()>>>(p, nT, d_pm.as<int>(), d_ycnt.as<int>());
+    LAKGB_CUDA(cudaGetLastError());
+    const dim3 grid((nW + 127) / 128, tensor ? A_pcols : 1, nT);
+    // every partial sum of T_tmp is an integer below patients * 2^B
+    const bool exact = B < 40 && (double)P * kBlockBits * (double)(1ll << B) <= 9007199254740992.0;
+    if (exact)
+      bitplane_tsum_kernel<true><<<grid, 128, 0, stream()>>>(p, d_pm.as<int>(), d_Tb.as<double>(), d_Tt.as<double>(),
+                                                             d_ys.as<long long>(), d_q2.as<double>());
+    else
+      bitplane_tsum_kernel<false><<<grid, 128, 0, stream()>>>(p, d_pm.as<int>(), d_Tb.as<double>(), d_Tt.as<double>(),
+                                                              d_ys.as<long long>(), d_q2.as<double>());
+    LAKGB_CUDA(cudaGetLastError());
+    count_launch(2);
+    if (tensor) {
+      bitplane_pairs_kernel<<<(npairs + 7) / 8, 256, 0, stream()>>>(p, d_Ab.as<double>(), d_zz.as<double2>());
+      LAKGB_CUDA(cudaGetLastError());
+      count_launch();
+    }
+  }
   if (defer) {
     BitplaneDeferred d;
     d.p = p;
-    d.nT = nT;
     d.host_out = out->lf;
     d.length = length;
     for (DBuf *b : {&mask, &d_at, &d_zt, &d_tt, &d_mw, &d_vS, &d_aA, &d_aZ, &d_oo, &d_to, &d_pm, &d_ycnt, &d_Tb, &d_Tt,
-                    &d_out})
+                    &d_ablk, &d_aBlk, &d_ys, &d_q2, &d_Ab, &d_zz, &d_out})
       d.keep.push_back(std::move(*b));
     t_bp.push_back(std::move(d));
     defer_register(bitplane_deferred_enqueue, bitplane_deferred_clear);
     return (int)length;
   }
-  const size_t smem = std::max((size_t)(kBP_M + kBP_N) * kLd * sizeof(uint32_t),
-                               (size_t)kBP_M * (kBP_N + 1) * sizeof(int) + (size_t)kBP_M * kBP_N * sizeof(double));
-  static std::once_flag attr;
-  std::call_once(attr, [&] {
-    LAKGB_CUDA(cudaFuncSetAttribute(bitplane_main_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  });
-  if (g_bitplane_impl.load(std::memory_order_relaxed) == LAKGB_IMPL_TENSOR && (B == 8 || B == 16 || B == 32)) {
-    launch_bitplane_tc(p, nT, stream());
+  if (tensor) {
+    run->launch(B);
   } else {
+    const size_t smem = std::max((size_t)(kBP_M + kBP_N) * kLd * sizeof(uint32_t),
+                                 (size_t)kBP_M * (kBP_N + 1) * sizeof(int) + (size_t)kBP_M * kBP_N * sizeof(double));
+    static std::once_flag attr;
+    std::call_once(attr, [&] {
+      LAKGB_CUDA(cudaFuncSetAttribute(bitplane_main_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    });
     dim3 grid((npairs + kBP_M - 1) / kBP_M, nT);
     bitplane_main_kernel<<<grid, kBP_T, smem, stream()>>>(p);
     LAKGB_CUDA(cudaGetLastError());

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 namespace lakgb {
 
 struct BitplaneParams {
@@ -17,7 +19,7 @@ struct BitplaneParams {
   int npairs;
   const uint8_t *Zt; const uint32_t *zt_rowb; long long zt_row_bytes;
   const uint32_t *mw_a;                         // a-index of each Wn row (j order)
-  int nW; int B; int ncols_per;
+  int nW; int B; int ncols_per; int nT;
   const int8_t *vS;                             // [t][mw] +/-1
   const double *aA; const double *aZ;           // per pair
   const int *ycnt;                              // per plane row: popcount(y & mask)
@@ -26,15 +28,37 @@ struct BitplaneParams {
   const unsigned long long *out_off;            // per pair: row index in the output
   const unsigned long long *t_off;              // per t: column offset (index * row_stride)
   double *out;
+  // tensor-core form
+  int chunks;                                   // 128-bit chunks that hold patients
+  const uint32_t *a_blk;                        // per pair: 1920-SNP block of the At row
+  const double *aBlk; int nblk;                 // a of every block
+  double inv_mlt;                               // RN(1 / mlt); 0: divide by mlt itself
+  const double *At_base;                        // [t][pair]
+  const double2 *zz;                            // per pair: 1 - aZ, -1 - aZ
+  const long long *ysum;                        // per Wn row: sum_k 2^k popcount(plane_k & mask)
+  const double *q2;                             // [t][block][mw]: (a T_base + a T_tmp) / mlt
 };
 
-// The tensor-core main kernel (bitplane_tc.cu), in place of
-// bitplane_main_kernel; requires B in {8, 16, 32}.
-void launch_bitplane_tc(const BitplaneParams &p, int nT, cudaStream_t s);
-// CTAs of one call (pair tiles x covariate columns), and many calls of the
-// same B in one launch: ps / tile0 in device memory, tile0 the prefix sums
-// of the calls' CTA counts, `tiles` their total.
-int bitplane_tc_tiles(const BitplaneParams &p, int nT);
-void launch_bitplane_tc_group(int B, const BitplaneParams *ps, const int *tile0, int n, int tiles, cudaStream_t s);
+// The tensor-core form (bitplane_tc.cu), in place of bitplane_main_kernel;
+// requires B in {8, 16, 32}.  A segment is a range of Wn rows of one (call,
+// covariate column); its terms, one per (pair, Wn row), go to a scratch array
+// and are then added up in order.  A batch is what one pair of launches
+// computes: as many segments as the scratch holds.
+struct BitplaneSeg {
+  int call, t, w0, w1;
+  int unit0;      // first (pair tile, N tile) unit of the segment in its batch
+  int block0;     // first block of the segment in the batch's adding launch
+  long long y0;   // its terms in the scratch: [w - w0][pair]
+};
+struct BitplaneBatch { int seg0, nseg, units, blocks; };
+// Segments and batches of calls (host parameters) of the same B; returns the
+// scratch's size in doubles.
+size_t bitplane_tc_plan(int B, const std::vector<BitplaneParams> &ps, std::vector<BitplaneSeg> *segs,
+                        std::vector<BitplaneBatch> *batches);
+void launch_bitplane_tc(int B, const BitplaneParams *d_ps, const BitplaneSeg *d_segs,
+                        const std::vector<BitplaneBatch> &batches, double *scratch, cudaStream_t s);
+// Most doubles of scratch (64 MB) that the terms of a batch take; one step of
+// Wn rows of one column always fits.
+constexpr size_t kBitplaneScratch = size_t(8) << 20;
 
 }  // namespace lakgb
