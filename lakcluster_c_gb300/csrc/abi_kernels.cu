@@ -118,13 +118,13 @@ int gram_entry(bool symmetric, int type_flag, int spacing_r, int spacing_c, M_ha
   p.symmetric = symmetric ? 1 : 0;
   st.flush();
   // A large host output of a non-symmetric Gram comes back in two parts: the
-  // Z rows are split at a multiple of 128 rows (whole tensor-core tiles) into
+  // Z rows are split at a whole number of tensor-core tiles into
   // two launches, and the output columns of the first part (a contiguous
   // range: column indices grow with the Z row) are downloaded while the
   // second part computes.  Every element is computed exactly as by one
   // launch.  (A symmetric Gram also writes the mirrored elements, which
   // cross the column split, so it comes back in one piece.)
-  const int zsplit = ((nZ / 2) + 127) / 128 * 128;
+  const int zsplit = (nZ / 2 + kGramTileN - 1) / kGramTileN * kGramTileN;
   if (!mo && !symmetric && length * sizeof(double) >= kSplitDownloadBytes && zsplit > 0 && zsplit < nZ &&
       std::is_sorted(outc.begin(), outc.end())) {
     GramParams q0 = p, q1 = p;

@@ -34,8 +34,7 @@ struct GramParams {
 // Several independent Grams launched as one (the tensor-core kernel's grouped
 // form): their parameters, the prefix sums of their tile counts (n + 1) and
 // of their block counts (n + 1, rows of the table array), all in device
-// memory.  Every instance has the same type; a symmetric instance has a
-// square tile grid.
+// memory.  Every instance has the same type.
 struct GramGroupDev {
   const GramParams *ps;
   const int *tile0;
@@ -43,8 +42,10 @@ struct GramGroupDev {
   int n;
 };
 
-// Tiles of one Gram on the tensor-core kernel's 128 x 128 grid (symmetric
-// with a square grid: the upper triangle).
+// Output tile of the tensor-core kernel (A rows x Z rows).
+constexpr int kGramTileM = 128, kGramTileN = 112;
+// Tiles of one Gram on the tensor-core kernel's grid (symmetric: those that
+// hold a pair i <= k).
 int gram_tc_tiles(const GramParams &p);
 
 // Enqueue the grouped tensor-core Gram on stream s: the table kernel for all

@@ -8,41 +8,49 @@
 // weighted popcounts of popcount_xor_lf / popcount_and_lf
 // (dir_c/popcount.c:310-423).
 //
-// Integer part on the tensor cores.  Every packed bit becomes one e4m3 byte:
-// 0x08 (= 2^-6) for a set bit, 0 otherwise, the mask applied to the A side.
-// One product is 2^-12, so the fp32 accumulator of a block holds
-// n_ikb * 2^-12 with n_ikb = popcount(A_i & mask & Z_k) <= 1920: an exact
-// value (11 significant bits).  The XOR count is c = pa_ib + pz_kb - 2 n_ikb
-// with the row counts pa = popcount(A_i & mask), pz = popcount(Z_k & mask)
-// that the producer threads take while they expand the bits.  Which bit goes
-// to which K position does not matter (a dot product is order-free) as long
-// as A and Z use the same map; the map used makes the expansion two integer
-// operations per output word: bit 8i+j of a 32-bit word goes to byte i of
-// output word j.
+// Integer part on the tensor cores.  Every packed bit becomes one e2m1 value
+// (4 bits, kind::mxf4 with unit scale factors), the mask applied to the A
+// side, so that a product of two set bits is 1 and the fp32 accumulator of a
+// block holds n_ikb = popcount(A_i & mask & Z_k) <= 1920 exactly.  The XOR
+// count is c = pa_ib + pz_kb - 2 n_ikb with the row counts
+// pa = popcount(A_i & mask), pz = popcount(Z_k & mask) that the producer
+// threads take while they expand the bits.  Which bit goes to which K position
+// does not matter (a dot product is order-free) as long as A and Z use the
+// same map (tc::expand_e2m1).  Against one e4m3 byte per bit this halves the
+// shared-memory bytes written by the producers and read by the MMAs, which
+// together were over half of the kernel's shared-memory traffic, and takes a
+// third of the expansion's integer operations.
 //
 // FP64 part on the CUDA cores, in the reference's order: acc = acc + D_b * c,
 // one rounding each, blocks ascending.  The product D_b * c is read from a
 // table T_b[c] (c = 0..1920), built once per launch with the same rounded
 // multiply, so the FP64 pipe -- slow on this part -- does only the add.
 //
-// Persistent CTAs, one per SM, each looping over 128 (A rows) x 128 (Z rows)
+// Persistent CTAs, one per SM, each looping over 128 (A rows) x 112 (Z rows)
 // output tiles; the pipeline runs on across tile boundaries.  25 warps:
 //   warps 0-7   producers, one tile row each (A rows 0-127, then Z rows
-//               0-127): per 128-column chunk, load the row's 16 bytes, mask,
-//               expand to 128 e4m3 bytes in shared memory (K-major, 128-byte
-//               swizzle), count pa / pz.
-//   warp 8      owns TMEM; lane 0 issues the MMAs (M=128, N=128, K=32; 4 per
+//               0-111): per 128-column chunk, read the row's 16 bytes from the
+//               raw buffer, mask, expand to 64 bytes of e2m1 in shared memory
+//               (K-major, 64-byte swizzle), count pa / pz.  Each warp brings
+//               its 32 rows' 240 bytes of the next block into its own raw
+//               buffer by cp.async, two rows per instruction: 16 bytes of its
+//               own row per thread took 32 wavefronts per warp load, and one
+//               bulk copy per row 68 cycles of the copy engine each (241 a
+//               block, 16400 cycles: slower than everything else).
+//   warp 8      owns TMEM; lane 0 issues the MMAs (M=128, N=112, K=64; 2 per
 //               chunk, 15 chunks per block) into one of two count buffers.
 //   warps 9-24  fold, four warps per lane quadrant (warp w reads TMEM lanes
-//               32*(w%4)..+31), each for 32 of the 128 columns: per block,
+//               32*(w%4)..+31), each for 28 of the 112 columns: per block,
 //               read the counts from TMEM, look up T_b[c], add into the FP64
-//               accumulators, which live in TMEM as well (columns 256..511,
+//               accumulators, which live in TMEM as well (columns 256..479,
 //               two 32-bit halves per value).
-// Shared memory: 6 stages x (16 KB A + 16 KB B) + 2 x T_b (15 KB) + counts.
+// Shared memory: 2 raw buffers (56 KB each) + 5 stages x (8 KB A + 7 KB B) +
+// 2 x T_b (15 KB) + counts.
 // The T_b buffers are filled by bulk copies on mbarriers, issued by whichever
 // fold warp finishes a block last, so fold warps drift apart by up to a block
 // instead of meeting at every block boundary.
-// TMEM: 512 columns (2 x 128 count columns + 256 accumulator columns).
+// TMEM: 2 x 112 count columns (0.., 128..), the scale factors (112..127) and
+// 224 accumulator columns; N = 112 leaves room for the scale factors.
 #include <algorithm>
 
 #include "gram.cuh"
@@ -58,16 +66,17 @@ static __device__ int g_withhold;
 
 namespace {
 
-constexpr int kBM = 128, kBN = 128;
-constexpr int kStages = 6;
+constexpr int kBM = kGramTileM, kBN = kGramTileN;
+constexpr int kStages = 5;
 constexpr int kChunks = 15;               // 128-bit chunks per 1920-bit block
-constexpr int kPrefetch = 3;              // producer loads in flight (divides kChunks)
-constexpr int kStageA = kBM * 128;        // bytes: 128 rows x 128 e4m3
-constexpr int kStageB = kBN * 128;
+constexpr int kRawRow = 240;              // bytes of one row of a block
+constexpr int kRawBytes = (kBM + kBN) * kRawRow;
+constexpr int kStageA = kBM * 64;         // bytes: 128 rows x 128 e2m1
+constexpr int kStageB = kBN * 64;
 constexpr int kStageBytes = kStageA + kStageB;
 constexpr int kTabStride = 1922;          // doubles per block table (1921 used, 16-byte multiple)
 constexpr int kTabBytes = kTabStride * 8;
-constexpr int kSBO = 8 * 128;             // bytes between 8-row swizzle atoms (8 rows of 128 B)
+constexpr int kSBO = 8 * 64;              // bytes between 8-row swizzle atoms (8 rows of 64 B)
 constexpr int kProducers = 256;           // warps 0-7
 constexpr int kMmaWarp = 8;
 constexpr int kFold = 512;                // warps 9-24
@@ -77,7 +86,13 @@ constexpr int kFoldCols = kBN / (kFold / 128);  // tile columns per fold warp
 constexpr int kRounds = kFoldCols / kRound;
 constexpr int kThreads = kProducers + 32 + kFold;
 constexpr uint32_t kTmemCols = 512;
-constexpr size_t kSmemBytes = (size_t)kStages * kStageBytes + 2 * kTabBytes + 2 * (kBM + kBN) * 4 + 1024;
+constexpr uint32_t kCntCols = 128;        // columns from one count buffer to the next
+constexpr uint32_t kSfCol = 112;          // scale factors: 16 columns of ones
+constexpr uint32_t kAccCol = 256;
+static_assert(kFoldCols % kRound == 0 && kBN <= (int)kSfCol && kAccCol + 2 * kBN <= kTmemCols, "TMEM layout");
+static_assert(kStageBytes % 512 == 0 && kRawBytes % 16 == 0, "swizzle atoms, 16-byte copies");
+constexpr size_t kSmemBytes =
+    (size_t)kStages * kStageBytes + 2 * kRawBytes + 2 * kTabBytes + 2 * 256 * 4 + 1024;
 
 struct Smem {
   uint64_t full[kStages], empty[kStages];
@@ -88,21 +103,6 @@ struct Smem {
   uint32_t tmem_base;
   int abort;
 };
-
-// Expand the 128 bits of x into the 128 e4m3 bytes of one tile row (a
-// 128-byte row of a 128-byte-swizzled atom): word q of x fills the 16-byte
-// chunks 2q and 2q+1, stored at chunk index c ^ sw (sw = row % 8).
-__device__ __forceinline__ void expand_row(uint32_t row_base, uint32_t sw, uint4 x) {
-  const uint32_t w[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const uint32_t v = w[q];
-    tc::st_shared_v4(row_base + (((2 * q) ^ sw) << 4), (v << 3) & 0x08080808u, (v << 2) & 0x08080808u,
-                     (v << 1) & 0x08080808u, v & 0x08080808u);
-    tc::st_shared_v4(row_base + (((2 * q + 1) ^ sw) << 4), (v >> 1) & 0x08080808u, (v >> 2) & 0x08080808u,
-                     (v >> 3) & 0x08080808u, (v >> 4) & 0x08080808u);
-  }
-}
 
 template <int R>
 __device__ __forceinline__ void tmem_ld_n(uint32_t taddr, uint32_t (&v)[R]) {
@@ -123,9 +123,9 @@ __device__ __forceinline__ uint4 and4(uint4 a, uint4 b) {
   return make_uint4(a.x & b.x, a.y & b.y, a.z & b.z, a.w & b.w);
 }
 
-// Counts decoded from the accumulator: n * 2^-12 -> n (exact for n < 2^22).
+// Counts decoded from the accumulator (exact for n < 2^22).
 __device__ __forceinline__ int decode_count(uint32_t bits) {
-  return __float_as_int(__fmaf_rn(__uint_as_float(bits), 4096.0f, 12582912.0f)) - 0x4B400000;
+  return __float_as_int(__fadd_rn(__uint_as_float(bits), 12582912.0f)) - 0x4B400000;
 }
 
 // 2.0 * x, exactly as __dmul_rn(2.0, x) rounds it: for a normal x whose
@@ -142,24 +142,26 @@ __device__ __forceinline__ double twice(double x) {
 // bands of kBand tile rows, each band column by column: the CTAs of a wave
 // (consecutive r) then share a few A row panels and a few Z row panels, a
 // working set that stays in L2 even when a whole side of the product does
-// not (32768-row bins: 2 MB per 128-row panel).  A symmetric Gram with a
-// square tile grid lists only the pairs on or above the diagonal, row by row.
+// not (32768-row bins: 2 MB per 128-row panel).  A symmetric Gram lists only
+// the tiles that hold a pair i <= k, row by row: those of tile row i from
+// tile column i * 128 / 112 on.
 constexpr int kBand = 8;
-__device__ __forceinline__ void tile_coords(int ntm, int ntn, bool tri, int r, int &tile_m, int &tile_n) {
-  if (!tri) {
+__device__ __forceinline__ void tile_coords(int ntm, int ntn, bool sym, int r, int &tile_m, int &tile_n) {
+  if (!sym) {
     const int band = r / (kBand * ntn), in = r - band * (kBand * ntn);
     const int rows = min(kBand, ntm - band * kBand);
     tile_m = (band * kBand + in % rows) * kBM;
     tile_n = (in / rows) * kBN;
     return;
   }
-  int i = 0;
-  while (r >= ntn - i) {  // row i of the upper triangle holds ntn - i tiles
-    r -= ntn - i;
+  int i = 0, first = 0;
+  while (r >= ntn - first) {
+    r -= ntn - first;
     ++i;
+    first = i * kBM / kBN;
   }
   tile_m = i * kBM;
-  tile_n = (i + r) * kBN;
+  tile_n = (first + r) * kBN;
 }
 
 // The instance of a grouped launch that holds global tile (or table row) k:
@@ -176,42 +178,20 @@ __device__ __forceinline__ int find_instance(const I *start, int n, long long k)
 
 // Tile order shared by every role: tile k of the launch's list goes to CTA
 // k % gridDim.x, so the active tiles, not all tiles, are spread evenly over
-// the CTAs.  A single Gram lists its own tiles (tile_coords; a symmetric call
-// with unequal row counts skips the tiles below the diagonal as it walks); a
-// grouped launch lists the tiles of its instances one instance after another.
+// the CTAs.  A single Gram lists its own tiles (tile_coords); a grouped launch
+// lists the tiles of its instances one instance after another.
 template <bool GRP>
 struct TileWalk {
-  int ntm, ntn, ntiles, k;
-  bool tri;
-  __device__ TileWalk(const GramParams &p, const GramGroupDev &g) : k((int)blockIdx.x - (int)gridDim.x) {
-    if (GRP) {
-      ntiles = g.tile0[g.n];
-      ntm = ntn = 0;
-      tri = false;
-    } else {
-      ntn = (p.nZ + kBN - 1) / kBN;
-      ntm = (p.nA + kBM - 1) / kBM;
-      tri = p.symmetric && ntm == ntn;
-      ntiles = tri ? ntn * (ntn + 1) / 2 : ntm * ntn;
-    }
-  }
+  int ntiles, k;
+  __device__ TileWalk(int tiles, const GramGroupDev &g)
+      : ntiles(GRP ? g.tile0[g.n] : tiles), k((int)blockIdx.x - (int)gridDim.x) {}
   __device__ bool next(const GramParams &p, const GramGroupDev &g, int &inst, int &tile_m, int &tile_n) {
-    if (GRP) {
-      k += gridDim.x;
-      if (k >= ntiles) return false;
-      inst = find_instance(g.tile0, g.n, k);
-      const GramParams &q = g.ps[inst];
-      const int n_z = (q.nZ + kBN - 1) / kBN, n_m = (q.nA + kBM - 1) / kBM;
-      tile_coords(n_m, n_z, q.symmetric && n_m == n_z, k - g.tile0[inst], tile_m, tile_n);
-      return true;
-    }
-    inst = 0;
-    for (;;) {
-      k += gridDim.x;
-      if (k >= ntiles) return false;
-      tile_coords(ntm, ntn, tri, k, tile_m, tile_n);
-      if (tri || !(p.symmetric && tile_m > tile_n + kBN - 1)) return true;
-    }
+    k += gridDim.x;
+    if (k >= ntiles) return false;
+    inst = GRP ? find_instance(g.tile0, g.n, k) : 0;
+    const GramParams &q = GRP ? g.ps[inst] : p;
+    tile_coords((q.nA + kBM - 1) / kBM, (q.nZ + kBN - 1) / kBN, q.symmetric, GRP ? k - g.tile0[inst] : k, tile_m, tile_n);
+    return true;
   }
 };
 
@@ -224,13 +204,14 @@ __device__ __forceinline__ const GramParams &params_of(const GramParams &p, cons
 
 template <int TYPE, bool GRP>
 __global__ void __launch_bounds__(kThreads, 1)
-    gram_tc_kernel(GramParams p, GramGroupDev grp, const double *__restrict__ T, int *status) {
+    gram_tc_kernel(GramParams p, GramGroupDev grp, int tiles, const double *__restrict__ T, int *status) {
   extern __shared__ __align__(128) uint8_t dsm[];
   __shared__ Smem sm;
   // stages first, on a 1024-byte boundary (swizzle atoms)
   uint8_t *stages = dsm + ((1024 - (tc::smem_u32(dsm) & 1023)) & 1023);
-  double *sT = reinterpret_cast<double *>(stages + (size_t)kStages * kStageBytes);  // [2][kTabStride]
-  int *s_cnt = reinterpret_cast<int *>(stages + (size_t)kStages * kStageBytes + 2 * kTabBytes);  // [2][256]
+  uint8_t *raw = stages + (size_t)kStages * kStageBytes;                       // [2][kRawBytes]
+  double *sT = reinterpret_cast<double *>(raw + 2 * (size_t)kRawBytes);        // [2][kTabStride]
+  int *s_cnt = reinterpret_cast<int *>(raw + 2 * (size_t)kRawBytes + 2 * kTabBytes);  // [2][256]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile int *abort = &sm.abort;
@@ -258,86 +239,126 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = sm.tmem_base;
-  TileWalk<GRP> walk(p, grp);
+  // unit scale factors in every lane: one warp per lane quadrant
+  if (warp > kMmaWarp && warp <= kMmaWarp + 4) {
+    uint32_t ones[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) ones[i] = tc::kScaleOnes;
+    tc::tmem_st16(tmem + kSfCol + ((uint32_t)(32 * (warp & 3)) << 16), ones);
+    tc::tmem_wait_st();
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  TileWalk<GRP> walk(tiles, grp);
   int inst, tile_m, tile_n;
 
   if (tid < kProducers) {
     // ---------------- producers ----------------
     const int side = tid >> 7, rr = tid & 127;  // side 0: A row rr, side 1: Z row rr
-    const uint32_t st0 = tc::smem_u32(stages);
-    const uint32_t my_row = st0 + side * kStageA + (uint32_t)((rr >> 3) * kSBO + (rr & 7) * 128);
-    const uint32_t my_sw = (uint32_t)(rr & 7);
+    const bool has_row = side == 0 || rr < kBN;
+    const uint32_t my_row = tc::smem_u32(stages) + side * kStageA + (uint32_t)(rr * 64);
+    const uint32_t my_sw = (uint32_t)((rr >> 1) & 3);
+    const int row0 = side * kBM + (rr & ~31);  // this warp's first tile row
+    const uint32_t my_raw = tc::smem_u32(raw) + (uint32_t)((row0 + (has_row ? lane : 0)) * kRawRow);
     // the test hook, read once: this thread withholds its first arrival
     bool withhold = g_withhold && blockIdx.x == 0 && tid == 0;
     bool ok = true;
+    // One position ahead of the block being expanded: its tile's parameters
+    // and this thread's row, and the copies of the block into raw buffer t.
+    struct Src {
+      const uint8_t *base, *mask;
+      long long row_bytes;
+      uint32_t row;  // row of the matrix, ~0 past its end
+      int P;
+    };
+    auto next_tile = [&](Src &v) {
+      if (!walk.next(p, grp, inst, tile_m, tile_n)) return false;
+      const GramParams &q = params_of<GRP>(p, grp, inst);
+      const int r = (side ? tile_n : tile_m) + rr;
+      v.base = side ? q.wZ : q.wA;
+      v.row_bytes = side ? q.z_row_bytes : q.a_row_bytes;
+      v.mask = q.mask;
+      v.P = q.P;
+      v.row = (has_row && r < (side ? q.nZ : q.nA)) ? (side ? q.z_rowb : q.a_rowb)[r] : 0xffffffffu;
+      return true;
+    };
+    const int half = lane >= kChunks, piece = lane - kChunks * half;  // lanes 0-14: even rows, 15-29: odd rows
+    auto fetch = [&](const Src &v, int b, int t) {
+      const uint8_t *src = v.base + (long long)b * kRawRow + 16 * piece;
+      uint8_t *dst = raw + (size_t)t * kRawBytes + row0 * kRawRow + 16 * piece;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const uint32_t r = __shfl_sync(0xffffffffu, v.row, 2 * i + half);
+        if (lane < 2 * kChunks && r != 0xffffffffu)
+          tc::cp_async16(dst + (2 * i + half) * kRawRow, src + (long long)r * v.row_bytes);
+      }
+    };
+    Src cur{}, nxt{};
+    bool have = next_tile(cur);
+    if (have) fetch(cur, 0, 0);
+    tc::cp_async_commit();
     // ring position of the next chunk: stage s, in pass `wrap` over the ring
     int s = 0, wrap = 0;
-    int gbb = 0;  // blocks this CTA has produced
-    while (walk.next(p, grp, inst, tile_m, tile_n)) {
-      const GramParams &q = params_of<GRP>(p, grp, inst);
-      const uint8_t *base = side ? q.wZ : q.wA;
-      const uint32_t *rowb = side ? q.z_rowb : q.a_rowb;
-      const long long row_bytes = side ? q.z_row_bytes : q.a_row_bytes;
-      const int nrows = side ? q.nZ : q.nA;
-      const uint8_t *mask = q.mask;
-      const int G = q.P * kChunks;
-      const int grow = (side ? tile_n : tile_m) + rr;
-      const long long ro = grow < nrows ? (long long)rowb[grow] * row_bytes : -1;
-      uint4 rm[kPrefetch], rx[kPrefetch];
-      // chunk g of the tile covers bytes 16g..16g+15 of each row (blocks of
-      // 240 bytes are contiguous)
-      auto load = [&](int g, uint4 &m, uint4 &x) {
-        m = x = make_uint4(0, 0, 0, 0);
-        if (g < G) {
-          m = __ldg(reinterpret_cast<const uint4 *>(mask) + g);
-          if (ro >= 0) x = __ldg(reinterpret_cast<const uint4 *>(base + ro) + g);
+    int gbb = 0, b = 0;  // blocks this CTA has produced; block of the tile
+    while (have) {
+      const int t = gbb & 1;
+      bool more = true;
+      int nb = b + 1;
+      nxt = cur;
+      if (nb == cur.P) {
+        nb = 0;
+        more = next_tile(nxt);
+      }
+      if (more) fetch(nxt, nb, t ^ 1);
+      tc::cp_async_commit();
+      tc::cp_async_wait<1>();
+      __syncwarp();
+      const uint32_t row = my_raw + t * kRawBytes;
+      const uint4 *mk = reinterpret_cast<const uint4 *>(cur.mask) + (long long)b * kChunks;
+      int cnt = 0;
+      uint4 x = tc::ld_shared_v4(row), m = __ldg(mk);
+#pragma unroll 3
+      for (int ch = 0; ch < kChunks; ++ch) {
+        const uint4 xm = and4(x, m);
+        // A rows enter masked; Z rows unmasked (the mask on A already
+        // restricts every product), their count masked
+        const uint4 e = side ? x : xm;
+        if (TYPE == 1) cnt += popc4(xm);
+        if (ch + 1 < kChunks) {
+          x = tc::ld_shared_v4(row + 16 * (ch + 1));
+          m = __ldg(mk + ch + 1);
         }
-      };
-#pragma unroll
-      for (int u = 0; u < kPrefetch; ++u) load(u, rm[u], rx[u]);
-      int cnt = 0, ch = 0;
-      for (int g0 = 0; g0 < G; g0 += kPrefetch) {
-#pragma unroll
-        for (int u = 0; u < kPrefetch; ++u) {
-          const int g = g0 + u;
-          const uint4 m = rm[u];
-          const uint4 xm = and4(rx[u], m);
-          // A rows enter masked; Z rows unmasked (the mask on A already
-          // restricts every product), their count masked
-          const uint4 x = side ? rx[u] : xm;
-          load(g + kPrefetch, rm[u], rx[u]);
-          if (TYPE == 1) cnt += popc4(xm);
-          if (wrap > 0 && ok) ok = tc::mbar_wait(&sm.empty[s], (uint32_t)((wrap - 1) & 1), abort, status, 1);
-          if (ok) {
-            expand_row(my_row + s * kStageBytes, my_sw, x);
-            tc::fence_proxy_async();
-          }
-          __syncwarp();
-          if (lane == 0 && !withhold) tc::mbar_arrive(&sm.full[s]);
-          withhold = false;
-          if (++s == kStages) {
-            s = 0;
-            ++wrap;
-          }
-          if (++ch == kChunks) {
-            // end of a block: publish the row counts
-            const int t = gbb & 1;
-            if (gbb >= 2 && ok)
-              ok = tc::mbar_wait(&sm.aux_empty[t], (uint32_t)(((gbb >> 1) - 1) & 1), abort, status, 2);
-            s_cnt[t * 256 + tid] = cnt;
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&sm.aux_full[t]);
-            cnt = 0;
-            ch = 0;
-            ++gbb;
-          }
+        if (wrap > 0 && ok) ok = tc::mbar_wait(&sm.empty[s], (uint32_t)((wrap - 1) & 1), abort, status, 1);
+        if (ok && has_row) {
+          if (side) tc::expand_e2m1<1>(my_row + s * kStageBytes, my_sw, e);
+          else tc::expand_e2m1<0>(my_row + s * kStageBytes, my_sw, e);
+          tc::fence_proxy_async();
+        }
+        __syncwarp();
+        if (lane == 0 && !withhold) tc::mbar_arrive(&sm.full[s]);
+        withhold = false;
+        if (++s == kStages) {
+          s = 0;
+          ++wrap;
         }
       }
+      // publish the row counts
+      if (gbb >= 2 && ok)
+        ok = tc::mbar_wait(&sm.aux_empty[t], (uint32_t)(((gbb >> 1) - 1) & 1), abort, status, 2);
+      s_cnt[t * 256 + tid] = cnt;
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&sm.aux_full[t]);
+      ++gbb;
+      b = nb;
+      cur = nxt;
+      have = more;
     }
+    tc::cp_async_wait<0>();
   } else if (warp == kMmaWarp) {
     // ---------------- MMA issue ----------------
     if (lane == 0) {
-      constexpr uint32_t idesc = tc::idesc_e4m3_f32(kBM, kBN);
+      constexpr uint32_t idesc = tc::idesc_mxf4_f32(kBM, kBN);
       const uint32_t st0 = tc::smem_u32(stages);
       bool ok = true;
       int s = 0, wrap = 0, gbb = 0;
@@ -359,11 +380,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             tc::fence_after_sync();
             const uint32_t sa = st0 + cs * kStageBytes, sb = sa + kStageA;
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-              const uint64_t ad = tc::smem_desc_sw128(sa + kk * 32, kSBO);
-              const uint64_t bd = tc::smem_desc_sw128(sb + kk * 32, kSBO);
-              tc::mma_e4m3(tmem + t * kBN, ad, bd, idesc, (ch | kk) != 0);
-            }
+            for (int kk = 0; kk < 2; ++kk)
+              tc::mma_mxf4(tmem + t * kCntCols, tc::smem_desc_sw64(sa + kk * 32, kSBO),
+                           tc::smem_desc_sw64(sb + kk * 32, kSBO), idesc, tmem + kSfCol, tmem + kSfCol + 4,
+                           (ch | kk) != 0);
             tc::mma_commit(&sm.empty[cs]);
           }
           if (ok) tc::mma_commit(&sm.acc_full[t]);
@@ -451,8 +471,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         uint32_t cn[2][kRound], a[2][2 * kRound];
         auto load_round = [&](int r, int buf) {
           const int c0 = col0 + r * kRound;
-          tmem_ld_n<kRound>(lane_base + t * kBN + c0, cn[buf]);
-          if (b > 0) tmem_ld_n<2 * kRound>(lane_base + 256 + 2 * c0, a[buf]);
+          tmem_ld_n<kRound>(lane_base + t * kCntCols + c0, cn[buf]);
+          if (b > 0) tmem_ld_n<2 * kRound>(lane_base + kAccCol + 2 * c0, a[buf]);
         };
         if (ok) {
           load_round(0, 0);
@@ -493,9 +513,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             a[cur][2 * j + 1] = (uint32_t)__double2hiint(v);
           }
           if (b + 1 < P) {
-            // accumulators of columns c0 + j: TMEM columns 256 + 2 (c0 + j)
+            // accumulators of columns c0 + j: TMEM columns kAccCol + 2 (c0 + j)
             // (low word) and + 1 (high word)
-            if (ok) tmem_st_n<2 * kRound>(lane_base + 256 + 2 * c0, a[cur]);
+            if (ok) tmem_st_n<2 * kRound>(lane_base + kAccCol + 2 * c0, a[cur]);
           } else if (ok && row_in) {
 #pragma unroll
             for (int j = 0; j < kRound; ++j) {
@@ -587,11 +607,13 @@ int sm_count() {
   return n;
 }
 
-// Tiles a launch computes (symmetric Grams: the tiles on or above the
-// diagonal of the square tile grid).
+// Tiles a launch computes (symmetric Grams: those that hold a pair i <= k).
 int active_tiles(const GramParams &p) {
   const int ntm = (p.nA + kBM - 1) / kBM, ntn = (p.nZ + kBN - 1) / kBN;
-  return (p.symmetric && ntm == ntn) ? ntn * (ntn + 1) / 2 : ntm * ntn;
+  if (!p.symmetric) return ntm * ntn;
+  int n = 0;
+  for (int i = 0; i < ntm; ++i) n += std::max(0, ntn - i * kBM / kBN);
+  return n;
 }
 
 template <int TYPE, bool GRP>
@@ -607,8 +629,8 @@ void configure_tc() {
 template <int TYPE>
 void launch_tc_type(const GramParams &p, const double *T, cudaStream_t s) {
   configure_tc<TYPE, false>();
-  const int grid = std::max(1, std::min(active_tiles(p), sm_count()));
-  gram_tc_kernel<TYPE, false><<<grid, kThreads, kSmemBytes, s>>>(p, GramGroupDev{}, T, tc_status_device_ptr());
+  const int tiles = active_tiles(p), grid = std::max(1, std::min(tiles, sm_count()));
+  gram_tc_kernel<TYPE, false><<<grid, kThreads, kSmemBytes, s>>>(p, GramGroupDev{}, tiles, T, tc_status_device_ptr());
   LAKGB_CUDA(cudaGetLastError());
   count_launch();
 }
@@ -617,7 +639,7 @@ template <int TYPE>
 void launch_tc_group_type(const GramGroupDev &g, int total_tiles, const double *T, cudaStream_t s) {
   configure_tc<TYPE, true>();
   const int grid = std::max(1, std::min(total_tiles, sm_count()));
-  gram_tc_kernel<TYPE, true><<<grid, kThreads, kSmemBytes, s>>>(GramParams{}, g, T, tc_status_device_ptr());
+  gram_tc_kernel<TYPE, true><<<grid, kThreads, kSmemBytes, s>>>(GramParams{}, g, total_tiles, T, tc_status_device_ptr());
   LAKGB_CUDA(cudaGetLastError());
   count_launch();
 }

@@ -172,6 +172,71 @@ __host__ __device__ constexpr uint32_t idesc_e4m3_f32(int M, int N) {
   return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// As smem_desc_sw128 with the 64-byte swizzle: rows of 64 bytes, 8-row atoms
+// of 512 bytes (512-byte aligned), the 16-byte chunk c of row r stored at chunk
+// c ^ (r / 2 % 4).
+__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t saddr, uint32_t sbo) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+  d |= (uint64_t)1 << 16;  // leading byte offset: unused by swizzled K-major layouts
+  d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
+  d |= (uint64_t)1 << 46;  // descriptor version
+  d |= (uint64_t)4 << 61;  // layout: 64-byte swizzle
+  return d;
+}
+
+// Instruction descriptor of kind::mxf4 with e2m1 A and B, ue8m0 scale factors
+// (data IDs 0), f32 accumulator, both operands K-major, K = 64, shape M x N.
+__host__ __device__ constexpr uint32_t idesc_mxf4_f32(int M, int N) {
+  return (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | (1u << 23) | ((uint32_t)(M >> 4) << 24);
+}
+
+// D[tmem] (+)= A * B^T with block scale factors (one per 32 elements of K) at
+// TMEM columns sfa / sfb, issued by one thread.
+__device__ __forceinline__ void mma_mxf4(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t sfa,
+                                         uint32_t sfb, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.b32 p, %6, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%4], [%5], p;\n}\n" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
+      : "memory");
+}
+// The scale factor 2^0 (ue8m0 127) in every byte of a 32-bit TMEM cell.
+constexpr uint32_t kScaleOnes = 0x7F7F7F7Fu;
+
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// 16 bytes from shared memory.
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+// The 128 bits of x as 128 e2m1 values in one 64-byte row of a 64-byte-swizzled
+// atom (sw = row / 2 % 4), two values per byte.  A clear bit is 0; bit class j
+// (bit 4i + j of a word) goes to 16-byte chunk j and becomes, in A and B rows
+// (SIDE 0 and 1), 0.5 and 2, 1 and 1, 2 and 0.5, 1 and 1, so that every
+// product of two set bits is 1: most classes are then one AND of the word with
+// a mask, with no shift (e2m1: 1 = 0.5, 2 = 1.0, 4 = 2.0).
+template <int SIDE>
+__device__ __forceinline__ void expand_e2m1(uint32_t row_base, uint32_t sw, uint4 x) {
+  const uint32_t v[4] = {x.x, x.y, x.z, x.w};
+  uint32_t o[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t d = v[i] >> 2;
+    o[0][i] = SIDE ? ((v[i] << 2) & 0x44444444u) : (v[i] & 0x11111111u);
+    o[1][i] = v[i] & 0x22222222u;
+    o[2][i] = SIDE ? (d & 0x11111111u) : (v[i] & 0x44444444u);
+    o[3][i] = d & 0x22222222u;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) st_shared_v4(row_base + ((j ^ sw) << 4), o[j][0], o[j][1], o[j][2], o[j][3]);
+}
+
 // D[tmem] (+)= A * B^T, issued by one thread.
 __device__ __forceinline__ void mma_e4m3(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                          uint32_t accumulate) {
@@ -273,10 +338,6 @@ __device__ __forceinline__ void cp_async_wait() {
 
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-
-__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
 }  // namespace tc
