@@ -29,22 +29,26 @@
 // Persistent CTAs, one per SM, each looping over 128 (A rows) x 112 (Z rows)
 // output tiles; the pipeline runs on across tile boundaries.  25 warps:
 //   warps 0-7   producers, one tile row each (A rows 0-127, then Z rows
-//               0-111): per 128-column chunk, read the row's 16 bytes from the
-//               raw buffer, mask, expand to 64 bytes of e2m1 in shared memory
-//               (K-major, 64-byte swizzle), count pa / pz.  Each warp brings
-//               its 32 rows' 240 bytes of the next block into its own raw
-//               buffer by cp.async, two rows per instruction: 16 bytes of its
-//               own row per thread took 32 wavefronts per warp load, and one
-//               bulk copy per row 68 cycles of the copy engine each (241 a
-//               block, 16400 cycles: slower than everything else).
-//   warp 8      owns TMEM; lane 0 issues the MMAs (M=128, N=112, K=64; 2 per
-//               chunk, 15 chunks per block) into one of two count buffers.
+//               0-111): per step of 384 columns, read the row's 48 bytes from
+//               the raw buffer, mask, expand to three 64-byte rows of e2m1 in
+//               shared memory (K-major, 64-byte swizzle), count pa / pz.  A
+//               producer warp works alone on its rows, so its time per step is
+//               instruction latency: three chunks of 128 columns at once give
+//               it independent instructions, and one wait, proxy fence and
+//               arrival serve all three.  Each warp brings its 32 rows' next
+//               steps into its own raw slots by cp.async, one block ahead, a
+//               fixed (row, 16 bytes) per lane and copy: 16 bytes of its own
+//               row per thread took 32 wavefronts per warp load, and one bulk
+//               copy per row 68 cycles of the copy engine each (241 a block,
+//               16400 cycles: slower than everything else).
+//   warp 8      owns TMEM; lane 0 issues the MMAs (M=128, N=112, K=64; 6 per
+//               step, 5 steps per block) into one of two count buffers.
 //   warps 9-24  fold, four warps per lane quadrant (warp w reads TMEM lanes
 //               32*(w%4)..+31), each for 28 of the 112 columns: per block,
 //               read the counts from TMEM, look up T_b[c], add into the FP64
 //               accumulators, which live in TMEM as well (columns 256..479,
 //               two 32-bit halves per value).
-// Shared memory: 2 raw buffers (56 KB each) + 5 stages x (8 KB A + 7 KB B) +
+// Shared memory: 6 raw slots (11 KB each) + 2 stages x 3 x (8 KB A + 7 KB B) +
 // 2 x T_b (15 KB) + counts.
 // The T_b buffers are filled by bulk copies on mbarriers, issued by whichever
 // fold warp finishes a block last, so fold warps drift apart by up to a block
@@ -67,13 +71,17 @@ static __device__ int g_withhold;
 namespace {
 
 constexpr int kBM = kGramTileM, kBN = kGramTileN;
-constexpr int kStages = 5;
-constexpr int kChunks = 15;               // 128-bit chunks per 1920-bit block
-constexpr int kRawRow = 240;              // bytes of one row of a block
+constexpr int kStages = 2;
+constexpr int kChunk = 3;                 // 128-column chunks per step
+constexpr int kSteps = 5;                 // steps per 1920-column block
+constexpr int kBlockRow = 240;            // bytes of one row of a block
+constexpr int kRawRow = 16 * kChunk;      // bytes of one row of a step
+constexpr int kRawSlots = kSteps + 1;
 constexpr int kRawBytes = (kBM + kBN) * kRawRow;
-constexpr int kStageA = kBM * 64;         // bytes: 128 rows x 128 e2m1
-constexpr int kStageB = kBN * 64;
-constexpr int kStageBytes = kStageA + kStageB;
+constexpr int kTileA = kBM * 64;          // bytes: 128 rows x 128 e2m1
+constexpr int kTileB = kBN * 64;
+constexpr int kChunkBytes = kTileA + kTileB;
+constexpr int kStageBytes = kChunk * kChunkBytes;
 constexpr int kTabStride = 1922;          // doubles per block table (1921 used, 16-byte multiple)
 constexpr int kTabBytes = kTabStride * 8;
 constexpr int kSBO = 8 * 64;              // bytes between 8-row swizzle atoms (8 rows of 64 B)
@@ -90,9 +98,9 @@ constexpr uint32_t kCntCols = 128;        // columns from one count buffer to th
 constexpr uint32_t kSfCol = 112;          // scale factors: 16 columns of ones
 constexpr uint32_t kAccCol = 256;
 static_assert(kFoldCols % kRound == 0 && kBN <= (int)kSfCol && kAccCol + 2 * kBN <= kTmemCols, "TMEM layout");
-static_assert(kStageBytes % 512 == 0 && kRawBytes % 16 == 0, "swizzle atoms, 16-byte copies");
+static_assert(kChunkBytes % 512 == 0 && kSteps * kRawRow == kBlockRow, "swizzle atoms, whole blocks");
 constexpr size_t kSmemBytes =
-    (size_t)kStages * kStageBytes + 2 * kRawBytes + 2 * kTabBytes + 2 * 256 * 4 + 1024;
+    (size_t)kStages * kStageBytes + kRawSlots * kRawBytes + 2 * kTabBytes + 2 * 256 * 4 + 1024;
 
 struct Smem {
   uint64_t full[kStages], empty[kStages];
@@ -209,9 +217,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   __shared__ Smem sm;
   // stages first, on a 1024-byte boundary (swizzle atoms)
   uint8_t *stages = dsm + ((1024 - (tc::smem_u32(dsm) & 1023)) & 1023);
-  uint8_t *raw = stages + (size_t)kStages * kStageBytes;                       // [2][kRawBytes]
-  double *sT = reinterpret_cast<double *>(raw + 2 * (size_t)kRawBytes);        // [2][kTabStride]
-  int *s_cnt = reinterpret_cast<int *>(raw + 2 * (size_t)kRawBytes + 2 * kTabBytes);  // [2][256]
+  uint8_t *raw = stages + (size_t)kStages * kStageBytes;                       // [kRawSlots][kRawBytes]
+  double *sT = reinterpret_cast<double *>(raw + kRawSlots * (size_t)kRawBytes);  // [2][kTabStride]
+  int *s_cnt = reinterpret_cast<int *>(sT + 2 * kTabStride);                   // [2][256]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile int *abort = &sm.abort;
@@ -257,50 +265,54 @@ __global__ void __launch_bounds__(kThreads, 1)
     // ---------------- producers ----------------
     const int side = tid >> 7, rr = tid & 127;  // side 0: A row rr, side 1: Z row rr
     const bool has_row = side == 0 || rr < kBN;
-    const uint32_t my_row = tc::smem_u32(stages) + side * kStageA + (uint32_t)(rr * 64);
+    const uint32_t my_row = tc::smem_u32(stages) + side * kTileA + (uint32_t)(rr * 64);
     const uint32_t my_sw = (uint32_t)((rr >> 1) & 3);
     const int row0 = side * kBM + (rr & ~31);  // this warp's first tile row
     const uint32_t my_raw = tc::smem_u32(raw) + (uint32_t)((row0 + (has_row ? lane : 0)) * kRawRow);
     // the test hook, read once: this thread withholds its first arrival
     bool withhold = g_withhold && blockIdx.x == 0 && tid == 0;
     bool ok = true;
-    // One position ahead of the block being expanded: its tile's parameters
-    // and this thread's row, and the copies of the block into raw buffer t.
+    // A tile's mask, blocks and the global addresses of this lane's kChunk
+    // copies of a step (copy j of a lane: piece i % 3 of the warp's row i / 3,
+    // i = lane + 32 j; null: a row past the matrix).
     struct Src {
-      const uint8_t *base, *mask;
-      long long row_bytes;
-      uint32_t row;  // row of the matrix, ~0 past its end
+      const uint8_t *mask, *piece[kChunk];
       int P;
     };
     auto next_tile = [&](Src &v) {
       if (!walk.next(p, grp, inst, tile_m, tile_n)) return false;
       const GramParams &q = params_of<GRP>(p, grp, inst);
-      const int r = (side ? tile_n : tile_m) + rr;
-      v.base = side ? q.wZ : q.wA;
-      v.row_bytes = side ? q.z_row_bytes : q.a_row_bytes;
       v.mask = q.mask;
       v.P = q.P;
-      v.row = (has_row && r < (side ? q.nZ : q.nA)) ? (side ? q.z_rowb : q.a_rowb)[r] : 0xffffffffu;
+      const int first = (side ? tile_n : tile_m) + (rr & ~31);
+      const int last = side ? min(q.nZ, tile_n + kBN) : q.nA;
+#pragma unroll
+      for (int j = 0; j < kChunk; ++j) {
+        const int i = lane + 32 * j, r = first + i / kChunk;
+        v.piece[j] = nullptr;
+        if (r < last)
+          v.piece[j] = (side ? q.wZ : q.wA) + (long long)(side ? q.z_rowb : q.a_rowb)[r] * (side ? q.z_row_bytes : q.a_row_bytes) +
+                       16 * (i % kChunk);
+      }
       return true;
     };
-    const int half = lane >= kChunks, piece = lane - kChunks * half;  // lanes 0-14: even rows, 15-29: odd rows
-    auto fetch = [&](const Src &v, int b, int t) {
-      const uint8_t *src = v.base + (long long)b * kRawRow + 16 * piece;
-      uint8_t *dst = raw + (size_t)t * kRawBytes + row0 * kRawRow + 16 * piece;
+    uint8_t *my_dst = raw + row0 * kRawRow + 16 * lane;  // copy j: + 512 j
+    auto fetch = [&](const Src &v, int step, int slot) {  // step: from the tile's first column
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const uint32_t r = __shfl_sync(0xffffffffu, v.row, 2 * i + half);
-        if (lane < 2 * kChunks && r != 0xffffffffu)
-          tc::cp_async16(dst + (2 * i + half) * kRawRow, src + (long long)r * v.row_bytes);
-      }
+      for (int j = 0; j < kChunk; ++j)
+        if (v.piece[j])
+          tc::cp_async16(my_dst + (size_t)slot * kRawBytes + 512 * j, v.piece[j] + (long long)step * kRawRow);
+      tc::cp_async_commit();
     };
     Src cur{}, nxt{};
     bool have = next_tile(cur);
-    if (have) fetch(cur, 0, 0);
-    tc::cp_async_commit();
-    // ring position of the next chunk: stage s, in pass `wrap` over the ring
-    int s = 0, wrap = 0;
-    int gbb = 0, b = 0;  // blocks this CTA has produced; block of the tile
+    for (int j = 0; j < kSteps; ++j) {
+      if (have) fetch(cur, j, j);
+      else tc::cp_async_commit();
+    }
+    int s = 0, wrap = 0;   // ring position of the next step: stage s, in pass `wrap` over the ring
+    int slot = 0;          // raw slot of the next step
+    int gbb = 0, b = 0;    // blocks this CTA has produced; block of the tile
     while (have) {
       const int t = gbb & 1;
       bool more = true;
@@ -310,29 +322,38 @@ __global__ void __launch_bounds__(kThreads, 1)
         nb = 0;
         more = next_tile(nxt);
       }
-      if (more) fetch(nxt, nb, t ^ 1);
-      tc::cp_async_commit();
-      tc::cp_async_wait<1>();
-      __syncwarp();
-      const uint32_t row = my_raw + t * kRawBytes;
-      const uint4 *mk = reinterpret_cast<const uint4 *>(cur.mask) + (long long)b * kChunks;
+      const uint4 *mk = reinterpret_cast<const uint4 *>(cur.mask) + (long long)b * (kSteps * kChunk);
       int cnt = 0;
-      uint4 x = tc::ld_shared_v4(row), m = __ldg(mk);
-#pragma unroll 3
-      for (int ch = 0; ch < kChunks; ++ch) {
-        const uint4 xm = and4(x, m);
-        // A rows enter masked; Z rows unmasked (the mask on A already
-        // restricts every product), their count masked
-        const uint4 e = side ? x : xm;
-        if (TYPE == 1) cnt += popc4(xm);
-        if (ch + 1 < kChunks) {
-          x = tc::ld_shared_v4(row + 16 * (ch + 1));
-          m = __ldg(mk + ch + 1);
-        }
+#pragma unroll 1
+      for (int j = 0; j < kSteps; ++j) {
+        // the step kSteps ahead, into the slot read before this one
+        if (more) fetch(nxt, nb * kSteps + j, slot ? slot - 1 : kRawSlots - 1);
+        else tc::cp_async_commit();
+        uint4 x[kChunk], m[kChunk];
+#pragma unroll
+        for (int u = 0; u < kChunk; ++u) m[u] = __ldg(mk + j * kChunk + u);
+        tc::cp_async_wait<kSteps>();
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < kChunk; ++u) x[u] = tc::ld_shared_v4(my_raw + slot * kRawBytes + 16 * u);
         if (wrap > 0 && ok) ok = tc::mbar_wait(&sm.empty[s], (uint32_t)((wrap - 1) & 1), abort, status, 1);
+#pragma unroll
+        for (int u = 0; u < kChunk; ++u) {
+          // A rows enter masked; Z rows unmasked (the mask on A already
+          // restricts every product), their count masked
+          const uint4 xm = and4(x[u], m[u]);
+          if (TYPE == 1) cnt += popc4(xm);
+          if (!side) x[u] = xm;
+        }
         if (ok && has_row) {
-          if (side) tc::expand_e2m1<1>(my_row + s * kStageBytes, my_sw, e);
-          else tc::expand_e2m1<0>(my_row + s * kStageBytes, my_sw, e);
+          const uint32_t dst = my_row + s * kStageBytes;
+          if (side) {
+#pragma unroll
+            for (int u = 0; u < kChunk; ++u) tc::expand_e2m1<1>(dst + u * kChunkBytes, my_sw, x[u]);
+          } else {
+#pragma unroll
+            for (int u = 0; u < kChunk; ++u) tc::expand_e2m1<0>(dst + u * kChunkBytes, my_sw, x[u]);
+          }
           tc::fence_proxy_async();
         }
         __syncwarp();
@@ -342,6 +363,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           s = 0;
           ++wrap;
         }
+        if (++slot == kRawSlots) slot = 0;
       }
       // publish the row counts
       if (gbb >= 2 && ok)
@@ -369,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (gbb >= 2)
             ok = tc::mbar_wait(&sm.acc_empty[t], (uint32_t)(((gbb >> 1) - 1) & 1), abort, status, 3);
           tc::fence_after_sync();
-          for (int ch = 0; ch < kChunks && ok; ++ch) {
+          for (int st = 0; st < kSteps && ok; ++st) {
             const int cs = s;
             ok = tc::mbar_wait(&sm.full[cs], (uint32_t)(wrap & 1), abort, status, 4);
             if (++s == kStages) {
@@ -378,12 +400,15 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             if (!ok) break;
             tc::fence_after_sync();
-            const uint32_t sa = st0 + cs * kStageBytes, sb = sa + kStageA;
 #pragma unroll
-            for (int kk = 0; kk < 2; ++kk)
-              tc::mma_mxf4(tmem + t * kCntCols, tc::smem_desc_sw64(sa + kk * 32, kSBO),
-                           tc::smem_desc_sw64(sb + kk * 32, kSBO), idesc, tmem + kSfCol, tmem + kSfCol + 4,
-                           (ch | kk) != 0);
+            for (int u = 0; u < kChunk; ++u) {
+              const uint32_t sa = st0 + cs * kStageBytes + u * kChunkBytes, sb = sa + kTileA;
+#pragma unroll
+              for (int kk = 0; kk < 2; ++kk)
+                tc::mma_mxf4(tmem + t * kCntCols, tc::smem_desc_sw64(sa + kk * 32, kSBO),
+                             tc::smem_desc_sw64(sb + kk * 32, kSBO), idesc, tmem + kSfCol, tmem + kSfCol + 4,
+                             (st | u | kk) != 0);
+            }
             tc::mma_commit(&sm.empty[cs]);
           }
           if (ok) tc::mma_commit(&sm.acc_full[t]);
