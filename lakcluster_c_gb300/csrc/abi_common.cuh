@@ -8,6 +8,7 @@
 
 #include <vector>
 
+#include "bcc_model.h"
 #include "lakgb_runtime.cuh"
 
 namespace lakgb {
@@ -21,18 +22,28 @@ inline unsigned long long spacing_length(int spacing, const M_handle *M) {
   }
 }
 
-// Index of the j-th retained row in the given spacing (AnZt_vv.c:71-77).
-inline std::vector<uint32_t> spacing_index(int spacing, const M_handle *M) {
-  std::vector<uint32_t> v((size_t)M->rpop_j);
-  for (long long j = 0; j < M->rpop_j; ++j) {
-    switch (spacing) {
-      case LAKGB_SPACING_j: v[j] = (uint32_t)j; break;
-      case LAKGB_SPACING_b: v[j] = M->m_b_[j]; break;
-      case LAKGB_SPACING_a: v[j] = M->m_a_[j]; break;
-      default: v[j] = 0; break;
-    }
+// Indices of the first n retained rows in the given spacing (AnZt_vv.c:71-77),
+// each times `mul`.  A solve makes some 10^4 calls whose lists have a few
+// thousand entries: one loop per spacing, without a test per element.
+template <class T>
+inline std::vector<T> spacing_index_of(int spacing, const M_handle *M, long long n, T mul = 1) {
+  std::vector<T> v((size_t)n);
+  T *o = v.data();
+  if (spacing == LAKGB_SPACING_j) {
+    for (long long j = 0; j < n; ++j) o[j] = (T)j * mul;
+  } else {
+    const unsigned int *from = spacing == LAKGB_SPACING_b ? M->m_b_ : M->m_a_;
+    for (long long j = 0; j < n; ++j) o[j] = (T)from[j] * mul;
   }
   return v;
+}
+
+// Index of the j-th retained row in the given spacing (zeros for none of the
+// three).
+inline std::vector<uint32_t> spacing_index(int spacing, const M_handle *M) {
+  if (spacing != LAKGB_SPACING_a && spacing != LAKGB_SPACING_b && spacing != LAKGB_SPACING_j)
+    return std::vector<uint32_t>((size_t)M->rpop_j, 0u);
+  return spacing_index_of<uint32_t>(spacing, M, M->rpop_j);
 }
 
 // Allocate (malloc, zero-filled) or check-and-zero the output, as the
@@ -75,15 +86,18 @@ struct HostOutputFill {
   }
 };
 
-inline int popcount_bytes(const unsigned char *p, long n) {
-  int c = 0;
-  for (long i = 0; i < n; ++i) c += __builtin_popcount((unsigned)p[i]);
-  return c;
-}
+inline int popcount_bytes(const unsigned char *p, long n) { return (int)lakbcc::popcount_bytes(p, n); }
 
 inline long long popcount_bytes_masked(const unsigned char *p, const unsigned char *m, long n) {
   long long c = 0;
-  for (long i = 0; i < n; ++i) c += __builtin_popcount((unsigned)(p[i] & m[i]));
+  long i = 0;
+  for (; i + 8 <= n; i += 8) {
+    uint64_t a, b;
+    memcpy(&a, p + i, 8);
+    memcpy(&b, m + i, 8);
+    c += __builtin_popcountll(a & b);
+  }
+  for (; i < n; ++i) c += __builtin_popcount((unsigned)(p[i] & m[i]));
   return c;
 }
 

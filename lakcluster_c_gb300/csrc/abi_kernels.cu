@@ -71,8 +71,8 @@ int gram_entry(bool symmetric, int type_flag, int spacing_r, int spacing_c, M_ha
   const void *wA = resident(M_An->wX, (size_t)M_An->rpop_b * M_An->mc_length);
   const void *wZ = resident(M_Zn->wX, (size_t)M_Zn->rpop_b * M_Zn->mc_length);
   DBuf mask = upload_bytes(M_An->mc_j, M_An->mc_length);
-  std::vector<uint32_t> arow(M_An->m_b_, M_An->m_b_ + nA), zrow(M_Zn->m_b_, M_Zn->m_b_ + nZ);
-  DBuf d_arow = upload_vec(arow), d_zrow = upload_vec(zrow);
+  DBuf d_arow = upload_bytes(M_An->m_b_, (size_t)nA * sizeof(uint32_t));
+  DBuf d_zrow = upload_bytes(M_Zn->m_b_, (size_t)nZ * sizeof(uint32_t));
   const std::vector<uint32_t> outc = spacing_index(spacing_c, M_Zn);
   DBuf d_outr = upload_vec(spacing_index(spacing_r, M_An));
   DBuf d_outc = upload_vec(outc);
@@ -90,8 +90,10 @@ int gram_entry(bool symmetric, int type_flag, int spacing_r, int spacing_c, M_ha
     std::vector<double> a((size_t)nA), z((size_t)nZ);
     std::vector<uint32_t> ia = spacing_index(lf_An_ajdk->spacing_row, M_An);
     std::vector<uint32_t> iz = spacing_index(lf_Zn_ajdk->spacing_row, M_Zn);
-    for (int i = 0; i < nA; ++i) a[i] = lf_An_ajdk->lf[ia[i] + kAjdk_1_1 * lf_An_ajdk->row_stride];
-    for (int k = 0; k < nZ; ++k) z[k] = lf_Zn_ajdk->lf[iz[k] + kAjdk_1_1 * lf_Zn_ajdk->row_stride];
+    const double *la = lf_An_ajdk->lf + kAjdk_1_1 * lf_An_ajdk->row_stride;
+    const double *lz = lf_Zn_ajdk->lf + kAjdk_1_1 * lf_Zn_ajdk->row_stride;
+    for (int i = 0; i < nA; ++i) a[i] = la[ia[i]];
+    for (int k = 0; k < nZ; ++k) z[k] = lz[iz[k]];
     d_lfA = upload_vec(a);
     d_lfZ = upload_vec(z);
   }
@@ -199,8 +201,7 @@ extern "C" int wrap_An_v__run(int *tidx, void **vpra, pthread_t *thread_in, int 
   Stager st;
   const void *w = resident(M_An->wX, (size_t)M_An->rpop_b * M_An->mc_length);
   DBuf mask = upload_bytes(M_An->mc_j, M_An->mc_length);
-  std::vector<uint32_t> rows(M_An->m_b_, M_An->m_b_ + n);
-  DBuf d_rows = upload_vec(rows), d_outr = upload_vec(spacing_index(output_spacing_r, M_An));
+  DBuf d_rows = upload_bytes(M_An->m_b_, (size_t)n * sizeof(uint32_t)), d_outr = upload_vec(spacing_index(output_spacing_r, M_An));
   st.flush();
   DBuf d_out(length * sizeof(double));
   d_out.zero();
@@ -229,20 +230,17 @@ extern "C" int wrap_An_ajdk_v(int *tidx, void **vpra, pthread_t *thread_in, int 
     return (int)length;
   }
   const int P = (int)(M_An->mc_length / kBlockBytes);
-  double base[LAKGB_AJDK_TOT];
-  for (int k = 0; k < LAKGB_AJDK_TOT; ++k) {
-    double s = 0.0;
-    for (int nc = 0; nc < P; ++nc)
-      s += A_ajdk[nc + k * P] * (double)popcount_bytes(M_An->mc_j + (long)nc * kBlockBytes, kBlockBytes);
-    base[k] = s;
+  double base[LAKGB_AJDK_TOT] = {0.0};
+  for (int nc = 0; nc < P; ++nc) {  // each sum in block order
+    const double c = (double)popcount_bytes(M_An->mc_j + (long)nc * kBlockBytes, kBlockBytes);
+    for (int k = 0; k < LAKGB_AJDK_TOT; ++k) base[k] += A_ajdk[nc + k * P] * c;
   }
   const int n = (int)M_An->rpop_j;
   if (n == 0) return (int)length;
   Stager st;
   const void *w = resident(M_An->wX, (size_t)M_An->rpop_b * M_An->mc_length);
   DBuf mask = upload_bytes(M_An->mc_j, M_An->mc_length);
-  std::vector<uint32_t> rows(M_An->m_b_, M_An->m_b_ + n);
-  DBuf d_rows = upload_vec(rows), d_outr = upload_vec(spacing_index(output_spacing_r, M_An));
+  DBuf d_rows = upload_bytes(M_An->m_b_, (size_t)n * sizeof(uint32_t)), d_outr = upload_vec(spacing_index(output_spacing_r, M_An));
   DBuf d_ajdk = upload_bytes(A_ajdk, (size_t)P * LAKGB_AJDK_TOT * sizeof(double));
   DBuf d_base = upload_bytes(base, sizeof(base));
   DBuf d_out(length * sizeof(double));

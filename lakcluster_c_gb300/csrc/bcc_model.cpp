@@ -61,10 +61,7 @@ MH *mh_make_owned(int nrows, int ncols) {
   return M;
 }
 
-static void mxget_excerpt(int n, const unsigned char *mb, const unsigned char *mj, long long *pop_b,
-                          long long *pop_j, unsigned int *a_, unsigned int *b_, long length) {
-  *pop_b = popcount_bytes(mb, length);
-  *pop_j = popcount_bytes(mj, length);
+long mask_lists(int n, const unsigned char *mb, const unsigned char *mj, unsigned int *a_, unsigned int *b_) {
   // The reference walks the n bits one at a time: every bit on in mb takes
   // the next b index, and those also on in mj are listed with their a and b
   // indices.  Same lists here, 64 elements at a time (bit 7 of a byte is its
@@ -72,7 +69,7 @@ static void mxget_excerpt(int n, const unsigned char *mb, const unsigned char *m
   // empty words are skipped, full words written as one run, and in the
   // others only the listed bits are visited, their b index being b plus the
   // mb bits before them.
-  if (n <= 0) return;
+  if (n <= 0) return 0;
   unsigned b = 0, j = 0;
   const long nwords = (long)n / 64;
   for (long w = 0; w < nwords; ++w) {
@@ -108,6 +105,14 @@ static void mxget_excerpt(int n, const unsigned char *mb, const unsigned char *m
       on_b &= ~bit;
     }
   }
+  return (long)j;
+}
+
+static void mxget_excerpt(int n, const unsigned char *mb, const unsigned char *mj, long long *pop_b,
+                          long long *pop_j, unsigned int *a_, unsigned int *b_, long length) {
+  *pop_b = popcount_bytes(mb, length);
+  *pop_j = popcount_bytes(mj, length);
+  mask_lists(n, mb, mj, a_, b_);
 }
 
 void mhandle_mxget(M_handle *h) {

@@ -75,6 +75,9 @@ MH *mh_make(int nrows, int ncols, unsigned char *rows, const unsigned char *mr_b
             const unsigned char *mc_b);
 // Same, owning a zeroed row buffer of nrows x bsize(ncols) bytes.
 MH *mh_make_owned(int nrows, int ncols);
+// The elements on in both masks (of n), in order: their positions (a_) and
+// their positions among the elements on in mb (b_); returns how many.
+long mask_lists(int n, const unsigned char *mb, const unsigned char *mj, unsigned int *a_, unsigned int *b_);
 // M_mxget (M_init.c:268-295): pops and index lists from the masks.
 void mh_mxget(MH *M);
 // The same on a bare M_handle whose mask and index arrays are already sized.

@@ -689,15 +689,16 @@ extern "C" int wrap_At_T_YnWt_S_Zn_ww__run(int *tidx, void **vpra, pthread_t *th
   const bool tensor = g_bitplane_impl.load(std::memory_order_relaxed) == LAKGB_IMPL_TENSOR &&
                       (B == 8 || B == 16 || B == 32);
 
-  std::vector<uint32_t> at_rowb(npairs), zt_rowb(npairs), a_blk(npairs), tt_rowb(nT), mw_a(nW);
+  const std::vector<uint32_t> at_rowb(M_At->m_b_, M_At->m_b_ + npairs), zt_rowb(M_Zt->m_b_, M_Zt->m_b_ + npairs),
+      mw_a(M_Wn->m_a_, M_Wn->m_a_ + nW);
+  std::vector<uint32_t> a_blk(npairs), tt_rowb(nT);
   std::vector<double> aA(npairs), aZ(npairs);
-  std::vector<unsigned long long> out_off(npairs), t_off(nT);
+  std::vector<unsigned long long> t_off(nT);
+  const auto out_off = spacing_index_of<unsigned long long>(spacing_a, M_At, npairs);
   for (int i = 0; i < npairs; ++i) {
-    at_rowb[i] = M_At->m_b_[i]; zt_rowb[i] = M_Zt->m_b_[i];
     a_blk[i] = M_At->m_a_[i] / lakbcc::POPLENGTH;
     aA[i] = a_An[a_blk[i]];
     aZ[i] = a_An[M_Zt->m_a_[i] / lakbcc::POPLENGTH];
-    out_off[i] = pick_u(spacing_a, i, M_At->m_b_[i], M_At->m_a_[i]);
   }
   std::vector<int8_t> vS((size_t)nT * nW);
   for (int t = 0; t < nT; ++t) {
@@ -706,7 +707,6 @@ extern "C" int wrap_At_T_YnWt_S_Zn_ww__run(int *tidx, void **vpra, pthread_t *th
     const unsigned char *st = M_St->wX + (size_t)M_St->m_b_[t] * M_St->mc_length;
     for (int mw = 0; mw < nW; ++mw) vS[(size_t)t * nW + mw] = (int8_t)lakbcc::bget_pm(st, M_Wn->m_a_[mw]);
   }
-  for (int mw = 0; mw < nW; ++mw) mw_a[mw] = M_Wn->m_a_[mw];
 
   // Inside a deferral scope the tensor-core main kernel waits for the scope's
   // end (its uploads are then owned buffers, not staging views).  Only with
@@ -847,9 +847,9 @@ extern "C" int wrap_An_ZtSn_ww__run(int *tidx, void **vpra, pthread_t *thread_in
     set_error(4, "wrap_An_ZtSn_ww__run: planes and rows of unequal length");
     return (int)length;
   }
-  std::vector<uint32_t> rowb(M_An->m_b_, M_An->m_b_ + n);
-  std::vector<unsigned long long> out_r(n), s_off(nS);
-  for (int i = 0; i < n; ++i) out_r[i] = pick_u(spacing_a, i, M_An->m_b_[i], M_An->m_a_[i]);
+  const std::vector<uint32_t> rowb(M_An->m_b_, M_An->m_b_ + n);
+  const auto out_r = spacing_index_of<unsigned long long>(spacing_a, M_An, n);
+  std::vector<unsigned long long> s_off(nS);
   for (int s = 0; s < nS; ++s) s_off[s] = pick_u(spacing_s, s, M_St->m_b_[s], M_St->m_a_[s]) * length_a;
   const int nplanes = nS * M_ZtSn->ncols_per_z;
   Stager st;

@@ -339,16 +339,13 @@ extern "C" int wrap_AnZt_S_WnYt_vv__run(int *tidx, void **vpra, pthread_t *threa
   out->spacing_col = output_spacing_s; out->col_stride = length_s;
   const int nA = (int)M_An->rpop_j, nZ = (int)M_Zn->rpop_j, nS = (int)M_St->rpop_j;
   if (!lf_AnZt || !lf_YnWt || nA == 0 || nS == 0) return (int)length;
-  std::vector<unsigned long long> a_r(nA), y_r(nA), out_r(nA), a_c(nZ), y_c(nZ), s_off(nS);
-  for (int i = 0; i < nA; ++i) {
-    a_r[i] = pick_u(lf_AnZt->spacing_row, i, M_An->m_b_[i], M_An->m_a_[i]);
-    y_r[i] = pick_u(lf_YnWt->spacing_row, i, M_An->m_b_[i], M_An->m_a_[i]);
-    out_r[i] = pick_u(output_spacing_a, i, M_An->m_b_[i], M_An->m_a_[i]);
-  }
-  for (int k = 0; k < nZ; ++k) {
-    a_c[k] = pick_u(lf_AnZt->spacing_col, k, M_Zn->m_b_[k], M_Zn->m_a_[k]) * lf_AnZt->row_stride;
-    y_c[k] = pick_u(lf_YnWt->spacing_col, k, M_Zn->m_b_[k], M_Zn->m_a_[k]) * lf_YnWt->row_stride;
-  }
+  using Idx = unsigned long long;
+  const auto a_r = spacing_index_of<Idx>(lf_AnZt->spacing_row, M_An, nA);
+  const auto y_r = spacing_index_of<Idx>(lf_YnWt->spacing_row, M_An, nA);
+  const auto out_r = spacing_index_of<Idx>(output_spacing_a, M_An, nA);
+  const auto a_c = spacing_index_of<Idx>(lf_AnZt->spacing_col, M_Zn, nZ, lf_AnZt->row_stride);
+  const auto y_c = spacing_index_of<Idx>(lf_YnWt->spacing_col, M_Zn, nZ, lf_YnWt->row_stride);
+  std::vector<Idx> s_off(nS);
   std::vector<int8_t> vS((size_t)nS * (nZ > 0 ? nZ : 1));
   for (int s = 0; s < nS; ++s) {
     s_off[s] = pick_u(output_spacing_s, s, M_St->m_b_[s], M_St->m_a_[s]) * length_a;
@@ -490,19 +487,15 @@ extern "C" int wrap_AtTYn____WtSZn_vv__run(int *tidx, void **vpra, pthread_t *th
   const int Y_pcols = (int)lakbcc::psize(M_Yt->nrows);
   const double *D_Yn = Y_ajdk + (size_t)lakbcc::AJDK_0_1 * Y_pcols;
   const L_handle *LA = lf_AtTYn, *LZ = lf_ZtSWn;
-  std::vector<unsigned long long> ay_a(npairs), zw_z(npairs), out_r(npairs), ay_y(ninner > 0 ? ninner : 1),
-      zw_w(ninner > 0 ? ninner : 1), ay_s(nS), zw_s(nS), s_off(nS);
-  std::vector<double> Dy(ninner > 0 ? ninner : 1);
-  for (int i = 0; i < npairs; ++i) {
-    ay_a[i] = pick_u(LA->spacing_row, i, M_At->m_b_[i], M_At->m_a_[i]);
-    zw_z[i] = pick_u(LZ->spacing_row, i, M_Zt->m_b_[i], M_Zt->m_a_[i]);
-    out_r[i] = pick_u(output_spacing_a, i, M_At->m_b_[i], M_At->m_a_[i]);
-  }
-  for (int k = 0; k < ninner; ++k) {
-    ay_y[k] = pick_u(LA->spacing_col, k, M_Yt->m_b_[k], M_Yt->m_a_[k]) * LA->row_stride;
-    zw_w[k] = pick_u(LZ->spacing_col, k, M_Wt->m_b_[k], M_Wt->m_a_[k]) * LZ->row_stride;
-    Dy[k] = D_Yn[M_Yt->m_a_[k] / lakbcc::POPLENGTH];
-  }
+  using Idx = unsigned long long;
+  const auto ay_a = spacing_index_of<Idx>(LA->spacing_row, M_At, npairs);
+  const auto zw_z = spacing_index_of<Idx>(LZ->spacing_row, M_Zt, npairs);
+  const auto out_r = spacing_index_of<Idx>(output_spacing_a, M_At, npairs);
+  const auto ay_y = spacing_index_of<Idx>(LA->spacing_col, M_Yt, ninner, LA->row_stride);
+  const auto zw_w = spacing_index_of<Idx>(LZ->spacing_col, M_Wt, ninner, LZ->row_stride);
+  std::vector<Idx> ay_s(nS), zw_s(nS), s_off(nS);
+  std::vector<double> Dy(ninner);
+  for (int k = 0; k < ninner; ++k) Dy[k] = D_Yn[M_Yt->m_a_[k] / lakbcc::POPLENGTH];
   for (int s = 0; s < nS; ++s) {
     ay_s[s] = pick_u(LA->spacing_lyr, s, M_St->m_b_[s], M_St->m_a_[s]) * LA->row_stride * LA->col_stride;
     zw_s[s] = pick_u(LZ->spacing_lyr, s, M_St->m_b_[s], M_St->m_a_[s]) * LZ->row_stride * LZ->col_stride;
@@ -594,26 +587,27 @@ int attyn_entry(bool symmetric, const char *who, int output_spacing_a, int outpu
   const int A_pcols = (int)lakbcc::psize(M_At->nrows), Y_pcols = (int)lakbcc::psize(M_Yt->nrows);
   const double *a_An = A_ajdk + (size_t)lakbcc::AJDK_1_0 * A_pcols;
   const double *a_Yn = Y_ajdk + (size_t)lakbcc::AJDK_1_0 * Y_pcols;
-  std::vector<uint32_t> a_rowb(M_At->m_b_, M_At->m_b_ + nA), y_rowb(M_Yt->m_b_, M_Yt->m_b_ + nY), t_rowb(nT);
+  const std::vector<uint32_t> a_rowb(M_At->m_b_, M_At->m_b_ + nA), y_rowb(M_Yt->m_b_, M_Yt->m_b_ + nY);
+  std::vector<uint32_t> t_rowb(nT);
   std::vector<double> hhAy((size_t)nT * nA), hhaY((size_t)nT * nY), hhay(nT), aA(nA), aY(nY);
-  std::vector<unsigned long long> out_a(nA), out_y(nY), out_t(nT);
-  for (int i = 0; i < nA; ++i) {
-    aA[i] = a_An[M_At->m_a_[i] / lakbcc::POPLENGTH];
-    out_a[i] = pick_u(output_spacing_a, i, M_At->m_b_[i], M_At->m_a_[i]);
-  }
-  for (int k = 0; k < nY; ++k) {
-    aY[k] = a_Yn[M_Yt->m_a_[k] / lakbcc::POPLENGTH];
-    out_y[k] = pick_u(output_spacing_y, k, M_Yt->m_b_[k], M_Yt->m_a_[k]) * la;
-  }
+  using Idx = unsigned long long;
+  const auto out_a = spacing_index_of<Idx>(output_spacing_a, M_At, nA);
+  const auto out_y = spacing_index_of<Idx>(output_spacing_y, M_Yt, nY, la);
+  std::vector<Idx> out_t(nT);
+  for (int i = 0; i < nA; ++i) aA[i] = a_An[M_At->m_a_[i] / lakbcc::POPLENGTH];
+  for (int k = 0; k < nY; ++k) aY[k] = a_Yn[M_Yt->m_a_[k] / lakbcc::POPLENGTH];
+  // row indices of the integer sums, read at their covariate's column
+  const auto ia = spacing_index_of<Idx>(lf_AtTn->spacing_row, M_At, nA);
+  const auto iy = spacing_index_of<Idx>(lf_YtTn->spacing_row, M_Yt, nY);
   for (int t = 0; t < nT; ++t) {
     const unsigned tb = M_Tt->m_b_[t], ta = M_Tt->m_a_[t];
     t_rowb[t] = tb;
     out_t[t] = pick_u(output_spacing_t, t, tb, ta) * la * ly;
     hhay[t] = (double)(-M_Tt->cpop_j + 2ll * popcount_bytes_masked(M_Tt->wX + (size_t)tb * M_Tt->mc_length, M_Tt->mc_j, (long)M_Tt->mc_length));
-    for (int i = 0; i < nA; ++i)
-      hhAy[(size_t)t * nA + i] = (double)(long long)(*lakbcc::L2_get(lf_AtTn, i, M_At->m_b_[i], M_At->m_a_[i], t, tb, ta));
-    for (int k = 0; k < nY; ++k)
-      hhaY[(size_t)t * nY + k] = (double)(long long)(*lakbcc::L2_get(lf_YtTn, k, M_Yt->m_b_[k], M_Yt->m_a_[k], t, tb, ta));
+    const double *ca = lf_AtTn->lf + lakbcc::pick(lf_AtTn->spacing_col, t, tb, ta) * lf_AtTn->row_stride;
+    const double *cy = lf_YtTn->lf + lakbcc::pick(lf_YtTn->spacing_col, t, tb, ta) * lf_YtTn->row_stride;
+    for (int i = 0; i < nA; ++i) hhAy[(size_t)t * nA + i] = (double)(long long)ca[ia[i]];
+    for (int k = 0; k < nY; ++k) hhaY[(size_t)t * nY + k] = (double)(long long)cy[iy[k]];
   }
   AtTYnParams p{};
   Stager st;
@@ -634,11 +628,8 @@ int attyn_entry(bool symmetric, const char *who, int output_spacing_a, int outpu
   DBuf d_oa2, d_oy2;
   if (symmetric) {
     // transposed positions: Yt row k as an output row, At row i as a column
-    std::vector<unsigned long long> out_a2(nY), out_y2(nA);
-    for (int k = 0; k < nY; ++k) out_a2[k] = pick_u(output_spacing_a, k, M_Yt->m_b_[k], M_Yt->m_a_[k]);
-    for (int i = 0; i < nA; ++i) out_y2[i] = pick_u(output_spacing_y, i, M_At->m_b_[i], M_At->m_a_[i]) * la;
-    d_oa2 = upload_vec(out_a2);
-    d_oy2 = upload_vec(out_y2);
+    d_oa2 = upload_vec(spacing_index_of<Idx>(output_spacing_a, M_Yt, nY));
+    d_oy2 = upload_vec(spacing_index_of<Idx>(output_spacing_y, M_At, nA, la));
     p.symmetric = 1;
     p.out_a2 = d_oa2.as<unsigned long long>();
     p.out_y2 = d_oy2.as<unsigned long long>();

@@ -441,11 +441,6 @@ double *noalloc_scratch() {
   return static_cast<double *>(g_noalloc_scratch[dev]);
 }
 
-inline bool bit_on(const unsigned char *b, long n) { return (b[n / 8] >> (7 - n % 8)) & 1; }
-inline unsigned long long pick(int s, unsigned long long j, unsigned long long b, unsigned long long a) {
-  return s == LAKGB_SPACING_j ? j : (s == LAKGB_SPACING_b ? b : a);
-}
-
 }  // namespace
 
 }  // namespace lakgb
@@ -553,26 +548,20 @@ extern "C" void wrap_xcalc(int *tidx, void **vpra, pthread_t *thread_in, unsigne
   const unsigned long long rs = lf_YnWt ? lf_YnWt->row_stride : 0;
   std::vector<long long> row_off_a((size_t)(Yn_nrows > 0 ? Yn_nrows : 1), -1), rows_j, cols_j;
   {
-    unsigned long long j = 0, b = 0;
-    for (int a = 0; a < Yn_nrows; ++a) {
-      if (!bit_on(mr_b, a)) continue;
-      if (bit_on(mr_j, a)) {
-        const long long o = trm_flag ? (long long)(pick(sc, j, b, a) * rs) : (long long)pick(sr, j, b, a);
-        row_off_a[a] = o;
-        rows_j.push_back(o);
-        ++j;
-      }
-      ++b;
-    }
-    j = 0; b = 0;
-    for (int a = 0; a < Wn_nrows; ++a) {
-      if (!bit_on(mc_b, a)) continue;
-      if (bit_on(mc_j, a)) {
-        cols_j.push_back(trm_flag ? (long long)pick(sr, j, b, a) : (long long)(pick(sc, j, b, a) * rs));
-        ++j;
-      }
-      ++b;
-    }
+    std::vector<unsigned> ia, ib;
+    // the retained elements' offsets in one dimension of lf
+    auto offsets = [&](int n, const unsigned char *mb, const unsigned char *mj, int spacing, unsigned long long stride,
+                       std::vector<long long> &out) {
+      ia.resize((size_t)(n > 0 ? n : 0));
+      ib.resize(ia.size());
+      const long cnt = lakbcc::mask_lists(n, mb, mj, ia.data(), ib.data());
+      out.resize((size_t)cnt);
+      const unsigned *from = spacing == LAKGB_SPACING_b ? ib.data() : spacing == LAKGB_SPACING_j ? nullptr : ia.data();
+      for (long i = 0; i < cnt; ++i) out[i] = (long long)((from ? from[i] : (unsigned long long)i) * stride);
+    };
+    offsets(Yn_nrows, mr_b, mr_j, trm_flag ? sc : sr, trm_flag ? rs : 1, rows_j);
+    for (size_t i = 0; i < rows_j.size(); ++i) row_off_a[ia[i]] = rows_j[i];
+    offsets(Wn_nrows, mc_b, mc_j, trm_flag ? sr : sc, trm_flag ? 1 : rs, cols_j);
   }
   long long max_off = 0;
   for (long long o : rows_j) max_off = o > max_off ? o : max_off;
@@ -595,8 +584,8 @@ extern "C" void wrap_xcalc(int *tidx, void **vpra, pthread_t *thread_in, unsigne
   int slot = -1;
   // Plane 0: the rows set in mr_j (xcalc.c:141).
   std::vector<unsigned char> row0((size_t)lakbcc::bsize(Yn_nrows), 0);
-  for (int a = 0; a < Yn_nrows; ++a)
-    if (bit_on(mr_j, a)) row0[a / 8] |= (unsigned char)(1 << (7 - a % 8));
+  memcpy(row0.data(), mr_j, (size_t)(Yn_nrows + 7) / 8);
+  if (Yn_nrows % 8) row0[Yn_nrows / 8] &= (unsigned char)(0xFF00 >> (Yn_nrows % 8));
   // no values: min 0, max 1 before the margins (xcalc.c:34)
   double min = 0.0 - 0.0625, max = 1.0 + 0.0625, mlt = (double)g_d_mlt / (max - min);
   if (values) {
@@ -686,9 +675,12 @@ extern "C" void wrap_xcalc(int *tidx, void **vpra, pthread_t *thread_in, unsigne
   M_X->mr_length = lakbcc::bsize(M_X->nrows);
   M_X->ncols_extend = (lakbcc::BITJ - (M_X->ncols % lakbcc::BITJ)) % lakbcc::BITJ;
   M_X->mc_length = lakbcc::bsize(M_X->ncols);
-  for (int j = 0; j < ncols_bZ; ++j) { lakbcc::bset_on(M_X->mr_b, j); lakbcc::bset_on(M_X->mr_j, j); }
+  memset(M_X->mr_b, 0xFF, (size_t)(ncols_bZ / 8));
+  memset(M_X->mr_j, 0xFF, (size_t)(ncols_bZ / 8));
+  for (int j = ncols_bZ / 8 * 8; j < ncols_bZ; ++j) { lakbcc::bset_on(M_X->mr_b, j); lakbcc::bset_on(M_X->mr_j, j); }
   M_X->rpop_b = ncols_bZ; M_X->rpop_j = ncols_bZ;
-  for (unsigned long i = 0; i < M_X->mc_length; ++i) { M_X->mc_b[i] = mr_b[i]; M_X->mc_j[i] = mr_j[i]; }
+  memcpy(M_X->mc_b, mr_b, M_X->mc_length);
+  memcpy(M_X->mc_j, mr_j, M_X->mc_length);
   M_X->cpop_b = rpop_b; M_X->cpop_j = rpop_j;
   M_X->wX = M_X->Ara;
   M_X->ncols_per_z = ncols_per;
