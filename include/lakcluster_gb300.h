@@ -557,9 +557,9 @@ void lakgb_call_profile_reset(void);
 #define LAKGB_IMPL_POPCOUNT 0
 #define LAKGB_IMPL_TENSOR 1
 #define LAKGB_IMPL_AUTO 2
-/* Gram only: the popcount kernel split over blocks (every 1920-column block
- * of every output tile counted by its own CTA, then the FP64 fold over the
- * blocks in order); for launches with few output tiles.  Bit-identical. */
+/* Gram only: tensor-core counts split over blocks (every 1920-column block of
+ * every output tile counted by its own CTA, then the FP64 fold over the blocks
+ * in order); for launches with few output tiles.  Bit-identical. */
 #define LAKGB_IMPL_SPLIT 3
 #define LAKGB_GRAM_POPCOUNT LAKGB_IMPL_POPCOUNT
 #define LAKGB_GRAM_TENSOR LAKGB_IMPL_TENSOR
@@ -568,10 +568,10 @@ void lakgb_set_gram_impl(int impl);
 int lakgb_gram_impl(void);
 /* LAKGB_GRAM_AUTO (the default) picks the Gram kernel and tile shape by
  * measurement: the first launch of each shape class (type, symmetric, log2 of
- * the A rows, Z rows and blocks) runs every candidate -- the tensor-core
- * kernel, two tile shapes of the popcount kernel and the popcount kernel
- * split over blocks, all bit-identical --
- * timed with CUDA events, and the fastest serves that class afterwards.
+ * the A rows, Z rows and blocks) below 1024 rows on a side runs the
+ * candidates -- the persistent tensor-core kernel and the counts split over
+ * blocks, bit-identical -- timed with CUDA events, and the faster serves that
+ * class afterwards (a kernel that was not timed reads -1 in the table).
  * lakgb_gram_autotune_table writes the table as JSON into buf (returns its
  * full length); lakgb_gram_autotune_reset clears it. */
 int lakgb_gram_autotune_table(char *buf, int buf_len);

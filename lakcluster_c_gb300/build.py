@@ -21,7 +21,7 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "liblakgb300.so")
 
 CU_SOURCES = ["lakgb_runtime.cu", "gram.cu", "gram_tc.cu", "rowvec.cu", "abi_kernels.cu", "xcalc.cu", "bitplane.cu",
-              "bitplane_tc.cu", "loopsum.cu", "lmirror.cu",
+              "bitplane_tc.cu", "tc_counts.cu", "loopsum.cu", "lmirror.cu",
               "vv_kernels.cu", "transpose.cu", "bed.cu", "condense.cu"]
 # Host-only translation units (the solve driver and its input reader).
 CPP_SOURCES = ["bcc_model.cpp", "bcc_sort.cpp", "bcc_driver.cpp", "bcc_io.cpp", "bcc_abi.cpp", "bcc_server.cpp"]

@@ -79,6 +79,7 @@ struct HostOutputFill {
   unsigned long long n = 0;
   bool copied = false;
   HostOutputFill() = default;
+  HostOutputFill(L_handle *out, unsigned long long length) : L(out), n(length) {}
   HostOutputFill(const HostOutputFill &) = delete;
   HostOutputFill &operator=(const HostOutputFill &) = delete;
   ~HostOutputFill() {

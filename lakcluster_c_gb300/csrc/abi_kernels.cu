@@ -188,7 +188,8 @@ extern "C" int wrap_An_v__run(int *tidx, void **vpra, pthread_t *thread_in, int 
   LAKGB_PROFILE_CALL("wrap_An_v__run");
   (void)tidx; (void)vpra; (void)thread_in;
   const unsigned long long length = spacing_length(output_spacing_r, M_An);
-  L_handle *out = ensure_output(output_An_v_p, length, "wrap_An_v__run");
+  L_handle *out = ensure_output(output_An_v_p, length, "wrap_An_v__run", false);
+  HostOutputFill fill{out, length};
   if (!out) return (int)length;
   out->spacing_row = output_spacing_r; out->row_stride = length;
   if (type_flag == LAKGB_TYPE_p0) {
@@ -210,7 +211,7 @@ extern "C" int wrap_An_v__run(int *tidx, void **vpra, pthread_t *thread_in, int 
   p.mask = mask.as<uint8_t>(); p.P = P; p.type = (type_flag == LAKGB_TYPE_pm) ? 1 : 2;
   p.cpop_j = M_An->cpop_j; p.out_r = d_outr.as<uint32_t>(); p.out = d_out.as<double>();
   launch_an_v(p);
-  copy_back(out->lf, d_out, length);
+  copy_back(out->lf, d_out, length, &fill);
   return (int)length;
 }
 
@@ -221,7 +222,8 @@ extern "C" int wrap_An_ajdk_v(int *tidx, void **vpra, pthread_t *thread_in, int 
   (void)tidx; (void)vpra; (void)thread_in;
   const unsigned long long length_r = spacing_length(output_spacing_r, M_An);
   const unsigned long long length = length_r * LAKGB_AJDK_TOT;
-  L_handle *out = ensure_output(output_An_ajdk_p, length, "wrap_An_ajdk_v");
+  L_handle *out = ensure_output(output_An_ajdk_p, length, "wrap_An_ajdk_v", false);
+  HostOutputFill fill{out, length};
   if (!out) return (int)length;
   out->spacing_row = output_spacing_r; out->row_stride = length_r;
   out->spacing_col = LAKGB_SPACING_a; out->col_stride = LAKGB_AJDK_TOT;
@@ -252,6 +254,6 @@ extern "C" int wrap_An_ajdk_v(int *tidx, void **vpra, pthread_t *thread_in, int 
   p.out_r = d_outr.as<uint32_t>(); p.out_stride = (long long)length_r; p.out = d_out.as<double>();
   st.flush();
   launch_an_ajdk(p);
-  copy_back(out->lf, d_out, length);
+  copy_back(out->lf, d_out, length, &fill);
   return (int)length;
 }

@@ -642,9 +642,8 @@ void bitplane_deferred_enqueue() {
     defer_flush();
     t_bp_runs.back().launch(B);
   }
-  for (const auto &d : t_bp)
-    if (d.length)
-      LAKGB_CUDA(cudaMemcpyAsync(d.host_out, d.p.out, d.length * sizeof(double), cudaMemcpyDeviceToHost, stream()));
+  // the outputs come back with the scope's other ones; their buffers stay in t_bp
+  for (const auto &d : t_bp) defer_copy(d.host_out, DBuf::view(d.p.out, d.length * sizeof(double)), d.length);
 }
 
 void bitplane_deferred_clear() {
@@ -664,7 +663,8 @@ extern "C" int wrap_At_T_YnWt_S_Zn_ww__run(int *tidx, void **vpra, pthread_t *th
   const unsigned long long length_a = spacing_length(spacing_a, M_At);
   const unsigned long long length_t = spacing_length(spacing_t, M_Tt);
   const unsigned long long length = length_a * length_t;
-  L_handle *out = ensure_output(output_p, length, "wrap_At_T_YnWt_S_Zn_ww__run");
+  L_handle *out = ensure_output(output_p, length, "wrap_At_T_YnWt_S_Zn_ww__run", false);
+  HostOutputFill fill{out, length};
   if (!out) return (int)length;
   out->spacing_row = spacing_a; out->row_stride = length_a;
   out->spacing_col = spacing_t; out->col_stride = length_t;
@@ -804,6 +804,7 @@ extern "C" int wrap_At_T_YnWt_S_Zn_ww__run(int *tidx, void **vpra, pthread_t *th
     d.p = p;
     d.host_out = out->lf;
     d.length = length;
+    fill.copied = true;
     for (DBuf *b : {&mask, &d_at, &d_zt, &d_tt, &d_mw, &d_vS, &d_aA, &d_aZ, &d_oo, &d_to, &d_pm, &d_ycnt, &d_Tb, &d_Tt,
                     &d_ablk, &d_aBlk, &d_ys, &d_q2, &d_Ab, &d_zz, &d_out})
       d.keep.push_back(std::move(*b));
@@ -825,7 +826,7 @@ extern "C" int wrap_At_T_YnWt_S_Zn_ww__run(int *tidx, void **vpra, pthread_t *th
     LAKGB_CUDA(cudaGetLastError());
     count_launch();
   }
-  copy_back(out->lf, d_out, length);
+  copy_back(out->lf, d_out, length, &fill);
   return (int)length;
 }
 
@@ -837,7 +838,8 @@ extern "C" int wrap_An_ZtSn_ww__run(int *tidx, void **vpra, pthread_t *thread_in
   const unsigned long long length_a = spacing_length(spacing_a, M_An);
   const unsigned long long length_s = spacing_length(spacing_s, M_St);
   const unsigned long long length = length_a * length_s;
-  L_handle *out = ensure_output(output_p, length, "wrap_An_ZtSn_ww__run");
+  L_handle *out = ensure_output(output_p, length, "wrap_An_ZtSn_ww__run", false);
+  HostOutputFill fill{out, length};
   if (!out) return (int)length;
   out->spacing_row = spacing_a; out->row_stride = length_a;
   out->spacing_col = spacing_s; out->col_stride = length_s;
@@ -887,7 +889,7 @@ extern "C" int wrap_An_ZtSn_ww__run(int *tidx, void **vpra, pthread_t *thread_in
   an_ztsn_finish_kernel<<<(unsigned)(((long long)n * nS + 255) / 256), 256, 0, stream()>>>(p);
   LAKGB_CUDA(cudaGetLastError());
   count_launch();
-  copy_back(out->lf, d_out, length);
+  copy_back(out->lf, d_out, length, &fill);
   return (int)length;
 }
 

@@ -14,9 +14,8 @@
 // shared memory (row pitch 61 words: conflict-free column reads), every
 // thread accumulates a TM x TN micro-tile of integer counts over the block's
 // 60 words, then folds them into FP64 accumulators with the block weight.
-// For launches with few tiles the same staging and counting run split over
-// blocks (one CTA per tile and block, counts to a scratch array), followed by
-// a kernel that does the fold in block order.
+// Launches of few tiles run on the tensor cores split over blocks
+// (tc_counts.cu).
 #include <string.h>
 
 #include <algorithm>
@@ -30,6 +29,7 @@
 
 #include "gram.cuh"
 #include "lakgb_runtime.cuh"
+#include "tc_counts.cuh"
 
 namespace lakgb {
 
@@ -169,66 +169,6 @@ gram_popc_kernel(GramParams p) {
   }
 }
 
-// Split over blocks, for launches with few output tiles (a few hundred rows
-// or fewer on a side), where one CTA per tile would walk all P blocks alone
-// while most SMs idle.  Every (tile, block) pair is its own CTA and writes
-// the tile's integer counts of that block (<= 1920, uint16) to a scratch
-// array cnt[(b * nZ + k) * nA + i]; the fold kernel then adds each element's
-// weighted counts over the blocks in ascending order, with the same multiply
-// and add as above, so the outputs are the same bit for bit.
-template <int BM, int BN, int TM, int TN, int TYPE>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
-gram_split_counts_kernel(GramParams p, uint16_t *__restrict__ cnt_out) {
-  constexpr int TX = BN / TN;
-  constexpr int TY = BM / TM;
-  constexpr int NT = TX * TY;
-  extern __shared__ uint32_t smem[];
-  uint32_t *As = smem;
-  uint32_t *Zs = smem + BM * kLd;
-  __shared__ long long a_off[BM];
-  __shared__ long long z_off[BN];
-
-  const int tile_n = blockIdx.x * BN;
-  const int tile_m = blockIdx.y * BM;
-  const int blk = blockIdx.z;
-  if (p.symmetric && tile_m > tile_n + BN - 1) return;
-  const int tid = threadIdx.x;
-  const int tx = tid % TX;
-  const int ty = tid / TX;
-  row_offsets<BM, BN>(p, tile_m, tile_n, a_off, z_off, tid, NT);
-  __syncthreads();
-  stage_block<BM, BN, NT>(p, blk, As, Zs, a_off, z_off, tid);
-  __syncthreads();
-  int cnt[TM][TN];
-  count_block<TM, TN, TX, TY, TYPE>(As, Zs, tx, ty, cnt);
-  uint16_t *o = cnt_out + (size_t)blk * p.nZ * p.nA;
-#pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int ga = tile_m + ty + i * TY;
-    if (ga >= p.nA) continue;
-#pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int gz = tile_n + tx + j * TX;
-      if (gz < p.nZ) o[(size_t)gz * p.nA + ga] = (uint16_t)cnt[i][j];
-    }
-  }
-}
-
-template <int TYPE>
-__global__ void __launch_bounds__(256) gram_split_fold_kernel(GramParams p, const uint16_t *__restrict__ cnt) {
-  const long long n = (long long)p.nA * p.nZ, plane = n;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int gz = (int)(e / p.nA), ga = (int)(e - (long long)gz * p.nA);
-    if (p.symmetric && ga > gz) continue;
-    double acc = 0.0;
-    for (int b = 0; b < p.P; ++b) {
-      const double d = p.D ? p.D[b] : 1.0;
-      acc = __dadd_rn(acc, __dmul_rn(d, (double)cnt[(size_t)b * plane + e]));
-    }
-    store_element<TYPE>(p, ga, gz, acc);
-  }
-}
-
 template <int BM, int BN, int TM, int TN, int TYPE>
 void launch_tile(const GramParams &p) {
   constexpr int NT = (BM / TM) * (BN / TN);
@@ -249,26 +189,10 @@ void launch_tile(const GramParams &p) {
 constexpr size_t kSplitMaxBytes = size_t(256) << 20;
 size_t split_bytes(const GramParams &p) { return (size_t)p.P * (size_t)p.nA * (size_t)p.nZ * sizeof(uint16_t); }
 
-template <int TYPE>
 void launch_split(const GramParams &p, cudaStream_t s) {
-  constexpr int BM = 64, BN = 64, TM = 4, TN = 4, NT = (BM / TM) * (BN / TN);
-  const size_t smem = (size_t)(BM + BN) * kLd * sizeof(uint32_t);
-  static bool configured = false;
-  if (!configured) {
-    LAKGB_CUDA(cudaFuncSetAttribute(gram_split_counts_kernel<BM, BN, TM, TN, TYPE>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
-  }
   uint16_t *cnt = nullptr;
   LAKGB_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&cnt), split_bytes(p), s));
-  dim3 grid((p.nZ + BN - 1) / BN, (p.nA + BM - 1) / BM, p.P);
-  gram_split_counts_kernel<BM, BN, TM, TN, TYPE><<<grid, NT, smem, s>>>(p, cnt);
-  LAKGB_CUDA(cudaGetLastError());
-  const long long n = (long long)p.nA * p.nZ;
-  const int blocks = (int)std::min<long long>((n + 255) / 256, 152ll * 8);
-  gram_split_fold_kernel<TYPE><<<blocks, 256, 0, s>>>(p, cnt);
-  LAKGB_CUDA(cudaGetLastError());
-  count_launch(2);
+  launch_gram_tc_split(p, cnt, s);
   LAKGB_CUDA(cudaFreeAsync(cnt, s));
 }
 
@@ -277,31 +201,31 @@ void launch_split(const GramParams &p, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 // Kernel choice.  Every candidate computes the same outputs bit for bit, so
 // the choice is a matter of speed only.  With LAKGB_IMPL_AUTO (the default)
-// a launch with at least kTensorRows rows on both sides takes the tensor-core
-// kernel (it wins there by 3x or more); for smaller launches the first one of
-// each shape class -- (type, symmetric, log2 of the A rows, of the Z rows and
-// of the blocks) -- runs the candidates (tensor kernel, popcount kernel with
-// two tile shapes, popcount kernel split over blocks) on its real arguments,
-// timed with CUDA events on the launching stream, and the fastest serves that
-// class from then on.
+// a launch with at least kTensorRows rows on both sides takes the persistent
+// tensor-core kernel; for smaller launches the first one of each shape class
+// -- (type, symmetric, log2 of the A rows, of the Z rows and of the blocks) --
+// runs that kernel and the tensor-core counts split over blocks (tc_counts.cu)
+// on its real arguments, timed with CUDA events on the launching stream, and
+// the faster serves that class from then on.  (Measured on the 120 classes of
+// a case/control solve, 9 blocks: split 17 to 34 us, persistent 60 to 81 us up
+// to 512 x 512 rows, 99 and 81 us at 512 x 4096; the popcount kernels, 113 to
+// 256 us, are the fastest in no class and are not timed.)
 
-enum GramVariant { kTensor = 0, kPopc128x64, kPopc64x64, kSplit64x64, kPopc64x128, kNumVariants };
-constexpr int kTunedVariants = 4;   // tensor, popcount 128x64, popcount 64x64, split over blocks
-constexpr int kTensorRows = 512;
-const char *const kVariantName[kNumVariants] = {"tensor_128x128", "popcount_128x64", "popcount_64x64",
-                                                "split_64x64", "popcount_64x128"};
+enum GramVariant { kTensor = 0, kPopc128x64, kPopc64x64, kSplit, kPopc64x128, kNumVariants };
+constexpr int kTuned[] = {kTensor, kSplit};
+constexpr int kTunedVariants = 2;
+constexpr int kTensorRows = 1024;
+const char *const kVariantName[kNumVariants] = {"tensor_128x112", "popcount_128x64", "popcount_64x64",
+                                                "split_128x64", "popcount_64x128"};
 
 void launch_variant(int v, const GramParams &p, cudaStream_t s) {
   GramParams q = p;
   q.stream = s;
-  if (v == kSplit64x64 && (split_bytes(q) > kSplitMaxBytes || q.P > 65535)) v = kPopc64x64;
+  if (v == kSplit && (split_bytes(q) > kSplitMaxBytes || q.P > 65535 || q.nA > 65535 * kCountsM)) v = kPopc64x64;
   if (v == kTensor) {
     launch_gram_tc(q, s);
-  } else if (v == kSplit64x64) {
-    if (q.type == 1)
-      launch_split<1>(q, s);
-    else
-      launch_split<2>(q, s);
+  } else if (v == kSplit) {
+    launch_split(q, s);
   } else if (q.type == 1) {
     if (v == kPopc128x64) launch_tile<128, 64, 8, 4, 1>(q);
     else if (v == kPopc64x64) launch_tile<64, 64, 4, 4, 1>(q);
@@ -348,31 +272,32 @@ int tuned_variant(const GramParams &p, cudaStream_t s, bool *ran) {
   // Measure the candidates on this launch; each overwrites the same output
   // elements with the same values, so the call's result is unaffected.  One
   // untimed round first (first launches can carry one-time costs such as
-  // module loading), then one timed round.
+  // module loading), then two timed ones, the shorter counting.
   TuneEntry e{};
   for (int v = 0; v < kNumVariants; ++v) e.ms[v] = -1.f;  // not measured
-  for (int v = 0; v < kTunedVariants; ++v) launch_variant(v, p, s);
-  constexpr int kRounds = 1;
+  for (int v : kTuned) launch_variant(v, p, s);
+  constexpr int kRounds = 2;
   cudaEvent_t ev[kRounds][kTunedVariants + 1];
   for (auto &r : ev)
     for (auto &x : r) LAKGB_CUDA(cudaEventCreate(&x));
   for (int r = 0; r < kRounds; ++r) {
     LAKGB_CUDA(cudaEventRecord(ev[r][0], s));
     for (int v = 0; v < kTunedVariants; ++v) {
-      launch_variant(v, p, s);
+      launch_variant(kTuned[v], p, s);
       LAKGB_CUDA(cudaEventRecord(ev[r][v + 1], s));
     }
   }
   LAKGB_CUDA(cudaEventSynchronize(ev[kRounds - 1][kTunedVariants]));
-  int best = 0;
+  int best = kTuned[0];
   for (int v = 0; v < kTunedVariants; ++v) {
-    e.ms[v] = 1e30f;
+    float &t = e.ms[kTuned[v]];
+    t = 1e30f;
     for (int r = 0; r < kRounds; ++r) {
       float ms = 0.f;
       LAKGB_CUDA(cudaEventElapsedTime(&ms, ev[r][v], ev[r][v + 1]));
-      e.ms[v] = std::min(e.ms[v], ms);
+      t = std::min(t, ms);
     }
-    if (e.ms[v] < e.ms[best]) best = v;
+    if (t < e.ms[best]) best = kTuned[v];
   }
   for (auto &r : ev)
     for (auto &x : r) LAKGB_CUDA(cudaEventDestroy(x));
@@ -395,7 +320,7 @@ void launch_gram(const GramParams &p) {
   if (impl == LAKGB_IMPL_TENSOR) {
     launch_variant(kTensor, p, s);
   } else if (impl == LAKGB_IMPL_SPLIT) {
-    launch_variant(kSplit64x64, p, s);
+    launch_variant(kSplit, p, s);
   } else if (impl == LAKGB_IMPL_POPCOUNT) {
     launch_variant(kPopc128x64, p, s);
   } else {

@@ -78,6 +78,10 @@ cudaStream_t copy_stream() {
 // --- per-thread staging arena -----------------------------------------------
 
 namespace {
+// One call's arena; a thread takes its kArenas arenas in turn, so that a call
+// can be prepared while the GPU still works on the calls before it.  (With one
+// arena every call waited for the previous call's copy, which the stream runs
+// only after that call's predecessor: host and GPU took turns.)
 struct Arena {
   unsigned char *host = nullptr;   // pinned
   unsigned char *dev = nullptr;
@@ -85,10 +89,10 @@ struct Arena {
   cudaEvent_t done = nullptr;      // the last flush's copy has completed
   bool pending = false;
 };
-Arena &arena() {
-  thread_local Arena a;
-  return a;
-}
+constexpr int kArenas = 8;
+thread_local Arena t_arenas[kArenas];
+thread_local int t_arena = 0;
+Arena &arena() { return t_arenas[t_arena]; }
 }  // namespace
 
 namespace {
@@ -113,6 +117,7 @@ DBuf upload_bytes(const void *h, size_t n) {
 
 void Stager::begin() {
   t_active = this;
+  t_arena = (t_arena + 1) % kArenas;
   Arena &a = arena();
   if (!a.host) {
     a.cap = kStageBytes;

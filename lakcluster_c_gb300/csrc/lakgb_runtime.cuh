@@ -90,9 +90,9 @@ struct DBuf {
 // each array (host bytes are copied into a pinned arena, the returned device
 // pointer is valid for kernels enqueued after flush()), flush() issues one
 // copy for all of them.  Arrays that do not fit the arena are uploaded on
-// their own.  One Stager per call; the arena is reused by the next call once
-// its copy has completed.
-constexpr size_t kStageBytes = 32u << 20;
+// their own.  One Stager per call; a thread's arenas are used in turn, each
+// again once its copy has completed.
+constexpr size_t kStageBytes = 4u << 20;
 // Arrays of at least this many bytes skip the arena (one direct copy each).
 constexpr size_t kDirectUploadBytes = 1u << 20;
 class Stager {

@@ -16,14 +16,13 @@
 //   hhAy = AtTn[na,t], hhaY = YtTn[ny,t] (integers read from FP64),
 //   hhay = -cpop_j(Tt) + 2*popcount(Tt_t & mc_j(Tt)), aA / aY the column
 //   means of the At / Yt rows' 1920-bit blocks.
-// The popcount is a tiled XOR Gram: per 1920-bit block the CTA stages
-// (At ^ Tt) & mask for 64 At rows and Yt & mask for 64 Yt rows, and each
-// thread accumulates a 4 x 4 tile of integer counts over all blocks.
+// The counts run on the tensor cores (tc_counts.cu).
 #include <optional>
 
 #include "abi_common.cuh"
 #include "lmirror.cuh"
 #include "bcc_model.h"
+#include "tc_counts.cuh"
 
 namespace lakgb {
 
@@ -181,105 +180,30 @@ thread_local std::vector<DeferCopy> t_copies;  // other calls' outputs
 // freed) when the outermost scope ends.
 struct UpChunk { uint8_t *h = nullptr; uint8_t *d = nullptr; size_t cap = 0, used = 0, sent = 0; };
 constexpr size_t kUpChunk = 4u << 20;
+
+// Page-locked buffer for a scope's small outputs: a copy into pageable memory
+// holds the host for about 8 us (and until the kernels before it are done), one
+// into page-locked memory under 1 us, so outputs of up to kDownEach bytes come
+// back there, as far as they fit, and are copied on after the scope's one wait.
+constexpr size_t kDownBytes = 8u << 20, kDownEach = 64u << 10;
+thread_local uint8_t *t_down = nullptr;
+struct DownCopy { double *host; size_t off, bytes; };
+
+// Enqueue the copy of `length` doubles of `dev` to `host`.
+void copy_down(double *host, const double *dev, unsigned long long length, size_t &used, std::vector<DownCopy> &later) {
+  const size_t bytes = length * sizeof(double);
+  if (!bytes) return;
+  if (bytes > kDownEach || used + bytes > kDownBytes) {
+    LAKGB_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, stream()));
+    return;
+  }
+  if (!t_down) LAKGB_CUDA(cudaHostAlloc((void **)&t_down, kDownBytes, cudaHostAllocDefault));
+  LAKGB_CUDA(cudaMemcpyAsync(t_down + used, dev, bytes, cudaMemcpyDeviceToHost, stream()));
+  later.push_back(DownCopy{host, used, bytes});
+  used += (bytes + 15) & ~(size_t)15;
+}
 thread_local std::vector<UpChunk> t_up;
 thread_local size_t t_up_cur = 0;
-
-constexpr int kLd = kBlockWords + 1;
-constexpr int kTY_M = 64, kTY_N = 64, kTY_TM = 4, kTY_TN = 4, kTY_T = 256;
-
-struct AtTYnParams {
-  const uint8_t *At; const uint32_t *a_rowb; int nA; long long a_row_bytes;
-  const uint8_t *Yt; const uint32_t *y_rowb; int nY; long long y_row_bytes;
-  const uint8_t *Tt; const uint32_t *t_rowb; long long t_row_bytes;
-  const uint8_t *mask; int P; long long cpop;
-  const double *hhAy;   // [t][na]
-  const double *hhaY;   // [t][ny]
-  const double *hhay;   // [t]
-  const double *aA; const double *aY;
-  const unsigned long long *out_a; const unsigned long long *out_y; const unsigned long long *out_t;
-  double *out;
-  // AtTAn (Yt = At): pairs na <= ny only, each also stored at
-  // out_a2[ny] + out_y2[na] (the transposed position).
-  int symmetric;
-  const unsigned long long *out_a2; const unsigned long long *out_y2;
-};
-
-__global__ void __launch_bounds__(kTY_T, 2) attyn_kernel(AtTYnParams p) {
-  extern __shared__ __align__(16) uint32_t smem[];
-  uint32_t *As = smem, *Ys = smem + kTY_M * kLd;
-  __shared__ long long a_off[kTY_M], y_off[kTY_N];
-  const int t = blockIdx.z;
-  const int n0 = blockIdx.x * kTY_N, m0 = blockIdx.y * kTY_M;
-  if (p.symmetric && m0 > n0 + kTY_N - 1) return;  // wholly below the diagonal
-  const int tid = threadIdx.x, tx = tid % (kTY_N / kTY_TN), ty = tid / (kTY_N / kTY_TN);
-  for (int i = tid; i < kTY_M; i += kTY_T) a_off[i] = m0 + i < p.nA ? (long long)p.a_rowb[m0 + i] * p.a_row_bytes : -1;
-  for (int i = tid; i < kTY_N; i += kTY_T) y_off[i] = n0 + i < p.nY ? (long long)p.y_rowb[n0 + i] * p.y_row_bytes : -1;
-  const uint8_t *trow = p.Tt + (long long)p.t_rowb[t] * p.t_row_bytes;
-  int c[kTY_TM][kTY_TN];
-#pragma unroll
-  for (int i = 0; i < kTY_TM; ++i)
-#pragma unroll
-    for (int j = 0; j < kTY_TN; ++j) c[i][j] = 0;
-  for (int blk = 0; blk < p.P; ++blk) {
-    __syncthreads();
-    const long long boff = (long long)blk * kBlockBytes;
-    const uint4 *mk = reinterpret_cast<const uint4 *>(p.mask + boff);
-    const uint4 *tk = reinterpret_cast<const uint4 *>(trow + boff);
-    for (int idx = tid; idx < kTY_M * 15; idx += kTY_T) {
-      const int r = idx / 15, v = idx - r * 15;
-      uint4 x = make_uint4(0u, 0u, 0u, 0u);
-      if (a_off[r] >= 0) {
-        const uint4 a = __ldg(reinterpret_cast<const uint4 *>(p.At + a_off[r] + boff) + v);
-        const uint4 tt = __ldg(tk + v), m = __ldg(mk + v);
-        x.x = (a.x ^ tt.x) & m.x; x.y = (a.y ^ tt.y) & m.y; x.z = (a.z ^ tt.z) & m.z; x.w = (a.w ^ tt.w) & m.w;
-      }
-      uint32_t *d = As + r * kLd + 4 * v;
-      d[0] = x.x; d[1] = x.y; d[2] = x.z; d[3] = x.w;
-    }
-    for (int idx = tid; idx < kTY_N * 15; idx += kTY_T) {
-      const int r = idx / 15, v = idx - r * 15;
-      uint4 x = make_uint4(0u, 0u, 0u, 0u);
-      if (y_off[r] >= 0) {
-        const uint4 y = __ldg(reinterpret_cast<const uint4 *>(p.Yt + y_off[r] + boff) + v);
-        const uint4 m = __ldg(mk + v);
-        x.x = y.x & m.x; x.y = y.y & m.y; x.z = y.z & m.z; x.w = y.w & m.w;
-      }
-      uint32_t *d = Ys + r * kLd + 4 * v;
-      d[0] = x.x; d[1] = x.y; d[2] = x.z; d[3] = x.w;
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int w = 0; w < kBlockWords; ++w) {
-      uint32_t a[kTY_TM], y[kTY_TN];
-#pragma unroll
-      for (int i = 0; i < kTY_TM; ++i) a[i] = As[(ty + 16 * i) * kLd + w];
-#pragma unroll
-      for (int j = 0; j < kTY_TN; ++j) y[j] = Ys[(tx + 16 * j) * kLd + w];
-#pragma unroll
-      for (int i = 0; i < kTY_TM; ++i)
-#pragma unroll
-        for (int j = 0; j < kTY_TN; ++j) c[i][j] += __popc(a[i] ^ y[j]);
-    }
-  }
-  const double hhay = p.hhay[t];
-#pragma unroll
-  for (int i = 0; i < kTY_TM; ++i) {
-    const int na = m0 + ty + 16 * i;
-    if (na >= p.nA) continue;
-    const double hhAy = p.hhAy[(long long)t * p.nA + na], aA = p.aA[na];
-#pragma unroll
-    for (int j = 0; j < kTY_TN; ++j) {
-      const int ny = n0 + tx + 16 * j;
-      if (ny >= p.nY || (p.symmetric && na > ny)) continue;
-      const double hhaY = p.hhaY[(long long)t * p.nY + ny], aY = p.aY[ny];
-      const double hhAY = (double)(2ll * c[i][j] - p.cpop);
-      const double v = __dadd_rn(__dsub_rn(__dsub_rn(hhAY, __dmul_rn(hhAy, aY)), __dmul_rn(aA, hhaY)),
-                                 __dmul_rn(__dmul_rn(aA, hhay), aY));
-      p.out[p.out_a[na] + p.out_y[ny] + p.out_t[t]] = v;
-      if (p.symmetric) p.out[p.out_a2[ny] + p.out_y2[na] + p.out_t[t]] = v;
-    }
-  }
-}
 
 }  // namespace
 
@@ -333,7 +257,8 @@ extern "C" int wrap_AnZt_S_WnYt_vv__run(int *tidx, void **vpra, pthread_t *threa
   const unsigned long long length_a = spacing_length(output_spacing_a, M_An);
   const unsigned long long length_s = spacing_length(output_spacing_s, M_St);
   const unsigned long long length = length_a * length_s;
-  L_handle *out = ensure_output(output_p, length, "wrap_AnZt_S_WnYt_vv__run");
+  L_handle *out = ensure_output(output_p, length, "wrap_AnZt_S_WnYt_vv__run", false);
+  HostOutputFill fill{out, length};
   if (!out) return (int)length;
   out->spacing_row = output_spacing_a; out->row_stride = length_a;
   out->spacing_col = output_spacing_s; out->col_stride = length_s;
@@ -388,6 +313,7 @@ extern "C" int wrap_AnZt_S_WnYt_vv__run(int *tidx, void **vpra, pthread_t *threa
     d.c = c;
     d.host_out = out->lf;
     d.length = length;
+    fill.copied = true;
     for (DBuf *b : {&dA, &dY, &d_ar, &d_yr, &d_ac, &d_yc, &d_vS, &d_or, &d_so, &d_out}) d.keep.push_back(std::move(*b));
     t_swnyt.push_back(std::move(d));
     return (int)length;
@@ -396,7 +322,7 @@ extern "C" int wrap_AnZt_S_WnYt_vv__run(int *tidx, void **vpra, pthread_t *threa
   anzt_s_wnyt_kernel<<<dim3((nA + kSW_R - 1) / kSW_R, nS), kSW_T, 0, stream()>>>(c);
   LAKGB_CUDA(cudaGetLastError());
   count_launch();
-  copy_back(out->lf, d_out, length);
+  copy_back(out->lf, d_out, length, &fill);
   return (int)length;
 }
 
@@ -446,16 +372,13 @@ extern "C" void lakgb_defer_end(void) {
       LAKGB_CUDA(cudaStreamSynchronize(stream()));
     }
     LAKGB_PROFILE_CALL("(copy back + sync)");
-    for (auto &d : t_swnyt)
-      if (d.length)
-        LAKGB_CUDA(cudaMemcpyAsync(d.host_out, d.c.out, d.length * sizeof(double), cudaMemcpyDeviceToHost, stream()));
-    for (auto &d : t_wtsz)
-      if (d.length)
-        LAKGB_CUDA(cudaMemcpyAsync(d.host_out, d.c.out, d.length * sizeof(double), cudaMemcpyDeviceToHost, stream()));
-    for (auto &c : t_copies)
-      if (c.length)
-        LAKGB_CUDA(cudaMemcpyAsync(c.host, c.dev.p, c.length * sizeof(double), cudaMemcpyDeviceToHost, stream()));
+    std::vector<DownCopy> later;
+    size_t used = 0;
+    for (auto &d : t_swnyt) copy_down(d.host_out, d.c.out, d.length, used, later);
+    for (auto &d : t_wtsz) copy_down(d.host_out, d.c.out, d.length, used, later);
+    for (auto &c : t_copies) copy_down(c.host, c.dev.as<double>(), c.length, used, later);
     LAKGB_CUDA(cudaStreamSynchronize(stream()));
+    for (const DownCopy &c : later) memcpy(c.host, t_down + c.off, c.bytes);
   }
   t_copies.clear();
   for (UpChunk &c : t_up) c.used = c.sent = 0;  // the stream has drained: reuse the chunks
@@ -475,7 +398,8 @@ extern "C" int wrap_AtTYn____WtSZn_vv__run(int *tidx, void **vpra, pthread_t *th
   const unsigned long long length_a = spacing_length(output_spacing_a, M_At);
   const unsigned long long length_s = spacing_length(output_spacing_s, M_St);
   const unsigned long long length = length_a * length_s;
-  L_handle *out = ensure_output(output_p, length, "wrap_AtTYn____WtSZn_vv__run");
+  L_handle *out = ensure_output(output_p, length, "wrap_AtTYn____WtSZn_vv__run", false);
+  HostOutputFill fill{out, length};
   if (!out) return (int)length;
   out->spacing_row = output_spacing_a; out->row_stride = length_a;
   out->spacing_col = output_spacing_s; out->col_stride = length_s;
@@ -535,6 +459,7 @@ extern "C" int wrap_AtTYn____WtSZn_vv__run(int *tidx, void **vpra, pthread_t *th
     d.c = c;
     d.host_out = out->lf;
     d.length = length;
+    fill.copied = true;
     for (DBuf *b : {&dA, &dZ, &d_aa, &d_ay, &d_as, &d_zz, &d_zw, &d_zs, &d_D, &d_or, &d_so, &d_out})
       d.keep.push_back(std::move(*b));
     t_wtsz.push_back(std::move(d));
@@ -544,7 +469,7 @@ extern "C" int wrap_AtTYn____WtSZn_vv__run(int *tidx, void **vpra, pthread_t *th
   attyn_wtszn_kernel<<<dim3((npairs + kWZ_T - 1) / kWZ_T, nS), kWZ_T, 0, stream()>>>(c);
   LAKGB_CUDA(cudaGetLastError());
   count_launch();
-  copy_back(out->lf, d_out, length);
+  copy_back(out->lf, d_out, length, &fill);
   return (int)length;
 }
 
@@ -642,12 +567,8 @@ int attyn_entry(bool symmetric, const char *who, int output_spacing_a, int outpu
     d_out.zero();
     p.out = d_out.as<double>();
   }
-  const size_t smem = (size_t)(kTY_M + kTY_N) * kLd * sizeof(uint32_t);
-  dim3 grid((nY + kTY_N - 1) / kTY_N, (nA + kTY_M - 1) / kTY_M, nT);
   st.flush();
-  attyn_kernel<<<grid, kTY_T, smem, stream()>>>(p);
-  LAKGB_CUDA(cudaGetLastError());
-  count_launch();
+  launch_attyn_tc(p, nT, stream());
   if (mo) return (int)length;
   copy_back(out->lf, d_out, length, &fill);
   return (int)length;
