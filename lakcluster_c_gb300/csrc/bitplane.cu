@@ -36,6 +36,7 @@
 #include "bcc_model.h"
 #include "bitplane.cuh"
 #include "gram.cuh"
+#include "tc_counts.cuh"
 
 namespace lakgb {
 
@@ -50,35 +51,58 @@ __device__ __forceinline__ int plane_row(int mw, int k, int ncols_per) {
   return mw * ncols_per + ncols_per - 1 - k;
 }
 
-// pmpm0 pieces for plane 0 / value planes against plane 0 combined with Tt:
-// warp per plane row.  pm[t][q] = 2*popcount(~(p0 ^ t) & y & m) - popcount(y & m)
-// for q = 0 (plane 0 itself) and q = 1 + mw*B + k (value plane of bit k).
-__global__ void bitplane_prep_kernel(BitplaneParams p, int nT, int *pm, int *ycnt) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// The counts that do not depend on (pair, plane): a warp per plane row and t,
+//   pm[t][q] = 2*popcount(~(p0 ^ t) & y & m) - popcount(y & m)
+// for q = 0 (plane 0 itself) and q = 1 + mw*B + k (value plane of bit k), and
+// ycnt[q] = popcount(y & m); then, for the tensor-core form (At_base not null),
+// a warp per pair: At_base = pmpm0(At, Tt, plane 0) * min * mlt for every t, and
+// the two values of vZ - aZ.
+__global__ void bitplane_prep_kernel(BitplaneParams p, int nT, int *pm, int *ycnt, double *At_base, double2 *zz) {
+  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int nq = 1 + p.nW * p.B;
-  if (warp >= nq * nT) return;
-  const int q = warp % nq, t = warp / nq;
-  const int prow = q == 0 ? 0 : plane_row((q - 1) / p.B, (q - 1) % p.B, p.ncols_per);
-  const uint32_t *y = reinterpret_cast<const uint32_t *>(p.planes + (long long)prow * p.plane_bytes);
+  const long long plane_warps = (long long)nq * nT;
   const uint32_t *p0 = reinterpret_cast<const uint32_t *>(p.planes);
-  const uint32_t *tt = reinterpret_cast<const uint32_t *>(p.Tt + (long long)p.tt_rowb[t] * p.tt_row_bytes);
   const uint32_t *m = reinterpret_cast<const uint32_t *>(p.mask);
   const int nw = p.P * kBlockWords;
-  int c = 0, yc = 0;
-  for (int i = lane; i < nw; i += 32) {
-    const uint32_t ym = __ldg(y + i) & __ldg(m + i);
-    yc += __popc(ym);
-    c += __popc(~(__ldg(p0 + i) ^ __ldg(tt + i)) & ym);
+  if (warp < plane_warps) {
+    const int q = (int)(warp % nq), t = (int)(warp / nq);
+    const int prow = q == 0 ? 0 : plane_row((q - 1) / p.B, (q - 1) % p.B, p.ncols_per);
+    const uint32_t *y = reinterpret_cast<const uint32_t *>(p.planes + (long long)prow * p.plane_bytes);
+    const uint32_t *tt = reinterpret_cast<const uint32_t *>(p.Tt + (long long)p.tt_rowb[t] * p.tt_row_bytes);
+    int c = 0, yc = 0;
+    for (int i = lane; i < nw; i += 32) {
+      const uint32_t ym = __ldg(y + i) & __ldg(m + i);
+      yc += __popc(ym);
+      c += __popc(~(__ldg(p0 + i) ^ __ldg(tt + i)) & ym);
+    }
+    c = __reduce_add_sync(0xffffffffu, c);
+    yc = __reduce_add_sync(0xffffffffu, yc);
+    if (lane == 0) {
+      pm[(long long)t * nq + q] = 2 * c - yc;
+      if (t == 0) ycnt[q] = yc;
+    }
+    return;
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    c += __shfl_xor_sync(0xffffffffu, c, o);
-    yc += __shfl_xor_sync(0xffffffffu, yc, o);
+  const long long pr = warp - plane_warps;
+  if (!At_base || pr >= p.npairs) return;
+  const uint32_t *aw = reinterpret_cast<const uint32_t *>(p.At + (long long)p.at_rowb[pr] * p.at_row_bytes);
+  for (int t = 0; t < nT; ++t) {
+    const uint32_t *tw = reinterpret_cast<const uint32_t *>(p.Tt + (long long)p.tt_rowb[t] * p.tt_row_bytes);
+    int c = 0, yc = 0;
+    for (int i = lane; i < nw; i += 32) {
+      const uint32_t ym = __ldg(m + i) & __ldg(p0 + i);
+      yc += __popc(ym);
+      c += __popc(~(__ldg(aw + i) ^ __ldg(tw + i)) & ym);
+    }
+    c = __reduce_add_sync(0xffffffffu, c);
+    yc = __reduce_add_sync(0xffffffffu, yc);
+    if (lane == 0)
+      At_base[(long long)t * p.npairs + pr] = __dmul_rn(__dmul_rn((double)(2ll * c - yc), p.min_d), p.mlt_d);
   }
   if (lane == 0) {
-    pm[(long long)t * nq + q] = 2 * c - yc;
-    if (t == 0) ycnt[q] = yc;
+    const double a = p.aZ[pr];
+    zz[pr] = make_double2(__dsub_rn(1.0, a), __dsub_rn(-1.0, a));
   }
 }
 
@@ -121,33 +145,6 @@ __global__ void bitplane_tsum_kernel(BitplaneParams p, const int *pm, double *T_
     const double a = p.aBlk[blk];
     q2[((long long)t * p.nblk + blk) * p.nW + mw] =
         __ddiv_rn(__dadd_rn(__dmul_rn(tb, a), __dmul_rn(s, a)), p.mlt_d);
-  }
-}
-
-// Per pair (a warp each): At_base = pmpm0(At, Tt, plane 0) * min * mlt for
-// every t, and the two values of vZ - aZ.
-__global__ void bitplane_pairs_kernel(BitplaneParams p, double *At_base, double2 *zz) {
-  const long long pr = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (pr >= p.npairs) return;
-  const uint32_t *aw = reinterpret_cast<const uint32_t *>(p.At + (long long)p.at_rowb[pr] * p.at_row_bytes);
-  const uint32_t *m = reinterpret_cast<const uint32_t *>(p.mask);
-  const uint32_t *p0 = reinterpret_cast<const uint32_t *>(p.planes);
-  const int nw = p.P * kBlockWords;
-  for (int t = 0; t < p.nT; ++t) {
-    const uint32_t *tw = reinterpret_cast<const uint32_t *>(p.Tt + (long long)p.tt_rowb[t] * p.tt_row_bytes);
-    int c = 0;
-    for (int i = lane; i < nw; i += 32) c += __popc(~(__ldg(aw + i) ^ __ldg(tw + i)) & __ldg(m + i) & __ldg(p0 + i));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if (lane == 0) {
-      const long long pm = 2ll * c - p.ycnt[0];
-      At_base[(long long)t * p.npairs + pr] = __dmul_rn(__dmul_rn((double)pm, p.min_d), p.mlt_d);
-    }
-  }
-  if (lane == 0) {
-    const double a = p.aZ[pr];
-    zz[pr] = make_double2(__dsub_rn(1.0, a), __dsub_rn(-1.0, a));
   }
 }
 
@@ -307,46 +304,53 @@ bitplane_main_kernel(BitplaneParams p) {
 // pos = popcount(a & y & mask) and all = popcount(y & mask) over the whole
 // row, each output is
 //   (pm0(a, plane 0) * min * mlt + sum_{mx = B..1} 2^(B-mx) pm0(a, plane(s, mx))) / mlt
-// in that order.  The pos counts of every (row, plane) pair are one
-// masked-AND Gram of the An rows against the plane rows (launch_gram with
-// unit block weights: its FP64 sums of integer block counts are exact), the
-// all counts one warp per plane, and the FP64 combination a thread per
-// (row, s).
+// in that order.  The pos counts of every (row, plane) pair and the all counts
+// come per 1920-column block from the tensor cores (tc_counts.cu); a thread per
+// (row, s) adds them and forms the output.
 struct AnZtSnFinish {
-  const double *pos;              // n x nplanes, pos[i + k*n]
-  const long long *all;           // per plane
-  int n, nS, ncols_per;
+  const uint16_t *cnt;            // [block][plane][row]
+  const uint16_t *zcnt;           // [block][plane]
+  int n, nplanes, P, nS, ncols_per;
+  int exact;                      // the FP64 sum over the planes is one of integers below 2^53
   double min_d, mlt_d;
   const unsigned long long *out_r; const unsigned long long *s_off;
   double *out;
 };
 
-__global__ void plane_counts_kernel(const uint8_t *planes, long long plane_bytes, const uint8_t *mask, int nwords,
-                                    int nplanes, long long *all) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= nplanes) return;
-  const uint32_t *y = reinterpret_cast<const uint32_t *>(planes + (long long)warp * plane_bytes);
-  const uint32_t *m = reinterpret_cast<const uint32_t *>(mask);
-  int c = 0;
-  for (int i = lane; i < nwords; i += 32) c += __popc(__ldg(y + i) & __ldg(m + i));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-  if (lane == 0) all[warp] = c;
-}
-
-__global__ void an_ztsn_finish_kernel(AnZtSnFinish p) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= (long long)p.n * p.nS) return;
-  const int i = (int)(t % p.n), s = (int)(t / p.n);
-  auto pm0 = [&](int k) { return 2ll * (long long)p.pos[i + (long long)k * p.n] - p.all[k]; };
+// The sum over the planes in FP64 would be a chain of 2 B operations of 80
+// cycles each (16.5 us a call at 2018 rows, 33 planes).
+__global__ void __launch_bounds__(128) an_ztsn_finish_kernel(AnZtSnFinish p) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, s = blockIdx.y;
+  if (i >= p.n) return;
+  auto pm0 = [&](int k) {
+    long long pos = 0, all = 0;
+    const uint16_t *c = p.cnt + (size_t)k * p.n + i, *z = p.zcnt + k;
+    for (int b = 0; b < p.P; ++b) {
+      pos += c[(size_t)b * p.nplanes * p.n];
+      all += z[(size_t)b * p.nplanes];
+    }
+    return 2ll * pos - all;
+  };
   const double base = __dmul_rn(__dmul_rn((double)pm0(0), p.min_d), p.mlt_d);
-  double tmp = 0.0, n2 = 1.0;
-  for (int mx = p.ncols_per - 1; mx > 0; --mx) {
-    tmp = __dadd_rn(tmp, __dmul_rn(n2, (double)pm0(p.ncols_per * s + mx)));
-    n2 *= 2.0;
+  double tmp = 0.0;
+  if (p.exact) {
+    long long t = 0;
+#pragma unroll 4
+    for (int k = 0; k < p.ncols_per - 1; ++k) t += pm0(p.ncols_per * s + p.ncols_per - 1 - k) << k;
+    tmp = (double)t;
+  } else {
+    double n2 = 1.0;
+    for (int mx = p.ncols_per - 1; mx > 0; --mx) {
+      tmp = __dadd_rn(tmp, __dmul_rn(n2, (double)pm0(p.ncols_per * s + mx)));
+      n2 *= 2.0;
+    }
   }
   p.out[p.out_r[i] + p.s_off[s]] = __ddiv_rn(__dadd_rn(base, tmp), p.mlt_d);
 }
+
+// Most bytes of per-block counts a call holds at a time; larger calls take
+// their rows in ranges.
+constexpr size_t kAnZtSnScratch = 256ull << 20;
 
 inline unsigned long long pick_u(int s, unsigned long long j, unsigned long long b, unsigned long long a) {
   return s == LAKGB_SPACING_j ? j : (s == LAKGB_SPACING_b ? b : a);
@@ -779,8 +783,9 @@ extern "C" int wrap_At_T_YnWt_S_Zn_ww__run(int *tidx, void **vpra, pthread_t *th
     run.emplace(std::vector<BitplaneParams>{p}, B, [](const auto &v) { return upload_vec(v); });
   if (st) st->flush();
   {
-    const long long warps = (long long)nq * nT;
-    bitplane_prep_kernel<<<(int)((warps * 32 + 255) / 256), 256, 0, stream()>>>(p, nT, d_pm.as<int>(), d_ycnt.as<int>());
+    const long long warps = (long long)nq * nT + (tensor ? npairs : 0);
+    bitplane_prep_kernel<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, stream()>>>(
+        p, nT, d_pm.as<int>(), d_ycnt.as<int>(), d_Ab.as<double>(), d_zz.as<double2>());
     LAKGB_CUDA(cudaGetLastError());
     const dim3 grid((nW + 127) / 128, tensor ? A_pcols : 1, nT);
     // every partial sum of T_tmp is an integer below patients * 2^B
@@ -793,11 +798,6 @@ extern "C" int wrap_At_T_YnWt_S_Zn_ww__run(int *tidx, void **vpra, pthread_t *th
                                                               d_ys.as<long long>(), d_q2.as<double>());
     LAKGB_CUDA(cudaGetLastError());
     count_launch(2);
-    if (tensor) {
-      bitplane_pairs_kernel<<<(npairs + 7) / 8, 256, 0, stream()>>>(p, d_Ab.as<double>(), d_zz.as<double2>());
-      LAKGB_CUDA(cudaGetLastError());
-      count_launch();
-    }
   }
   if (defer) {
     BitplaneDeferred d;
@@ -857,38 +857,35 @@ extern "C" int wrap_An_ZtSn_ww__run(int *tidx, void **vpra, pthread_t *thread_in
   Stager st;
   const uint8_t *An = (const uint8_t *)resident(M_An->wX, (size_t)M_An->rpop_b * M_An->mc_length);
   const uint8_t *planes = (const uint8_t *)resident(M_ZtSn->wX, (size_t)M_ZtSn->nrows * M_ZtSn->mc_length);
-  std::vector<uint32_t> zrow(nplanes), orow(n), ocol(nplanes);
-  for (int k = 0; k < nplanes; ++k) zrow[k] = ocol[k] = (uint32_t)k;
-  for (int i = 0; i < n; ++i) orow[i] = (uint32_t)i;
+  std::vector<uint32_t> zrow(nplanes);
+  for (int k = 0; k < nplanes; ++k) zrow[k] = (uint32_t)k;
   DBuf d_rowb = upload_vec(rowb), d_or = upload_vec(out_r), d_so = upload_vec(s_off);
-  DBuf d_zrow = upload_vec(zrow), d_orow = upload_vec(orow), d_ocol = upload_vec(ocol);
+  DBuf d_zrow = upload_vec(zrow);
   DBuf mask = upload_bytes(M_An->mc_j, M_An->mc_length);
-  DBuf d_pos((size_t)n * nplanes * sizeof(double)), d_all((size_t)nplanes * sizeof(long long));
+  const int P = (int)(M_An->mc_length / kBlockBytes), B = M_ZtSn->ncols_per_z - 1;
+  const size_t per_row = (size_t)nplanes * P * sizeof(uint16_t);
+  const int range = (int)std::min<long long>(n, std::max<long long>(128, (long long)(kAnZtSnScratch / std::max<size_t>(per_row, 1)) / 128 * 128));
+  DBuf d_cnt((size_t)range * per_row), d_zcnt(per_row);
   DBuf d_out(length * sizeof(double));
   d_out.zero();
   st.flush();
-  GramParams g{};
-  g.wA = An; g.a_rowb = d_rowb.as<uint32_t>(); g.nA = n; g.a_row_bytes = (long long)M_An->mc_length;
-  g.wZ = planes; g.z_rowb = d_zrow.as<uint32_t>(); g.nZ = nplanes; g.z_row_bytes = (long long)M_ZtSn->mc_length;
-  g.mask = mask.as<uint8_t>(); g.P = (int)(M_An->mc_length / kBlockBytes);
-  g.D = nullptr; g.type = 2;  // masked AND counts
-  g.out_r = d_orow.as<uint32_t>(); g.out_c = d_ocol.as<uint32_t>(); g.out_stride = n; g.out = d_pos.as<double>();
-  launch_gram(g);
-  const int nwords = (int)(M_An->mc_length / 4);
-  plane_counts_kernel<<<(nplanes * 32 + 255) / 256, 256, 0, stream()>>>(planes, (long long)M_ZtSn->mc_length,
-                                                                     mask.as<uint8_t>(), nwords, nplanes,
-                                                                     d_all.as<long long>());
-  LAKGB_CUDA(cudaGetLastError());
-  count_launch();
-  AnZtSnFinish p{};
-  p.pos = d_pos.as<double>(); p.all = d_all.as<long long>();
-  p.n = n; p.nS = nS; p.ncols_per = M_ZtSn->ncols_per_z;
-  p.min_d = M_ZtSn->min_d; p.mlt_d = M_ZtSn->mlt_d;
-  p.out_r = d_or.as<unsigned long long>(); p.s_off = d_so.as<unsigned long long>();
-  p.out = d_out.as<double>();
-  an_ztsn_finish_kernel<<<(unsigned)(((long long)n * nS + 255) / 256), 256, 0, stream()>>>(p);
-  LAKGB_CUDA(cudaGetLastError());
-  count_launch();
+  for (int r0 = 0; r0 < n; r0 += range) {
+    GramParams g{};
+    g.wA = An; g.a_rowb = d_rowb.as<uint32_t>() + r0; g.nA = std::min(range, n - r0); g.a_row_bytes = (long long)M_An->mc_length;
+    g.wZ = planes; g.z_rowb = d_zrow.as<uint32_t>(); g.nZ = nplanes; g.z_row_bytes = (long long)M_ZtSn->mc_length;
+    g.mask = mask.as<uint8_t>(); g.P = P; g.type = 2;
+    if (P > 0 && nplanes > 0) launch_and_counts_tc(g, d_cnt.as<uint16_t>(), d_zcnt.as<uint16_t>(), stream());
+    AnZtSnFinish p{};
+    p.cnt = d_cnt.as<uint16_t>(); p.zcnt = d_zcnt.as<uint16_t>();
+    p.n = g.nA; p.nplanes = nplanes; p.P = P; p.nS = nS; p.ncols_per = M_ZtSn->ncols_per_z;
+    p.exact = B < 40 && (double)P * kBlockBits * (double)(1ll << B) <= 9007199254740992.0;
+    p.min_d = M_ZtSn->min_d; p.mlt_d = M_ZtSn->mlt_d;
+    p.out_r = d_or.as<unsigned long long>() + r0; p.s_off = d_so.as<unsigned long long>();
+    p.out = d_out.as<double>();
+    an_ztsn_finish_kernel<<<dim3((g.nA + 127) / 128, nS), 128, 0, stream()>>>(p);
+    LAKGB_CUDA(cudaGetLastError());
+    count_launch();
+  }
   copy_back(out->lf, d_out, length, &fill);
   return (int)length;
 }

@@ -5,9 +5,7 @@
 // AtTYn____WtSZn_vv (dir_c/AtTYn____WtSZn_vv.c:5-115, wrapper :117-159): over
 // paired rows (na with nz) and paired inner rows (ny with nw), in order,
 //   out[na, s] = sum (AtTYn[na,ny,s] * D_Yn[ny]) * ZtSWn[nz,nw,s]
-// Both are sequential FP64 sums; one thread per output element runs the
-// reference's recurrence (left-to-right, no FMA), with adjacent threads on
-// adjacent rows so the column-major loads coalesce.
+// Both are sequential FP64 sums, added left to right by one lane per output.
 //
 // AtTYn_vv (dir_c/AtTYn_vv.c:5-202, wrapper :204-235):
 //   out[na, ny, t] = ((hhAY - hhAy*aY) - aA*hhaY) + (aA*hhay)*aY
@@ -52,12 +50,14 @@ DBuf upload_L(const L_handle *L, bool three_d) {
   return d;
 }
 
-// One CTA per 16 rows: all 256 threads compute the products of a 16 x 128
-// (row, mz) tile into shared memory -- reads of consecutive rows for one mz are
-// contiguous in the column-major matrix -- then 16 threads add their row's
-// products in mz order.  The additions stay sequential per row; the loads
-// and multiplies run 256 wide.
-constexpr int kSW_R = 16, kSW_Z = 128, kSW_T = 256;
+// Both sums: one CTA per 32 rows (or pairs) and covariate.  Warps 1-8 form the
+// terms of kTerms columns into one half of a shared buffer -- the lane's row,
+// so that reads of one column are contiguous in the column-major matrix --
+// while warp 0 adds the other half's in order, a lane per row.  The chain of
+// one FP64 add (80 cycles) per term bounds a row; a sum and its products in one
+// thread took three operations per term, and 16 rows per CTA with the two
+// phases one after the other twice the adding warps.
+constexpr int kSumRows = 32, kTerms = 64, kSumT = 32 + 256;
 struct SwnytCall {
   const double *A; const unsigned long long *a_r, *a_c;
   const double *Y; const unsigned long long *y_r, *y_c;
@@ -65,62 +65,6 @@ struct SwnytCall {
   const unsigned long long *out_r, *s_off;
   double *out;
   int tile0;  // grouped launch: first CTA of this call
-};
-
-// CTA (row tile rt, covariate s) of one call.
-__device__ __forceinline__ void anzt_s_wnyt_tile(const SwnytCall &c, int rt, int s) {
-  __shared__ double prod[kSW_Z][kSW_R + 1];
-  const int r0 = rt * kSW_R;
-  const int8_t *vs = c.vS + (long long)s * c.nZ;
-  const int lr = threadIdx.x % kSW_R, lz = threadIdx.x / kSW_R;   // 16 rows x 16 columns per pass
-  const int ma = r0 + lr;
-  const unsigned long long ar = ma < c.nA ? c.a_r[ma] : 0, yr = ma < c.nA ? c.y_r[ma] : 0;
-  double acc = 0.0;
-  for (int z0 = 0; z0 < c.nZ; z0 += kSW_Z) {
-    const int zn = min(kSW_Z, c.nZ - z0);
-    __syncthreads();
-    for (int z = lz; z < zn; z += kSW_T / kSW_R) {
-      double v = 0.0;
-      if (ma < c.nA) {
-        const int mz = z0 + z;
-        v = __dmul_rn(__dmul_rn(c.A[ar + c.a_c[mz]], (double)vs[mz]), c.Y[yr + c.y_c[mz]]);
-      }
-      prod[z][lr] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < kSW_R)
-      for (int z = 0; z < zn; ++z) acc = __dadd_rn(acc, prod[z][threadIdx.x]);
-  }
-  if (threadIdx.x < kSW_R && r0 + threadIdx.x < c.nA) c.out[c.out_r[r0 + threadIdx.x] + c.s_off[s]] = acc;
-}
-
-__global__ void __launch_bounds__(kSW_T) anzt_s_wnyt_kernel(SwnytCall c) {
-  anzt_s_wnyt_tile(c, blockIdx.x, blockIdx.y);
-}
-
-// Several calls in one launch (a deferred group, lakgb_defer_end): CTA k
-// belongs to the last call whose tile0 <= k; within it, row tile (k - tile0)
-// % row tiles, covariate (k - tile0) / row tiles.
-__global__ void __launch_bounds__(kSW_T) anzt_s_wnyt_group_kernel(const SwnytCall *calls, int n) {
-  const int k = blockIdx.x;
-  int lo = 0, hi = n - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (calls[mid].tile0 <= k) lo = mid; else hi = mid - 1;
-  }
-  const SwnytCall &c = calls[lo];
-  const int rtiles = (c.nA + kSW_R - 1) / kSW_R;
-  const int j = k - c.tile0;
-  anzt_s_wnyt_tile(c, j % rtiles, j / rtiles);
-}
-
-// The calls a deferral scope holds back (this host thread): their device
-// inputs and outputs, and where each output goes on the host.
-struct SwnytDeferred {
-  SwnytCall c{};
-  std::vector<DBuf> keep;   // uploads and the device output
-  double *host_out = nullptr;
-  unsigned long long length = 0;
 };
 
 struct WtszCall {
@@ -131,34 +75,104 @@ struct WtszCall {
   double *out;
   int tile0;  // grouped launch: first CTA of this call
 };
-constexpr int kWZ_T = 128;
 
-// Thread = (pair i, covariate s): the sum over the inner rows in order.
-__device__ __forceinline__ void attyn_wtszn_one(const WtszCall &c, int i, int s) {
-  if (i >= c.npairs || s >= c.nS) return;
-  const unsigned long long a0 = c.ay_a[i] + c.ay_s[s], z0 = c.zw_z[i] + c.zw_s[s];
+// The terms of row i and covariate s: reference order of the operations; the
+// product with vS = +1 / -1 is exact.
+struct SwnytTerm {
+  const double *A, *Y;
+  const unsigned long long *a_c, *y_c;
+  const int8_t *vs;
+  __device__ SwnytTerm(const SwnytCall &c, int i, int s)
+      : A(c.A + c.a_r[i]), Y(c.Y + c.y_r[i]), a_c(c.a_c), y_c(c.y_c), vs(c.vS + (long long)s * c.nZ) {}
+  __device__ __forceinline__ double operator()(int z) const {
+    const double a = A[a_c[z]];
+    return __dmul_rn(vs[z] < 0 ? -a : a, Y[y_c[z]]);
+  }
+};
+struct WtszTerm {
+  const double *AY, *ZW, *Dy;
+  const unsigned long long *ay_y, *zw_w;
+  __device__ WtszTerm(const WtszCall &c, int i, int s)
+      : AY(c.AY + c.ay_a[i] + c.ay_s[s]), ZW(c.ZW + c.zw_z[i] + c.zw_s[s]), Dy(c.Dy), ay_y(c.ay_y), zw_w(c.zw_w) {}
+  __device__ __forceinline__ double operator()(int k) const {
+    return __dmul_rn(__dmul_rn(AY[ay_y[k]], Dy[k]), ZW[zw_w[k]]);
+  }
+};
+__host__ __device__ inline int sum_rows(const SwnytCall &c) { return c.nA; }
+__host__ __device__ inline int sum_rows(const WtszCall &c) { return c.npairs; }
+__device__ inline int sum_terms(const SwnytCall &c) { return c.nZ; }
+__device__ inline int sum_terms(const WtszCall &c) { return c.ninner; }
+
+// CTA (row tile rt, covariate s) of one call.
+template <class Term, class Call>
+__device__ __forceinline__ void ordered_sum_tile(const Call &c, int rt, int s) {
+  __shared__ double term[2][kTerms][kSumRows];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rows = sum_rows(c), n = sum_terms(c), i = rt * kSumRows + lane;
+  const Term t(c, min(i, rows - 1), s);
+  const int tiles = (n + kTerms - 1) / kTerms;
   double acc = 0.0;
-  for (int k = 0; k < c.ninner; ++k)
-    acc = __dadd_rn(acc, __dmul_rn(__dmul_rn(c.AY[a0 + c.ay_y[k]], c.Dy[k]), c.ZW[z0 + c.zw_w[k]]));
-  c.out[c.out_r[i] + c.s_off[s]] = acc;
+  for (int j = 0; j <= tiles; ++j) {
+    if (warp > 0) {
+      if (j < tiles) {
+        double v[kTerms / 8];
+#pragma unroll
+        for (int u = 0; u < kTerms / 8; ++u) {
+          const int k = j * kTerms + (warp - 1) + 8 * u;
+          v[u] = k < n ? t(k) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < kTerms / 8; ++u) term[j & 1][(warp - 1) + 8 * u][lane] = v[u];
+      }
+    } else if (j > 0) {
+      const int m = min(kTerms, n - (j - 1) * kTerms);
+      const double(*q)[kSumRows] = term[(j - 1) & 1];
+#pragma unroll 8
+      for (int k = 0; k < m; ++k) acc = __dadd_rn(acc, q[k][lane]);
+    }
+    __syncthreads();
+  }
+  if (warp == 0 && i < rows) c.out[c.out_r[i] + c.s_off[s]] = acc;
 }
 
-__global__ void attyn_wtszn_kernel(WtszCall c) {
-  attyn_wtszn_one(c, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y);
+__global__ void __launch_bounds__(kSumT) anzt_s_wnyt_kernel(SwnytCall c) {
+  ordered_sum_tile<SwnytTerm>(c, blockIdx.x, blockIdx.y);
+}
+__global__ void __launch_bounds__(kSumT) attyn_wtszn_kernel(WtszCall c) {
+  ordered_sum_tile<WtszTerm>(c, blockIdx.x, blockIdx.y);
 }
 
-__global__ void attyn_wtszn_group_kernel(const WtszCall *calls, int n) {
+// Several calls in one launch (a deferred group, lakgb_defer_end): CTA k
+// belongs to the last call whose tile0 <= k; within it, row tile (k - tile0)
+// % row tiles, covariate (k - tile0) / row tiles.
+template <class Term, class Call>
+__device__ __forceinline__ void ordered_sum_group(const Call *calls, int n) {
   const int k = blockIdx.x;
   int lo = 0, hi = n - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (calls[mid].tile0 <= k) lo = mid; else hi = mid - 1;
   }
-  const WtszCall &c = calls[lo];
-  const int ptiles = (c.npairs + kWZ_T - 1) / kWZ_T;
+  const Call c = calls[lo];
+  const int rtiles = (sum_rows(c) + kSumRows - 1) / kSumRows;
   const int j = k - c.tile0;
-  attyn_wtszn_one(c, (j % ptiles) * kWZ_T + threadIdx.x, j / ptiles);
+  ordered_sum_tile<Term>(c, j % rtiles, j / rtiles);
 }
+__global__ void __launch_bounds__(kSumT) anzt_s_wnyt_group_kernel(const SwnytCall *calls, int n) {
+  ordered_sum_group<SwnytTerm>(calls, n);
+}
+__global__ void __launch_bounds__(kSumT) attyn_wtszn_group_kernel(const WtszCall *calls, int n) {
+  ordered_sum_group<WtszTerm>(calls, n);
+}
+
+// The calls a deferral scope holds back (this host thread): their device
+// inputs and outputs, and where each output goes on the host.
+struct SwnytDeferred {
+  SwnytCall c{};
+  std::vector<DBuf> keep;   // uploads and the device output
+  double *host_out = nullptr;
+  unsigned long long length = 0;
+};
 
 struct WtszDeferred {
   WtszCall c{};
@@ -319,7 +333,7 @@ extern "C" int wrap_AnZt_S_WnYt_vv__run(int *tidx, void **vpra, pthread_t *threa
     return (int)length;
   }
   st->flush();
-  anzt_s_wnyt_kernel<<<dim3((nA + kSW_R - 1) / kSW_R, nS), kSW_T, 0, stream()>>>(c);
+  anzt_s_wnyt_kernel<<<dim3((nA + kSumRows - 1) / kSumRows, nS), kSumT, 0, stream()>>>(c);
   LAKGB_CUDA(cudaGetLastError());
   count_launch();
   copy_back(out->lf, d_out, length, &fill);
@@ -342,12 +356,12 @@ extern "C" void lakgb_defer_end(void) {
   int tiles1 = 0, tiles2 = 0;
   for (auto &d : t_swnyt) {
     d.c.tile0 = tiles1;
-    tiles1 += ((d.c.nA + kSW_R - 1) / kSW_R) * d.c.nS;
+    tiles1 += ((d.c.nA + kSumRows - 1) / kSumRows) * d.c.nS;
     c1.push_back(d.c);
   }
   for (auto &d : t_wtsz) {
     d.c.tile0 = tiles2;
-    tiles2 += ((d.c.npairs + kWZ_T - 1) / kWZ_T) * d.c.nS;
+    tiles2 += ((d.c.npairs + kSumRows - 1) / kSumRows) * d.c.nS;
     c2.push_back(d.c);
   }
   {
@@ -355,14 +369,14 @@ extern "C" void lakgb_defer_end(void) {
     if (!c1.empty()) {
       d_c1 = defer_upload(c1);
       defer_flush();
-      anzt_s_wnyt_group_kernel<<<tiles1, kSW_T, 0, stream()>>>(d_c1.as<SwnytCall>(), (int)c1.size());
+      anzt_s_wnyt_group_kernel<<<tiles1, kSumT, 0, stream()>>>(d_c1.as<SwnytCall>(), (int)c1.size());
       LAKGB_CUDA(cudaGetLastError());
       count_launch();
     }
     if (!c2.empty()) {
       d_c2 = defer_upload(c2);
       defer_flush();
-      attyn_wtszn_group_kernel<<<tiles2, kWZ_T, 0, stream()>>>(d_c2.as<WtszCall>(), (int)c2.size());
+      attyn_wtszn_group_kernel<<<tiles2, kSumT, 0, stream()>>>(d_c2.as<WtszCall>(), (int)c2.size());
       LAKGB_CUDA(cudaGetLastError());
       count_launch();
     }
@@ -466,7 +480,7 @@ extern "C" int wrap_AtTYn____WtSZn_vv__run(int *tidx, void **vpra, pthread_t *th
     return (int)length;
   }
   st->flush();
-  attyn_wtszn_kernel<<<dim3((npairs + kWZ_T - 1) / kWZ_T, nS), kWZ_T, 0, stream()>>>(c);
+  attyn_wtszn_kernel<<<dim3((npairs + kSumRows - 1) / kSumRows, nS), kSumT, 0, stream()>>>(c);
   LAKGB_CUDA(cudaGetLastError());
   count_launch();
   copy_back(out->lf, d_out, length, &fill);

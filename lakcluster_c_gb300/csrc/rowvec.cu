@@ -8,18 +8,15 @@
 //          and one add per block and no FMA, as popcount_lf (popcount.c:252-308).
 //
 // An_v: one warp per row; lanes 0..29 read the 240-byte block as 8-byte
-// words and the warp reduces the block count with shuffles.  An_ajdk: the
-// same counts for two rows per warp, whose 2 x 15 FP64 accumulators sit on
-// lanes 0..14 and 16..30.
+// words and the warp reduces the block count with shuffles.  An_ajdk: two rows
+// per warp, one 16-byte piece of a row per lane.
 #include "lakgb_runtime.cuh"
 #include "rowvec.cuh"
+#include "weigh.cuh"
 
 namespace lakgb {
 
 namespace {
-
-// Rows from which An_ajdk runs two rows per warp.
-constexpr int kAjdkTwoRows = 16384;
 
 __device__ __forceinline__ int block_count(const uint8_t *row, const uint8_t *mask, int lane) {
   int c = 0;
@@ -47,32 +44,55 @@ __global__ void an_v_kernel(RowvecParams p) {
   }
 }
 
-// RPW rows per warp.  With two, lanes 0..14 carry the 15 accumulators of row
-// 2w and lanes 16..30 those of row 2w+1, so each FP64 multiply and add
-// instruction (which holds the sub-partition's FP64 unit whatever its active
-// lanes) serves both rows: 1.7x faster on 32768 rows; small launches keep one
-// row per warp, which gives them twice the warps.
-template <int RPW>
-__global__ void an_ajdk_kernel(RowvecParams p) {
+// Two rows per warp: lanes 0..14 read the pieces of row 2w's block, lanes
+// 15..29 those of row 2w + 1, kAhead blocks ahead; one warp reduction gives both
+// counts (16 bits each), and lanes 0..14 and 16..30 carry the two rows' 15 FP64
+// sums.  The products with the counts are formed in integers, so a block costs
+// one FP64 instruction (80 cycles of its sub-partition's FP64 pipe) per two
+// rows: the floor beside the memory's.  8192 rows x 65536 columns: 64 us with
+// two FP64 instructions per row and no loads ahead.
+constexpr int kAhead = 4;
+__global__ void __launch_bounds__(256) an_ajdk_kernel(RowvecParams p) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  const int r0 = RPW * warp;
+  const int r0 = 2 * warp;
   if (r0 >= p.n) return;
-  const bool two = RPW == 2 && r0 + 1 < p.n;
-  const uint8_t *rowA = p.w + (long long)p.rowb[r0] * p.row_bytes;
-  const uint8_t *rowB = two ? p.w + (long long)p.rowb[r0 + 1] * p.row_bytes : rowA;
+  const bool two = r0 + 1 < p.n;
+  const int piece = lane < 15 ? lane : lane - 15;
+  const bool reads = lane < 30;
+  const uint4 *row = reinterpret_cast<const uint4 *>(p.w + (long long)p.rowb[lane >= 15 && two ? r0 + 1 : r0] * p.row_bytes) + piece;
+  const uint4 *mask = reinterpret_cast<const uint4 *>(p.mask) + piece;
   const int k = lane & 15;
   const bool mine = k < 15 && (lane < 16 || two);
-  double s = 0.0;
-  for (int b = 0; b < p.P; ++b) {
-    const long long bo = (long long)b * kBlockBytes;
-    const int cA = block_count(rowA + bo, p.mask + bo, lane);
-    int c = cA;
-    if (RPW == 2) {
-      const int cB = block_count(rowB + bo, p.mask + bo, lane);
-      c = lane < 16 ? cA : cB;
+  const double *w = p.ajdk + (long long)(k < 15 ? k : 0) * p.P;
+  uint4 x[kAhead], m[kAhead];
+  double d[kAhead];
+  auto load = [&](int b, int u) {
+    x[u] = m[u] = make_uint4(0u, 0u, 0u, 0u);
+    d[u] = 0.0;
+    if (b < p.P) {
+      if (reads) {
+        x[u] = __ldg(row + 15 * b);
+        m[u] = __ldg(mask + 15 * b);
+      }
+      d[u] = __ldg(w + b);
     }
-    if (mine) s = __dadd_rn(s, __dmul_rn(p.ajdk[b + (long long)k * p.P], (double)c));
+  };
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u) load(u, u);
+  double s = 0.0;
+  for (int b0 = 0; b0 < p.P; b0 += kAhead) {
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int b = b0 + u;
+      if (b >= p.P) break;
+      const uint32_t c = (uint32_t)(__popc(x[u].x & m[u].x) + __popc(x[u].y & m[u].y) + __popc(x[u].z & m[u].z) +
+                                    __popc(x[u].w & m[u].w));
+      const uint32_t both = __reduce_add_sync(0xffffffffu, lane < 15 ? c : c << 16);
+      const double v = times_count(d[u], lane < 16 ? both & 0xffffu : both >> 16);
+      load(b + kAhead, u);
+      s = __dadd_rn(s, v);
+    }
   }
   if (mine) {
     double o = (p.type == 1) ? __dadd_rn(-p.base[k], __dmul_rn(2.0, s)) : s;
@@ -94,12 +114,8 @@ void launch_an_v(const RowvecParams &p) {
 void launch_an_ajdk(const RowvecParams &p) {
   if (p.n <= 0) return;
   const int threads = 256;
-  if (p.n >= kAjdkTwoRows) {
-    const long long warps = ((long long)p.n + 1) / 2;
-    an_ajdk_kernel<2><<<(int)((warps * 32 + threads - 1) / threads), threads, 0, stream()>>>(p);
-  } else {
-    an_ajdk_kernel<1><<<(int)(((long long)p.n * 32 + threads - 1) / threads), threads, 0, stream()>>>(p);
-  }
+  const long long warps = ((long long)p.n + 1) / 2;
+  an_ajdk_kernel<<<(int)((warps * 32 + threads - 1) / threads), threads, 0, stream()>>>(p);
   LAKGB_CUDA(cudaGetLastError());
   count_launch();
 }

@@ -27,6 +27,7 @@
 #include "lakgb_runtime.cuh"
 #include "tc_counts.cuh"
 #include "tc_ptx.cuh"
+#include "weigh.cuh"
 
 namespace lakgb {
 
@@ -210,7 +211,7 @@ __device__ __forceinline__ int decode_count(uint32_t bits) {
 
 template <int TYPE>
 __global__ void __launch_bounds__(kThreads, 2)
-    gram_counts_tc_kernel(GramParams p, uint16_t *__restrict__ out, int *status) {
+    gram_counts_tc_kernel(GramParams p, uint16_t *__restrict__ out, uint16_t *__restrict__ zcnt, int *status) {
   extern __shared__ __align__(128) uint8_t dsm[];
   __shared__ Smem sm;
   const int m0 = blockIdx.y * kM, n0 = blockIdx.x * kN, b = blockIdx.z;
@@ -220,6 +221,8 @@ __global__ void __launch_bounds__(kThreads, 2)
   tile.setup(&sm, dsm, t, m0, n0);
   tile.block(t, b, true, false, status);
   tile.wait_mma(status);
+  if (zcnt && m0 == 0 && threadIdx.x < kN && n0 + (int)threadIdx.x < p.nZ)
+    zcnt[(size_t)b * p.nZ + n0 + threadIdx.x] = (uint16_t)tile.cnt[kM + threadIdx.x];
   if (tile.ok) {
     uint32_t v[32];
     tile.read(v);
@@ -237,17 +240,6 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
   }
   tile.finish();
-}
-
-// RN(D c) for a positive normal D = dm 2^(ed - 1075) and 0 < c < 2^11, in
-// integers: dm c < 2^64 is exact and is rounded to 53 bits, ties to even.  (An
-// FP64 multiply holds the sub-partition's FP64 pipe for 80 cycles per warp,
-// beside the add that has to be one.)
-__device__ __forceinline__ double weigh(unsigned long long dm, int ed, uint32_t c) {
-  const unsigned long long x = dm * c;
-  const int sh = 11 - __clzll((long long)x);  // bits past 53
-  const unsigned long long r = (x + ((1ull << sh) >> 1) - (sh > 0) + ((x >> sh) & (sh > 0 ? 1ull : 0ull))) >> sh;
-  return __longlong_as_double((long long)(((unsigned long long)(ed + sh - 1) << 52) + r));
 }
 
 // The weighted counts of every element added over the blocks in order, then
@@ -268,16 +260,8 @@ __global__ void __launch_bounds__(256) gram_fold_kernel(GramParams p, const uint
     } else {
 #pragma unroll 4
       for (int b = 0; b < p.P; ++b) {
-        const double d = __ldg(p.D + b);
-        const unsigned long long bits = (unsigned long long)__double_as_longlong(d);
-        const int ed = (int)(bits >> 52);  // sign and exponent
-        const uint32_t c = ce[(size_t)b * n];
-        double x;
-        if (ed > 0 && ed < 2000) {
-          x = c ? weigh((bits & 0x000fffffffffffffull) | 0x0010000000000000ull, ed, c) : 0.0;
-        } else {
-          x = __dmul_rn(d, (double)c);
-        }
+        // the multiply in integers, beside the add that has to be FP64
+        const double x = times_count(__ldg(p.D + b), ce[(size_t)b * n]);
         acc = __dadd_rn(acc, x);
       }
     }
@@ -368,20 +352,26 @@ void allow_smem(K kernel) {
 }
 
 template <int TYPE>
-void launch_split_type(const GramParams &p, uint16_t *cnt, cudaStream_t s) {
+void launch_counts(const GramParams &p, uint16_t *cnt, uint16_t *zcnt, cudaStream_t s) {
   static const bool configured = [] {
     allow_smem(gram_counts_tc_kernel<TYPE>);
     return true;
   }();
   (void)configured;
   const dim3 grid((p.nZ + kN - 1) / kN, (p.nA + kM - 1) / kM, p.P);
-  gram_counts_tc_kernel<TYPE><<<grid, kThreads, kSmemBytes, s>>>(p, cnt, tc_status_device_ptr());
+  gram_counts_tc_kernel<TYPE><<<grid, kThreads, kSmemBytes, s>>>(p, cnt, zcnt, tc_status_device_ptr());
   LAKGB_CUDA(cudaGetLastError());
+  count_launch();
+}
+
+template <int TYPE>
+void launch_split_type(const GramParams &p, uint16_t *cnt, cudaStream_t s) {
+  launch_counts<TYPE>(p, cnt, nullptr, s);
   const int bx = std::min(256, (p.nA + 31) / 32 * 32), by = 256 / bx;
   const dim3 fold((p.nA + bx - 1) / bx, std::min((p.nZ + by - 1) / by, 65535));
   gram_fold_kernel<TYPE><<<fold, dim3(bx, by), 0, s>>>(p, cnt);
   LAKGB_CUDA(cudaGetLastError());
-  count_launch(2);
+  count_launch();
 }
 
 }  // namespace
@@ -391,6 +381,10 @@ void launch_gram_tc_split(const GramParams &p, uint16_t *cnt, cudaStream_t s) {
     launch_split_type<1>(p, cnt, s);
   else
     launch_split_type<2>(p, cnt, s);
+}
+
+void launch_and_counts_tc(const GramParams &p, uint16_t *cnt, uint16_t *zcnt, cudaStream_t s) {
+  launch_counts<2>(p, cnt, zcnt, s);
 }
 
 void launch_attyn_tc(const AtTYnParams &p, int nT, cudaStream_t s) {

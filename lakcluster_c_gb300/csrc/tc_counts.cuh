@@ -14,6 +14,10 @@ constexpr int kCountsM = 128, kCountsN = 64;  // tile rows of A and Z
 // and a fold over the blocks in order.  P <= 65535.
 void launch_gram_tc_split(const GramParams &p, uint16_t *cnt, cudaStream_t s);
 
+// The per-block counts alone: cnt as above (popcount(A & Z & mask)) and zcnt,
+// P x nZ: popcount(Z & mask).
+void launch_and_counts_tc(const GramParams &p, uint16_t *cnt, uint16_t *zcnt, cudaStream_t s);
+
 // AtTYn_vv and, with `symmetric`, AtTAn_vv.
 struct AtTYnParams {
   const uint8_t *At; const uint32_t *a_rowb; int nA; long long a_row_bytes;
