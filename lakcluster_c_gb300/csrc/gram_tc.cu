@@ -1,4 +1,4 @@
-// +/-1 Gram of packed bit rows on the tensor cores (tcgen05, e4m3 operands).
+// +/-1 Gram of packed bit rows on the tensor cores (tcgen05, e2m1 operands).
 //
 // Computes exactly what the popcount kernel (gram.cu) computes, bit for bit:
 //   out[i,k] = a0d1 - 2*S_ik - ((lfA_i + lfZ_k) - a2d1),  S_ik = sum_b D_b * c_ikb

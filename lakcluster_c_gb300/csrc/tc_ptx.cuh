@@ -139,42 +139,11 @@ __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// Shared-memory matrix descriptor, K-major operand without swizzle: core
-// matrices of 8 rows x 16 bytes; lbo = byte distance between core matrices
-// adjacent in K, sbo = byte distance between core matrices adjacent in M/N.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-  d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;  // descriptor version
-  return d;
-}
-
-// Shared-memory matrix descriptor, K-major operand with the 128-byte swizzle:
-// rows of 128 bytes, 8-row atoms of 1024 bytes (1024-byte aligned), the
-// 16-byte chunk c of row r stored at chunk c ^ (r % 8); sbo = byte distance
-// between 8-row atoms.  A start address inside the first row of an atom
-// selects the K offset.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-  d |= (uint64_t)1 << 16;  // leading byte offset: unused by swizzled K-major layouts
-  d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;  // descriptor version
-  d |= (uint64_t)2 << 61;  // layout: 128-byte swizzle
-  return d;
-}
-
-// Instruction descriptor of kind::f8f6f4 with e4m3 A and B, f32 accumulator,
-// both operands K-major, shape M x N.
-__host__ __device__ constexpr uint32_t idesc_e4m3_f32(int M, int N) {
-  return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-
-// As smem_desc_sw128 with the 64-byte swizzle: rows of 64 bytes, 8-row atoms
-// of 512 bytes (512-byte aligned), the 16-byte chunk c of row r stored at chunk
-// c ^ (r / 2 % 4).
+// Shared-memory matrix descriptor, K-major operand with the 64-byte swizzle:
+// rows of 64 bytes, 8-row atoms of 512 bytes (512-byte aligned), the 16-byte
+// chunk c of row r stored at chunk c ^ (r / 2 % 4); sbo = byte distance between
+// 8-row atoms.  A start address inside the first row of an atom selects the K
+// offset.
 __device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t saddr, uint32_t sbo) {
   uint64_t d = 0;
   d |= (uint64_t)((saddr >> 4) & 0x3FFF);
@@ -235,16 +204,6 @@ __device__ __forceinline__ void expand_e2m1(uint32_t row_base, uint32_t sw, uint
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j) st_shared_v4(row_base + ((j ^ sw) << 4), o[j][0], o[j][1], o[j][2], o[j][3]);
-}
-
-// D[tmem] (+)= A * B^T, issued by one thread.
-__device__ __forceinline__ void mma_e4m3(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
 }
 
 // Arrive on `bar` once all previously issued tcgen05 MMAs of this thread

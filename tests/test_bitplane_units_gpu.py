@@ -57,3 +57,9 @@ def test_tensor_bitplane_equals_oracle(gpu_lib, snps, ny, nw, B, nt, keep, mlt):
     got = _call(gpu_lib.wrap_At_T_YnWt_S_Zn_ww__run, h, snps, nt, (C.byref(C.c_int(0)), None, None))
     assert gpu_lib.lakgb_device_status() == 0
     assert np.array_equal(got.view(np.uint64), want.view(np.uint64))
+
+
+@pytest.mark.parametrize("ny,nw,B", [(383, 28, 8), (384, 29, 8), (385, 14, 16), (769, 15, 16), (1537, 7, 32),
+                                     (3841, 6, 32)])
+def test_units_of_224_planes_and_steps_of_384_patients(gpu_lib, ny, nw, B):
+    test_tensor_bitplane_equals_oracle(gpu_lib, 130, ny, nw, B, 2, 0.9, 2.9)
