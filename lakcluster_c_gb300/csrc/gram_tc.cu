@@ -57,6 +57,7 @@
 // 224 accumulator columns; N = 112 leaves room for the scale factors.
 #include <algorithm>
 
+#include "fixed_fp64.cuh"
 #include "gram.cuh"
 #include "lakgb_runtime.cuh"
 #include "tc_ptx.cuh"
@@ -136,16 +137,6 @@ __device__ __forceinline__ int decode_count(uint32_t bits) {
   return __float_as_int(__fadd_rn(__uint_as_float(bits), 12582912.0f)) - 0x4B400000;
 }
 
-// 2.0 * x, exactly as __dmul_rn(2.0, x) rounds it: for a normal x whose
-// double does not overflow, one more in the exponent field; otherwise (zero,
-// subnormal, near-overflow, inf, nan) the multiply itself.  Keeps the FP64
-// pipe for the adds.
-__device__ __forceinline__ double twice(double x) {
-  const long long bits = __double_as_longlong(x);
-  const int e = (int)((bits >> 52) & 0x7FF);
-  return (e >= 1 && e <= 2045) ? __longlong_as_double(bits + (1ll << 52)) : __dmul_rn(2.0, x);
-}
-
 // (tile_m, tile_n) of tile r of one Gram's list.  A full grid is walked in
 // bands of kBand tile rows, each band column by column: the CTAs of a wave
 // (consecutive r) then share a few A row panels and a few Z row panels, a
@@ -208,6 +199,69 @@ template <bool GRP>
 __device__ __forceinline__ const GramParams &params_of(const GramParams &p, const GramGroupDev &g, int inst) {
   if constexpr (GRP) return g.ps[inst];
   else return p;
+}
+
+// The results of a fold warp's 32 rows x kFoldCols columns from its sums S in
+// TMEM (acc): a0d1 - 2 S - ((lfA + lfZ) - a2d1).  As four FP64 operations and a
+// predicated multiply for 2 S that took 52000 cycles a tile (a block's fold:
+// 10400): S doubles in its bits, and the row terms, known before the sums, are
+// added in fixed point where all of the warp's have one (fixed_fp64.cuh).
+template <int TYPE>
+__device__ __forceinline__ void write_results(const GramParams &pp, int tile_m, int tile_n, int col0, int row, int lane,
+                                              uint32_t acc) {
+  const int ga = tile_m + row, gl = tile_n + col0 + lane;
+  const bool row_in = ga < pp.nA, lf = pp.lfA && pp.lfZ;
+  const double lfa = (lf && row_in) ? pp.lfA[ga] : 0.0, a0 = pp.a0d1, a2 = pp.a2d1;
+  const long long orow = row_in ? (long long)pp.out_r[ga] : 0;
+  const long long ocol2 = (pp.symmetric && row_in) ? (long long)pp.out_c2[ga] * pp.out_stride : 0;
+  long long fa = 0, fz = 0, f2 = 0;
+  int emax = 0;
+  bool fixed = false;
+  if (lf) {
+    // lane l holds the term of the warp's column l
+    const double lfz = (lane < kFoldCols && gl < pp.nZ) ? pp.lfZ[gl] : 0.0;
+    const uint32_t e = max(max((uint32_t)__double2hiint(lfa) << 1, (uint32_t)__double2hiint(lfz) << 1),
+                           (uint32_t)__double2hiint(a2) << 1);
+    emax = (int)(__reduce_max_sync(0xffffffffu, e) >> 21);
+    const bool good = fixed::from_bits((unsigned long long)__double_as_longlong(lfa), emax, &fa) &
+                      fixed::from_bits((unsigned long long)__double_as_longlong(lfz), emax, &fz) &
+                      fixed::from_bits((unsigned long long)__double_as_longlong(a2), emax, &f2);
+    fixed = __all_sync(0xffffffffu, good && fixed::in_range(emax));
+  }
+#pragma unroll 1
+  for (int r = 0; r < kRounds; ++r) {
+    uint32_t a[2 * kRound];
+    __syncwarp();
+    tmem_ld_n<2 * kRound>(acc + 2 * r * kRound, a);
+    double f[kRound];
+    if (fixed) {
+#pragma unroll
+      for (int j = 0; j < kRound; ++j) {
+        const long long z = __shfl_sync(0xffffffffu, fz, r * kRound + j);
+        f[j] = __longlong_as_double((long long)fixed::to_bits(fixed::round53(fa + z) - f2, emax));
+      }
+    } else if (lf) {
+      // read here, so that the compiler can not hoist the FP64 operations above
+      // the branch
+#pragma unroll
+      for (int j = 0; j < kRound; ++j)
+        f[j] = __dsub_rn(__dadd_rn(lfa, __ldcv(pp.lfZ + min(tile_n + col0 + r * kRound + j, pp.nZ - 1))), a2);
+    }
+    tc::tmem_wait_ld();
+    tc::reg_fence(a);
+#pragma unroll
+    for (int j = 0; j < kRound; ++j) {
+      const int gz = tile_n + col0 + r * kRound + j;
+      const double v = __hiloint2double((int)a[2 * j + 1], (int)a[2 * j]);
+      double o = v;
+      if (TYPE == 1)
+        o = __dsub_rn(a0, __longlong_as_double((long long)fixed::twice_bits((unsigned long long)__double_as_longlong(v))));
+      if (lf) o = __dsub_rn(o, f[j]);
+      if (!row_in || gz >= pp.nZ || (pp.symmetric && ga > gz)) continue;
+      pp.out[orow + (long long)pp.out_c[gz] * pp.out_stride] = o;
+      if (pp.symmetric) pp.out[(long long)pp.out_r2[gz] + ocol2] = o;
+    }
+  }
 }
 
 template <int TYPE, bool GRP>
@@ -474,11 +528,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     while (walk.next(p, grp, inst, tile_m, tile_n)) {
       const GramParams &pp = params_of<GRP>(p, grp, inst);
       const int P = pp.P;
-      const int ga = tile_m + row;
-      const bool row_in = ga < pp.nA;
-      const double lfa = (pp.lfA && row_in) ? pp.lfA[ga] : 0.0;
-      const long long orow = row_in ? (long long)pp.out_r[ga] : 0;
-      const long long ocol2 = (pp.symmetric && row_in) ? (long long)pp.out_c2[ga] * pp.out_stride : 0;
       for (int b = 0; b < P; ++b) {
         const long long gbb = gb0 + b;
         const int t = (int)(gbb & 1);
@@ -537,22 +586,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             a[cur][2 * j] = (uint32_t)__double2loint(v);
             a[cur][2 * j + 1] = (uint32_t)__double2hiint(v);
           }
-          if (b + 1 < P) {
-            // accumulators of columns c0 + j: TMEM columns kAccCol + 2 (c0 + j)
-            // (low word) and + 1 (high word)
-            if (ok) tmem_st_n<2 * kRound>(lane_base + kAccCol + 2 * c0, a[cur]);
-          } else if (ok && row_in) {
-#pragma unroll
-            for (int j = 0; j < kRound; ++j) {
-              const int gz = tile_n + c0 + j;
-              if (gz >= pp.nZ || (pp.symmetric && ga > gz)) continue;
-              const double v = __hiloint2double((int)a[cur][2 * j + 1], (int)a[cur][2 * j]);
-              double o = (TYPE == 1) ? __dsub_rn(pp.a0d1, twice(v)) : v;
-              if (pp.lfA && pp.lfZ) o = __dsub_rn(o, __dsub_rn(__dadd_rn(lfa, pp.lfZ[gz]), pp.a2d1));
-              pp.out[orow + (long long)pp.out_c[gz] * pp.out_stride] = o;
-              if (pp.symmetric) pp.out[(long long)pp.out_r2[gz] + ocol2] = o;
-            }
-          }
+          // accumulators of columns c0 + j: TMEM columns kAccCol + 2 (c0 + j)
+          // (low word) and + 1 (high word)
+          if (ok) tmem_st_n<2 * kRound>(lane_base + kAccCol + 2 * c0, a[cur]);
           if (ok && r + 1 < kRounds) {
             tc::tmem_wait_ld();
             tc::reg_fence(cn[nxt]);
@@ -581,6 +617,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&sm.aux_empty[t]);
       }
+      if (ok) write_results<TYPE>(pp, tile_m, tile_n, col0, row, lane, lane_base + kAccCol + 2 * col0);
       gb0 += P;
       ++jt;
     }
