@@ -4,9 +4,9 @@
 // half the time and leaves the pipe to others.
 //
 // With emax the largest biased exponent of the values, a fixed-point number is
-// a multiple of 2^(emax - 1083): the largest value has 61 bits, so two of them
-// and the difference to a third stay below 2^63.  A value is representable if
-// it has no bits below that unit (any value down to 2^-8 of the largest, smaller
+// a multiple of 2^(emax - 1082): the largest value has 60 bits, so sums and
+// differences of up to eight stay below 2^63.  A value is representable if it
+// has no bits below that unit (any value down to 2^-7 of the largest, smaller
 // ones if their low bits are clear); the others take the FP64 operations.
 #pragma once
 #include <stdint.h>
@@ -19,6 +19,8 @@
 
 namespace lakgb {
 namespace fixed {
+
+constexpr int kBelow = 7;  // binades below the largest
 
 LAKGB_HD int clz32(uint32_t x) {
 #ifdef __CUDA_ARCH__
@@ -46,7 +48,7 @@ LAKGB_HD bool from_bits(unsigned long long x, int emax, long long *out) {
   const int e = (int)((x >> 52) & 0x7FF);
   if (e == 0 || e == 0x7FF) return false;
   unsigned long long m = (x & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
-  const int sh = e - emax + 8;
+  const int sh = e - emax + kBelow;
   if (sh >= 0) {
     m <<= sh;
   } else {
@@ -78,7 +80,7 @@ LAKGB_HD unsigned long long to_bits(long long s, int emax) {
   n <<= z;
   const unsigned long long b = n >> 11;
   const uint32_t up = (((uint32_t)n & 0x7FFu) + 0x3FFu + ((uint32_t)b & 1u)) >> 11;
-  return sign | ((((unsigned long long)(emax + 2 - z)) << 52) + b + up);
+  return sign | ((((unsigned long long)(emax + 10 - kBelow - z)) << 52) + b + up);
 }
 
 // 2 x on the bits, as the FP64 multiply rounds it: one more in the exponent,

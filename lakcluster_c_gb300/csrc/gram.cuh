@@ -49,9 +49,9 @@ constexpr int kGramTileM = 128, kGramTileN = 112;
 int gram_tc_tiles(const GramParams &p);
 
 // Enqueue the grouped tensor-core Gram on stream s: the table kernel for all
-// instances' blocks into T (total_blocks x 1922 doubles), then one
+// instances' blocks into T (total_blocks table rows), then one
 // persistent launch over all instances' tiles.
-void launch_gram_tc_group(const GramGroupDev &g, int type, int total_tiles, long long total_blocks, double *T,
+void launch_gram_tc_group(const GramGroupDev &g, int type, int total_tiles, long long total_blocks, void *T,
                           cudaStream_t s);
 // Bytes of one table row (per instance block) of the grouped launch.
 size_t gram_tc_table_row_bytes();

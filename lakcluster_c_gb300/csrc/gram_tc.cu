@@ -21,10 +21,31 @@
 // together were over half of the kernel's shared-memory traffic, and takes a
 // third of the expansion's integer operations.
 //
-// FP64 part on the CUDA cores, in the reference's order: acc = acc + D_b * c,
-// one rounding each, blocks ascending.  The product D_b * c is read from a
-// table T_b[c] (c = 0..1920), built once per launch with the same rounded
-// multiply, so the FP64 pipe -- slow on this part -- does only the add.
+// FP64 part on the CUDA cores, in the reference's order: acc = RN(acc + x),
+// x = RN(D_b * c), blocks ascending.  An FP64 instruction of a warp holds its
+// sub-partition's FP64 pipe for 80 cycles, so one FP64 add per element and
+// block bounds the kernel (8960 cycles per tile and block; whole kernel 75.9 ms
+// on 16384 x 16384 rows x 131072 columns of three bins, 60.3 ms with half of
+// the adds left out), and integer adds alone are more instructions than the SM
+// issues in that time (88 ms).  So rounds of four columns add with FP64 and with
+// integers in turn: 62.7 ms (two or four of seven in integers: 63.8 and 64.7;
+// two columns of every round: 64.8, a warp that waits for one pipe can not
+// issue to the other).  Neither pipe is full then: of the issue slots 55 % are
+// used, and the warps wait for TMEM, table and add latencies with no registers
+// left for more of them.
+// FP64: x comes from a table of the block's products.
+// Integers: while acc lies in one binade its bit pattern counts units in the
+// last place, and adding x is adding the integer RN(x / ulp), ties to even.
+// For two exponents the table holds, for every count c and parity of acc,
+//   RN(x / ulp) - c * floor(D / ulp)   (at most c + 1: 12 bits)
+// and on which side of x / ulp that lies, so that an add is a 32 x 64-bit
+// multiply-add and one more add.  A sum that leaves its binade is rounded once
+// more, one bit up.  A round of which an element has another exponent or no
+// entry (zero sums; negative, tiny or non-finite weights) is done again with
+// FP64.
+// The two exponents lie around the block's expected sums, estimated from a few
+// row pairs when the table is made; the estimate decides only how often that
+// happens.
 //
 // Persistent CTAs, one per SM, each looping over 128 (A rows) x 112 (Z rows)
 // output tiles; the pipeline runs on across tile boundaries.  25 warps:
@@ -45,12 +66,12 @@
 //               step, 5 steps per block) into one of two count buffers.
 //   warps 9-24  fold, four warps per lane quadrant (warp w reads TMEM lanes
 //               32*(w%4)..+31), each for 28 of the 112 columns: per block,
-//               read the counts from TMEM, look up T_b[c], add into the FP64
-//               accumulators, which live in TMEM as well (columns 256..479,
+//               read the counts from TMEM, look up the table, add into the
+//               FP64 sums, which live in TMEM as well (columns 256..479,
 //               two 32-bit halves per value).
 // Shared memory: 6 raw slots (11 KB each) + 2 stages x 3 x (8 KB A + 7 KB B) +
-// 2 x T_b (15 KB) + counts.
-// The T_b buffers are filled by bulk copies on mbarriers, issued by whichever
+// 2 block tables (30 KB) + counts.
+// The table buffers are filled by bulk copies on mbarriers, issued by whichever
 // fold warp finishes a block last, so fold warps drift apart by up to a block
 // instead of meeting at every block boundary.
 // TMEM: 2 x 112 count columns (0.., 128..), the scale factors (112..127) and
@@ -84,7 +105,18 @@ constexpr int kTileB = kBN * 64;
 constexpr int kChunkBytes = kTileA + kTileB;
 constexpr int kStageBytes = kChunk * kChunkBytes;
 constexpr int kTabStride = 1922;          // doubles per block table (1921 used, 16-byte multiple)
-constexpr int kTabBytes = kTabStride * 8;
+constexpr int kTabExps = 2;               // exponents of the integer entries
+constexpr int kTabInt = kTabStride * 8;   // their place in a block's table
+constexpr int kTabExpBytes = kTabStride * 4;
+constexpr int kTabHdr = kTabInt + kTabExps * kTabExpBytes;
+struct TabHdr {
+  unsigned long long unit[kTabExps];      // floor(D / ulp) of exponent etop, etop - 1
+  uint32_t etop, pad[3];                  // biased exponent
+};
+constexpr int kTabBytes = kTabHdr + (int)sizeof(TabHdr);
+constexpr uint32_t kTabInvalid = 0xFFFFu, kTabValue = 0xFFFu;
+constexpr int kTabRestShift = 12;         // x / ulp - RN(x / ulp): 0 zero, 1 above, 2 below
+static_assert(kTabInt % 16 == 0 && kTabHdr % 16 == 0 && kTabBytes % 16 == 0, "bulk copies");
 constexpr int kSBO = 8 * 64;              // bytes between 8-row swizzle atoms (8 rows of 64 B)
 constexpr int kProducers = 256;           // warps 0-7
 constexpr int kMmaWarp = 8;
@@ -102,6 +134,7 @@ static_assert(kFoldCols % kRound == 0 && kBN <= (int)kSfCol && kAccCol + 2 * kBN
 static_assert(kChunkBytes % 512 == 0 && kSteps * kRawRow == kBlockRow, "swizzle atoms, whole blocks");
 constexpr size_t kSmemBytes =
     (size_t)kStages * kStageBytes + kRawSlots * kRawBytes + 2 * kTabBytes + 2 * 256 * 4 + 1024;
+static_assert(kSmemBytes + 512 <= 227 * 1024, "one CTA per SM");
 
 struct Smem {
   uint64_t full[kStages], empty[kStages];
@@ -201,79 +234,158 @@ __device__ __forceinline__ const GramParams &params_of(const GramParams &p, cons
   else return p;
 }
 
+// Rounds of kRound columns of a fold warp that hold results: not those past
+// the last Z row or, in a symmetric Gram, left of the warp's first row.  A warp
+// past the last A row has none.  [first, end)
+__device__ __forceinline__ void live_rounds(const GramParams &pp, int row0, int colbase, int &first, int &end) {
+  first = 0;
+  end = row0 < pp.nA ? min(kRounds, (max(pp.nZ - colbase, 0) + kRound - 1) / kRound) : 0;
+  if (pp.symmetric && row0 > colbase) first = min((row0 - colbase) / kRound, end);
+}
+
 // The results of a fold warp's 32 rows x kFoldCols columns from its sums S in
 // TMEM (acc): a0d1 - 2 S - ((lfA + lfZ) - a2d1).  As four FP64 operations and a
 // predicated multiply for 2 S that took 52000 cycles a tile (a block's fold:
-// 10400): S doubles in its bits, and the row terms, known before the sums, are
-// added in fixed point where all of the warp's have one (fixed_fp64.cuh).
+// 10400), now about 25000 (2018 x 2025 rows x 820 columns: 65.3 -> 49 us).  So S doubles in its bits; where all of the warp's terms have a
+// fixed-point form (fixed_fp64.cuh), every other round is computed in integers,
+// the even ones by half of a sub-partition's warps and the odd ones by the other.
 template <int TYPE>
 __device__ __forceinline__ void write_results(const GramParams &pp, int tile_m, int tile_n, int col0, int row, int lane,
-                                              uint32_t acc) {
+                                              int first, int end, int phase, uint32_t acc) {
   const int ga = tile_m + row, gl = tile_n + col0 + lane;
   const bool row_in = ga < pp.nA, lf = pp.lfA && pp.lfZ;
-  const double lfa = (lf && row_in) ? pp.lfA[ga] : 0.0, a0 = pp.a0d1, a2 = pp.a2d1;
-  const long long orow = row_in ? (long long)pp.out_r[ga] : 0;
-  const long long ocol2 = (pp.symmetric && row_in) ? (long long)pp.out_c2[ga] * pp.out_stride : 0;
-  long long fa = 0, fz = 0, f2 = 0;
+  const double lfa = (lf && row_in) ? pp.lfA[ga] : 0.0, a0 = TYPE == 1 ? pp.a0d1 : 0.0, a2 = pp.a2d1;
+  // Everything else that a result needs is read here, before the first store
+  // (which may change any of it, for all the compiler knows); lane l holds what
+  // belongs to the warp's column l.
+  const bool sym = pp.symmetric, col_in = lane < kFoldCols && gl < pp.nZ;
+  const long long stride = pp.out_stride;
+  const int nZ = pp.nZ;
+  const double *plfz = pp.lfZ;
+  const double lfz = (lf && col_in) ? plfz[gl] : 0.0;
+  const uint32_t oc = col_in ? pp.out_c[gl] : 0u, or2 = (sym && col_in) ? pp.out_r2[gl] : 0u;
+  double *out = pp.out + (row_in ? (long long)pp.out_r[ga] : 0);
+  double *out2 = pp.out + ((sym && row_in) ? (long long)pp.out_c2[ga] * stride : 0);
+  long long fa = 0, fz = 0, f0 = 0, f2 = 0;
   int emax = 0;
   bool fixed = false;
   if (lf) {
-    // lane l holds the term of the warp's column l
-    const double lfz = (lane < kFoldCols && gl < pp.nZ) ? pp.lfZ[gl] : 0.0;
     const uint32_t e = max(max((uint32_t)__double2hiint(lfa) << 1, (uint32_t)__double2hiint(lfz) << 1),
-                           (uint32_t)__double2hiint(a2) << 1);
+                           max((uint32_t)__double2hiint(a0) << 1, (uint32_t)__double2hiint(a2) << 1));
     emax = (int)(__reduce_max_sync(0xffffffffu, e) >> 21);
     const bool good = fixed::from_bits((unsigned long long)__double_as_longlong(lfa), emax, &fa) &
                       fixed::from_bits((unsigned long long)__double_as_longlong(lfz), emax, &fz) &
+                      fixed::from_bits((unsigned long long)__double_as_longlong(a0), emax, &f0) &
                       fixed::from_bits((unsigned long long)__double_as_longlong(a2), emax, &f2);
     fixed = __all_sync(0xffffffffu, good && fixed::in_range(emax));
   }
 #pragma unroll 1
-  for (int r = 0; r < kRounds; ++r) {
+  for (int r = first; r < end; ++r) {
     uint32_t a[2 * kRound];
     __syncwarp();
     tmem_ld_n<2 * kRound>(acc + 2 * r * kRound, a);
-    double f[kRound];
-    if (fixed) {
-#pragma unroll
-      for (int j = 0; j < kRound; ++j) {
-        const long long z = __shfl_sync(0xffffffffu, fz, r * kRound + j);
-        f[j] = __longlong_as_double((long long)fixed::to_bits(fixed::round53(fa + z) - f2, emax));
-      }
-    } else if (lf) {
-      // read here, so that the compiler can not hoist the FP64 operations above
-      // the branch
-#pragma unroll
-      for (int j = 0; j < kRound; ++j)
-        f[j] = __dsub_rn(__dadd_rn(lfa, __ldcv(pp.lfZ + min(tile_n + col0 + r * kRound + j, pp.nZ - 1))), a2);
-    }
+    double o[kRound];
     tc::tmem_wait_ld();
     tc::reg_fence(a);
+    // in integers where every S has a fixed-point form too (not a zero, a
+    // smaller or larger S)
+    bool good = fixed && ((r ^ phase) & 1);
+#pragma unroll
+    for (int j = 0; j < kRound; ++j)
+      good = good && (a[2 * j + 1] >> 20) - (uint32_t)(emax - fixed::kBelow) <= (uint32_t)fixed::kBelow;
+    if (__all_sync(0xffffffffu, good || (!row_in && fixed && ((r ^ phase) & 1)))) {
+#pragma unroll
+      for (int j = 0; j < kRound; ++j) {
+        const uint32_t sh = ((a[2 * j + 1] >> 20) - (uint32_t)(emax - fixed::kBelow)) & 15u;
+        const long long v = (long long)(((unsigned long long)((a[2 * j + 1] & 0xFFFFFu) | 0x100000u) << 32 | a[2 * j]) << sh);
+        const long long t = fixed::round53(fixed::round53(fa + __shfl_sync(0xffffffffu, fz, r * kRound + j)) - f2);
+        const long long u = TYPE == 1 ? fixed::round53(f0 - 2 * v) : v;
+        o[j] = __longlong_as_double((long long)fixed::to_bits(u - t, emax));
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < kRound; ++j) {
+        const unsigned long long s = (unsigned long long)a[2 * j + 1] << 32 | a[2 * j];
+        o[j] = TYPE == 1 ? __dsub_rn(a0, __longlong_as_double((long long)fixed::twice_bits(s))) : __longlong_as_double((long long)s);
+        // read here, so that the compiler can not hoist the FP64 operations
+        // above the branch
+        if (lf)
+          o[j] = __dsub_rn(o[j], __dsub_rn(__dadd_rn(lfa, __ldcv(plfz + min(tile_n + col0 + r * kRound + j, nZ - 1))), a2));
+      }
+    }
 #pragma unroll
     for (int j = 0; j < kRound; ++j) {
       const int gz = tile_n + col0 + r * kRound + j;
-      const double v = __hiloint2double((int)a[2 * j + 1], (int)a[2 * j]);
-      double o = v;
-      if (TYPE == 1)
-        o = __dsub_rn(a0, __longlong_as_double((long long)fixed::twice_bits((unsigned long long)__double_as_longlong(v))));
-      if (lf) o = __dsub_rn(o, f[j]);
-      if (!row_in || gz >= pp.nZ || (pp.symmetric && ga > gz)) continue;
-      pp.out[orow + (long long)pp.out_c[gz] * pp.out_stride] = o;
-      if (pp.symmetric) pp.out[(long long)pp.out_r2[gz] + ocol2] = o;
+      const uint32_t c = __shfl_sync(0xffffffffu, oc, r * kRound + j), r2 = __shfl_sync(0xffffffffu, or2, r * kRound + j);
+      if (!row_in || gz >= nZ || (sym && ga > gz)) continue;
+      out[(long long)c * stride] = o[j];
+      if (sym) out2[r2] = o[j];
+    }
+  }
+}
+
+// acc = RN(acc + RN(D c)) for the warp's 32 x kRound sums (a: low and high
+// words; old: the same in TMEM), in integers as described at the top.
+// Lanes without a row hold no sums.
+__device__ __forceinline__ void add_round(const uint8_t *tab, uint32_t etop, const int (&c)[kRound],
+                                          uint32_t (&a)[2 * kRound], uint32_t old, bool row_in) {
+  uint32_t far = 0u, left = 0u, last = 0u, below = 0u, ent[kRound];
+#pragma unroll
+  for (int j = 0; j < kRound; ++j) {
+    const uint32_t lo = a[2 * j], hi = a[2 * j + 1], x = etop - (hi >> 20), xi = x & 1u;
+    ent[j] = *reinterpret_cast<const uint16_t *>(tab + kTabInt + xi * kTabExpBytes + 4 * c[j] + 2 * (lo & 1u));
+    const unsigned long long unit = reinterpret_cast<const TabHdr *>(tab + kTabHdr)->unit[xi];
+    const unsigned long long v =
+        (((unsigned long long)hi << 32) | lo) + (unsigned)c[j] * unit + (ent[j] & kTabValue);
+    a[2 * j] = (uint32_t)v;
+    a[2 * j + 1] = (uint32_t)(v >> 32);
+    far |= x;
+    below |= xi << j;
+    left |= a[2 * j + 1] ^ hi;
+    last = max(last, ent[j]);
+  }
+  const bool bad = row_in && (far > 1u || last == kTabInvalid);
+  if (__any_sync(0xffffffffu, bad || (row_in && (left >> 20)))) {
+    if (__any_sync(0xffffffffu, bad)) {
+      tmem_ld_n<2 * kRound>(old, a);
+      tc::tmem_wait_ld();
+      tc::reg_fence(a);
+#pragma unroll
+      for (int j = 0; j < kRound; ++j) {
+        const double v = __dadd_rn(__hiloint2double((int)a[2 * j + 1], (int)a[2 * j]),
+                                   reinterpret_cast<const double *>(tab)[c[j]]);
+        a[2 * j] = (uint32_t)__double2loint(v);
+        a[2 * j + 1] = (uint32_t)__double2hiint(v);
+      }
+    } else {
+      // Sums that left their binade e: v counts (e << 52) + m - 2^52 with m in
+      // [2^53, 2^54) and becomes (e << 52) + RN(m / 2), m odd rounded by what
+      // the first rounding left.
+#pragma unroll
+      for (int j = 0; j < kRound; ++j) {
+        const uint32_t e = etop - ((below >> j) & 1u);
+        if ((a[2 * j + 1] >> 20) == e) continue;
+        const uint32_t lo = a[2 * j], hi = a[2 * j + 1] - (e << 20) + 0x00100000u;
+        const uint32_t rest = ent[j] >> kTabRestShift, half = __funnelshift_r(lo, hi, 1);
+        const uint32_t up = lo & 1u & (rest == 0u ? half : rest);
+        const unsigned long long h = (((unsigned long long)((hi >> 1) + (e << 20))) << 32 | half) + up;
+        a[2 * j] = (uint32_t)h;
+        a[2 * j + 1] = (uint32_t)(h >> 32);
+      }
     }
   }
 }
 
 template <int TYPE, bool GRP>
 __global__ void __launch_bounds__(kThreads, 1)
-    gram_tc_kernel(GramParams p, GramGroupDev grp, int tiles, const double *__restrict__ T, int *status) {
+    gram_tc_kernel(GramParams p, GramGroupDev grp, int tiles, const uint8_t *__restrict__ T, int *status) {
   extern __shared__ __align__(128) uint8_t dsm[];
   __shared__ Smem sm;
   // stages first, on a 1024-byte boundary (swizzle atoms)
   uint8_t *stages = dsm + ((1024 - (tc::smem_u32(dsm) & 1023)) & 1023);
   uint8_t *raw = stages + (size_t)kStages * kStageBytes;                       // [kRawSlots][kRawBytes]
-  double *sT = reinterpret_cast<double *>(raw + kRawSlots * (size_t)kRawBytes);  // [2][kTabStride]
-  int *s_cnt = reinterpret_cast<int *>(sT + 2 * kTabStride);                   // [2][256]
+  uint8_t *sT = raw + kRawSlots * (size_t)kRawBytes;                           // [2][kTabBytes]
+  int *s_cnt = reinterpret_cast<int *>(sT + 2 * kTabBytes);                    // [2][256]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile int *abort = &sm.abort;
@@ -484,6 +596,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int et = tid - (kProducers + 32);  // 0..kFold-1
     const int q = warp & 3;
     const int col0 = (et >> 7) * kFoldCols;   // this warp's columns of the tile
+    const int phase = et >> 7;
     const int row = 32 * q + lane;
     const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16);
     // The table T_b of the CTA's g-th block goes into buffer g & 1 by one
@@ -512,10 +625,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       } else {
         blk = boff % p.P;
       }
-      const double *src = T + ((GRP ? grp.blk0[in] : 0ll) + blk) * (long long)kTabStride;
+      const uint8_t *src = T + ((GRP ? grp.blk0[in] : 0ll) + blk) * (long long)kTabBytes;
       tc::fence_proxy_async();
       tc::mbar_arrive_expect_tx(&sm.tab_full[t], kTabBytes);
-      tc::bulk_g2s(sT + t * kTabStride, src, kTabBytes, &sm.tab_full[t]);
+      tc::bulk_g2s(sT + t * kTabBytes, src, kTabBytes, &sm.tab_full[t]);
       atomicAdd(&sm.tab_issued[t], 1u);
     };
     if (et == 0) {
@@ -528,6 +641,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     while (walk.next(p, grp, inst, tile_m, tile_n)) {
       const GramParams &pp = params_of<GRP>(p, grp, inst);
       const int P = pp.P;
+      int first, end;
+      live_rounds(pp, tile_m + 32 * q, tile_n + col0, first, end);
+      const bool row_in = tile_m + row < pp.nA;
       for (int b = 0; b < P; ++b) {
         const long long gbb = gb0 + b;
         const int t = (int)(gbb & 1);
@@ -536,7 +652,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         w = w && tc::mbar_wait(&sm.acc_full[t], (uint32_t)((gbb >> 1) & 1), abort, status, 7);
         ok = __all_sync(0xffffffffu, w);
         tc::fence_after_sync();
-        const double *Tb = sT + t * kTabStride;
+        const uint8_t *tab = sT + t * kTabBytes;
+        const double *Tb = reinterpret_cast<const double *>(tab);
+        const uint32_t etop = reinterpret_cast<const TabHdr *>(tab + kTabHdr)->etop;
         const int pa = s_cnt[t * 256 + row];
         const int *pzb = s_cnt + t * 256 + 128;
         // Rounds of kRound columns, software-pipelined: the TMEM loads of
@@ -548,51 +666,67 @@ __global__ void __launch_bounds__(kThreads, 1)
           tmem_ld_n<kRound>(lane_base + t * kCntCols + c0, cn[buf]);
           if (b > 0) tmem_ld_n<2 * kRound>(lane_base + kAccCol + 2 * c0, a[buf]);
         };
-        if (ok) {
-          load_round(0, 0);
-          tc::tmem_wait_ld();
-          tc::reg_fence(cn[0]);
-          tc::reg_fence(a[0]);
-        }
-#pragma unroll
-        for (int r = 0; r < kRounds; ++r) {
-          const int cur = r & 1, nxt = cur ^ 1;
-          const int c0 = col0 + r * kRound;
-          if (!ok) {
-#pragma unroll
-            for (int j = 0; j < kRound; ++j) cn[cur][j] = 0;
-          }
-          if (ok && r + 1 < kRounds) load_round(r + 1, nxt);
-          if (r == kRounds - 1) {
-            // all this warp's count columns of buffer t have been read
-            tc::fence_before_sync();
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&sm.acc_empty[t]);
-          }
-          // the four columns' Z row counts in one 16-byte load (c0 is a
-          // multiple of kRound = 4)
-          static_assert(kRound == 4, "one int4 of Z row counts per round");
-          const int4 pz4 = *reinterpret_cast<const int4 *>(pzb + c0);
-          const int pzr[4] = {pz4.x, pz4.y, pz4.z, pz4.w};
-#pragma unroll
-          for (int j = 0; j < kRound; ++j) {
-            const int n = decode_count(cn[cur][j]);
-            const int c = (TYPE == 1) ? pa + pzr[j] - 2 * n : n;
-            // 0 <= c <= 1920 for counts of a completed block; anything else
-            // (counts of an aborted pipeline) reads the NaN entry 1921
-            const double x = Tb[min((unsigned)c, (unsigned)(kTabStride - 1))];
-            const double v =
-                (b > 0) ? __dadd_rn(__hiloint2double((int)a[cur][2 * j + 1], (int)a[cur][2 * j]), x) : x;
-            a[cur][2 * j] = (uint32_t)__double2loint(v);
-            a[cur][2 * j + 1] = (uint32_t)__double2hiint(v);
-          }
-          // accumulators of columns c0 + j: TMEM columns kAccCol + 2 (c0 + j)
-          // (low word) and + 1 (high word)
-          if (ok) tmem_st_n<2 * kRound>(lane_base + kAccCol + 2 * c0, a[cur]);
-          if (ok && r + 1 < kRounds) {
+        if (first == end) {  // no results: no sums
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&sm.acc_empty[t]);
+        } else {
+          if (ok) {
+            load_round(0, 0);
             tc::tmem_wait_ld();
-            tc::reg_fence(cn[nxt]);
-            tc::reg_fence(a[nxt]);
+            tc::reg_fence(cn[0]);
+            tc::reg_fence(a[0]);
+          }
+#pragma unroll
+          for (int r = 0; r < kRounds; ++r) {
+            const int cur = r & 1, nxt = cur ^ 1;
+            const int c0 = col0 + r * kRound;
+            if (!ok) {
+#pragma unroll
+              for (int j = 0; j < kRound; ++j) cn[cur][j] = 0;
+            }
+            if (ok && r + 1 < kRounds) load_round(r + 1, nxt);
+            if (r == kRounds - 1) {
+              // all this warp's count columns of buffer t have been read
+              tc::fence_before_sync();
+              __syncwarp();
+              if (lane == 0) tc::mbar_arrive(&sm.acc_empty[t]);
+            }
+            // the four columns' Z row counts in one 16-byte load (c0 is a
+            // multiple of kRound = 4)
+            static_assert(kRound == 4, "one int4 of Z row counts per round");
+            const int4 pz4 = *reinterpret_cast<const int4 *>(pzb + c0);
+            const int pzr[4] = {pz4.x, pz4.y, pz4.z, pz4.w};
+            int c[kRound];
+#pragma unroll
+            for (int j = 0; j < kRound; ++j) {
+              const int n = decode_count(cn[cur][j]);
+              // 0 <= c <= 1920 for counts of a completed block; anything else
+              // (counts of an aborted pipeline) reads the NaN entry 1921
+              c[j] = (int)min((unsigned)((TYPE == 1) ? pa + pzr[j] - 2 * n : n), (unsigned)(kTabStride - 1));
+            }
+            // (not staggered between warps: both forms of every round in the
+            // code take 75 ms)
+            if (b > 0 && (r & 1)) {
+              if (ok) add_round(tab, etop, c, a[cur], lane_base + kAccCol + 2 * c0, row_in);
+            } else {
+#pragma unroll
+              for (int j = 0; j < kRound; ++j) {
+                const double x = Tb[c[j]];
+                const double v =
+                    (b > 0) ? __dadd_rn(__hiloint2double((int)a[cur][2 * j + 1], (int)a[cur][2 * j]), x) : x;
+                a[cur][2 * j] = (uint32_t)__double2loint(v);
+                a[cur][2 * j + 1] = (uint32_t)__double2hiint(v);
+              }
+            }
+            // accumulators of columns c0 + j: TMEM columns kAccCol + 2 (c0 + j)
+            // (low word) and + 1 (high word)
+            if (ok) tmem_st_n<2 * kRound>(lane_base + kAccCol + 2 * c0, a[cur]);
+            if (ok && r + 1 < kRounds) {
+              tc::tmem_wait_ld();
+              tc::reg_fence(cn[nxt]);
+              tc::reg_fence(a[nxt]);
+            }
           }
         }
         // this warp no longer reads T buffer t; the last of the fold warps
@@ -617,7 +751,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&sm.aux_empty[t]);
       }
-      if (ok) write_results<TYPE>(pp, tile_m, tile_n, col0, row, lane, lane_base + kAccCol + 2 * col0);
+      if (ok) write_results<TYPE>(pp, tile_m, tile_n, col0, row, lane, first, end, phase, lane_base + kAccCol + 2 * col0);
       gb0 += P;
       ++jt;
     }
@@ -641,22 +775,119 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-__device__ __forceinline__ void write_table_row(double d, double *__restrict__ row) {
-  for (int c = threadIdx.x; c < kTabStride; c += blockDim.x)
-    row[c] = c < kTabStride - 1 ? __dmul_rn(d, (double)c) : __longlong_as_double(0x7ff8dead00000000ll);
+// The table of block b of Gram p, shared out over kTableParts CTAs of 256
+// threads (each makes the same estimate).
+constexpr int kTableParts = 4;
+__device__ void write_block_table(const GramParams &p, int b, uint8_t *__restrict__ tab) {
+  __shared__ double s_sum[8];
+  __shared__ int s_diff[8], s_all[8];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const double D = p.D ? p.D[b] : 1.0;
+  double *prod = reinterpret_cast<double *>(tab);
+  if (b == 0) {  // the first block's products are the sums: no integer entries
+    for (int c = tid + blockDim.x * blockIdx.y; c < kTabStride; c += blockDim.x * kTableParts)
+      prod[c] = c < kTabStride - 1 ? __dmul_rn(D, (double)c) : __longlong_as_double(0x7ff8dead00000000ll);
+    return;
+  }
+  // Expected sums before this block: the earlier blocks' weighted mask counts,
+  // times the share of differing (TYPE_pm) or common (TYPE_00) bits of four
+  // row pairs in this block (first A rows against last Z rows).
+  double sum = 0.0;
+  for (int i = tid; i < b; i += blockDim.x) {
+    const uint4 *m = reinterpret_cast<const uint4 *>(p.mask + (long long)i * kBlockRow);
+    int n = 0;
+    for (int v = 0; v < kBlockRow / 16; ++v) n += popc4(__ldg(m + v));
+    sum = __dadd_rn(sum, __dmul_rn(p.D ? p.D[i] : 1.0, (double)n));
+  }
+  int diff = 0, all = 0;
+  if (tid < 4 * (kBlockRow / 4)) {
+    const int pair = tid / (kBlockRow / 4), w = tid % (kBlockRow / 4);
+    const long long off = (long long)b * kBlockRow + 4 * w;
+    const uint32_t m = __ldg(reinterpret_cast<const uint32_t *>(p.mask + off));
+    const uint32_t ai = p.a_rowb[min(pair, p.nA - 1)], zi = p.z_rowb[max(p.nZ - 1 - pair, 0)];
+    const uint32_t x = __ldg(reinterpret_cast<const uint32_t *>(p.wA + (long long)ai * p.a_row_bytes + off));
+    const uint32_t z = __ldg(reinterpret_cast<const uint32_t *>(p.wZ + (long long)zi * p.z_row_bytes + off));
+    diff = __popc((p.type == 1 ? x ^ z : x & z) & m);
+    all = __popc(m);
+  }
+  diff = __reduce_add_sync(0xffffffffu, diff);
+  all = __reduce_add_sync(0xffffffffu, all);
+  if (32 * warp < b)
+    for (int o = 16; o > 0; o >>= 1) sum = __dadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, o));
+  if (lane == 0) {
+    s_sum[warp] = sum;
+    s_diff[warp] = diff;
+    s_all[warp] = all;
+  }
+  __syncthreads();
+  sum = s_sum[0];
+  diff = all = 0;
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+    if (w && 32 * w < b) sum = __dadd_rn(sum, s_sum[w]);
+    diff += s_diff[w];
+    all += s_all[w];
+  }
+  const double share = (diff > 0 && all > 0) ? (double)diff / (double)all : 0.25;
+  // two exponents: the expected sum's, and the one above where its mantissa
+  // is above about sqrt(2), else the one below
+  const uint32_t est = (uint32_t)__double2hiint(__dmul_rn(sum, share));
+  const int etop = (int)((est >> 20) & 0x7ff) + ((est & 0xFFFFF) > 0x6A000 ? 1 : 0);
+
+  const unsigned long long db = (unsigned long long)__double_as_longlong(D);
+  const int ed = (int)((db >> 52) & 0x7ff);
+  const unsigned long long dm = (db & 0x000fffffffffffffull) | 0x0010000000000000ull;
+  const bool ok_d = !(db >> 63) && ed >= 64 && ed <= 1900;
+  for (int c = tid + blockDim.x * blockIdx.y; c < kTabStride; c += blockDim.x * kTableParts) {
+    const double x = c < kTabStride - 1 ? __dmul_rn(D, (double)c) : __longlong_as_double(0x7ff8dead00000000ll);
+    prod[c] = x;
+    const unsigned long long xb = (unsigned long long)__double_as_longlong(x);
+    const int ex = (int)((xb >> 52) & 0x7ff);
+    const unsigned long long xm = (xb & 0x000fffffffffffffull) | 0x0010000000000000ull;
+    for (int j = 0; j < kTabExps; ++j) {
+      const int e = etop - j, k = e - ed, sh = e - ex;
+      uint32_t entry = kTabInvalid | kTabInvalid << 16;
+      if (ok_d && k >= 0 && k <= 52 && e >= 64 && e <= 2000 && c < kTabStride - 1) {
+        if (c == 0) {
+          entry = 0u;
+        } else if (sh >= 0) {
+          // floor(x / ulp) and its fraction: 0, below, at, above one half
+          unsigned long long f = 0ull;
+          uint32_t code = 1u;
+          if (sh <= 60) {
+            f = xm >> sh;
+            const unsigned long long rem = xm & ((1ull << sh) - 1ull), half = (1ull << sh) >> 1;
+            code = rem == 0ull ? 0u : rem < half ? 1u : rem == half ? 2u : 3u;
+          }
+          const uint32_t d = (uint32_t)(f - (unsigned long long)c * (dm >> k));  // at most c
+          entry = 0u;
+          for (uint32_t odd = 0; odd < 2; ++odd) {
+            const uint32_t up = (code + (((uint32_t)f ^ odd) & 1u) + 1u) >> 2;
+            entry |= (d + up | (code == 0u ? 0u : up ? 2u : 1u) << kTabRestShift) << (16 * odd);
+          }
+        }
+      }
+      reinterpret_cast<uint32_t *>(tab + kTabInt + j * kTabExpBytes)[c] = entry;
+    }
+  }
+  if (tid == 0 && blockIdx.y == 0) {
+    TabHdr *h = reinterpret_cast<TabHdr *>(tab + kTabHdr);
+    for (int j = 0; j < kTabExps; ++j) {
+      const int k = etop - j - ed;
+      h->unit[j] = k >= 0 && k <= 52 ? dm >> k : 0ull;
+    }
+    h->etop = (uint32_t)etop;
+  }
 }
 
-__global__ void gram_table_kernel(const double *__restrict__ D, int P, double *__restrict__ T) {
-  const int b = blockIdx.x;
-  write_table_row(D ? D[b] : 1.0, T + (size_t)b * kTabStride);
+__global__ void __launch_bounds__(256) gram_table_kernel(GramParams p, uint8_t *__restrict__ T) {
+  write_block_table(p, blockIdx.x, T + (size_t)blockIdx.x * kTabBytes);
 }
 
 // Table rows of a grouped launch: row r is block r - blk0[i] of instance i.
-__global__ void gram_table_group_kernel(GramGroupDev g, double *__restrict__ T) {
+__global__ void __launch_bounds__(256) gram_table_group_kernel(GramGroupDev g, uint8_t *__restrict__ T) {
   const long long r = blockIdx.x;
   const int in = find_instance(g.blk0, g.n, r);
-  const double *D = g.ps[in].D;
-  write_table_row(D ? D[r - g.blk0[in]] : 1.0, T + (size_t)r * kTabStride);
+  write_block_table(g.ps[in], (int)(r - g.blk0[in]), T + (size_t)r * kTabBytes);
 }
 
 int sm_count() {
@@ -689,7 +920,7 @@ void configure_tc() {
 }
 
 template <int TYPE>
-void launch_tc_type(const GramParams &p, const double *T, cudaStream_t s) {
+void launch_tc_type(const GramParams &p, const uint8_t *T, cudaStream_t s) {
   configure_tc<TYPE, false>();
   const int tiles = active_tiles(p), grid = std::max(1, std::min(tiles, sm_count()));
   gram_tc_kernel<TYPE, false><<<grid, kThreads, kSmemBytes, s>>>(p, GramGroupDev{}, tiles, T, tc_status_device_ptr());
@@ -698,7 +929,7 @@ void launch_tc_type(const GramParams &p, const double *T, cudaStream_t s) {
 }
 
 template <int TYPE>
-void launch_tc_group_type(const GramGroupDev &g, int total_tiles, const double *T, cudaStream_t s) {
+void launch_tc_group_type(const GramGroupDev &g, int total_tiles, const uint8_t *T, cudaStream_t s) {
   configure_tc<TYPE, true>();
   const int grid = std::max(1, std::min(total_tiles, sm_count()));
   gram_tc_kernel<TYPE, true><<<grid, kThreads, kSmemBytes, s>>>(GramParams{}, g, total_tiles, T, tc_status_device_ptr());
@@ -709,9 +940,9 @@ void launch_tc_group_type(const GramGroupDev &g, int total_tiles, const double *
 }  // namespace
 
 void launch_gram_tc(const GramParams &p, cudaStream_t s) {
-  double *T = nullptr;
+  uint8_t *T = nullptr;
   LAKGB_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&T), (size_t)p.P * kTabBytes, s));
-  gram_table_kernel<<<p.P, 256, 0, s>>>(p.D, p.P, T);
+  gram_table_kernel<<<dim3(p.P, kTableParts), 256, 0, s>>>(p, T);
   LAKGB_CUDA(cudaGetLastError());
   count_launch();
   if (p.type == 1)
@@ -725,16 +956,17 @@ int gram_tc_tiles(const GramParams &p) { return active_tiles(p); }
 
 size_t gram_tc_table_row_bytes() { return (size_t)kTabBytes; }
 
-void launch_gram_tc_group(const GramGroupDev &g, int type, int total_tiles, long long total_blocks, double *T,
+void launch_gram_tc_group(const GramGroupDev &g, int type, int total_tiles, long long total_blocks, void *T,
                           cudaStream_t s) {
+  uint8_t *tab = static_cast<uint8_t *>(T);
   if (total_tiles <= 0 || total_blocks <= 0) return;
-  gram_table_group_kernel<<<(unsigned)total_blocks, 256, 0, s>>>(g, T);
+  gram_table_group_kernel<<<dim3((unsigned)total_blocks, kTableParts), 256, 0, s>>>(g, tab);
   LAKGB_CUDA(cudaGetLastError());
   count_launch();
   if (type == 1)
-    launch_tc_group_type<1>(g, total_tiles, T, s);
+    launch_tc_group_type<1>(g, total_tiles, tab, s);
   else
-    launch_tc_group_type<2>(g, total_tiles, T, s);
+    launch_tc_group_type<2>(g, total_tiles, tab, s);
 }
 
 // The status word of the calling host thread's launches: every thread (a
