@@ -318,33 +318,49 @@ struct AnZtSnFinish {
 };
 
 // The sum over the planes in FP64 would be a chain of 2 B operations of 80
-// cycles each (16.5 us a call at 2018 rows, 33 planes).
-__global__ void __launch_bounds__(128) an_ztsn_finish_kernel(AnZtSnFinish p) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, s = blockIdx.y;
-  if (i >= p.n) return;
-  auto pm0 = [&](int k) {
-    long long pos = 0, all = 0;
-    const uint16_t *c = p.cnt + (size_t)k * p.n + i, *z = p.zcnt + k;
-    for (int b = 0; b < p.P; ++b) {
-      pos += c[(size_t)b * p.nplanes * p.n];
-      all += z[(size_t)b * p.nplanes];
-    }
-    return 2ll * pos - all;
-  };
-  const double base = __dmul_rn(__dmul_rn((double)pm0(0), p.min_d), p.mlt_d);
-  double tmp = 0.0;
-  if (p.exact) {
-    long long t = 0;
+// cycles each (16.5 us a call at 2018 rows, 33 planes), and one thread per row
+// reading its counts plane after plane is a chain of loads (33 us at 4000 rows,
+// 33 planes, several blocks).  So a warp's lanes are 32 rows and its CTA's eight
+// warps share their planes out; one warp adds the planes up, in order.
+constexpr int kFinishRows = 32, kFinishPlanes = 64, kFinishWarps = 8;
+__global__ void __launch_bounds__(32 * kFinishWarps) an_ztsn_finish_kernel(AnZtSnFinish p) {
+  __shared__ long long pm[kFinishPlanes][kFinishRows];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = blockIdx.y;
+  const int row = blockIdx.x * kFinishRows + lane, i = min(row, p.n - 1);
+  double base = 0.0, tmp = 0.0, n2 = 1.0;
+  long long t = 0;
+  // plane j of the sum: the mask plane, then the value planes from the lowest
+  // bit up
+  for (int j0 = 0; j0 < p.ncols_per; j0 += kFinishPlanes) {
+    const int j1 = min(j0 + kFinishPlanes, p.ncols_per);
+    for (int j = j0 + warp; j < j1; j += kFinishWarps) {
+      const int k = j ? p.ncols_per * s + p.ncols_per - j : 0;
+      const uint16_t *c = p.cnt + (size_t)k * p.n + i, *z = p.zcnt + k;
+      long long pos = 0, all = 0;
 #pragma unroll 4
-    for (int k = 0; k < p.ncols_per - 1; ++k) t += pm0(p.ncols_per * s + p.ncols_per - 1 - k) << k;
-    tmp = (double)t;
-  } else {
-    double n2 = 1.0;
-    for (int mx = p.ncols_per - 1; mx > 0; --mx) {
-      tmp = __dadd_rn(tmp, __dmul_rn(n2, (double)pm0(p.ncols_per * s + mx)));
-      n2 *= 2.0;
+      for (int b = 0; b < p.P; ++b) {
+        pos += c[(size_t)b * p.nplanes * p.n];
+        all += z[(size_t)b * p.nplanes];
+      }
+      pm[j - j0][lane] = 2ll * pos - all;
     }
+    __syncthreads();
+    if (warp == 0) {
+      int j = j0;
+      if (j == 0) base = __dmul_rn(__dmul_rn((double)pm[j++][lane], p.min_d), p.mlt_d);
+      if (p.exact) {
+        for (; j < j1; ++j) t += pm[j - j0][lane] << (j - 1);
+      } else {
+        for (; j < j1; ++j) {
+          tmp = __dadd_rn(tmp, __dmul_rn(n2, (double)pm[j - j0][lane]));
+          n2 *= 2.0;
+        }
+      }
+    }
+    __syncthreads();
   }
+  if (warp != 0 || row >= p.n) return;
+  if (p.exact) tmp = (double)t;
   p.out[p.out_r[i] + p.s_off[s]] = __ddiv_rn(__dadd_rn(base, tmp), p.mlt_d);
 }
 
@@ -882,7 +898,7 @@ extern "C" int wrap_An_ZtSn_ww__run(int *tidx, void **vpra, pthread_t *thread_in
     p.min_d = M_ZtSn->min_d; p.mlt_d = M_ZtSn->mlt_d;
     p.out_r = d_or.as<unsigned long long>() + r0; p.s_off = d_so.as<unsigned long long>();
     p.out = d_out.as<double>();
-    an_ztsn_finish_kernel<<<dim3((g.nA + 127) / 128, nS), 128, 0, stream()>>>(p);
+    an_ztsn_finish_kernel<<<dim3((g.nA + kFinishRows - 1) / kFinishRows, nS), 32 * kFinishWarps, 0, stream()>>>(p);
     LAKGB_CUDA(cudaGetLastError());
     count_launch();
   }

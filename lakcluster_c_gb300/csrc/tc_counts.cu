@@ -23,6 +23,7 @@
 // (tc_ptx.cuh); a pipeline error is recorded in the tensor-core status word.
 #include <algorithm>
 
+#include "fixed_fp64.cuh"
 #include "gram.cuh"
 #include "lakgb_runtime.cuh"
 #include "tc_counts.cuh"
@@ -116,10 +117,12 @@ struct Tile {
 
   // Count block b: the accumulators become (first) or gain its counts, the row
   // counts likewise.  On return the MMAs may still run.
+  // ROWS: tile rows in use (kM and some Z rows).
+  template <int ROWS>
   __device__ __forceinline__ void block(const TileRows &t, int b, bool first, bool more_before, int *status) {
     const int tid = threadIdx.x;
     const long long boff = (long long)b * kRow;
-    for (int i = tid; i < kRows * kChunks; i += kThreads) {
+    for (int i = tid; i < ROWS * kChunks; i += kThreads) {
       const int r = i / kChunks, v = i - r * kChunks;
       const long long o = off[r];
       if (o >= 0) tc::cp_async16(raw + r * kRow + 16 * v, (r < kM ? t.wA : t.wZ) + o + boff + 16 * v);
@@ -134,8 +137,8 @@ struct Tile {
     const uint32_t st = tc::smem_u32(stage), rw = tc::smem_u32(raw), mk = tc::smem_u32(mask), xr = tc::smem_u32(xrow);
     for (int g = 0; g < kChunks / kGroup; ++g) {
       if (g > 0 || more_before) wait_mma(status);
-      for (int i = tid; i < kRows * kGroup; i += kThreads) {
-        const int u = i / kRows, r = i - u * kRows, ch = g * kGroup + u;
+      for (int i = tid; i < ROWS * kGroup; i += kThreads) {
+        const int u = i / ROWS, r = i - u * ROWS, ch = g * kGroup + u;
         uint4 x = tc::ld_shared_v4(rw + r * kRow + 16 * ch);
         const uint32_t dst = st + u * kChunkBytes;
         if (r < kM) {
@@ -167,7 +170,7 @@ struct Tile {
       ++phase;
     }
     // the row counts, while the last group's MMAs run
-    if (tid < kRows) {
+    if (tid < ROWS) {
       int c = 0;
 #pragma unroll 5
       for (int ch = 0; ch < kChunks; ++ch) {
@@ -184,10 +187,13 @@ struct Tile {
     __syncthreads();  // the raw rows have been read
   }
 
-  // This warp's 32 columns of the accumulators (the lane's row).
-  __device__ __forceinline__ void read(uint32_t (&v)[32]) {
+  // This warp's NC columns of the accumulators (the lane's row).
+  template <int NC>
+  __device__ __forceinline__ void read(uint32_t (&v)[NC]) {
     const int warp = threadIdx.x >> 5;
-    tc::tmem_ld32(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 32 * (warp >> 2), v);
+    const uint32_t at = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + NC * (warp >> 2);
+    if constexpr (NC == 32) tc::tmem_ld32(at, v);
+    else tc::tmem_ld8(at, v);
     tc::tmem_wait_ld();
     tc::reg_fence(v);
   }
@@ -219,7 +225,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   const TileRows t{p.wA, p.a_rowb, p.nA, p.a_row_bytes, p.wZ, p.z_rowb, p.nZ, p.z_row_bytes, p.mask, nullptr};
   Tile tile;
   tile.setup(&sm, dsm, t, m0, n0);
-  tile.block(t, b, true, false, status);
+  tile.block<kRows>(t, b, true, false, status);
   tile.wait_mma(status);
   if (zcnt && m0 == 0 && threadIdx.x < kN && n0 + (int)threadIdx.x < p.nZ)
     zcnt[(size_t)b * p.nZ + n0 + threadIdx.x] = (uint16_t)tile.cnt[kM + threadIdx.x];
@@ -265,81 +271,101 @@ __global__ void __launch_bounds__(256) gram_fold_kernel(GramParams p, const uint
         acc = __dadd_rn(acc, x);
       }
     }
-    double o = TYPE == 1 ? __dsub_rn(p.a0d1, __dmul_rn(2.0, acc)) : acc;
+    double o = acc;
+    if (TYPE == 1)
+      o = __dsub_rn(p.a0d1, __longlong_as_double((long long)fixed::twice_bits((unsigned long long)__double_as_longlong(acc))));
     if (p.lfA && p.lfZ) o = __dsub_rn(o, __dsub_rn(__dadd_rn(p.lfA[ga], p.lfZ[gz]), p.a2d1));
     p.out[(long long)p.out_r[ga] + (long long)p.out_c[gz] * p.out_stride] = o;
     if (p.symmetric) p.out[(long long)p.out_r2[gz] + (long long)p.out_c2[ga] * p.out_stride] = o;
   }
 }
 
+// v as a double (the conversion is an instruction of the FP64 pipe).
+__device__ __forceinline__ double int_to_double(int v) {
+  const uint32_t n = v < 0 ? 0u - (uint32_t)v : (uint32_t)v;
+  const int z = __clz((int)n);
+  const uint32_t m = n << (z & 31);
+  const uint32_t hi = ((uint32_t)v & 0x80000000u) | (((uint32_t)(1053 - z) << 20) + (m >> 11));
+  return n ? __hiloint2double((int)hi, (int)(m << 21)) : 0.0;
+}
+
 // out = ((hhAY - hhAy aY) - aA hhaY) + (aA hhay) aY.  A thread holds one At row
-// and 32 Yt rows: the products with aY are formed again only where aY changes
-// (once per 1920 SNPs), and aA hhaY of the 32 Yt rows one per lane where the
-// warp's rows share aA, so an element costs three FP64 operations instead of
-// seven.
+// and NC Yt rows: where a warp's rows share aA and its columns share aY (both
+// change once per 1920 SNPs) the products with aY are formed once and aA hhaY
+// of the NC Yt rows one per lane, so an element costs three FP64 operations
+// instead of seven.  Those bound a CTA's time (80 cycles a warp each), so a
+// product of few tiles takes NC = 8: four times as many CTAs with a quarter of
+// the elements each.
+template <int NC>
 __global__ void __launch_bounds__(kThreads, 2) attyn_tc_kernel(AtTYnParams p, int *status) {
   extern __shared__ __align__(128) uint8_t dsm[];
   __shared__ Smem sm;
-  const int m0 = blockIdx.y * kM, n0 = blockIdx.x * kN, t = blockIdx.z;
-  if (p.symmetric && m0 > n0 + kN - 1) return;
-  const TileRows rows{p.At, p.a_rowb, p.nA, p.a_row_bytes, p.Yt, p.y_rowb, p.nY, p.y_row_bytes, p.mask,
+  const int m0 = blockIdx.y * kM, n0 = blockIdx.x * 2 * NC, t = blockIdx.z;
+  if (p.symmetric && m0 > n0 + 2 * NC - 1) return;
+  const TileRows rows{p.At, p.a_rowb, p.nA, p.a_row_bytes, p.Yt, p.y_rowb, min(p.nY, n0 + 2 * NC), p.y_row_bytes, p.mask,
                       p.Tt + (long long)p.t_rowb[t] * p.t_row_bytes};
   Tile tile;
   tile.setup(&sm, dsm, rows, m0, n0);
-  int n[32];
+  int n[NC];
 #pragma unroll
-  for (int j = 0; j < 32; ++j) n[j] = 0;
+  for (int j = 0; j < NC; ++j) n[j] = 0;
   // kExactBlocks blocks at a time: their counts stay below 2^24
   for (int b0 = 0; b0 < p.P; b0 += kExactBlocks) {
-    for (int b = b0; b < min(p.P, b0 + kExactBlocks); ++b) tile.block(rows, b, b == b0, b > b0, status);
+    for (int b = b0; b < min(p.P, b0 + kExactBlocks); ++b) tile.block<kM + 2 * NC>(rows, b, b == b0, b > b0, status);
     tile.wait_mma(status);
     if (tile.ok) {
-      uint32_t v[32];
+      uint32_t v[NC];
       tile.read(v);
 #pragma unroll
-      for (int j = 0; j < 32; ++j) n[j] += decode_count(v[j]);
+      for (int j = 0; j < NC; ++j) n[j] += decode_count(v[j]);
     }
     tc::fence_before_sync();
     __syncthreads();  // read before the next blocks' MMAs overwrite them
   }
   if (tile.ok) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row = 32 * (warp & 3) + lane, c0 = 32 * (warp >> 2), na = m0 + row;
+    const int row = 32 * (warp & 3) + lane, c0 = NC * (warp >> 2), na = m0 + row;
     const bool live = na < p.nA;
-    const int nac = live ? na : p.nA - 1;  // every lane takes part in the shuffles
+    const int nac = live ? na : p.nA - 1;  // every lane takes part in the votes
     const double aA = p.aA[nac], hhAy = p.hhAy[(long long)t * p.nA + nac];
     const double aAh = __dmul_rn(aA, p.hhay[t]);
     const unsigned long long oa = p.out_a[nac] + p.out_t[t];
     const long long base = 2ll * tile.cnt[row] - p.cpop;
-    const bool shared_a = __all_sync(0xffffffffu, __double_as_longlong(aA) ==
-                                                      __shfl_sync(0xffffffffu, __double_as_longlong(aA), 0));
-    // this warp's 32 Yt rows, in the operand tiles' shared memory (the MMAs
-    // have read them): hhaY, aY and aA hhaY
+    // this warp's Yt rows, one per lane, in the operand tiles' shared memory
+    // (the MMAs have read them): hhaY, aY and aA hhaY
     double *y = reinterpret_cast<double *>(tile.stage) + 96 * warp;
-    const int nyl = min(n0 + c0 + lane, p.nY - 1);
-    y[lane] = p.hhaY[(long long)t * p.nY + nyl];
-    y[32 + lane] = p.aY[nyl];
-    y[64 + lane] = __dmul_rn(aA, y[lane]);
+    const int nyl = min(n0 + c0 + min(lane, NC - 1), p.nY - 1);
+    const double aYl = p.aY[nyl], hhaYl = p.hhaY[(long long)t * p.nY + nyl];
+    y[lane] = hhaYl;
+    y[32 + lane] = aYl;
+    y[64 + lane] = __dmul_rn(aA, hhaYl);
     __syncwarp();
-    double q1 = 0.0, q3 = 0.0;
-    long long prev = 0;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
+    const long long aA0 = __shfl_sync(0xffffffffu, __double_as_longlong(aA), 0);
+    const long long aY0 = __shfl_sync(0xffffffffu, __double_as_longlong(aYl), 0);
+    // (counts below 2^30 for the conversion)
+    const bool shared = __all_sync(0xffffffffu, __double_as_longlong(aA) == aA0 && __double_as_longlong(aYl) == aY0) &&
+                        p.P < (1 << 30) / (2 * kBlockBits);
+    auto store = [&](int j, double o) {
       const int ny = n0 + c0 + j;
-      const double aY = y[32 + j];
-      if (j == 0 || __double_as_longlong(aY) != prev) {  // the same for the whole warp
-        q1 = __dmul_rn(hhAy, aY);
-        q3 = __dmul_rn(aAh, aY);
-        prev = __double_as_longlong(aY);
-      }
-      double q2 = y[64 + j];
-      if (!shared_a) q2 = __dmul_rn(aA, y[j]);
-      // 2 (pa + py - 2 n) - cpop
-      const double hhAY = (double)(base + 2ll * tile.cnt[kM + c0 + j] - 4ll * n[j]);
-      const double o = __dadd_rn(__dsub_rn(__dsub_rn(hhAY, q1), q2), q3);
       if (live && ny < p.nY && !(p.symmetric && na > ny)) {
         p.out[oa + p.out_y[ny]] = o;
         if (p.symmetric) p.out[p.out_a2[ny] + p.out_y2[na] + p.out_t[t]] = o;
+      }
+    };
+    // hhAY = 2 (pa + py - 2 n) - cpop
+    if (shared) {
+      const double q1 = __dmul_rn(hhAy, aYl), q3 = __dmul_rn(aAh, aYl);
+#pragma unroll
+      for (int j = 0; j < NC; ++j) {
+        const double hhAY = int_to_double((int)base + 2 * tile.cnt[kM + c0 + j] - 4 * n[j]);
+        store(j, __dadd_rn(__dsub_rn(__dsub_rn(hhAY, q1), y[64 + j]), q3));
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < NC; ++j) {
+        const volatile double *yj = y + j;  // read here: no FP64 operation above the branch
+        const double aY = yj[32], hhAY = (double)(base + 2ll * tile.cnt[kM + c0 + j] - 4ll * n[j]);
+        store(j, __dadd_rn(__dsub_rn(__dsub_rn(hhAY, __dmul_rn(hhAy, aY)), __dmul_rn(aA, yj[0])), __dmul_rn(aAh, aY)));
       }
     }
   }
@@ -387,16 +413,29 @@ void launch_and_counts_tc(const GramParams &p, uint16_t *cnt, uint16_t *zcnt, cu
   launch_counts<2>(p, cnt, zcnt, s);
 }
 
-void launch_attyn_tc(const AtTYnParams &p, int nT, cudaStream_t s) {
+namespace {
+template <int NC>
+void launch_attyn(const AtTYnParams &p, int nT, cudaStream_t s) {
   static const bool configured = [] {
-    allow_smem(attyn_tc_kernel);
+    allow_smem(attyn_tc_kernel<NC>);
     return true;
   }();
   (void)configured;
-  const dim3 grid((p.nY + kN - 1) / kN, (p.nA + kM - 1) / kM, nT);
-  attyn_tc_kernel<<<grid, kThreads, kSmemBytes, s>>>(p, tc_status_device_ptr());
+  const dim3 grid((p.nY + 2 * NC - 1) / (2 * NC), (p.nA + kM - 1) / kM, nT);
+  attyn_tc_kernel<NC><<<grid, kThreads, kSmemBytes, s>>>(p, tc_status_device_ptr());
   LAKGB_CUDA(cudaGetLastError());
   count_launch();
+}
+}  // namespace
+
+void launch_attyn_tc(const AtTYnParams &p, int nT, cudaStream_t s) {
+  // Narrow tiles while all of them still fit the 304 places at once; above,
+  // expanding the A rows four times would cost more than it gains.
+  const long long tiles = (long long)((p.nY + kN - 1) / kN) * ((p.nA + kM - 1) / kM) * nT;
+  if (4 * tiles <= 304)
+    launch_attyn<8>(p, nT, s);
+  else
+    launch_attyn<32>(p, nT, s);
 }
 
 }  // namespace lakgb
