@@ -32,6 +32,11 @@ int gram_entry(bool symmetric, int type_flag, int spacing_r, int spacing_c, M_ha
   const unsigned long long length_r = spacing_length(spacing_r, M_An);
   const unsigned long long length_c = spacing_length(spacing_c, M_Zn);
   const unsigned long long length = length_r * length_c;
+  // The Gram writes every element where every row and column of the output is
+  // retained; otherwise the rest is zero.
+  const bool all = type_flag != LAKGB_TYPE_p0 && M_An->mc_length >= kBlockBytes &&
+                   (unsigned long long)M_An->rpop_j * (unsigned long long)M_Zn->rpop_j == length &&
+                   (!symmetric || M_An == M_Zn);
   // A mirrored output (lmirror.cu) is produced on the device only.
   Mirror *mo = *out_p ? find_mirror(*out_p) : nullptr;
   L_handle *out = nullptr;
@@ -42,7 +47,7 @@ int gram_entry(bool symmetric, int type_flag, int spacing_r, int spacing_c, M_ha
       set_error(2, "output length %llu < %llu in %s", out->length, length, who);
       return (int)length;
     }
-    if (length) LAKGB_CUDA(cudaMemsetAsync(mo->d, 0, length * sizeof(double), stream()));
+    if (length && !all) LAKGB_CUDA(cudaMemsetAsync(mo->d, 0, length * sizeof(double), stream()));
     mo->host_stale = true;
   } else {
     out = ensure_output(out_p, length, who, false);
@@ -103,7 +108,7 @@ int gram_entry(bool symmetric, int type_flag, int spacing_r, int spacing_c, M_ha
     dout = mo->d;
   } else {
     d_out = DBuf(length * sizeof(double));
-    d_out.zero();
+    if (!all) d_out.zero();
     dout = d_out.as<double>();
   }
 
@@ -205,7 +210,7 @@ extern "C" int wrap_An_v__run(int *tidx, void **vpra, pthread_t *thread_in, int 
   DBuf d_rows = upload_bytes(M_An->m_b_, (size_t)n * sizeof(uint32_t)), d_outr = upload_vec(spacing_index(output_spacing_r, M_An));
   st.flush();
   DBuf d_out(length * sizeof(double));
-  d_out.zero();
+  if ((unsigned long long)n != length) d_out.zero();
   RowvecParams p{};
   p.w = (const uint8_t *)w; p.rowb = d_rows.as<uint32_t>(); p.n = n; p.row_bytes = (long long)M_An->mc_length;
   p.mask = mask.as<uint8_t>(); p.P = P; p.type = (type_flag == LAKGB_TYPE_pm) ? 1 : 2;
@@ -246,7 +251,7 @@ extern "C" int wrap_An_ajdk_v(int *tidx, void **vpra, pthread_t *thread_in, int 
   DBuf d_ajdk = upload_bytes(A_ajdk, (size_t)P * LAKGB_AJDK_TOT * sizeof(double));
   DBuf d_base = upload_bytes(base, sizeof(base));
   DBuf d_out(length * sizeof(double));
-  d_out.zero();
+  if ((unsigned long long)n != length_r) d_out.zero();
   RowvecParams p{};
   p.w = (const uint8_t *)w; p.rowb = d_rows.as<uint32_t>(); p.n = n; p.row_bytes = (long long)M_An->mc_length;
   p.mask = mask.as<uint8_t>(); p.P = P; p.type = (type_flag == LAKGB_TYPE_pm) ? 1 : 2;

@@ -789,7 +789,8 @@ extern "C" int wrap_At_T_YnWt_S_Zn_ww__run(int *tidx, void **vpra, pthread_t *th
     d_zz = DBuf((size_t)npairs * sizeof(double2));
   }
   DBuf d_out(length * sizeof(double));
-  d_out.zero();
+  // the kernels write every pair and covariate column
+  if (nW == 0 || (unsigned long long)npairs * nT != length) d_out.zero();
   p.ycnt = d_ycnt.as<int>(); p.T_base = d_Tb.as<double>(); p.T_tmp = d_Tt.as<double>();
   p.At_base = d_Ab.as<double>(); p.zz = d_zz.as<double2>();
   p.ysum = d_ys.as<long long>(); p.q2 = d_q2.as<double>();
@@ -883,7 +884,7 @@ extern "C" int wrap_An_ZtSn_ww__run(int *tidx, void **vpra, pthread_t *thread_in
   const int range = (int)std::min<long long>(n, std::max<long long>(128, (long long)(kAnZtSnScratch / std::max<size_t>(per_row, 1)) / 128 * 128));
   DBuf d_cnt((size_t)range * per_row), d_zcnt(per_row);
   DBuf d_out(length * sizeof(double));
-  d_out.zero();
+  if ((unsigned long long)n * nS != length) d_out.zero();
   st.flush();
   for (int r0 = 0; r0 < n; r0 += range) {
     GramParams g{};

@@ -316,7 +316,7 @@ extern "C" int wrap_AnZt_S_WnYt_vv__run(int *tidx, void **vpra, pthread_t *threa
   DBuf d_vS = up(vS), d_or = up(out_r), d_so = up(s_off);
   if (defer) defer_flush();
   DBuf d_out(length * sizeof(double));
-  d_out.zero();
+  if ((unsigned long long)nA * nS != length) d_out.zero();
   SwnytCall c{};
   c.A = pA; c.a_r = d_ar.as<unsigned long long>(); c.a_c = d_ac.as<unsigned long long>();
   c.Y = pY; c.y_r = d_yr.as<unsigned long long>(); c.y_c = d_yc.as<unsigned long long>();
@@ -460,7 +460,7 @@ extern "C" int wrap_AtTYn____WtSZn_vv__run(int *tidx, void **vpra, pthread_t *th
   DBuf d_D = up(Dy), d_or = up(out_r), d_so = up(s_off);
   if (defer) defer_flush();
   DBuf d_out(length * sizeof(double));
-  d_out.zero();
+  if ((unsigned long long)npairs * nS != length) d_out.zero();
   WtszCall c{};
   c.AY = pA; c.ay_a = d_aa.as<unsigned long long>(); c.ay_y = d_ay.as<unsigned long long>();
   c.ay_s = d_as.as<unsigned long long>();
@@ -496,6 +496,9 @@ int attyn_entry(bool symmetric, const char *who, int output_spacing_a, int outpu
   const unsigned long long ly = spacing_length(output_spacing_y, M_Yt);
   const unsigned long long lt = spacing_length(output_spacing_t, M_Tt);
   const unsigned long long length = la * ly * lt;
+  // every element is written where all rows are retained; otherwise the rest is zero
+  const bool all = (unsigned long long)M_At->rpop_j * (unsigned long long)M_Yt->rpop_j * (unsigned long long)M_Tt->rpop_j == length &&
+                   M_Yt->mc_length == M_At->mc_length && M_Tt->mc_length == M_At->mc_length && (!symmetric || M_At == M_Yt);
   // A mirrored output (lmirror.cu) is produced on the device only.
   Mirror *mo = *output_p ? find_mirror(*output_p) : nullptr;
   L_handle *out = nullptr;
@@ -506,7 +509,7 @@ int attyn_entry(bool symmetric, const char *who, int output_spacing_a, int outpu
       set_error(2, "output length %llu < %llu in %s", out->length, length, who);
       return (int)length;
     }
-    if (length) LAKGB_CUDA(cudaMemsetAsync(mo->d, 0, length * sizeof(double), stream()));
+    if (length && !all) LAKGB_CUDA(cudaMemsetAsync(mo->d, 0, length * sizeof(double), stream()));
     mo->host_stale = true;
   } else {
     out = ensure_output(output_p, length, who, false);
@@ -578,7 +581,7 @@ int attyn_entry(bool symmetric, const char *who, int output_spacing_a, int outpu
     p.out = mo->d;
   } else {
     d_out = DBuf(length * sizeof(double));
-    d_out.zero();
+    if (!all) d_out.zero();
     p.out = d_out.as<double>();
   }
   st.flush();
