@@ -61,6 +61,7 @@ __global__ void bitplane_prep_kernel(BitplaneParams p, int nT, int *pm, int *ycn
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int nq = 1 + p.nW * p.B;
+  release_next();
   const long long plane_warps = (long long)nq * nT;
   const uint32_t *p0 = reinterpret_cast<const uint32_t *>(p.planes);
   const uint32_t *m = reinterpret_cast<const uint32_t *>(p.mask);
@@ -117,6 +118,8 @@ __global__ void bitplane_tsum_kernel(BitplaneParams p, const int *pm, double *T_
                                      double *q2) {
   const int mw = blockIdx.x * blockDim.x + threadIdx.x, blk = blockIdx.y, t = blockIdx.z;
   const int nq = 1 + p.nW * p.B;
+  await_previous();
+  release_next();
   if (mw >= p.nW) return;
   const int *row = pm + (long long)t * nq;
   const double tb = __dmul_rn(__dmul_rn((double)row[0], p.min_d), p.mlt_d);
@@ -327,6 +330,7 @@ __global__ void __launch_bounds__(32 * kFinishWarps) an_ztsn_finish_kernel(AnZtS
   __shared__ long long pm[kFinishPlanes][kFinishRows];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = blockIdx.y;
   const int row = blockIdx.x * kFinishRows + lane, i = min(row, p.n - 1);
+  await_previous();
   double base = 0.0, tmp = 0.0, n2 = 1.0;
   long long t = 0;
   // plane j of the sum: the mask plane, then the value planes from the lowest
@@ -808,11 +812,11 @@ extern "C" int wrap_At_T_YnWt_S_Zn_ww__run(int *tidx, void **vpra, pthread_t *th
     // every partial sum of T_tmp is an integer below patients * 2^B
     const bool exact = B < 40 && (double)P * kBlockBits * (double)(1ll << B) <= 9007199254740992.0;
     if (exact)
-      bitplane_tsum_kernel<true><<<grid, 128, 0, stream()>>>(p, d_pm.as<int>(), d_Tb.as<double>(), d_Tt.as<double>(),
-                                                             d_ys.as<long long>(), d_q2.as<double>());
+      launch_after(bitplane_tsum_kernel<true>, grid, 128, 0, stream(), p, d_pm.as<int>(), d_Tb.as<double>(),
+                   d_Tt.as<double>(), d_ys.as<long long>(), d_q2.as<double>());
     else
-      bitplane_tsum_kernel<false><<<grid, 128, 0, stream()>>>(p, d_pm.as<int>(), d_Tb.as<double>(), d_Tt.as<double>(),
-                                                              d_ys.as<long long>(), d_q2.as<double>());
+      launch_after(bitplane_tsum_kernel<false>, grid, 128, 0, stream(), p, d_pm.as<int>(), d_Tb.as<double>(),
+                   d_Tt.as<double>(), d_ys.as<long long>(), d_q2.as<double>());
     LAKGB_CUDA(cudaGetLastError());
     count_launch(2);
   }
@@ -899,7 +903,7 @@ extern "C" int wrap_An_ZtSn_ww__run(int *tidx, void **vpra, pthread_t *thread_in
     p.min_d = M_ZtSn->min_d; p.mlt_d = M_ZtSn->mlt_d;
     p.out_r = d_or.as<unsigned long long>() + r0; p.s_off = d_so.as<unsigned long long>();
     p.out = d_out.as<double>();
-    an_ztsn_finish_kernel<<<dim3((g.nA + kFinishRows - 1) / kFinishRows, nS), 32 * kFinishWarps, 0, stream()>>>(p);
+    launch_after(an_ztsn_finish_kernel, dim3((g.nA + kFinishRows - 1) / kFinishRows, nS), 32 * kFinishWarps, 0, stream(), p);
     LAKGB_CUDA(cudaGetLastError());
     count_launch();
   }

@@ -172,6 +172,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kMmaWarp) tc::tmem_alloc(&sm.tmem_base, kTmemCols);
+  await_previous();
   const BitplaneParams *ps = g_ps;
   const BitplaneSeg *segs = g_segs;
   const int call0 = g_segs[0].call, ncalls = g_segs[nseg - 1].call - call0 + 1;
@@ -424,6 +425,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   }
 
+  release_next();
   tc::fence_before_sync();
   __syncthreads();
   if (warp == kMmaWarp) {
@@ -437,6 +439,9 @@ __global__ void __launch_bounds__(kThreads, 1)
 // carrying the sum on from the output where the segment does not start at the
 // first Wn row.  A chain of one FP64 add (80 cycles) per term: small blocks
 // put the few warps of a small call on as many SMs.
+// Not started while the tensor kernel runs: its blocks were then packed onto the
+// first SMs that fall free, many to an FP64 pipe (the 4096 x 1000 x 1024 product
+// took 240 us longer).
 constexpr int kAddThreads = 32, kAddAhead = 16;
 __global__ void __launch_bounds__(kAddThreads)
     bitplane_add_kernel(const BitplaneParams *__restrict__ ps, const BitplaneSeg *__restrict__ segs, int nseg,
@@ -483,8 +488,8 @@ void launch_b(const BitplaneParams *ps, const BitplaneSeg *segs, const BitplaneB
     LAKGB_CUDA(cudaFuncSetAttribute(bitplane_tc_kernel<B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)kSmemBytes));
   });
-  bitplane_tc_kernel<B><<<std::min(bt.units, 152), kThreads, kSmemBytes, s>>>(ps, segs + bt.seg0, bt.nseg, bt.units, Y,
-                                                                            tc_status_device_ptr());
+  launch_after(bitplane_tc_kernel<B>, std::min(bt.units, 152), kThreads, kSmemBytes, s, ps, segs + bt.seg0, bt.nseg,
+               bt.units, Y, tc_status_device_ptr());
   LAKGB_CUDA(cudaGetLastError());
   bitplane_add_kernel<<<bt.blocks, kAddThreads, 0, s>>>(ps, segs + bt.seg0, bt.nseg, Y);
   LAKGB_CUDA(cudaGetLastError());

@@ -631,6 +631,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       tc::bulk_g2s(sT + t * kTabBytes, src, kTabBytes, &sm.tab_full[t]);
       atomicAdd(&sm.tab_issued[t], 1u);
     };
+    await_previous();  // the tables; nothing before the first block's fold needs them
     if (et == 0) {
       issue_table(0, 0, 0);
       issue_table(1, 0, 1);
@@ -781,6 +782,7 @@ constexpr int kTableParts = 4;
 __device__ void write_block_table(const GramParams &p, int b, uint8_t *__restrict__ tab) {
   __shared__ double s_sum[8];
   __shared__ int s_diff[8], s_all[8];
+  release_next();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const double D = p.D ? p.D[b] : 1.0;
   double *prod = reinterpret_cast<double *>(tab);
@@ -923,7 +925,7 @@ template <int TYPE>
 void launch_tc_type(const GramParams &p, const uint8_t *T, cudaStream_t s) {
   configure_tc<TYPE, false>();
   const int tiles = active_tiles(p), grid = std::max(1, std::min(tiles, sm_count()));
-  gram_tc_kernel<TYPE, false><<<grid, kThreads, kSmemBytes, s>>>(p, GramGroupDev{}, tiles, T, tc_status_device_ptr());
+  launch_after(gram_tc_kernel<TYPE, false>, grid, kThreads, kSmemBytes, s, p, GramGroupDev{}, tiles, T, tc_status_device_ptr());
   LAKGB_CUDA(cudaGetLastError());
   count_launch();
 }
@@ -932,7 +934,8 @@ template <int TYPE>
 void launch_tc_group_type(const GramGroupDev &g, int total_tiles, const uint8_t *T, cudaStream_t s) {
   configure_tc<TYPE, true>();
   const int grid = std::max(1, std::min(total_tiles, sm_count()));
-  gram_tc_kernel<TYPE, true><<<grid, kThreads, kSmemBytes, s>>>(GramParams{}, g, total_tiles, T, tc_status_device_ptr());
+  launch_after(gram_tc_kernel<TYPE, true>, grid, kThreads, kSmemBytes, s, GramParams{}, g, total_tiles, T,
+               tc_status_device_ptr());
   LAKGB_CUDA(cudaGetLastError());
   count_launch();
 }

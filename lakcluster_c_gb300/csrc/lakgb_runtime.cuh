@@ -30,6 +30,31 @@ cudaStream_t stream();
 cudaStream_t copy_stream();
 void count_launch(unsigned long long n = 1);
 
+// A launch that may start while the kernel before it on the stream still runs
+// (programmatic stream serialisation).  The kernel calls await_previous()
+// before it reads or writes anything that the one before it writes or reads;
+// that one calls release_next() once the rest of it needs no more room than it
+// has.  Saves the launch gap, about 1.5 us, and whatever the kernel does before
+// it waits.
+template <class... P, class... A>
+inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  LAKGB_CUDA(cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...));
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 // Device allocation on the library stream (stream-ordered allocator).
 void *dalloc(size_t bytes);
 void dfree(void *p);

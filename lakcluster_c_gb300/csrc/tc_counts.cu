@@ -221,6 +221,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   extern __shared__ __align__(128) uint8_t dsm[];
   __shared__ Smem sm;
   const int m0 = blockIdx.y * kM, n0 = blockIdx.x * kN, b = blockIdx.z;
+  release_next();
   if (p.symmetric && m0 > n0 + kN - 1) return;  // no pair i <= k
   const TileRows t{p.wA, p.a_rowb, p.nA, p.a_row_bytes, p.wZ, p.z_rowb, p.nZ, p.z_row_bytes, p.mask, nullptr};
   Tile tile;
@@ -254,6 +255,7 @@ template <int TYPE>
 __global__ void __launch_bounds__(256) gram_fold_kernel(GramParams p, const uint16_t *__restrict__ cnt) {
   const size_t n = (size_t)p.nA * p.nZ;
   const int ga = blockIdx.x * blockDim.x + threadIdx.x;
+  await_previous();
   if (ga >= p.nA) return;
   for (int gz = blockIdx.y * blockDim.y + threadIdx.y; gz < p.nZ; gz += gridDim.y * blockDim.y) {
     if (p.symmetric && ga > gz) continue;
@@ -395,7 +397,7 @@ void launch_split_type(const GramParams &p, uint16_t *cnt, cudaStream_t s) {
   launch_counts<TYPE>(p, cnt, nullptr, s);
   const int bx = std::min(256, (p.nA + 31) / 32 * 32), by = 256 / bx;
   const dim3 fold((p.nA + bx - 1) / bx, std::min((p.nZ + by - 1) / by, 65535));
-  gram_fold_kernel<TYPE><<<fold, dim3(bx, by), 0, s>>>(p, cnt);
+  launch_after(gram_fold_kernel<TYPE>, fold, dim3(bx, by), 0, s, p, cnt);
   LAKGB_CUDA(cudaGetLastError());
   count_launch();
 }

@@ -156,6 +156,7 @@ template <bool SKIP_NAN>
 __global__ void __launch_bounds__(kMinMaxThreads, 5)
     xcalc_minmax_kernel(const double *lf, const long long *rows_j, int nr, const long long *cols_j, int nc,
                         ulonglong2 *part, unsigned *ticket, long long d_mlt, XcalcScalars *out) {
+  release_next();
   unsigned long long kmn = ~0ull, kmx = 0ull;  // empty: kmn > kmx
   const int stride = gridDim.x * blockDim.x;
   for (int rb = blockIdx.x * blockDim.x + threadIdx.x; rb < nr; rb += kMinMaxRows * stride) {
@@ -290,6 +291,7 @@ __global__ void __launch_bounds__(kPlaneThreads, kPlaneBlocks) xcalc_planes_kern
   const int lane = threadIdx.x & 31;
   const int ngroups = max(1, (p.nrows_a + kPlaneRows - 1) / kPlaneRows);
   const int g = warp % ngroups;
+  await_previous();
   if (warp / ngroups >= cstep) return;
   const long long pad0 = g == ngroups - 1 ? 32ll * ngroups : p.brows;  // padding this warp clears
   const XcalcScalars s = *p.sc;
@@ -390,11 +392,11 @@ void launch_planes(const XcalcParams &p, cudaStream_t s) {
   const bool wide = (p.brows & 15) == 0 && (reinterpret_cast<uintptr_t>(p.planes) & 15) == 0;
   const bool narrow = p.ncols_per - 1 <= 32 && p.dmax <= 0xffffffffull;
   if (wide && narrow)
-    xcalc_planes_kernel<true, uint32_t><<<blocks, kPlaneThreads, 0, s>>>(p, cstep);
+    launch_after(xcalc_planes_kernel<true, uint32_t>, blocks, kPlaneThreads, 0, s, p, cstep);
   else if (wide)
-    xcalc_planes_kernel<true, unsigned long long><<<blocks, kPlaneThreads, 0, s>>>(p, cstep);
+    launch_after(xcalc_planes_kernel<true, unsigned long long>, blocks, kPlaneThreads, 0, s, p, cstep);
   else
-    xcalc_planes_kernel<false, unsigned long long><<<blocks, kPlaneThreads, 0, s>>>(p, cstep);
+    launch_after(xcalc_planes_kernel<false, unsigned long long>, blocks, kPlaneThreads, 0, s, p, cstep);
   LAKGB_CUDA(cudaGetLastError());
   count_launch();
 }
