@@ -50,14 +50,18 @@ DBuf upload_L(const L_handle *L, bool three_d) {
   return d;
 }
 
-// Both sums: one CTA per 32 rows (or pairs) and covariate.  Warps 1-8 form the
+// Both sums: one CTA per 32 rows (or pairs) and covariate.  Nine warps form the
 // terms of kTerms columns into one half of a shared buffer -- the lane's row,
 // so that reads of one column are contiguous in the column-major matrix --
-// while warp 0 adds the other half's in order, a lane per row.  The chain of
+// while one warp adds the other half's in order, a lane per row.  The chain of
 // one FP64 add (80 cycles) per term bounds a row; a sum and its products in one
 // thread took three operations per term, and 16 rows per CTA with the two
-// phases one after the other twice the adding warps.
-constexpr int kSumRows = 32, kTerms = 64, kSumT = 32 + 256;
+// phases one after the other twice the adding warps.  Two warps do nothing:
+// they share the adding warp's FP64 pipe, which their products held for a fifth (two of
+// eight forming warps there, one product a term) to a third of the time.  Which
+// quarter of the warps that is goes round with the CTA, so that several CTAs on
+// an SM add on different pipes.
+constexpr int kSumRows = 32, kFormWarps = 9, kTermsPerWarp = 4, kTerms = kFormWarps * kTermsPerWarp, kSumT = 32 * 12;
 struct SwnytCall {
   const double *A; const unsigned long long *a_r, *a_c;
   const double *Y; const unsigned long long *y_r, *y_c;
@@ -76,27 +80,40 @@ struct WtszCall {
   int tile0;  // grouped launch: first CTA of this call
 };
 
-// The terms of row i and covariate s: reference order of the operations; the
-// product with vS = +1 / -1 is exact.
+// The terms of row i and covariate s: where term k's operands are, the operands
+// and the product, in the reference's order of operations; the product with
+// vS = +1 / -1 is exact.
 struct SwnytTerm {
   const double *A, *Y;
   const unsigned long long *a_c, *y_c;
   const int8_t *vs;
   __device__ SwnytTerm(const SwnytCall &c, int i, int s)
       : A(c.A + c.a_r[i]), Y(c.Y + c.y_r[i]), a_c(c.a_c), y_c(c.y_c), vs(c.vS + (long long)s * c.nZ) {}
-  __device__ __forceinline__ double operator()(int z) const {
-    const double a = A[a_c[z]];
-    return __dmul_rn(vs[z] < 0 ? -a : a, Y[y_c[z]]);
+  // few rows and long chains: operands ahead pay (a call 203 -> 139 us)
+  static constexpr bool kAhead = true;
+  static constexpr int kCtas = 2;
+  struct At { unsigned long long a, y; int8_t v; };
+  struct Of { double a, y; };
+  __device__ __forceinline__ At at(int z) const { return {a_c[z], y_c[z], vs[z]}; }
+  __device__ __forceinline__ Of of(const At &p) const {
+    const double a = A[p.a];
+    return {p.v < 0 ? -a : a, Y[p.y]};
   }
+  __device__ __forceinline__ double operator()(const Of &o) const { return __dmul_rn(o.a, o.y); }
 };
 struct WtszTerm {
   const double *AY, *ZW, *Dy;
   const unsigned long long *ay_y, *zw_w;
   __device__ WtszTerm(const WtszCall &c, int i, int s)
       : AY(c.AY + c.ay_a[i] + c.ay_s[s]), ZW(c.ZW + c.zw_z[i] + c.zw_s[s]), Dy(c.Dy), ay_y(c.ay_y), zw_w(c.zw_w) {}
-  __device__ __forceinline__ double operator()(int k) const {
-    return __dmul_rn(__dmul_rn(AY[ay_y[k]], Dy[k]), ZW[zw_w[k]]);
-  }
+  // many rows: more CTAs per SM hide the loads, the registers go to them
+  static constexpr bool kAhead = false;
+  static constexpr int kCtas = 3;
+  struct At { unsigned long long a, z; double d; };
+  struct Of { double a, d, z; };
+  __device__ __forceinline__ At at(int k) const { return {ay_y[k], zw_w[k], Dy[k]}; }
+  __device__ __forceinline__ Of of(const At &p) const { return {AY[p.a], p.d, ZW[p.z]}; }
+  __device__ __forceinline__ double operator()(const Of &o) const { return __dmul_rn(__dmul_rn(o.a, o.d), o.z); }
 };
 __host__ __device__ inline int sum_rows(const SwnytCall &c) { return c.nA; }
 __host__ __device__ inline int sum_rows(const WtszCall &c) { return c.npairs; }
@@ -112,19 +129,44 @@ __device__ __forceinline__ void ordered_sum_tile(const Call &c, int rt, int s) {
   const Term t(c, min(i, rows - 1), s);
   const int tiles = (n + kTerms - 1) / kTerms;
   double acc = 0.0;
-  for (int j = 0; j <= tiles; ++j) {
-    if (warp > 0) {
-      if (j < tiles) {
-        double v[kTerms / 8];
+  // kAhead: the operands of the next tile and the places of the one after are on
+  // their way while a tile's terms are formed.  (Past the last term: the last
+  // one's.)
+  const int quarter = (int)(blockIdx.x + blockIdx.x / 152) & 3, own = warp & 3;
+  const int w = 3 * (warp >> 2) + own - (own > quarter);
+  const bool adds = warp == quarter, forms = own != quarter && n > 0;
+  typename Term::At at[kTermsPerWarp];
+  typename Term::Of of[kTermsPerWarp];
+  auto places = [&](int j) {
 #pragma unroll
-        for (int u = 0; u < kTerms / 8; ++u) {
-          const int k = j * kTerms + (warp - 1) + 8 * u;
-          v[u] = k < n ? t(k) : 0.0;
+    for (int u = 0; u < kTermsPerWarp; ++u) at[u] = t.at(min(j * kTerms + w + kFormWarps * u, n - 1));
+  };
+  auto operands = [&]() {
+#pragma unroll
+    for (int u = 0; u < kTermsPerWarp; ++u) of[u] = t.of(at[u]);
+  };
+  if (forms && Term::kAhead) {
+    places(0);
+    operands();
+    places(1);
+  }
+  for (int j = 0; j <= tiles; ++j) {
+    if (forms) {
+      if (j < tiles) {
+        double v[kTermsPerWarp];
+#pragma unroll
+        for (int u = 0; u < kTermsPerWarp; ++u) {
+          if (!Term::kAhead) of[u] = t.of(t.at(min(j * kTerms + w + kFormWarps * u, n - 1)));
+          v[u] = t(of[u]);
+        }
+        if (Term::kAhead) {
+          operands();
+          places(j + 2);
         }
 #pragma unroll
-        for (int u = 0; u < kTerms / 8; ++u) term[j & 1][(warp - 1) + 8 * u][lane] = v[u];
+        for (int u = 0; u < kTermsPerWarp; ++u) term[j & 1][w + kFormWarps * u][lane] = v[u];
       }
-    } else if (j > 0) {
+    } else if (adds && j > 0) {
       const int m = min(kTerms, n - (j - 1) * kTerms);
       const double(*q)[kSumRows] = term[(j - 1) & 1];
 #pragma unroll 8
@@ -132,13 +174,13 @@ __device__ __forceinline__ void ordered_sum_tile(const Call &c, int rt, int s) {
     }
     __syncthreads();
   }
-  if (warp == 0 && i < rows) c.out[c.out_r[i] + c.s_off[s]] = acc;
+  if (adds && i < rows) c.out[c.out_r[i] + c.s_off[s]] = acc;
 }
 
-__global__ void __launch_bounds__(kSumT) anzt_s_wnyt_kernel(SwnytCall c) {
+__global__ void __launch_bounds__(kSumT, SwnytTerm::kCtas) anzt_s_wnyt_kernel(SwnytCall c) {
   ordered_sum_tile<SwnytTerm>(c, blockIdx.x, blockIdx.y);
 }
-__global__ void __launch_bounds__(kSumT) attyn_wtszn_kernel(WtszCall c) {
+__global__ void __launch_bounds__(kSumT, WtszTerm::kCtas) attyn_wtszn_kernel(WtszCall c) {
   ordered_sum_tile<WtszTerm>(c, blockIdx.x, blockIdx.y);
 }
 
@@ -158,10 +200,10 @@ __device__ __forceinline__ void ordered_sum_group(const Call *calls, int n) {
   const int j = k - c.tile0;
   ordered_sum_tile<Term>(c, j % rtiles, j / rtiles);
 }
-__global__ void __launch_bounds__(kSumT) anzt_s_wnyt_group_kernel(const SwnytCall *calls, int n) {
+__global__ void __launch_bounds__(kSumT, SwnytTerm::kCtas) anzt_s_wnyt_group_kernel(const SwnytCall *calls, int n) {
   ordered_sum_group<SwnytTerm>(calls, n);
 }
-__global__ void __launch_bounds__(kSumT) attyn_wtszn_group_kernel(const WtszCall *calls, int n) {
+__global__ void __launch_bounds__(kSumT, WtszTerm::kCtas) attyn_wtszn_group_kernel(const WtszCall *calls, int n) {
   ordered_sum_group<WtszTerm>(calls, n);
 }
 
