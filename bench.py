@@ -416,7 +416,7 @@ def large_pass_headline(args, lib, stream, sh, rank, world, local):
     roof = {
         "bound": "tensor", "achieved": tflops, "peak": peak_tf, "unit": "TFLOP/s", "frac": tflops / peak_tf,
         "traffic": traffic,
-        "kernel": "gram_tc_kernel<1> (tcgen05 e4m3 counts + FP64 fold), one persistent launch per product",
+        "kernel": "gram_tc_kernel<1> (tcgen05 e2m1 counts + FP64 and integer fold), one persistent launch per product",
         "note": ("bit pairs of the pass (full square for AnAt) counted as 2 ops (one MAC) per step time, which "
                  "also holds the 15 table launches (a few us each), against the %s dense bf16 burst peak; frac against "
                  "the sustained peak %.3f. traffic: DRAM bytes per launch scaled by work from the committed ncu "
@@ -599,7 +599,7 @@ def run_gpu(args):
         line = {
             "metric": METRIC, "value": head["value"], "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": head["ms"], "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": "e4m3-bit-mma+f64", "data": "synthetic",
+            "vs_baseline": None, "dtype": "e2m1-bit-mma+f64", "data": "synthetic",
             "config": dict(CONFIG, parallelism="replicas" if world > 1 else "single"),
             "pass_form": "one persistent tcgen05 launch per product (lakgb_gram_device, 15 per step, each after "
                          "its table launch); grouped_pass has the pass as one grouped launch",

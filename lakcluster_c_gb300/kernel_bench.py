@@ -117,8 +117,8 @@ def bench_attyn(lib, rng, reps):
         lib.wrap_AtTYn_vv__run(*_thread(), abi.SPACING_a, abi.SPACING_a, abi.SPACING_a, At.ptr, Tt.ptr, At.ptr,
                                aj.ctypes.data_as(_DP), aj.ctypes.data_as(_DP), lt.ptr, lt.ptr, C.byref(out))
     s = _time(call, reps)
-    return {"seconds": s, "bitops": float(nsnp) * nsnp * At.s.mc_length * 8, "kernel": "attyn_kernel",
-            "bound": "integer pipe", "note": "the call downloads the 4096 x 4096 FP64 output (134 MB)"}
+    return {"seconds": s, "bitops": float(nsnp) * nsnp * At.s.mc_length * 8, "kernel": "attyn_tc_kernel",
+            "bound": "download", "note": "the call downloads the 4096 x 4096 FP64 output (134 MB)"}
 
 
 def bench_an_ztsn(lib, rng, reps):
@@ -134,8 +134,8 @@ def bench_an_ztsn(lib, rng, reps):
                                  C.byref(out))
     s = _time(call, reps)
     return {"seconds": s, "bitops": float(n) * (B + 1) * An.s.mc_length * 8, "bytes": An.s.rpop_b * An.s.mc_length,
-            "kernel": "the masked-AND Gram of the An rows against the 33 planes (gram kernels), an_ztsn_finish_kernel",
-            "bound": "integer or tensor pipe (the Gram)"}
+            "kernel": "gram_counts_tc_kernel (the An rows against the 33 planes), an_ztsn_finish_kernel",
+            "bound": "tensor-core counts, then latency"}
 
 
 def bench_anzt_s_wnyt(lib, rng, reps):
