@@ -426,7 +426,8 @@ def large_pass_headline(args, lib, stream, sh, rank, world, local):
                       "achieved_ops_per_s": elems * fp64_per_elem / (ms / 1000.0),
                       "peak_adds_per_s": fp64_rate,
                       "frac": elems * fp64_per_elem / (ms / 1000.0) / fp64_rate,
-                      "note": "the fold's FP64 operations (%d per computed element) against the add rate measured "
+                      "note": "the fold's additions and the results' operations (%d per computed element; three of seven "
+                              "rounds of additions and half of the results run in integers) against the FP64 add rate measured "
                               "live on this GPU" % fp64_per_elem},
         "vs_int_pipe_roofline": {"achieved_bitops": work / (ms / 1000.0), "int_pipe_peak_bitops": popc_peak,
                                  "ratio": (work / (ms / 1000.0)) / popc_peak,
