@@ -150,7 +150,7 @@ __device__ void make_scalars(unsigned long long kmn, unsigned long long kmx, boo
 // SKIP_NAN: a NaN is left out of the extremes unless it is the first retained
 // value, which then gives NaN (the comparisons of xcalc.c:25 in order).
 constexpr int kMinMaxRows = 4, kMinMaxCols = 2, kMinMaxThreads = 256;
-constexpr int kMinMaxBlocks = 152 * 8;  // most blocks of a launch (760, one wave: 1 % faster)
+constexpr int kMinMaxBlocks = 152 * 8;  // most blocks of a launch
 
 template <bool SKIP_NAN>
 __global__ void __launch_bounds__(kMinMaxThreads, 5)
