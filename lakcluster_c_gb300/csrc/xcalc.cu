@@ -66,7 +66,9 @@ struct XcalcParams {
   const uint8_t *row0;       // first plane's bytes (null: zeros)
   long long row_max;         // largest row offset
   unsigned long long lf_n, planes_n;  // elements of lf, bytes of planes (bounds checks)
-  int *bad;                  // set when an index would leave its buffer (access skipped)
+  // set when an index would leave its buffer (access skipped); null: the
+  // caller's offsets, negative ones among them, are taken as they are
+  int *bad;
   const XcalcScalars *sc;
 };
 
@@ -269,6 +271,10 @@ __device__ __forceinline__ unsigned long long quantise_fixed(double x, const Xca
   return v < 1ull ? 1ull : v;
 }
 
+__device__ __forceinline__ void note_bad(int *bad, int code) {
+  if (bad) atomicCAS(bad, 0, code);
+}
+
 // Warp per 256-row group (32 bytes of every plane row), for the columns
 // c, c + step, ...: the row offsets stay in registers, lane l quantises rows
 // 256g + 32k + l, k = 0..7 (eight independent coalesced loads).  Per k, the
@@ -306,8 +312,8 @@ __global__ void __launch_bounds__(kPlaneThreads, kPlaneBlocks) xcalc_planes_kern
   const long long byte0 = 32ll * g;
   for (int c = warp / ngroups; c < p.ncols_j; c += cstep) {
     const long long co = p.col_off[c];
-    const bool inside = (unsigned long long)(p.row_max + co) < p.lf_n;
-    if (!inside) atomicCAS(p.bad, 0, 1);
+    const bool inside = !p.bad || (unsigned long long)(p.row_max + co) < p.lf_n;
+    if (!inside) note_bad(p.bad, 1);
     double x[R];
     unsigned live = 0u;
 #pragma unroll
@@ -351,7 +357,7 @@ __global__ void __launch_bounds__(kPlaneThreads, kPlaneBlocks) xcalc_planes_kern
 #pragma unroll
           for (int h = 0; h < 2; ++h)
             if (byte0 + 16 * h < p.brows) {
-              if (off + 16 * h + 16 > p.planes_n) atomicCAS(p.bad, 0, 2);
+              if (off + 16 * h + 16 > p.planes_n) note_bad(p.bad, 2);
               else *reinterpret_cast<uint4 *>(p.planes + off + 16 * h) =
                   make_uint4(o[4 * h], o[4 * h + 1], o[4 * h + 2], o[4 * h + 3]);
             }
@@ -362,7 +368,7 @@ __global__ void __launch_bounds__(kPlaneThreads, kPlaneBlocks) xcalc_planes_kern
 #pragma unroll
           for (int k = 0; k < R; ++k)
             if (byte0 + 4 * k < p.brows) {
-              if (off + 4 * k + 4 > p.planes_n) atomicCAS(p.bad, 0, 2);
+              if (off + 4 * k + 4 > p.planes_n) note_bad(p.bad, 2);
               else *reinterpret_cast<uint32_t *>(p.planes + off + 4 * k) = o[k];
             }
           for (long long b = pad0; b < p.brows; b += 4)
@@ -375,7 +381,7 @@ __global__ void __launch_bounds__(kPlaneThreads, kPlaneBlocks) xcalc_planes_kern
     const long long mask_end = pad0 < p.brows ? p.brows : min(p.brows, byte0 + 32);
     for (long long b = byte0 + lane; b < mask_end; b += 32) {
       const unsigned long long off = (unsigned long long)(first * p.brows + b);
-      if (off >= p.planes_n) atomicCAS(p.bad, 0, 2);
+      if (off >= p.planes_n) note_bad(p.bad, 2);
       else p.planes[off] = (c == 0 && p.row0) ? p.row0[b] : (uint8_t)0;
     }
   }
@@ -751,7 +757,6 @@ extern "C" int lakgb_xcalc_noalloc(const struct lakgb_xcalc_noalloc_args *a) {
     p.dmax = (unsigned long long)(a->d_mlt - 1); p.ncols_per = ncols_per; p.brows = a->brows;
     p.planes = a->planes; p.row0 = a->row0;
     p.sc = sc;
-    p.lf_n = ~0ull;  // the caller's offsets are taken as they are
     p.planes_n = (unsigned long long)nbytes;
     launch_planes(p, s);
   }
