@@ -537,6 +537,10 @@ int lakgb_thread_error_take(char *msg, int msg_len);
  * for the length of the solve whatever this setting is. */
 void lakgb_set_residency(int on);
 void lakgb_forget_host_buffer(const void *host_ptr);
+/* Staging buffers (page-locked and device memory) that host threads which have
+ * ended left for the next ones; returns their bytes and, with release != 0,
+ * frees them.  At most eight threads' buffers are kept. */
+long long lakgb_idle_buffers(int release);
 /* D_MLT used by wrap_xcalc (the reference's GLOBAL_D_MLT, default 2^32). */
 void lakgb_set_d_mlt(long long d_mlt);
 /* Number of CUDA kernels this library has launched since load. */

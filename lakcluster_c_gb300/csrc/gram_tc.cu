@@ -974,29 +974,19 @@ void launch_gram_tc_group(const GramGroupDev &g, int type, int total_tiles, long
 
 // The status word of the calling host thread's launches: every thread (a
 // solve, a server worker) has its own, so a pipeline timeout in one solve is
-// reported to that solve alone.  Zeroed on the thread's own stream (which
-// does not wait for the legacy default stream).
-namespace {
-thread_local int *t_status = nullptr;
-}
-
-int *tc_status_device_ptr() {
-  if (!t_status) {
-    LAKGB_CUDA(cudaMalloc(reinterpret_cast<void **>(&t_status), sizeof(int)));
-    LAKGB_CUDA(cudaMemsetAsync(t_status, 0, sizeof(int), stream()));
-  }
-  return t_status;
-}
+// reported to that solve alone.
+int *tc_status_device_ptr() { return thread_word(kTcStatus); }
 
 // Read and clear the calling thread's status word (after every launch made
 // so far has finished: the launches may be on a caller's stream).
 int tc_status_take() {
-  if (!t_status) return 0;
+  int *status = thread_word(kTcStatus, false);
+  if (!status) return 0;
   int v = 0;
   LAKGB_CUDA(cudaDeviceSynchronize());
-  LAKGB_CUDA(cudaMemcpy(&v, t_status, sizeof v, cudaMemcpyDeviceToHost));
+  LAKGB_CUDA(cudaMemcpy(&v, status, sizeof v, cudaMemcpyDeviceToHost));
   if (v) {
-    LAKGB_CUDA(cudaMemsetAsync(t_status, 0, sizeof(int), stream()));
+    LAKGB_CUDA(cudaMemsetAsync(status, 0, sizeof(int), stream()));
     LAKGB_CUDA(cudaStreamSynchronize(stream()));
   }
   return v;
@@ -1005,12 +995,13 @@ int tc_status_take() {
 // As tc_status_take, for launches on the calling thread's own stream only
 // (a whole solve): waits for that stream, not for the device.
 int tc_status_take_stream() {
-  if (!t_status) return 0;
+  int *status = thread_word(kTcStatus, false);
+  if (!status) return 0;
   int v = 0;
-  LAKGB_CUDA(cudaMemcpyAsync(&v, t_status, sizeof v, cudaMemcpyDeviceToHost, stream()));
+  LAKGB_CUDA(cudaMemcpyAsync(&v, status, sizeof v, cudaMemcpyDeviceToHost, stream()));
   LAKGB_CUDA(cudaStreamSynchronize(stream()));
   if (v) {
-    LAKGB_CUDA(cudaMemsetAsync(t_status, 0, sizeof(int), stream()));
+    LAKGB_CUDA(cudaMemsetAsync(status, 0, sizeof(int), stream()));
     LAKGB_CUDA(cudaStreamSynchronize(stream()));
   }
   return v;

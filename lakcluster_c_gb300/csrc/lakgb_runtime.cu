@@ -4,7 +4,9 @@
 #include <stdarg.h>
 #include <stdlib.h>
 #include <string.h>
+#include <unistd.h>
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <map>
@@ -55,44 +57,139 @@ void check_cuda(cudaError_t e, const char *what, const char *file, int line) {
   exit(1);  // RET_NOMEM-style hard stop, as the reference does on fatal errors
 }
 
-// One non-blocking stream per host thread: solves run from different
-// threads overlap on the device, while the calls of one solve stay ordered.
-cudaStream_t stream() {
-  thread_local cudaStream_t s = nullptr;
-  if (!s) {
-    cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+// --- per-thread streams and buffers -------------------------------------------
+
+namespace {
+std::mutex g_idle_mu;
+// Never destroyed: threads may end after the library's static objects have gone.
+std::vector<ThreadBuffers *> &idle_buffers() {
+  static auto *v = new std::vector<ThreadBuffers *>;
+  return *v;
+}
+
+long long buffer_bytes(const ThreadBuffers &b) {
+  long long n = b.down ? (long long)kDownBytes : 0;
+  for (const Arena &a : b.arenas) n += a.host ? 2 * (long long)a.cap : 0;
+  for (const UpChunk &c : b.up) n += 2 * (long long)c.cap;
+  return n;
+}
+
+// (Nothing of the set is in flight.)
+void free_up_chunks(ThreadBuffers &b, size_t keep) {
+  for (; b.up.size() > keep; b.up.pop_back()) {
+    cudaFreeHost(b.up.back().h);
+    cudaFree(b.up.back().d);
+  }
+}
+void free_buffers(ThreadBuffers &b) {
+  free_up_chunks(b, 0);
+  for (Arena &a : b.arenas) {
+    if (!a.host) continue;
+    cudaFreeHost(a.host);
+    cudaFree(a.dev);
+    cudaEventDestroy(a.done);
+    a = Arena{};
+  }
+  if (b.down) cudaFreeHost(b.down);
+  b.down = nullptr;
+}
+
+thread_local ThreadBuffers *t_buffers = nullptr;
+
+// Leaves the thread's set to others when the thread ends.
+struct BuffersOwner {
+  bool used = false;
+  ~BuffersOwner() {
+    ThreadBuffers *b = t_buffers;
+    t_buffers = nullptr;
+    if (!b || b->pid != getpid()) return;  // (a forked child has no device)
+    // another thread's capture does not forbid what follows
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    // a set whose stream has failed, or is being captured, is not used again
+    if (b->words && cudaMemsetAsync(b->words, 0, kThreadWords * sizeof(int), b->stream) != cudaSuccess) return;
+    if (cudaStreamSynchronize(b->stream) != cudaSuccess) return;
+    if (b->copy && cudaStreamSynchronize(b->copy) != cudaSuccess) return;
+    for (Arena &a : b->arenas) a.pending = false;
+    b->up_cur = 0;
+    for (UpChunk &c : b->up) c.used = c.sent = 0;
+    std::sort(b->up.begin(), b->up.end(), [](const UpChunk &x, const UpChunk &y) { return x.cap < y.cap; });
+    size_t keep = 0;
+    while (keep < b->up.size() && keep < (size_t)kIdleUpChunks && b->up[keep].cap == kUpChunk) ++keep;
+    std::lock_guard<std::mutex> lk(g_idle_mu);
+    int full = 0;
+    for (const ThreadBuffers *i : idle_buffers()) full += buffer_bytes(*i) > 0;
+    if (full < kIdleBuffers)
+      free_up_chunks(*b, keep);
+    else
+      free_buffers(*b);
+    idle_buffers().push_back(b);
+  }
+};
+thread_local BuffersOwner t_owner;
+}  // namespace
+
+ThreadBuffers &thread_buffers() {
+  if (t_buffers) return *t_buffers;
+  t_owner.used = true;  // its destructor runs when the thread ends
+  int dev = 0;
+  cudaGetDevice(&dev);
+  ThreadBuffers *b = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(g_idle_mu);
+    auto &idle = idle_buffers();
+    // the set left last, so that those beyond the usual number stay untouched
+    for (size_t i = idle.size(); i-- > 0 && !b;)
+      if (idle[i]->device == dev) {
+        b = idle[i];
+        idle.erase(idle.begin() + (long)i);
+      }
+  }
+  if (!b) {
+    b = new ThreadBuffers;
+    b->device = dev;
+    b->pid = getpid();
+    cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
       fprintf(stderr, " %% Error! no CUDA device usable by liblakgb300: %s\n", cudaGetErrorString(e));
       exit(1);
     }
   }
-  return s;
+  t_buffers = b;
+  return *b;
 }
+
+int *thread_word(ThreadWord w, bool make) {
+  if (!make && (!t_buffers || !t_buffers->words)) return nullptr;
+  ThreadBuffers &b = thread_buffers();
+  if (!b.words) {
+    LAKGB_CUDA(cudaMalloc(reinterpret_cast<void **>(&b.words), kThreadWords * sizeof(int)));
+    LAKGB_CUDA(cudaMemsetAsync(b.words, 0, kThreadWords * sizeof(int), b.stream));
+  }
+  return b.words + w;
+}
+
+// One non-blocking stream per host thread: solves run from different
+// threads overlap on the device, while the calls of one solve stay ordered.
+cudaStream_t stream() { return thread_buffers().stream; }
 
 cudaStream_t copy_stream() {
-  thread_local cudaStream_t s = nullptr;
-  if (!s) LAKGB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-  return s;
+  ThreadBuffers &b = thread_buffers();
+  if (!b.copy) LAKGB_CUDA(cudaStreamCreateWithFlags(&b.copy, cudaStreamNonBlocking));
+  return b.copy;
 }
 
-// --- per-thread staging arena -----------------------------------------------
+// --- staging arenas -------------------------------------------------------------
 
-namespace {
 // One call's arena; a thread takes its kArenas arenas in turn, so that a call
 // can be prepared while the GPU still works on the calls before it.  (With one
 // arena every call waited for the previous call's copy, which the stream runs
 // only after that call's predecessor: host and GPU took turns.)
-struct Arena {
-  unsigned char *host = nullptr;   // pinned
-  unsigned char *dev = nullptr;
-  size_t cap = 0, used = 0;
-  cudaEvent_t done = nullptr;      // the last flush's copy has completed
-  bool pending = false;
-};
-constexpr int kArenas = 8;
-thread_local Arena t_arenas[kArenas];
-thread_local int t_arena = 0;
-Arena &arena() { return t_arenas[t_arena]; }
+namespace {
+Arena &arena() {
+  ThreadBuffers &b = thread_buffers();
+  return b.arenas[b.arena];
+}
 }  // namespace
 
 namespace {
@@ -117,7 +214,8 @@ DBuf upload_bytes(const void *h, size_t n) {
 
 void Stager::begin() {
   t_active = this;
-  t_arena = (t_arena + 1) % kArenas;
+  ThreadBuffers &b = thread_buffers();
+  b.arena = (b.arena + 1) % kArenas;
   Arena &a = arena();
   if (!a.host) {
     a.cap = kStageBytes;
@@ -416,6 +514,16 @@ bool host_planes_wanted() { return !t_device_only_planes || !residency_enabled()
 // Inside a solve: bit planes made by wrap_xcalc stay on the device only (the
 // driver reads them through the residency cache, never on the host).
 extern "C" void lakgb_device_only_planes(int on) { lakgb::t_device_only_planes = on ? 1 : 0; }
+
+extern "C" long long lakgb_idle_buffers(int release) {
+  std::lock_guard<std::mutex> lk(lakgb::g_idle_mu);
+  long long n = 0;
+  for (lakgb::ThreadBuffers *b : lakgb::idle_buffers()) {
+    n += lakgb::buffer_bytes(*b);
+    if (release) lakgb::free_buffers(*b);
+  }
+  return n;
+}
 
 extern "C" void lakgb_residency_scope(int enter) {
   thread_local std::vector<lakgb::ResidencyScope *> scopes;

@@ -28,6 +28,45 @@ cudaStream_t stream();
 // A second per-thread stream (non-blocking) for downloads that overlap the
 // kernels on stream().
 cudaStream_t copy_stream();
+
+// What a host thread keeps from call to call: its streams, its staging arenas
+// (Stager), the page-locked chunks of its deferral scopes (loopsum.cu) and the
+// device words its kernels report in.  A set belongs to one living thread; a
+// thread that ends waits for its streams and leaves the set to the next thread
+// on the same device, so that a server whose workers come and go allocates what
+// its most workers at a time need.  (Kept by the threads alone, every batch of
+// solves with eight workers lost 256 MB of device and 320 MB of page-locked
+// memory.)  The sets of kIdleBuffers ended threads keep their buffers, further
+// ones free them, lakgb_idle_buffers(1) frees all of them.  Streams and words
+// stay for the life of the process: a captured graph may hold a word's address.
+struct Arena {
+  unsigned char *host = nullptr;   // pinned
+  unsigned char *dev = nullptr;
+  size_t cap = 0, used = 0;
+  cudaEvent_t done = nullptr;      // the last flush's copy has completed
+  bool pending = false;
+};
+struct UpChunk { uint8_t *h = nullptr; uint8_t *d = nullptr; size_t cap = 0, used = 0, sent = 0; };
+constexpr int kArenas = 8;
+constexpr size_t kUpChunk = 4u << 20;      // bytes of an ordinary UpChunk
+constexpr int kIdleBuffers = 8, kIdleUpChunks = 4;
+struct ThreadBuffers {
+  int device = 0, pid = 0;
+  cudaStream_t stream = nullptr, copy = nullptr;
+  Arena arenas[kArenas];
+  int arena = 0;
+  std::vector<UpChunk> up;
+  size_t up_cur = 0;
+  uint8_t *down = nullptr;         // page-locked, kDownBytes
+  int *words = nullptr;            // device: the words below
+};
+enum ThreadWord { kTcStatus, kXcalcBad, kXcalcTicket, kThreadWords };
+constexpr size_t kDownBytes = 8u << 20;
+ThreadBuffers &thread_buffers();
+// The calling thread's word, zero when the thread first has it (zeroed on its
+// own stream: that one does not wait for the legacy default stream); null, if
+// `make` is false and the thread has no words yet.
+int *thread_word(ThreadWord w, bool make = true);
 void count_launch(unsigned long long n = 1);
 
 // A launch that may start while the kernel before it on the stream still runs

@@ -233,16 +233,13 @@ thread_local std::vector<DeferCopy> t_copies;  // other calls' outputs
 // Page-locked host chunks and their device twins for held-back calls'
 // inputs: bump-allocated, 16-byte aligned; `sent` is how much has been
 // copied.  Arrays larger than a chunk get a chunk of their own.  Reset (not
-// freed) when the outermost scope ends.
-struct UpChunk { uint8_t *h = nullptr; uint8_t *d = nullptr; size_t cap = 0, used = 0, sent = 0; };
-constexpr size_t kUpChunk = 4u << 20;
+// freed) when the outermost scope ends; kept in the thread's ThreadBuffers.
 
 // Page-locked buffer for a scope's small outputs: a copy into pageable memory
 // holds the host for about 8 us (and until the kernels before it are done), one
 // into page-locked memory under 1 us, so outputs of up to kDownEach bytes come
 // back there, as far as they fit, and are copied on after the scope's one wait.
-constexpr size_t kDownBytes = 8u << 20, kDownEach = 64u << 10;
-thread_local uint8_t *t_down = nullptr;
+constexpr size_t kDownEach = 64u << 10;
 struct DownCopy { double *host; size_t off, bytes; };
 
 // Enqueue the copy of `length` doubles of `dev` to `host`.
@@ -253,30 +250,29 @@ void copy_down(double *host, const double *dev, unsigned long long length, size_
     LAKGB_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, stream()));
     return;
   }
-  if (!t_down) LAKGB_CUDA(cudaHostAlloc((void **)&t_down, kDownBytes, cudaHostAllocDefault));
-  LAKGB_CUDA(cudaMemcpyAsync(t_down + used, dev, bytes, cudaMemcpyDeviceToHost, stream()));
+  uint8_t *&down = thread_buffers().down;
+  if (!down) LAKGB_CUDA(cudaHostAlloc((void **)&down, kDownBytes, cudaHostAllocDefault));
+  LAKGB_CUDA(cudaMemcpyAsync(down + used, dev, bytes, cudaMemcpyDeviceToHost, stream()));
   later.push_back(DownCopy{host, used, bytes});
   used += (bytes + 15) & ~(size_t)15;
 }
-thread_local std::vector<UpChunk> t_up;
-thread_local size_t t_up_cur = 0;
-
 }  // namespace
 
 bool defer_active() { return t_defer_depth > 0; }
 
 const void *defer_put(const void *h, size_t n) {
+  ThreadBuffers &b = thread_buffers();
   const size_t need = (n + 15) & ~(size_t)15;
-  while (t_up_cur < t_up.size() && t_up[t_up_cur].used + need > t_up[t_up_cur].cap) ++t_up_cur;
-  if (t_up_cur == t_up.size()) {
-    if (!t_up.empty()) defer_flush();  // the earlier chunks' pending bytes go first
+  while (b.up_cur < b.up.size() && b.up[b.up_cur].used + need > b.up[b.up_cur].cap) ++b.up_cur;
+  if (b.up_cur == b.up.size()) {
+    if (!b.up.empty()) defer_flush();  // the earlier chunks' pending bytes go first
     UpChunk c;
     c.cap = std::max(kUpChunk, need);
     LAKGB_CUDA(cudaHostAlloc((void **)&c.h, c.cap, cudaHostAllocDefault));
     LAKGB_CUDA(cudaMalloc((void **)&c.d, c.cap));
-    t_up.push_back(c);
+    b.up.push_back(c);
   }
-  UpChunk &c = t_up[t_up_cur];
+  UpChunk &c = b.up[b.up_cur];
   if (n) memcpy(c.h + c.used, h, n);
   const void *d = c.d + c.used;
   c.used += need;
@@ -284,7 +280,7 @@ const void *defer_put(const void *h, size_t n) {
 }
 
 void defer_flush() {
-  for (UpChunk &c : t_up) {
+  for (UpChunk &c : thread_buffers().up) {
     if (c.used > c.sent)
       LAKGB_CUDA(cudaMemcpyAsync(c.d + c.sent, c.h + c.sent, c.used - c.sent, cudaMemcpyHostToDevice, stream()));
     c.sent = c.used;
@@ -434,11 +430,11 @@ extern "C" void lakgb_defer_end(void) {
     for (auto &d : t_wtsz) copy_down(d.host_out, d.c.out, d.length, used, later);
     for (auto &c : t_copies) copy_down(c.host, c.dev.as<double>(), c.length, used, later);
     LAKGB_CUDA(cudaStreamSynchronize(stream()));
-    for (const DownCopy &c : later) memcpy(c.host, t_down + c.off, c.bytes);
+    for (const DownCopy &c : later) memcpy(c.host, thread_buffers().down + c.off, c.bytes);
   }
   t_copies.clear();
-  for (UpChunk &c : t_up) c.used = c.sent = 0;  // the stream has drained: reuse the chunks
-  t_up_cur = 0;
+  for (UpChunk &c : thread_buffers().up) c.used = c.sent = 0;  // the stream has drained: reuse the chunks
+  thread_buffers().up_cur = 0;
   t_swnyt.clear();
   t_wtsz.clear();
   for (const DeferKind &k : t_kinds) k.clear();

@@ -459,30 +459,11 @@ extern "C" void lakgb_set_d_mlt(long long d_mlt) { g_d_mlt = d_mlt; }
 
 namespace lakgb {
 namespace {
-// Per-thread device flag of the planes kernel's bounds checks.  It is
-// zeroed on the thread's own stream: that stream does not wait for the
-// legacy default stream (it is created non-blocking), so a plain cudaMemset
-// could still be pending when the first read of the flag runs, which would
-// then see whatever the allocation held before.
-int *bad_flag() {
-  thread_local int *d = nullptr;
-  if (!d) {
-    LAKGB_CUDA(cudaMalloc(&d, sizeof(int)));
-    LAKGB_CUDA(cudaMemsetAsync(d, 0, sizeof(int), stream()));
-  }
-  return d;
-}
-
-// The ticket of the extremes kernel's last block, per host thread (its
-// launches follow one another on the thread's stream); zero between launches.
-unsigned *minmax_ticket() {
-  thread_local unsigned *d = nullptr;
-  if (!d) {
-    LAKGB_CUDA(cudaMalloc(&d, sizeof(unsigned)));
-    LAKGB_CUDA(cudaMemsetAsync(d, 0, sizeof(unsigned), stream()));
-  }
-  return d;
-}
+// The flag of the planes kernel's bounds checks and the ticket of the extremes
+// kernel's last block (its launches follow one another on the thread's stream;
+// zero between launches), per host thread.
+int *bad_flag() { return thread_word(kXcalcBad); }
+unsigned *minmax_ticket() { return reinterpret_cast<unsigned *>(thread_word(kXcalcTicket)); }
 
 // Calls inside a deferral scope: their scalars stay on the device (one
 // XcalcScalars per call, in chunks of kSlots calls) until the scope ends;
