@@ -308,12 +308,12 @@ bitplane_main_kernel(BitplaneParams p) {
 // row, each output is
 //   (pm0(a, plane 0) * min * mlt + sum_{mx = B..1} 2^(B-mx) pm0(a, plane(s, mx))) / mlt
 // in that order.  The pos counts of every (row, plane) pair and the all counts
-// come per 1920-column block from the tensor cores (tc_counts.cu); a thread per
-// (row, s) adds them and forms the output.
+// come per span of 1920-column blocks from the tensor cores (tc_counts.cu); a
+// thread per (row, s) adds them and forms the output.
 struct AnZtSnFinish {
-  const uint16_t *cnt;            // [block][plane][row]
-  const uint16_t *zcnt;           // [block][plane]
-  int n, nplanes, P, nS, ncols_per;
+  const uint16_t *cnt;            // [span][plane][row]
+  const uint16_t *zcnt;           // [span][plane]
+  int n, nplanes, spans, nS, ncols_per;
   int exact;                      // the FP64 sum over the planes is one of integers below 2^53
   double min_d, mlt_d;
   const unsigned long long *out_r; const unsigned long long *s_off;
@@ -328,49 +328,52 @@ struct AnZtSnFinish {
 constexpr int kFinishRows = 32, kFinishPlanes = 64, kFinishWarps = 8;
 __global__ void __launch_bounds__(32 * kFinishWarps) an_ztsn_finish_kernel(AnZtSnFinish p) {
   __shared__ long long pm[kFinishPlanes][kFinishRows];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = blockIdx.y;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row = blockIdx.x * kFinishRows + lane, i = min(row, p.n - 1);
   await_previous();
-  double base = 0.0, tmp = 0.0, n2 = 1.0;
-  long long t = 0;
-  // plane j of the sum: the mask plane, then the value planes from the lowest
-  // bit up
-  for (int j0 = 0; j0 < p.ncols_per; j0 += kFinishPlanes) {
-    const int j1 = min(j0 + kFinishPlanes, p.ncols_per);
-    for (int j = j0 + warp; j < j1; j += kFinishWarps) {
-      const int k = j ? p.ncols_per * s + p.ncols_per - j : 0;
-      const uint16_t *c = p.cnt + (size_t)k * p.n + i, *z = p.zcnt + k;
-      long long pos = 0, all = 0;
+  for (int s = blockIdx.y; s < p.nS; s += gridDim.y) {
+    double base = 0.0, tmp = 0.0, n2 = 1.0;
+    long long t = 0;
+    // plane j of the sum: the mask plane, then the value planes from the lowest
+    // bit up
+    for (int j0 = 0; j0 < p.ncols_per; j0 += kFinishPlanes) {
+      const int j1 = min(j0 + kFinishPlanes, p.ncols_per);
+      for (int j = j0 + warp; j < j1; j += kFinishWarps) {
+        const int k = j ? p.ncols_per * s + p.ncols_per - j : 0;
+        const uint16_t *c = p.cnt + (size_t)k * p.n + i, *z = p.zcnt + k;
+        long long pos = 0, all = 0;
 #pragma unroll 4
-      for (int b = 0; b < p.P; ++b) {
-        pos += c[(size_t)b * p.nplanes * p.n];
-        all += z[(size_t)b * p.nplanes];
+        for (int b = 0; b < p.spans; ++b) {
+          pos += c[(size_t)b * p.nplanes * p.n];
+          all += z[(size_t)b * p.nplanes];
+        }
+        pm[j - j0][lane] = 2ll * pos - all;
       }
-      pm[j - j0][lane] = 2ll * pos - all;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      int j = j0;
-      if (j == 0) base = __dmul_rn(__dmul_rn((double)pm[j++][lane], p.min_d), p.mlt_d);
-      if (p.exact) {
-        for (; j < j1; ++j) t += pm[j - j0][lane] << (j - 1);
-      } else {
-        for (; j < j1; ++j) {
-          tmp = __dadd_rn(tmp, __dmul_rn(n2, (double)pm[j - j0][lane]));
-          n2 *= 2.0;
+      __syncthreads();
+      if (warp == 0) {
+        int j = j0;
+        if (j == 0) base = __dmul_rn(__dmul_rn((double)pm[j++][lane], p.min_d), p.mlt_d);
+        if (p.exact) {
+          for (; j < j1; ++j) t += pm[j - j0][lane] << (j - 1);
+        } else {
+          for (; j < j1; ++j) {
+            tmp = __dadd_rn(tmp, __dmul_rn(n2, (double)pm[j - j0][lane]));
+            n2 *= 2.0;
+          }
         }
       }
+      __syncthreads();
     }
-    __syncthreads();
+    if (warp == 0 && row < p.n) {
+      if (p.exact) tmp = (double)t;
+      p.out[p.out_r[i] + p.s_off[s]] = __ddiv_rn(__dadd_rn(base, tmp), p.mlt_d);
+    }
   }
-  if (warp != 0 || row >= p.n) return;
-  if (p.exact) tmp = (double)t;
-  p.out[p.out_r[i] + p.s_off[s]] = __ddiv_rn(__dadd_rn(base, tmp), p.mlt_d);
 }
 
-// Most bytes of per-block counts a call holds at a time; larger calls take
-// their rows in ranges.
-constexpr size_t kAnZtSnScratch = 256ull << 20;
+// Most bytes of counts a call holds at a time (seven rounds of CTAs); larger
+// calls take their rows in ranges.
+constexpr size_t kAnZtSnScratch = 32ull << 20;
 
 inline unsigned long long pick_u(int s, unsigned long long j, unsigned long long b, unsigned long long a) {
   return s == LAKGB_SPACING_j ? j : (s == LAKGB_SPACING_b ? b : a);
@@ -884,8 +887,10 @@ extern "C" int wrap_An_ZtSn_ww__run(int *tidx, void **vpra, pthread_t *thread_in
   DBuf d_zrow = upload_vec(zrow);
   DBuf mask = upload_bytes(M_An->mc_j, M_An->mc_length);
   const int P = (int)(M_An->mc_length / kBlockBytes), B = M_ZtSn->ncols_per_z - 1;
-  const size_t per_row = (size_t)nplanes * P * sizeof(uint16_t);
-  const int range = (int)std::min<long long>(n, std::max<long long>(128, (long long)(kAnZtSnScratch / std::max<size_t>(per_row, 1)) / 128 * 128));
+  const int span = and_counts_span(n, nplanes, P), spans = (P + span - 1) / span;
+  const size_t per_row = (size_t)nplanes * spans * sizeof(uint16_t);
+  const long long fit = std::max<long long>(kCountsM, (long long)(kAnZtSnScratch / std::max<size_t>(per_row, 1)) / kCountsM * kCountsM);
+  const int range = (int)std::min<long long>(n, std::min<long long>(fit, kCountsMaxRows));
   DBuf d_cnt((size_t)range * per_row), d_zcnt(per_row);
   DBuf d_out(length * sizeof(double));
   if ((unsigned long long)n * nS != length) d_out.zero();
@@ -895,15 +900,15 @@ extern "C" int wrap_An_ZtSn_ww__run(int *tidx, void **vpra, pthread_t *thread_in
     g.wA = An; g.a_rowb = d_rowb.as<uint32_t>() + r0; g.nA = std::min(range, n - r0); g.a_row_bytes = (long long)M_An->mc_length;
     g.wZ = planes; g.z_rowb = d_zrow.as<uint32_t>(); g.nZ = nplanes; g.z_row_bytes = (long long)M_ZtSn->mc_length;
     g.mask = mask.as<uint8_t>(); g.P = P; g.type = 2;
-    if (P > 0 && nplanes > 0) launch_and_counts_tc(g, d_cnt.as<uint16_t>(), d_zcnt.as<uint16_t>(), stream());
+    if (P > 0 && nplanes > 0) launch_and_counts_tc(g, span, d_cnt.as<uint16_t>(), d_zcnt.as<uint16_t>(), stream());
     AnZtSnFinish p{};
     p.cnt = d_cnt.as<uint16_t>(); p.zcnt = d_zcnt.as<uint16_t>();
-    p.n = g.nA; p.nplanes = nplanes; p.P = P; p.nS = nS; p.ncols_per = M_ZtSn->ncols_per_z;
+    p.n = g.nA; p.nplanes = nplanes; p.spans = spans; p.nS = nS; p.ncols_per = M_ZtSn->ncols_per_z;
     p.exact = B < 40 && (double)P * kBlockBits * (double)(1ll << B) <= 9007199254740992.0;
     p.min_d = M_ZtSn->min_d; p.mlt_d = M_ZtSn->mlt_d;
     p.out_r = d_or.as<unsigned long long>() + r0; p.s_off = d_so.as<unsigned long long>();
     p.out = d_out.as<double>();
-    launch_after(an_ztsn_finish_kernel, dim3((g.nA + kFinishRows - 1) / kFinishRows, nS), 32 * kFinishWarps, 0, stream(), p);
+    launch_after(an_ztsn_finish_kernel, dim3((g.nA + kFinishRows - 1) / kFinishRows, std::min(nS, 65535)), 32 * kFinishWarps, 0, stream(), p);
     LAKGB_CUDA(cudaGetLastError());
     count_launch();
   }

@@ -2,11 +2,12 @@
 // launches are too small for the persistent Gram kernel (gram_tc.cu) or have
 // no per-block FP64 fold:
 //
-//   gram_counts_tc_kernel  the counts of one 1920-column block per CTA, written
-//       as 16-bit integers to scratch; gram_fold_kernel then adds each
-//       element's weighted counts in block order.  For launches of few tiles:
-//       every (tile, block) pair is its own CTA, where one CTA per tile would
-//       walk all blocks alone while most SMs idle.
+//   gram_counts_tc_kernel  the counts of a span of 1920-column blocks per CTA,
+//       written as 16-bit integers to scratch.  A Gram weighs its blocks, so its
+//       spans are single blocks; gram_fold_kernel then adds each element's
+//       weighted counts in block order.  For launches of few tiles: every
+//       (tile, block) pair is its own CTA, where one CTA per tile would walk all
+//       blocks alone while most SMs idle.
 //   attyn_tc_kernel        AtTYn_vv / AtTAn_vv (dir_c/AtTYn_vv.c:5-202,
 //       dir_c/AtTAn_vv.c:5-172): the counts of ((At ^ Tt) & mask) xor Yt over
 //       all blocks stay in TMEM, and the epilogue forms the outputs.
@@ -42,6 +43,7 @@ constexpr int kTileA = kM * 64, kTileB = kN * 64, kChunkBytes = kTileA + kTileB;
 constexpr int kSBO = 8 * 64;
 constexpr uint32_t kTmemCols = 128, kSfCol = 64;
 constexpr int kStageBytes = kGroup * kChunkBytes;
+constexpr int kSpanMax = 65535 / kBlockBits;  // blocks whose counts fit 16 bits
 constexpr int kExactBlocks = (1 << 24) / kBlockBits;  // whole blocks whose counts an fp32 sum holds exactly
 constexpr size_t kSmemBytes = 1024 + kStageBytes + (size_t)kRows * kRow + 2 * 256 + kRows * (8 + 4);
 static_assert(2 * (kSmemBytes + 1024 + 64) <= 228 * 1024, "two CTAs per SM");
@@ -215,9 +217,10 @@ __device__ __forceinline__ int decode_count(uint32_t bits) {
   return (int)__float2int_rn(__uint_as_float(bits));
 }
 
+// Span blockIdx.z: blocks [span * z, span * z + span) of p.P, span <= kSpanMax.
 template <int TYPE>
 __global__ void __launch_bounds__(kThreads, 2)
-    gram_counts_tc_kernel(GramParams p, uint16_t *__restrict__ out, uint16_t *__restrict__ zcnt, int *status) {
+    gram_counts_tc_kernel(GramParams p, int span, uint16_t *__restrict__ out, uint16_t *__restrict__ zcnt, int *status) {
   extern __shared__ __align__(128) uint8_t dsm[];
   __shared__ Smem sm;
   const int m0 = blockIdx.y * kM, n0 = blockIdx.x * kN, b = blockIdx.z;
@@ -226,7 +229,8 @@ __global__ void __launch_bounds__(kThreads, 2)
   const TileRows t{p.wA, p.a_rowb, p.nA, p.a_row_bytes, p.wZ, p.z_rowb, p.nZ, p.z_row_bytes, p.mask, nullptr};
   Tile tile;
   tile.setup(&sm, dsm, t, m0, n0);
-  tile.block<kRows>(t, b, true, false, status);
+  const int b0 = span * b;
+  for (int k = b0; k < min(p.P, b0 + span); ++k) tile.block<kRows>(t, k, k == b0, k > b0, status);
   tile.wait_mma(status);
   if (zcnt && m0 == 0 && threadIdx.x < kN && n0 + (int)threadIdx.x < p.nZ)
     zcnt[(size_t)b * p.nZ + n0 + threadIdx.x] = (uint16_t)tile.cnt[kM + threadIdx.x];
@@ -380,21 +384,21 @@ void allow_smem(K kernel) {
 }
 
 template <int TYPE>
-void launch_counts(const GramParams &p, uint16_t *cnt, uint16_t *zcnt, cudaStream_t s) {
+void launch_counts(const GramParams &p, int span, uint16_t *cnt, uint16_t *zcnt, cudaStream_t s) {
   static const bool configured = [] {
     allow_smem(gram_counts_tc_kernel<TYPE>);
     return true;
   }();
   (void)configured;
-  const dim3 grid((p.nZ + kN - 1) / kN, (p.nA + kM - 1) / kM, p.P);
-  gram_counts_tc_kernel<TYPE><<<grid, kThreads, kSmemBytes, s>>>(p, cnt, zcnt, tc_status_device_ptr());
+  const dim3 grid((p.nZ + kN - 1) / kN, (p.nA + kM - 1) / kM, (p.P + span - 1) / span);
+  gram_counts_tc_kernel<TYPE><<<grid, kThreads, kSmemBytes, s>>>(p, span, cnt, zcnt, tc_status_device_ptr());
   LAKGB_CUDA(cudaGetLastError());
   count_launch();
 }
 
 template <int TYPE>
 void launch_split_type(const GramParams &p, uint16_t *cnt, cudaStream_t s) {
-  launch_counts<TYPE>(p, cnt, nullptr, s);
+  launch_counts<TYPE>(p, 1, cnt, nullptr, s);
   const int bx = std::min(256, (p.nA + 31) / 32 * 32), by = 256 / bx;
   const dim3 fold((p.nA + bx - 1) / bx, std::min((p.nZ + by - 1) / by, 65535));
   launch_after(gram_fold_kernel<TYPE>, fold, dim3(bx, by), 0, s, p, cnt);
@@ -411,8 +415,18 @@ void launch_gram_tc_split(const GramParams &p, uint16_t *cnt, cudaStream_t s) {
     launch_split_type<2>(p, cnt, s);
 }
 
-void launch_and_counts_tc(const GramParams &p, uint16_t *cnt, uint16_t *zcnt, cudaStream_t s) {
-  launch_counts<2>(p, cnt, zcnt, s);
+// As many blocks as leave two rounds of the 304 CTAs that run at once (one or
+// four rounds: within 10 % either way).  A CTA per block writes, and the sum
+// reads, the counts of every block: for 16384 rows x 99 planes x 69 blocks, 224
+// MB of them, 503 us and 200 us, a call of 780 us where one CTA per tile walking
+// all blocks had taken 667; with spans it takes 440.
+int and_counts_span(long long nA, long long nZ, int P) {
+  const long long tiles = ((nA + kM - 1) / kM) * ((nZ + kN - 1) / kN);
+  return (int)std::max(1ll, std::min<long long>(kSpanMax, tiles * P / 608));
+}
+
+void launch_and_counts_tc(const GramParams &p, int span, uint16_t *cnt, uint16_t *zcnt, cudaStream_t s) {
+  launch_counts<2>(p, span, cnt, zcnt, s);
 }
 
 namespace {

@@ -9,14 +9,17 @@ namespace lakgb {
 struct GramParams;
 
 constexpr int kCountsM = 128, kCountsN = 64;  // tile rows of A and Z
+constexpr int kCountsMaxRows = 65535 * kCountsM;
 
 // The Gram p as per-block counts (cnt: P x nZ x nA 16-bit integers of scratch)
 // and a fold over the blocks in order.  P <= 65535.
 void launch_gram_tc_split(const GramParams &p, uint16_t *cnt, cudaStream_t s);
 
-// The per-block counts alone: cnt as above (popcount(A & Z & mask)) and zcnt,
-// P x nZ: popcount(Z & mask).
-void launch_and_counts_tc(const GramParams &p, uint16_t *cnt, uint16_t *zcnt, cudaStream_t s);
+// The counts alone, per span of blocks: cnt (spans x nZ x nA 16-bit integers:
+// popcount(A & Z & mask)) and zcnt (spans x nZ: popcount(Z & mask)), with
+// ceil(P / span) spans of and_counts_span(...) blocks; nA <= kCountsMaxRows.
+int and_counts_span(long long nA, long long nZ, int P);
+void launch_and_counts_tc(const GramParams &p, int span, uint16_t *cnt, uint16_t *zcnt, cudaStream_t s);
 
 // AtTYn_vv and, with `symmetric`, AtTAn_vv.
 struct AtTYnParams {
