@@ -382,9 +382,10 @@ void lakgb_server_destroy(struct lakgb_server *s);
 #define LAKGB_E_DEADLINE 7
 long long lakgb_bcc_footprint(const struct lakgb_bcc_problem *p);
 /* High-water mark (bytes) of the device memory held by the library's
- * stream-ordered allocations (the device's default memory pool) since the
- * last reset; reset != 0 restarts it from the current use.  Lets a caller
- * compare lakgb_bcc_footprint with what a solve really held. */
+ * stream-ordered allocations (the device's default memory pool, and the pool
+ * of the Grams' scratch) since the last reset; reset != 0 restarts it from the
+ * current use.  Lets a caller compare lakgb_bcc_footprint with what a solve
+ * really held. */
 long long lakgb_pool_high_water(int reset);
 /* Solve n problems on a server of `workers` threads; returns the number that
  * failed (per-problem status in rcs, may be NULL). */
@@ -537,9 +538,10 @@ int lakgb_thread_error_take(char *msg, int msg_len);
  * for the length of the solve whatever this setting is. */
 void lakgb_set_residency(int on);
 void lakgb_forget_host_buffer(const void *host_ptr);
-/* Staging buffers (page-locked and device memory) that host threads which have
- * ended left for the next ones; returns their bytes and, with release != 0,
- * frees them.  At most eight threads' buffers are kept. */
+/* Memory kept for later calls: staging buffers (page-locked and device memory)
+ * that host threads which have ended left for the next ones, at most eight
+ * threads', and up to 64 MB of the Grams' device scratch.  Returns the bytes and,
+ * with release != 0, frees them. */
 long long lakgb_idle_buffers(int release);
 /* D_MLT used by wrap_xcalc (the reference's GLOBAL_D_MLT, default 2^32). */
 void lakgb_set_d_mlt(long long d_mlt);

@@ -190,8 +190,7 @@ constexpr size_t kSplitMaxBytes = size_t(256) << 20;
 size_t split_bytes(const GramParams &p) { return (size_t)p.P * (size_t)p.nA * (size_t)p.nZ * sizeof(uint16_t); }
 
 void launch_split(const GramParams &p, cudaStream_t s) {
-  uint16_t *cnt = nullptr;
-  LAKGB_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&cnt), split_bytes(p), s));
+  uint16_t *cnt = static_cast<uint16_t *>(scratch_alloc(split_bytes(p), s));
   launch_gram_tc_split(p, cnt, s);
   LAKGB_CUDA(cudaFreeAsync(cnt, s));
 }

@@ -943,8 +943,7 @@ void launch_tc_group_type(const GramGroupDev &g, int total_tiles, const uint8_t 
 }  // namespace
 
 void launch_gram_tc(const GramParams &p, cudaStream_t s) {
-  uint8_t *T = nullptr;
-  LAKGB_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&T), (size_t)p.P * kTabBytes, s));
+  uint8_t *T = static_cast<uint8_t *>(scratch_alloc((size_t)p.P * kTabBytes, s));
   gram_table_kernel<<<dim3(p.P, kTableParts), 256, 0, s>>>(p, T);
   LAKGB_CUDA(cudaGetLastError());
   count_launch();

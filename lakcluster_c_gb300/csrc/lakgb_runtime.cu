@@ -273,6 +273,41 @@ void dfree(void *p) {
   if (p) LAKGB_CUDA(cudaFreeAsync(p, stream()));
 }
 
+namespace {
+constexpr int kMaxDevices = 64;
+std::mutex g_scratch_mu;
+cudaMemPool_t g_scratch_pool[kMaxDevices] = {nullptr};
+
+// The current device's scratch pool; null if there is none and `make` is false.
+cudaMemPool_t scratch_pool(bool make) {
+  int dev = 0;
+  LAKGB_CUDA(cudaGetDevice(&dev));
+  if (dev >= kMaxDevices) return nullptr;
+  std::lock_guard<std::mutex> lk(g_scratch_mu);
+  cudaMemPool_t &pool = g_scratch_pool[dev];
+  if (!pool && make) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    LAKGB_CUDA(cudaMemPoolCreate(&pool, &props));
+    uint64_t kept = kScratchKept;
+    LAKGB_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept));
+  }
+  return pool;
+}
+}  // namespace
+
+void *scratch_alloc(size_t bytes, cudaStream_t s) {
+  void *p = nullptr;
+  cudaMemPool_t pool = capturing(s) ? nullptr : scratch_pool(true);
+  if (pool)
+    LAKGB_CUDA(cudaMallocFromPoolAsync(&p, bytes, pool, s));
+  else
+    LAKGB_CUDA(cudaMallocAsync(&p, bytes, s));
+  return p;
+}
+
 void DBuf::upload(const void *h, size_t bytes) {
   if (bytes) LAKGB_CUDA(cudaMemcpyAsync(p, h, bytes, cudaMemcpyHostToDevice, stream()));
 }
@@ -456,19 +491,22 @@ using namespace lakgb;
 
 // High-water mark of the device memory the library's stream-ordered
 // allocations hold (the current device's default memory pool, from which
-// every working buffer, mirror and resident copy comes), optionally reset.
+// every working buffer, mirror and resident copy comes, and the scratch pool;
+// the sum of their marks), optionally reset.
 extern "C" long long lakgb_pool_high_water(int reset) {
   int dev = 0;
   LAKGB_CUDA(cudaGetDevice(&dev));
-  cudaMemPool_t pool;
-  LAKGB_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
-  unsigned long long v = 0;
-  LAKGB_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemHigh, &v));
-  if (reset) {
-    unsigned long long zero = 0;
-    LAKGB_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrUsedMemHigh, &zero));
+  cudaMemPool_t pools[2] = {nullptr, scratch_pool(false)};
+  LAKGB_CUDA(cudaDeviceGetDefaultMemPool(&pools[0], dev));
+  unsigned long long sum = 0;
+  for (cudaMemPool_t pool : pools) {
+    if (!pool) continue;
+    unsigned long long v = 0, zero = 0;
+    LAKGB_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemHigh, &v));
+    if (reset) LAKGB_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrUsedMemHigh, &zero));
+    sum += v;
   }
-  return (long long)v;
+  return (long long)sum;
 }
 
 extern "C" int lakgb_thread_error_take(char *msg, int msg_len) {
@@ -521,6 +559,13 @@ extern "C" long long lakgb_idle_buffers(int release) {
   for (lakgb::ThreadBuffers *b : lakgb::idle_buffers()) {
     n += lakgb::buffer_bytes(*b);
     if (release) lakgb::free_buffers(*b);
+  }
+  if (cudaMemPool_t pool = lakgb::scratch_pool(false)) {
+    unsigned long long reserved = 0, used = 0;
+    LAKGB_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+    LAKGB_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+    if (reserved > used) n += (long long)(reserved - used);
+    if (release) LAKGB_CUDA(cudaMemPoolTrimTo(pool, 0));
   }
   return n;
 }

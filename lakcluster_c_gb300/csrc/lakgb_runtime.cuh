@@ -98,6 +98,14 @@ __device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.la
 void *dalloc(size_t bytes);
 void dfree(void *p);
 
+// Scratch of a kernel on stream s, freed by cudaFreeAsync(p, s).  From a pool that
+// keeps up to kScratchKept bytes when the stream is waited for: the default pool
+// gives unused memory back at every synchronisation, and a call that found it
+// empty took 190 us where its kernels take 20.  lakgb_idle_buffers(1) gives it
+// back.  (While s is captured the memory belongs to the graph.)
+constexpr size_t kScratchKept = 64u << 20;
+void *scratch_alloc(size_t bytes, cudaStream_t s);
+
 // Device copy of a host buffer.  With residency on (residency_enabled()),
 // buffers are cached by (host pointer, size) and reused without re-upload;
 // otherwise the copy goes into the call's staging arena (the caller holds a
