@@ -185,7 +185,7 @@ void launch_tile(const GramParams &p) {
   count_launch();
 }
 
-// Scratch bytes of the split launch; above kSplitMaxBytes it is not used.
+// Scratch bytes of the split launch; above kSplitMaxBytes the persistent kernel runs.
 constexpr size_t kSplitMaxBytes = size_t(256) << 20;
 size_t split_bytes(const GramParams &p) { return (size_t)p.P * (size_t)p.nA * (size_t)p.nZ * sizeof(uint16_t); }
 
@@ -199,41 +199,49 @@ void launch_split(const GramParams &p, cudaStream_t s) {
 
 // ---------------------------------------------------------------------------
 // Kernel choice.  Every candidate computes the same outputs bit for bit, so
-// the choice is a matter of speed only.  With LAKGB_IMPL_AUTO (the default)
-// a launch with at least kTensorRows rows on both sides takes the persistent
-// tensor-core kernel; for smaller launches the first one of each shape class
-// -- (type, symmetric, log2 of the A rows, of the Z rows and of the blocks) --
-// runs that kernel and the tensor-core counts split over blocks (tc_counts.cu)
-// on its real arguments, timed with CUDA events on the launching stream, and
-// the faster serves that class from then on.  (Measured on the 120 classes of
-// a case/control solve, 9 blocks: split 17 to 34 us, persistent 60 to 81 us up
-// to 512 x 512 rows, 99 and 81 us at 512 x 4096; the popcount kernels, 113 to
-// 256 us, are the fastest in no class and are not timed.)
+// the choice is a matter of speed only.  With LAKGB_IMPL_AUTO (the default) the
+// number of 128 x 112 tiles decides, and between the bounds a measurement: the
+// persistent tensor-core kernel walks the blocks of a tile in one CTA, the
+// counts split over blocks (tc_counts.cu) give every (tile, block) its own.
+// Measured at 1 to 64 blocks, 1 x 1000 to 1020 x 30000 rows: up to 60 tiles the
+// split is faster at every number of blocks (7x at 40 x 300 rows, 1.0 to 1.2x
+// at 54 to 60 tiles), from 96 tiles on the persistent kernel is (1.1 to 2x; 0.93x at 1
+// x 30000 rows x 1 block), and between them the faster is ahead by up to 1.4x
+// either way.  So launches of 96 tiles or more, with 1024 rows on both sides or
+// with more counts than the split's scratch takes the persistent kernel; below,
+// the first launch of each shape class -- (type, symmetric, up to 60 tiles or
+// more, log2 of the A rows, of the Z rows and of the blocks) -- runs both on its
+// real arguments, timed with CUDA events on the launching stream, and the faster
+// serves that class from then on.  (Without the tile counts in the class, 520 x
+// 1030 rows chose the split for 1020 x 2040 x 64 blocks: 925 us, persistent 326.)
+// The popcount kernel, 21 to 56 us at one block where the faster of them takes 18 to 43,
+// is the fastest nowhere and is not timed.
 
+// (popcount_64x64 and popcount_64x128 are names of the table only: those tiles
+// are built no more.)
 enum GramVariant { kTensor = 0, kPopc128x64, kPopc64x64, kSplit, kPopc64x128, kNumVariants };
 constexpr int kTuned[] = {kTensor, kSplit};
 constexpr int kTunedVariants = 2;
-constexpr int kTensorRows = 1024;
+constexpr int kTensorRows = 1024, kTensorTiles = 96, kSplitTiles = 60;
 const char *const kVariantName[kNumVariants] = {"tensor_128x112", "popcount_128x64", "popcount_64x64",
                                                 "split_128x64", "popcount_64x128"};
+
+bool split_fits(const GramParams &p) {
+  return p.P <= 65535 && p.nA <= kCountsMaxRows && split_bytes(p) <= kSplitMaxBytes;
+}
 
 void launch_variant(int v, const GramParams &p, cudaStream_t s) {
   GramParams q = p;
   q.stream = s;
-  if (v == kSplit && (split_bytes(q) > kSplitMaxBytes || q.P > 65535 || q.nA > 65535 * kCountsM)) v = kPopc64x64;
-  if (v == kTensor) {
+  if (v == kSplit && !split_fits(q)) v = kTensor;
+  if (v == kTensor)
     launch_gram_tc(q, s);
-  } else if (v == kSplit) {
+  else if (v == kSplit)
     launch_split(q, s);
-  } else if (q.type == 1) {
-    if (v == kPopc128x64) launch_tile<128, 64, 8, 4, 1>(q);
-    else if (v == kPopc64x64) launch_tile<64, 64, 4, 4, 1>(q);
-    else launch_tile<64, 128, 4, 8, 1>(q);
-  } else {
-    if (v == kPopc128x64) launch_tile<128, 64, 8, 4, 2>(q);
-    else if (v == kPopc64x64) launch_tile<64, 64, 4, 4, 2>(q);
-    else launch_tile<64, 128, 4, 8, 2>(q);
-  }
+  else if (q.type == 1)
+    launch_tile<128, 64, 8, 4, 1>(q);
+  else
+    launch_tile<128, 64, 8, 4, 2>(q);
 }
 
 inline int log2_bucket(long long n) {
@@ -243,9 +251,9 @@ inline int log2_bucket(long long n) {
 }
 
 struct TuneKey {
-  int type, sym, la, lz, lp;
+  int type, sym, la, lz, lp, many;  // many: more than kSplitTiles tiles
   bool operator<(const TuneKey &o) const {
-    return std::tie(type, sym, la, lz, lp) < std::tie(o.type, o.sym, o.la, o.lz, o.lp);
+    return std::tie(type, sym, la, lz, lp, many) < std::tie(o.type, o.sym, o.la, o.lz, o.lp, o.many);
   }
 };
 
@@ -258,8 +266,10 @@ std::mutex g_tune_mu;
 std::map<TuneKey, TuneEntry> g_tune;
 
 int tuned_variant(const GramParams &p, cudaStream_t s, bool *ran) {
-  if (p.nA >= kTensorRows && p.nZ >= kTensorRows) return kTensor;
-  const TuneKey key{p.type, p.symmetric ? 1 : 0, log2_bucket(p.nA), log2_bucket(p.nZ), log2_bucket(p.P)};
+  const int tiles = gram_tc_tiles(p);
+  if ((p.nA >= kTensorRows && p.nZ >= kTensorRows) || tiles >= kTensorTiles || !split_fits(p)) return kTensor;
+  const TuneKey key{p.type, p.symmetric ? 1 : 0, log2_bucket(p.nA), log2_bucket(p.nZ), log2_bucket(p.P),
+                    tiles > kSplitTiles ? 1 : 0};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
@@ -347,9 +357,9 @@ extern "C" int lakgb_gram_autotune_table(char *buf, int buf_len) {
     for (const auto &kv : g_tune) {
       char line[512];
       int n = snprintf(line, sizeof line, "%s{\"type\":%d,\"symmetric\":%d,\"log2_rows_a\":%d,\"log2_rows_z\":%d,"
-                       "\"log2_blocks\":%d,\"choice\":\"%s\",\"ms\":{",
+                       "\"log2_blocks\":%d,\"over_%d_tiles\":%d,\"choice\":\"%s\",\"ms\":{",
                        first ? "" : ",", kv.first.type, kv.first.sym, kv.first.la, kv.first.lz, kv.first.lp,
-                       kVariantName[kv.second.choice]);
+                       kSplitTiles, kv.first.many, kVariantName[kv.second.choice]);
       for (int v = 0; v < kNumVariants; ++v)
         n += snprintf(line + n, sizeof line - n, "%s\"%s\":%.4f", v ? "," : "", kVariantName[v], kv.second.ms[v]);
       snprintf(line + n, sizeof line - n, "}}");
