@@ -18,6 +18,7 @@
 // alone.
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -32,6 +33,7 @@
 #include "../../include/lakcluster_gb300.h"
 #include "bcc_driver.h"
 #include "bcc_model.h"
+#include "scratch_limits.h"
 
 namespace {
 
@@ -79,7 +81,8 @@ struct OwnedProblem {
 // Device bytes a solve holds at its peak (an upper estimate): the packed
 // matrices and their transposes, the FP64 Gram matrices of every bin pair
 // with their low-rank updates (kept on the device for the whole solve), the
-// bit planes of the initial loop product, and the SNP x SNP low-rank blocks.
+// bit planes of the initial loop product, the SNP x SNP low-rank blocks, and the
+// scratch of the kernels, one at a time of each kind.
 long long footprint(const lakgb_bcc_problem &p) {
   const long long m = lakbcc::bsize(p.ncols) * 8;  // padded columns
   long long bytes = 0, rows_total = 0;
@@ -96,8 +99,19 @@ long long footprint(const lakgb_bcc_problem &p) {
   bytes += 8 * 3 * (long long)p.ncols * cdrop * p.nbins;        // SNP x SNP blocks
   if (p.QR_strategy && strstr(p.QR_strategy, "condense"))
     bytes += 8 * (rows_total + rows_total) * cdrop;             // dense removed columns, their uploads
-  bytes += 64ll << 20;                                          // terms of the bit-plane product
-  return bytes + (64ll << 20);                                // staging arena, scratch
+  long long counts = 0, split = 0;
+  const long long blocks = m / lakbcc::POPLENGTH, planes = (long long)(p.B_MLT + 1) * std::max(1, p.T_ncols);
+  for (int a = 0; a < p.nbins; ++a)
+    for (int b = 0; b < p.nbins; ++b) {
+      const long long na = p.bins[a].A_nrows, n = std::max(p.bins[b].Z_nrows, p.bins[b].A_nrows);
+      counts = std::max(counts, 2 * std::max(na, n) * planes * blocks);
+      split = std::max(split, 2 * na * n * blocks);
+    }
+  bytes += std::min<long long>(counts, lakgb::kAnZtSnScratch);   // counts of An_ZtSn
+  bytes += std::min<long long>(split, lakgb::kSplitMaxBytes);    // counts of a split Gram
+  bytes += lakgb::kBitplaneScratchBytes;                        // terms of the bit-plane product
+  bytes += lakgb::kArenas * lakgb::kArenaBytes + lakgb::kIdleUpChunks * lakgb::kUpChunk;  // the thread's staging
+  return bytes + (64ll << 20);                                // block tables, small arrays
 }
 
 struct Job {

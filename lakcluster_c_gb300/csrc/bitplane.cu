@@ -371,10 +371,6 @@ __global__ void __launch_bounds__(32 * kFinishWarps) an_ztsn_finish_kernel(AnZtS
   }
 }
 
-// Most bytes of counts a call holds at a time (seven rounds of CTAs); larger
-// calls take their rows in ranges.
-constexpr size_t kAnZtSnScratch = 32ull << 20;
-
 inline unsigned long long pick_u(int s, unsigned long long j, unsigned long long b, unsigned long long a) {
   return s == LAKGB_SPACING_j ? j : (s == LAKGB_SPACING_b ? b : a);
 }
@@ -888,6 +884,8 @@ extern "C" int wrap_An_ZtSn_ww__run(int *tidx, void **vpra, pthread_t *thread_in
   DBuf mask = upload_bytes(M_An->mc_j, M_An->mc_length);
   const int P = (int)(M_An->mc_length / kBlockBytes), B = M_ZtSn->ncols_per_z - 1;
   const int span = and_counts_span(n, nplanes, P), spans = (P + span - 1) / span;
+  // at most kAnZtSnScratch bytes of counts at a time (seven rounds of CTAs): larger
+  // calls take their rows in ranges
   const size_t per_row = (size_t)nplanes * spans * sizeof(uint16_t);
   const long long fit = std::max<long long>(kCountsM, (long long)(kAnZtSnScratch / std::max<size_t>(per_row, 1)) / kCountsM * kCountsM);
   const int range = (int)std::min<long long>(n, std::min<long long>(fit, kCountsMaxRows));

@@ -6,6 +6,8 @@
 
 #include <vector>
 
+#include "scratch_limits.h"
+
 namespace lakgb {
 
 struct BitplaneParams {
@@ -57,8 +59,8 @@ size_t bitplane_tc_plan(int B, const std::vector<BitplaneParams> &ps, std::vecto
                         std::vector<BitplaneBatch> *batches);
 void launch_bitplane_tc(int B, const BitplaneParams *d_ps, const BitplaneSeg *d_segs,
                         const std::vector<BitplaneBatch> &batches, double *scratch, cudaStream_t s);
-// Most doubles of scratch (64 MB) that the terms of a batch take; one step of
-// Wn rows of one column always fits.
-constexpr size_t kBitplaneScratch = size_t(8) << 20;
+// Most doubles of scratch that the terms of a batch take; one step of Wn rows of
+// one column always fits.
+constexpr size_t kBitplaneScratch = kBitplaneScratchBytes / sizeof(double);
 
 }  // namespace lakgb

@@ -186,7 +186,6 @@ void launch_tile(const GramParams &p) {
 }
 
 // Scratch bytes of the split launch; above kSplitMaxBytes the persistent kernel runs.
-constexpr size_t kSplitMaxBytes = size_t(256) << 20;
 size_t split_bytes(const GramParams &p) { return (size_t)p.P * (size_t)p.nA * (size_t)p.nZ * sizeof(uint16_t); }
 
 void launch_split(const GramParams &p, cudaStream_t s) {

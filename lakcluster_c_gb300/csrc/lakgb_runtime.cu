@@ -218,7 +218,7 @@ void Stager::begin() {
   b.arena = (b.arena + 1) % kArenas;
   Arena &a = arena();
   if (!a.host) {
-    a.cap = kStageBytes;
+    a.cap = kArenaBytes;
     LAKGB_CUDA(cudaMallocHost((void **)&a.host, a.cap));
     LAKGB_CUDA(cudaMalloc((void **)&a.dev, a.cap));
     LAKGB_CUDA(cudaEventCreateWithFlags(&a.done, cudaEventDisableTiming));

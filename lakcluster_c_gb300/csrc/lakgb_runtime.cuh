@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/lakcluster_gb300.h"
+#include "scratch_limits.h"
 
 namespace lakgb {
 
@@ -47,9 +48,7 @@ struct Arena {
   bool pending = false;
 };
 struct UpChunk { uint8_t *h = nullptr; uint8_t *d = nullptr; size_t cap = 0, used = 0, sent = 0; };
-constexpr int kArenas = 8;
-constexpr size_t kUpChunk = 4u << 20;      // bytes of an ordinary UpChunk
-constexpr int kIdleBuffers = 8, kIdleUpChunks = 4;
+constexpr int kIdleBuffers = 8;
 struct ThreadBuffers {
   int device = 0, pid = 0;
   cudaStream_t stream = nullptr, copy = nullptr;
@@ -164,7 +163,6 @@ struct DBuf {
 // copy for all of them.  Arrays that do not fit the arena are uploaded on
 // their own.  One Stager per call; a thread's arenas are used in turn, each
 // again once its copy has completed.
-constexpr size_t kStageBytes = 4u << 20;
 // Arrays of at least this many bytes skip the arena (one direct copy each).
 constexpr size_t kDirectUploadBytes = 1u << 20;
 class Stager {
