@@ -768,10 +768,11 @@ extern "C" int wrap_At_T_YnWt_S_Zn_ww__run(int *tidx, void **vpra, pthread_t *th
     while (last >= 0 && !M_At->mc_j[last]) --last;
     p.chunks = (int)(last / 16 + (last >= 0 ? 1 : 0));
     // The division by mlt as multiplications by its reciprocal (bitplane_tc.cu)
-    // needs quotients and remainders far from overflow and underflow.
+    // needs quotients and remainders far from overflow and underflow (a
+    // numerator may be the minimum's term alone).
     const double lim = 1.2676506002282294e30;  // 2^100
-    const double m = M_YnWt->mlt_d, lo = M_YnWt->min_d;
-    if (m >= 1.0 / lim && m <= lim && lo >= -lim && lo <= lim) p.inv_mlt = 1.0 / m;
+    const double m = M_YnWt->mlt_d, lo = fabs(M_YnWt->min_d);
+    if (m >= 1.0 / lim && m <= lim && (lo == 0.0 || (lo >= 1.0 / lim && lo <= lim))) p.inv_mlt = 1.0 / m;
   }
   if (defer) defer_flush();
   p.at_rowb = d_at.as<uint32_t>(); p.zt_rowb = d_zt.as<uint32_t>(); p.tt_rowb = d_tt.as<uint32_t>();
