@@ -242,11 +242,26 @@ thread_local std::vector<DeferCopy> t_copies;  // other calls' outputs
 constexpr size_t kDownEach = 64u << 10;
 struct DownCopy { double *host; size_t off, bytes; };
 
-// Enqueue the copy of `length` doubles of `dev` to `host`.
+// Wait for the copies into the page-locked buffer and pass them on.
+void finish_down(std::vector<DownCopy> &later) {
+  LAKGB_CUDA(cudaStreamSynchronize(stream()));
+  for (const DownCopy &c : later) memcpy(c.host, thread_buffers().down + c.off, c.bytes);
+  later.clear();
+}
+
+// Enqueue the copy of `length` doubles of `dev` to `host`.  Where two calls of a
+// scope write the same host memory the later copy's values stay: a direct copy
+// comes after the held-back ones that it overlaps.
 void copy_down(double *host, const double *dev, unsigned long long length, size_t &used, std::vector<DownCopy> &later) {
   const size_t bytes = length * sizeof(double);
   if (!bytes) return;
   if (bytes > kDownEach || used + bytes > kDownBytes) {
+    const auto at = [](const double *p) { return reinterpret_cast<uintptr_t>(p); };
+    for (const DownCopy &c : later)
+      if (at(c.host) < at(host) + bytes && at(host) < at(c.host) + c.bytes) {
+        finish_down(later);
+        break;
+      }
     LAKGB_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, stream()));
     return;
   }
@@ -429,8 +444,7 @@ extern "C" void lakgb_defer_end(void) {
     for (auto &d : t_swnyt) copy_down(d.host_out, d.c.out, d.length, used, later);
     for (auto &d : t_wtsz) copy_down(d.host_out, d.c.out, d.length, used, later);
     for (auto &c : t_copies) copy_down(c.host, c.dev.as<double>(), c.length, used, later);
-    LAKGB_CUDA(cudaStreamSynchronize(stream()));
-    for (const DownCopy &c : later) memcpy(c.host, thread_buffers().down + c.off, c.bytes);
+    finish_down(later);
   }
   t_copies.clear();
   for (UpChunk &c : thread_buffers().up) c.used = c.sent = 0;  // the stream has drained: reuse the chunks
