@@ -794,7 +794,7 @@ extern "C" int wrap_At_T_YnWt_S_Zn_ww__run(int *tidx, void **vpra, pthread_t *th
   }
   DBuf d_out(length * sizeof(double));
   // the kernels write every pair and covariate column
-  if (nW == 0 || (unsigned long long)npairs * nT != length) d_out.zero();
+  if ((unsigned long long)npairs * nT != length) d_out.zero();
   p.ycnt = d_ycnt.as<int>(); p.T_base = d_Tb.as<double>(); p.T_tmp = d_Tt.as<double>();
   p.At_base = d_Ab.as<double>(); p.zz = d_zz.as<double2>();
   p.ysum = d_ys.as<long long>(); p.q2 = d_q2.as<double>();

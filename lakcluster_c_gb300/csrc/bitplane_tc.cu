@@ -425,7 +425,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   }
 
-  release_next();
   tc::fence_before_sync();
   __syncthreads();
   if (warp == kMmaWarp) {

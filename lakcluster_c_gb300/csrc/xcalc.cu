@@ -137,7 +137,7 @@ __device__ void make_scalars(unsigned long long kmn, unsigned long long kmx, boo
     r.frac = -1;
   } else {
     const unsigned long long mb = (unsigned long long)__double_as_longlong(r.mlt);
-    const int s = (int)(mb >> 52) - 1075 + e + 2 + r.frac;  // 6 <= s <= 10: 2^58 < K <= 2^63
+    const int s = (int)(mb >> 52) - 1075 + e + 2 + r.frac;  // 9 <= s <= 11: 2^61 < K <= 2^63
     r.K = ((mb & 0x000fffffffffffffull) | 0x0010000000000000ull) << s;
   }
   *out = r;
