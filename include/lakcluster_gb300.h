@@ -486,12 +486,11 @@ void lakgb_defer_end(void);
  * must not allocate device memory -- e.g. a process whose device memory is
  * fully reserved up front by its own pool (the serving loop admits solves by
  * HBM footprint), or code on a path where a cudaMalloc would synchronise the
- * device.  Its scratch is one static device array of
- * 3 * LAKGB_XCALC_NOALLOC_MAX_COLS + 4 doubles (786,464 bytes), so at most
- * LAKGB_XCALC_NOALLOC_MAX_COLS retained columns; larger problems are rejected
- * with an error.  The array is shared by every call on a device: calls whose
- * kernels overlap on the GPU race.  The first call on a device looks the array
- * up (cudaGetSymbolAddress) and should come before any stream capture.
+ * device.  Its scratch is one static device array of about 20 KB, shared by
+ * every call on a device: calls whose kernels overlap on the GPU race.  More
+ * than LAKGB_XCALC_NOALLOC_MAX_COLS retained columns are rejected with an
+ * error.  The first call on a device looks the array up (cudaGetSymbolAddress)
+ * and should come before any stream capture.
  * The call is synchronous: it returns once its GPU work is done (it reads
  * {min, max, mlt} back into host memory).
  * Inputs (device): lf, the element offset of each Yn a-row (-1 = not

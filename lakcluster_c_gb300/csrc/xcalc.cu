@@ -51,7 +51,6 @@ struct XcalcScalars {
   unsigned long long span;    // largest value - lo in fixed point
   int shift0, frac;
 };
-static_assert(sizeof(XcalcScalars) <= 64, "eight doubles of scratch");
 
 struct XcalcParams {
   const double *lf;
@@ -418,14 +417,16 @@ dim3 minmax_grid(int nr, int nc) {
 //
 // lakgb_xcalc_noalloc runs the same kernels on caller-owned device buffers
 // for callers that cannot allocate device memory.  Its only scratch is this
-// file-scope array (786,464 bytes): the blocks' partial extremes, the scalars
-// and the ticket of the last block.  Every entry a call reads is written
-// earlier in the same call; the array is shared by every call on a device, so
-// calls whose kernels overlap on the GPU race.
+// file-scope array: the blocks' partial extremes, the scalars and the ticket of
+// the last block.  Every entry a call reads is written earlier in the same call;
+// the array is shared by every call on a device, so calls whose kernels overlap
+// on the GPU race.  (The scratch does not grow with the columns any more; their
+// limit is one of the interface.)
 constexpr int kNoAllocMaxCols = LAKGB_XCALC_NOALLOC_MAX_COLS;
-static __device__ __align__(256) double g_xcalc_noalloc_scratch[3 * kNoAllocMaxCols + 4];
 constexpr int kScratchScalars = 2 * kMinMaxBlocks;       // doubles from the start
-constexpr int kScratchTicket = kScratchScalars + 8;
+constexpr int kScratchTicket = kScratchScalars + (int)(sizeof(XcalcScalars) / sizeof(double));
+static __device__ __align__(256) double g_xcalc_noalloc_scratch[kScratchTicket + 1];
+static_assert(sizeof(ulonglong2) == 2 * sizeof(double) && sizeof(XcalcScalars) % sizeof(double) == 0, "whole doubles");
 
 std::mutex g_noalloc_mu;
 void *g_noalloc_scratch[64] = {nullptr};
