@@ -571,13 +571,12 @@ void lakgb_call_profile_reset(void);
 #define LAKGB_GRAM_AUTO LAKGB_IMPL_AUTO
 void lakgb_set_gram_impl(int impl);
 int lakgb_gram_impl(void);
-/* LAKGB_GRAM_AUTO (the default) picks the Gram kernel by the number of output
- * tiles of 128 x 112 and, below 96 tiles and 1024 rows on a side, by measurement:
- * the first launch of each shape class (type, symmetric, up to 60 tiles or more,
- * log2 of the A rows, Z rows and blocks) runs the candidates -- the persistent
- * tensor-core kernel and the counts split over blocks, bit-identical -- timed
- * with CUDA events, and the faster serves that class afterwards (a kernel that
- * was not timed reads -1 in the table).
+/* LAKGB_GRAM_AUTO (the default) takes the persistent tensor-core kernel from 1024
+ * rows on both sides, the cheaper of it and the counts split over blocks (both
+ * bit-identical) by their costs above 60 output tiles of 128 x 112, and measures up
+ * to 60 tiles: the first launch of each shape class (type, symmetric, log2 of the A
+ * rows, Z rows and blocks) runs both, timed with CUDA events, and the faster serves
+ * that class afterwards (a kernel that was not timed reads -1 in the table).
  * lakgb_gram_autotune_table writes the table as JSON into buf (returns its
  * full length); lakgb_gram_autotune_reset clears it. */
 int lakgb_gram_autotune_table(char *buf, int buf_len);

@@ -26,6 +26,7 @@
 #include <tuple>
 #include <vector>
 #include <climits>
+#include <cmath>
 
 #include "gram.cuh"
 #include "lakgb_runtime.cuh"
@@ -199,20 +200,18 @@ void launch_split(const GramParams &p, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 // Kernel choice.  Every candidate computes the same outputs bit for bit, so
 // the choice is a matter of speed only.  With LAKGB_IMPL_AUTO (the default) the
-// number of 128 x 112 tiles decides, and between the bounds a measurement: the
-// persistent tensor-core kernel walks the blocks of a tile in one CTA, the
-// counts split over blocks (tc_counts.cu) give every (tile, block) its own.
-// Measured at 1 to 64 blocks, 1 x 1000 to 1020 x 30000 rows: up to 60 tiles the
-// split is faster at every number of blocks (7x at 40 x 300 rows, 1.0 to 1.2x
-// at 54 to 60 tiles), from 96 tiles on the persistent kernel is (1.1 to 2x; 0.93x at 1
-// x 30000 rows x 1 block), and between them the faster is ahead by up to 1.4x
-// either way.  So launches of 96 tiles or more, with 1024 rows on both sides or
-// with more counts than the split's scratch takes the persistent kernel; below,
-// the first launch of each shape class -- (type, symmetric, up to 60 tiles or
-// more, log2 of the A rows, of the Z rows and of the blocks) -- runs both on its
-// real arguments, timed with CUDA events on the launching stream, and the faster
-// serves that class from then on.  (Without the tile counts in the class, 520 x
-// 1030 rows chose the split for 1020 x 2040 x 64 blocks: 925 us, persistent 326.)
+// number of 128 x 112 tiles decides how: the persistent tensor-core kernel walks the
+// blocks of a tile in one CTA, the counts split over blocks (tc_counts.cu) give every
+// (tile, block) its own.
+// 1024 rows on both sides, or more counts than the split's scratch: persistent.
+// Above 60 tiles: the cheaper by split_is_cheaper's costs.  Up to 60 tiles, where the
+// split is nearly always faster (7x at 40 x 300 rows, 1.0 to 1.2x at 54 to 60 tiles),
+// the first launch of each shape class -- (type, symmetric, log2 of the A rows, of
+// the Z rows and of the blocks) -- runs both on its real arguments, timed with CUDA
+// events, and the faster serves that class from then on.  (Classes above 60 tiles
+// hold both kinds: 520 x 1030 rows chose the split for 1020 x 2040 x 64 blocks, 925 us
+// where the persistent kernel takes 326; the number of tiles alone, persistent from 96
+// on, took 43 us for 6454 x 113 x 2 blocks and 57 for 300 x 6454 x 1, split 30 and 45.)
 // The popcount kernel, 21 to 56 us at one block where the faster of them takes 18 to 43,
 // is the fastest nowhere and is not timed.
 
@@ -221,12 +220,31 @@ void launch_split(const GramParams &p, cudaStream_t s) {
 enum GramVariant { kTensor = 0, kPopc128x64, kPopc64x64, kSplit, kPopc64x128, kNumVariants };
 constexpr int kTuned[] = {kTensor, kSplit};
 constexpr int kTunedVariants = 2;
-constexpr int kTensorRows = 1024, kTensorTiles = 96, kSplitTiles = 60;
+constexpr int kTensorRows = 1024, kSplitTiles = 60;
 const char *const kVariantName[kNumVariants] = {"tensor_128x112", "popcount_128x64", "popcount_64x64",
                                                 "split_128x64", "popcount_64x128"};
 
 bool split_fits(const GramParams &p) {
   return p.P <= 65535 && p.nA <= kCountsMaxRows && split_bytes(p) <= kSplitMaxBytes;
+}
+
+// Times of the two kernels in us, fitted to 306 shapes (1 to 400 rows on one side, 3000
+// to 30000 on the other, 1 to 69 blocks).  On 260 other shapes, drawn up to 150 blocks,
+// the kernel taken is 0.5 % slower than the faster one on average, at most 15 %.
+// Persistent: every tile of the CTA with the most costs 4.4 a block and 15.3 for
+// results of full width.  Split: 304
+// CTAs count at a time, 9.1 a round (the first in the constant); the fold costs 9.5 per
+// million elements and 2.1 more per block.
+bool split_is_cheaper(const GramParams &p, int tiles) {
+  const auto up = [](long long n, long long d) { return (n + d - 1) / d; };
+  const double tn = (double)up(p.nZ, kGramTileN), blocks = (double)p.P;
+  const double active = tiles / (tn * (double)up(p.nA, kGramTileM));  // 1, about 1/2 for a symmetric Gram
+  const double waves = (double)up(tiles, 152), width = p.nZ / (tn * kGramTileN);
+  const double rounds = active * (double)(up(p.nA, kCountsM) * up(p.nZ, kCountsN)) * blocks / 304.0;
+  const double elements = active * (double)p.nA * (double)p.nZ * 1e-6;
+  const double persistent = 17.5 + waves * (4.4 * blocks + 15.3 * width);
+  const double split = 19.5 + elements * (9.5 + 2.1 * blocks) + 9.1 * (std::ceil(rounds) - 1.0);
+  return split < persistent;
 }
 
 void launch_variant(int v, const GramParams &p, cudaStream_t s) {
@@ -250,9 +268,9 @@ inline int log2_bucket(long long n) {
 }
 
 struct TuneKey {
-  int type, sym, la, lz, lp, many;  // many: more than kSplitTiles tiles
+  int type, sym, la, lz, lp;
   bool operator<(const TuneKey &o) const {
-    return std::tie(type, sym, la, lz, lp, many) < std::tie(o.type, o.sym, o.la, o.lz, o.lp, o.many);
+    return std::tie(type, sym, la, lz, lp) < std::tie(o.type, o.sym, o.la, o.lz, o.lp);
   }
 };
 
@@ -266,9 +284,9 @@ std::map<TuneKey, TuneEntry> g_tune;
 
 int tuned_variant(const GramParams &p, cudaStream_t s, bool *ran) {
   const int tiles = gram_tc_tiles(p);
-  if ((p.nA >= kTensorRows && p.nZ >= kTensorRows) || tiles >= kTensorTiles || !split_fits(p)) return kTensor;
-  const TuneKey key{p.type, p.symmetric ? 1 : 0, log2_bucket(p.nA), log2_bucket(p.nZ), log2_bucket(p.P),
-                    tiles > kSplitTiles ? 1 : 0};
+  if ((p.nA >= kTensorRows && p.nZ >= kTensorRows) || !split_fits(p)) return kTensor;
+  if (tiles > kSplitTiles) return split_is_cheaper(p, tiles) ? kSplit : kTensor;
+  const TuneKey key{p.type, p.symmetric ? 1 : 0, log2_bucket(p.nA), log2_bucket(p.nZ), log2_bucket(p.P)};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
@@ -356,9 +374,9 @@ extern "C" int lakgb_gram_autotune_table(char *buf, int buf_len) {
     for (const auto &kv : g_tune) {
       char line[512];
       int n = snprintf(line, sizeof line, "%s{\"type\":%d,\"symmetric\":%d,\"log2_rows_a\":%d,\"log2_rows_z\":%d,"
-                       "\"log2_blocks\":%d,\"over_%d_tiles\":%d,\"choice\":\"%s\",\"ms\":{",
+                       "\"log2_blocks\":%d,\"choice\":\"%s\",\"ms\":{",
                        first ? "" : ",", kv.first.type, kv.first.sym, kv.first.la, kv.first.lz, kv.first.lp,
-                       kSplitTiles, kv.first.many, kVariantName[kv.second.choice]);
+                       kVariantName[kv.second.choice]);
       for (int v = 0; v < kNumVariants; ++v)
         n += snprintf(line + n, sizeof line - n, "%s\"%s\":%.4f", v ? "," : "", kVariantName[v], kv.second.ms[v]);
       snprintf(line + n, sizeof line - n, "}}");
