@@ -426,9 +426,9 @@ def large_pass_headline(args, lib, stream, sh, rank, world, local):
                       "achieved_ops_per_s": elems * fp64_per_elem / (ms / 1000.0),
                       "peak_adds_per_s": fp64_rate,
                       "frac": elems * fp64_per_elem / (ms / 1000.0) / fp64_rate,
-                      "note": "the fold's additions and the results' operations (%d per computed element; three of seven "
-                              "rounds of additions and half of the results run in integers) against the FP64 add rate measured "
-                              "live on this GPU" % fp64_per_elem},
+                      "note": "the fold's additions and the results' operations (%d per computed element) against the FP64 add "
+                              "rate measured live on this GPU; three of seven rounds of additions and half of the results "
+                              "run in integers, so the pipe itself is less active (47 %% in the committed capture)" % fp64_per_elem},
         "vs_int_pipe_roofline": {"achieved_bitops": work / (ms / 1000.0), "int_pipe_peak_bitops": popc_peak,
                                  "ratio": (work / (ms / 1000.0)) / popc_peak,
                                  "note": "against the integer-pipe roofline of any popcount Gram (POPC 16 lanes/clk"

@@ -30,8 +30,8 @@
 // issues in that time (88 ms).  So rounds of four columns add with FP64 and with
 // integers in turn: 62.7 ms (two or four of seven in integers: 63.8 and 64.7;
 // two columns of every round: 64.8, a warp that waits for one pipe can not
-// issue to the other).  Neither pipe is full then: of the issue slots 55 % are
-// used, and the warps wait for TMEM, table and add latencies with no registers
+// issue to the other).  Neither pipe is full then: of the issue slots 58 % (9
+// blocks) to 70 % (69 blocks) are used, and the warps wait for TMEM, table and add latencies with no registers
 // left for more of them.
 // FP64: x comes from a table of the block's products.
 // Integers: while acc lies in one binade its bit pattern counts units in the

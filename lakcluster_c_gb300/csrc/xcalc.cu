@@ -283,8 +283,8 @@ __device__ __forceinline__ void note_bad(int *bad, int code) {
 // written, the first plane and (by the last group's warp) the padding past the
 // rows included, so the planes need no zero-fill before.  WIDE: plane rows and the array are 16-byte
 // aligned (16-byte stores); otherwise 4-byte ones.  T: holds b_mlt bits.
-// Bound: the integer pipe (57 % active; about 100 operations per value, 30 of
-// them the transpose), then load latency.  4096 x 4001 values to 32 bits
+// Bound: the integer pipe (71 % active at 8192 x 8192; about 100 operations per value,
+// 30 of them the transpose), then load latency.  4096 x 4001 values to 32 bits
 // through lakgb_xcalc_noalloc: 1463 us a call before (a warp per 32 rows, FP64
 // operations, 4-byte stores, one thread folding the columns' extremes), 130 us
 // now; this kernel 76 us, the extremes 37 us.
